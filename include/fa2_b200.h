@@ -61,7 +61,15 @@ typedef struct fa2_fwd_args {
   const int32_t* cu_seqlens_k;
   int32_t total_q, total_k;
   int32_t zero_tensors; /* packed mode: clear out (0) and LSE (-inf) first, as the reference's flag does */
+  /* Optional scratch memory of fa2_fwd_workspace_bytes() bytes, 256-byte aligned, contents irrelevant. With it a
+   * call whose (batch, head) work does not fill the GPU is split along the keys as well. May be NULL. */
+  void* workspace;
+  int64_t workspace_bytes;
 } fa2_fwd_args;
+
+/* Bytes of scratch memory the dense forward can use for these arguments (0: none); reads the shapes, the window
+ * and the pointers' device only. */
+FA2_API int64_t fa2_fwd_workspace_bytes(const fa2_fwd_args* args);
 
 /* Dense forward. Replaces launch_forward + flash_attn_fwd of the reference
  * (flash-attn2-rs/src/host/forward/mod.rs:449-813, src/device/forward/dense.rs:472-590).

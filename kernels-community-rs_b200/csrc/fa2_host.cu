@@ -7,6 +7,9 @@
 
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <climits>
 #include <cmath>
 #include <cstdarg>
@@ -178,6 +181,96 @@ __global__ void fill_f32_kernel(float* dst, int64_t n, float value) {
   if (i < n) dst[i] = value;
 }
 
+// ---- dense forward with few query rows per kv head (fwd_decode_sm100.cu)
+struct DecodePlan {
+  int rows = 0;            // query rows per kv head; 0: the path does not take this call
+  int tile_lo = 0, tiles = 0;
+  int grid = 0;            // CTAs when there is a workspace
+  int64_t counter_bytes = 0, workspace_bytes = 0;
+};
+DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
+  DecodePlan d;
+  const int64_t rows = static_cast<int64_t>(a->seqlen_q) * (a->heads / a->heads_k);
+  if (rows <= 0 || rows > fa2::kDecodeMaxRows || a->seqlen_k <= 0) return d;
+  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
+  const int64_t off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q;
+  int64_t lo = 0, hi = a->seqlen_k;
+  if (w.left >= 0) lo = std::max<int64_t>(0, off - w.left);
+  if (w.right >= 0) hi = std::min<int64_t>(hi, a->seqlen_q - 1 + off + w.right + 1);
+  if (hi <= lo) return d;  // no row sees a key
+  d.rows = static_cast<int>(rows);
+  d.tile_lo = static_cast<int>(lo / 128);
+  d.tiles = static_cast<int>((hi + 127) / 128) - d.tile_lo;
+  // One CTA per SM, each with an equal share of the tiles; a unit is split only as long as the shares keep three
+  // tiles (the merge of the parts costs about as much as two).
+  const int64_t units = static_cast<int64_t>(a->batch) * a->heads_k, n = units * d.tiles;
+  d.grid = static_cast<int>(std::min<int64_t>(sm_count, std::max(units, (n + 2) / 3)));
+  if (n % d.grid != 0 || (n / d.grid) % d.tiles != 0) {  // some share ends inside a unit
+    const int64_t dim = (a->head_dim + 63) / 64 * 64;
+    d.counter_bytes = (static_cast<int64_t>(d.grid) * 8 + 255) / 256 * 256;
+    d.workspace_bytes = d.counter_bytes + 2 * static_cast<int64_t>(d.grid) * 16 * fa2::decode_row_tiles(d.rows) * (dim + 2) * 4;
+  }
+  return d;
+}
+
+int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, Runtime* rt, cudaStream_t stream) {
+  fa2::DecodeParams p;
+  memset(&p, 0, sizeof(p));
+  int rc;
+  if ((rc = make_map(&p.tm_k, a->k, a->dtype, 2, a->head_dim, a->heads_k, a->seqlen_k, a->batch, a->k_stride[2], a->k_stride[1],
+                     a->k_stride[0], 64, 128, "k")) != FA2_OK) return rc;
+  if ((rc = make_map(&p.tm_v, a->v, a->dtype, 2, a->head_dim, a->heads_k, a->seqlen_k, a->batch, a->v_stride[2], a->v_stride[1],
+                     a->v_stride[0], 64, 128, "v")) != FA2_OK) return rc;
+  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
+  p.q_ptr = a->q;
+  p.o_ptr = a->out;
+  p.lse_ptr = a->lse;
+  p.alibi = a->alibi_slopes;
+  p.alibi_batch_stride = a->alibi_batch_stride;
+  p.q_batch_stride = a->q_stride[0];
+  p.q_row_stride = a->q_stride[1];
+  p.q_head_stride = a->q_stride[2];
+  p.o_batch_stride = a->o_stride[0];
+  p.o_row_stride = a->o_stride[1];
+  p.o_head_stride = a->o_stride[2];
+  p.lse_head_stride = a->seqlen_q;
+  p.lse_batch_stride = static_cast<int64_t>(a->heads) * a->seqlen_q;
+  p.units = a->batch * a->heads_k;
+  p.heads_k = a->heads_k;
+  p.group = a->heads / a->heads_k;
+  p.rows = d.rows;
+  p.tiles_per_unit = d.tiles;
+  p.tile_lo = d.tile_lo;
+  p.seqlen_k = a->seqlen_k;
+  p.off = a->seqlen_k - a->seqlen_q;
+  p.full_lo = w.left >= 0 ? a->seqlen_q - 1 + p.off - w.left : 0;
+  p.full_hi = w.right >= 0 ? std::min<int64_t>(a->seqlen_k, static_cast<int64_t>(p.off) + w.right + 1) : a->seqlen_k;
+  p.window_left = w.left;
+  p.window_right = w.right;
+  p.causal_alibi = w.causal_alibi;
+  p.scale = a->softmax_scale;
+  p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
+  p.softcap = a->softcap > 0.f ? a->softcap : 0.f;
+  p.head_dim = a->head_dim;
+  p.status = rt->status;
+  int grid = d.grid;
+  if (d.workspace_bytes > 0) {
+    if (a->workspace != nullptr && a->workspace_bytes >= d.workspace_bytes && reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0) {
+      // The counters in the workspace are tagged with this number, so their old contents do not matter.
+      static std::atomic<unsigned long long> launches{static_cast<unsigned long long>(
+          std::chrono::steady_clock::now().time_since_epoch().count())};
+      p.launch_tag = launches.fetch_add(1) + 1;
+      p.counters = static_cast<unsigned long long*>(a->workspace);
+      p.partials = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + d.counter_bytes);
+    } else {
+      grid = p.units;  // one CTA per unit: no share ends inside one
+    }
+  }
+  const cudaError_t e = fa2::launch_fwd_decode(p, grid, a->dtype == FA2_BF16, stream);
+  if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "forward launch failed: %s", cudaGetErrorString(e));
+  return FA2_OK;
+}
+
 int fwd_common(const fa2_fwd_args* a, void* stream_v, bool packed) {
   if (a == nullptr) return fail(FA2_E_VALUE, "args is null");
   if (a->dtype != FA2_F16 && a->dtype != FA2_BF16) return fail(FA2_E_TYPE, "q, k, v must be float16 or bfloat16");
@@ -260,6 +353,10 @@ int fwd_common(const fa2_fwd_args* a, void* stream_v, bool packed) {
   if ((rc = check_layout(a->v, vs, ns, "v")) != FA2_OK) return rc;
   if ((rc = check_layout(a->out, os, ns, "out")) != FA2_OK) return rc;
 
+  if (!packed) {
+    const DecodePlan plan = decode_plan(a, rt->sm_count);
+    if (plan.rows > 0) return fwd_decode(a, plan, rt, stream);
+  }
   if ((rc = make_map(&p.tm_q, a->q, a->dtype, 2, d, a->heads, rows_q, nbatch, a->q_stride[2], a->q_stride[1],
                      a->q_stride[0], 64, 128, "q")) != FA2_OK)
     return rc;
@@ -741,6 +838,16 @@ int fa2_bwd_static_status(int device) {
   return rc != FA2_OK ? rc : word;
 }
 
+
+int64_t fa2_fwd_workspace_bytes(const fa2_fwd_args* args) {
+  if (args == nullptr || args->heads_k <= 0 || args->heads <= 0 || args->heads % args->heads_k != 0 || args->batch <= 0 ||
+      args->seqlen_q <= 0 || args->seqlen_k <= 0 || args->head_dim <= 0)
+    return 0;
+  const DeviceScope scope(args->q);
+  Runtime* rt = nullptr;
+  if (get_runtime(scope.device(), &rt) != FA2_OK) return 0;
+  return decode_plan(args, rt->sm_count).workspace_bytes;
+}
 
 int fa2_fwd(const fa2_fwd_args* args, void* stream) { return fwd_common(args, stream, false); }
 

@@ -12,6 +12,12 @@ cudaError_t launch_fwd(const FwdParams& p, int head_dim, bool bf16, int num_sms,
 // p.tm_v carry boxes of 64 rows.
 cudaError_t launch_fwd_wide(const FwdParams& p, int head_dim, bool bf16, cudaStream_t stream);
 
+// Dense forward with at most kDecodeMaxRows query rows per kv head, head_dim a multiple of 8 up to 256; `grid` CTAs
+// share the tile list evenly. The workspace behind p.partials and p.counters holds 2 * grid partial results of
+// 16 * decode_row_tiles(rows) rows x (D + 2) floats (D: head_dim rounded up to 64) and grid 8-byte counters.
+int decode_row_tiles(int rows);
+cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, cudaStream_t stream);
+
 // dQ / dK / dV for head_dim a multiple of 8 up to 128; the fp32 dQ accumulator behind p.tm_dqa (and the turn
 // counters p.dq_turn, when given) must be zero.
 cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream);

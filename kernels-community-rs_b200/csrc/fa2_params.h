@@ -20,6 +20,7 @@ enum WaitSite : int {
   kWaitEpiFinal = 41,
   kWaitEpiPvDone = 42,
   kWaitBwd = 50,
+  kWaitDecode = 80,
 };
 
 struct FwdParams {
@@ -43,6 +44,32 @@ struct FwdParams {
   float softcap;                       // 0 = off
   int* status;                         // device status word (0 = ok)
   int head_dim;                         // real head dim (<= the kernel's D; columns beyond it are padding)
+};
+
+// Forward for few query rows (fwd_decode_sm100.cu). A unit is one (batch, kv head): its rows are the query rows of all
+// the group's heads, row r = query r / group, head r % group.
+constexpr int kDecodeMaxRows = 64;
+struct DecodeParams {
+  CUtensorMap tm_k, tm_v;              // box (64, 1, 128, 1)
+  const void* q_ptr;
+  void* o_ptr;
+  float* lse_ptr;
+  const float* alibi;
+  float* partials;                     // 2 slots per CTA (null when no unit is split)
+  unsigned long long* counters;        // one per CTA: the unit that starts in it and ends in another
+  unsigned long long launch_tag;
+  int64_t q_row_stride, q_head_stride, q_batch_stride;  // elements
+  int64_t o_row_stride, o_head_stride, o_batch_stride;
+  int64_t lse_head_stride, lse_batch_stride;
+  int alibi_batch_stride;
+  int units, heads_k, group, rows;     // rows = seqlen_q * group
+  int tiles_per_unit, tile_lo;         // 128-key tiles [tile_lo, tile_lo + tiles_per_unit) hold every visible key
+  int seqlen_k, off;                   // off = seqlen_k - seqlen_q
+  int full_lo, full_hi;                // every row sees all of the keys [full_lo, full_hi)
+  int window_left, window_right, causal_alibi;
+  float scale, scale_log2, softcap;
+  int head_dim;
+  int* status;
 };
 
 struct BwdParams {

@@ -304,6 +304,13 @@ Any fwd_impl(const AnyView* args, int32_t n, bool lse_only) {
   a.window_left = static_cast<int32_t>(wl);
   a.window_right = static_cast<int32_t>(wr);
   a.softcap = static_cast<float>(softcap);
+  Optional<Tensor> workspace;
+  const int64_t need = fa2_fwd_workspace_bytes(&a);
+  if (need > 0) {
+    workspace = alloc({need / 4}, kF32, dev);
+    a.workspace = workspace.value().data_ptr();
+    a.workspace_bytes = need;
+  }
   check(fa2_fwd(&a, stream_of(dev)));
   if (copy_out) {
     const Tensor& o = supplied.value();

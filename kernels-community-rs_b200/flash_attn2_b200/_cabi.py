@@ -27,6 +27,7 @@ class FwdArgs(C.Structure):
         ("window_left", C.c_int32), ("window_right", C.c_int32), ("softcap", C.c_float),
         ("cu_seqlens_q", C.c_void_p), ("cu_seqlens_k", C.c_void_p),
         ("total_q", C.c_int32), ("total_k", C.c_int32), ("zero_tensors", C.c_int32),
+        ("workspace", C.c_void_p), ("workspace_bytes", C.c_int64),
     ]
 
 
@@ -60,7 +61,7 @@ class BwdArgs(C.Structure):
 
 # Every symbol include/fa2_b200.h declares; the CPU test suite checks that the library exports them.
 EXPORTS = (
-    "fa2_fwd", "fa2_varlen_fwd", "fa2_bwd_preprocess", "fa2_bwd_workspace_bytes", "fa2_bwd",
+    "fa2_fwd", "fa2_fwd_workspace_bytes", "fa2_varlen_fwd", "fa2_bwd_preprocess", "fa2_bwd_workspace_bytes", "fa2_bwd",
     "fa2_bwd_static", "fa2_bwd_static_status", "fa2_layout_is_addressable", "fa2_pack_16bit", "fa2_copy_16bit",
     "fa2_last_error", "fa2_device_status", "fa2_sm_count",
 )
@@ -81,6 +82,8 @@ def load() -> C.CDLL:
         for name in ("fa2_fwd", "fa2_varlen_fwd"):
             getattr(lib, name).argtypes = [C.POINTER(FwdArgs), C.c_void_p]
             getattr(lib, name).restype = C.c_int
+        lib.fa2_fwd_workspace_bytes.argtypes = [C.POINTER(FwdArgs)]
+        lib.fa2_fwd_workspace_bytes.restype = C.c_int64
         if hasattr(lib, "fa2_bwd_preprocess"):
             lib.fa2_bwd_preprocess.argtypes = [C.POINTER(BwdPreprocessArgs), C.c_void_p]
             lib.fa2_bwd_preprocess.restype = C.c_int

@@ -91,6 +91,10 @@ def fwd(q, k, v, *, out=None, alibi_slopes=None, softmax_scale=None, causal=Fals
     a.window_left, a.window_right = int(window_left), int(window_right)
     a.softcap = float(softcap)
     with torch.cuda.device(q.device):
+        need = lib.fa2_fwd_workspace_bytes(C.byref(a))
+        if need > 0:
+            workspace = _alloc((need // 4,), torch.float32, q.device)
+            a.workspace, a.workspace_bytes = workspace.data_ptr(), need
         _cabi.check(lib.fa2_fwd(C.byref(a), _stream(q)))
     return out, lse
 
