@@ -2,6 +2,7 @@
 
   lib/libfa2_b200.so            CUDA kernels + the C ABI declared in include/fa2_b200.h
   lib/libflash_attn2_b200.so    tvm-ffi operator symbols (__tvm_ffi_fwd, ...) on top of the C ABI
+  lib/_fa2_torch.so             Python module: the dense calls on torch tensors, on top of the C ABI
 
 Run as `python build.py` or call build(); a library is rebuilt only when a source is newer.
 """
@@ -88,9 +89,29 @@ def build_tvm_ffi() -> Path | None:
     return out
 
 
+def build_torch_calls() -> Path:
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    src = CSRC / "torch_calls.cc"
+    out = LIB / "_fa2_torch.so"
+    if _newer(out, [src, INCLUDE / "fa2_b200.h", LIB / "libfa2_b200.so"]):
+        libdir = Path(torch.__file__).resolve().parent / "lib"
+        incs = [*include_paths(), sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+        _run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+              *[a for p in incs for a in ("-isystem", str(p))], f"-I{INCLUDE}", str(src), "-o", str(out),
+              f"-L{LIB}", "-lfa2_b200", f"-L{libdir}", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda",
+              "-lc10", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{libdir}"])
+    return out
+
+
 def build(verbose: bool = False) -> None:
     build_kernels(verbose)
     build_tvm_ffi()
+    build_torch_calls()
 
 
 if __name__ == "__main__":

@@ -185,8 +185,9 @@ __global__ void fill_f32_kernel(float* dst, int64_t n, float value) {
 struct DecodePlan {
   int rows = 0;            // query rows per kv head; 0: the path does not take this call
   int tile_lo = 0, tiles = 0;
-  int grid = 0;            // CTAs when there is a workspace
-  int64_t counter_bytes = 0, workspace_bytes = 0;
+  int grid = 0, whole_grid = 0;  // CTAs with a workspace, and without one
+  bool split = false;            // some unit is shared by CTAs (needs the workspace)
+  int64_t flag_bytes = 0, workspace_bytes = 0;
 };
 DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
   DecodePlan d;
@@ -201,14 +202,25 @@ DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
   d.rows = static_cast<int>(rows);
   d.tile_lo = static_cast<int>(lo / 128);
   d.tiles = static_cast<int>((hi + 127) / 128) - d.tile_lo;
-  // One CTA per SM, each with an equal share of the tiles; a unit is split only as long as the shares keep three
-  // tiles (the merge of the parts costs about as much as two).
-  const int64_t units = static_cast<int64_t>(a->batch) * a->heads_k, n = units * d.tiles;
-  d.grid = static_cast<int>(std::min<int64_t>(sm_count, std::max(units, (n + 2) / 3)));
-  if (n % d.grid != 0 || (n / d.grid) % d.tiles != 0) {  // some share ends inside a unit
+  const int64_t units = static_cast<int64_t>(a->batch) * a->heads_k, n = units * d.tiles, sms = sm_count;
+  // Whole units per CTA, as evenly as that goes: what happens without a workspace.
+  const int64_t per_cta = (units + sms - 1) / sms;
+  d.whole_grid = d.grid = static_cast<int>((units + per_cta - 1) / per_cta);
+  // Splitting units over CTAs costs about 5 us at the end (parts to memory, flags, merge), as much as a CTA takes for
+  // four tiles of its own. Few units: each is cut into as many equal parts as the SMs allow and leave three tiles; at
+  // most 24, because one CTA merges them. More units than SMs: equal shares of the whole list when the last,
+  // incomplete round of whole units would take more than five tiles longer.
+  if (units <= sms) {
+    const int64_t parts = std::min<int64_t>({sms / units, 24, d.tiles / 3});
+    if (parts > 1) d.grid = static_cast<int>(units * parts);
+  } else if (per_cta * d.tiles - n / sms > 5) {
+    d.grid = sm_count;
+  }
+  d.split = d.grid != d.whole_grid || (units > sms && d.grid == sm_count && units % sms != 0);
+  if (d.split) {
     const int64_t dim = (a->head_dim + 63) / 64 * 64;
-    d.counter_bytes = (static_cast<int64_t>(d.grid) * 8 + 255) / 256 * 256;
-    d.workspace_bytes = d.counter_bytes + 2 * static_cast<int64_t>(d.grid) * 16 * fa2::decode_row_tiles(d.rows) * (dim + 2) * 4;
+    d.flag_bytes = (2 * static_cast<int64_t>(d.grid) * 8 + 255) / 256 * 256;
+    d.workspace_bytes = d.flag_bytes + 2 * static_cast<int64_t>(d.grid) * 16 * fa2::decode_row_tiles(d.rows) * (dim + 2) * 4;
   }
   return d;
 }
@@ -253,18 +265,16 @@ int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, Runtime* rt, cudaStre
   p.softcap = a->softcap > 0.f ? a->softcap : 0.f;
   p.head_dim = a->head_dim;
   p.status = rt->status;
-  int grid = d.grid;
-  if (d.workspace_bytes > 0) {
-    if (a->workspace != nullptr && a->workspace_bytes >= d.workspace_bytes && reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0) {
-      // The counters in the workspace are tagged with this number, so their old contents do not matter.
-      static std::atomic<unsigned long long> launches{static_cast<unsigned long long>(
-          std::chrono::steady_clock::now().time_since_epoch().count())};
-      p.launch_tag = launches.fetch_add(1) + 1;
-      p.counters = static_cast<unsigned long long*>(a->workspace);
-      p.partials = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + d.counter_bytes);
-    } else {
-      grid = p.units;  // one CTA per unit: no share ends inside one
-    }
+  int grid = d.whole_grid;
+  if (d.split && a->workspace != nullptr && a->workspace_bytes >= d.workspace_bytes &&
+      reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0) {
+    grid = d.grid;
+    // The flags in the workspace are set to this number, so their old contents do not matter.
+    static std::atomic<unsigned long long> launches{static_cast<unsigned long long>(
+        std::chrono::steady_clock::now().time_since_epoch().count())};
+    p.launch_tag = (launches.fetch_add(1) + 1) | (1ull << 63);  // never the cleared value
+    p.flags = static_cast<unsigned long long*>(a->workspace);
+    p.partials = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + d.flag_bytes);
   }
   const cudaError_t e = fa2::launch_fwd_decode(p, grid, a->dtype == FA2_BF16, stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "forward launch failed: %s", cudaGetErrorString(e));

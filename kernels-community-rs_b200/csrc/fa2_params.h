@@ -56,7 +56,7 @@ struct DecodeParams {
   float* lse_ptr;
   const float* alibi;
   float* partials;                     // 2 slots per CTA (null when no unit is split)
-  unsigned long long* counters;        // one per CTA: the unit that starts in it and ends in another
+  unsigned long long* flags;           // one per partial slot: launch_tag once the part is in memory
   unsigned long long launch_tag;
   int64_t q_row_stride, q_head_stride, q_batch_stride;  // elements
   int64_t o_row_stride, o_head_stride, o_batch_stride;

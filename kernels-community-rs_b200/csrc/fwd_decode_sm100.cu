@@ -7,8 +7,8 @@
 //     head r % group) are the M dimension of one problem, and K and V cross the memory system once per kv head.
 //   * The key tiles of all (batch, kv head) units form one list that is cut into equal contiguous shares, one per
 //     CTA, one CTA per SM. A share may end in the middle of a unit; the CTA then leaves a partial result (fp32 O, row
-//     maximum, row sum) in the workspace and the CTA that finishes a unit last adds the partials up. Which CTA that
-//     is is decided by a counter per split unit, tagged with the launch's number, so the workspace needs no clearing.
+//     maximum, row sum) in the workspace and the CTA that finishes a unit last adds the partials up. Which CTA that is
+//     is seen from a flag per part that holds the launch's number, so the workspace needs no clearing.
 //   * One warp keeps a ring of 196 KB of K and V tiles filled by TMA (23 B/clk per SM is an SM's share of HBM; a
 //     round trip of about 2000 cycles needs 46 KB in flight), eight warps consume it. Each consumer owns 16 x MT keys
 //     of a 128-key tile and 16 query rows and never waits for another consumer until the share's unit ends.
@@ -60,10 +60,10 @@ __device__ __forceinline__ void ldsm4_trans(uint32_t addr, uint32_t* r) {
 template <bool BF16>
 __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   if constexpr (BF16) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   } else {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
 }
@@ -88,9 +88,16 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
   volatile int* s_last = reinterpret_cast<volatile int*>(smem + Cfg::kMiscOff + 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
-  // this CTA's share of the tile list
+  // this CTA's share of the tile list; without parts (no workspace for them) it is whole units
   const int64_t n_tiles = static_cast<int64_t>(p.units) * p.tiles_per_unit;
-  const int lo = static_cast<int>(blockIdx.x * n_tiles / gridDim.x), hi = static_cast<int>((blockIdx.x + 1) * n_tiles / gridDim.x);
+  int lo, hi;
+  if (p.partials != nullptr) {
+    lo = static_cast<int>(blockIdx.x * n_tiles / gridDim.x);
+    hi = static_cast<int>((blockIdx.x + 1) * n_tiles / gridDim.x);
+  } else {
+    lo = static_cast<int>(static_cast<int64_t>(blockIdx.x) * p.units / gridDim.x) * p.tiles_per_unit;
+    hi = static_cast<int>(static_cast<int64_t>(blockIdx.x + 1) * p.units / gridDim.x) * p.tiles_per_unit;
+  }
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -157,210 +164,141 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
     const float inv_cap = p.softcap > 0.f ? p.scale / p.softcap : 0.f;
     const float cap_l2 = p.softcap * 1.4426950408889634f;
     uint32_t slot = 0, phase = 0;
-    uint32_t qf[A <= 2 ? D / 16 : 1][4];  // Q fragments stay in registers up to head dim 128
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    float o[kOT][4];
-    float slope0 = 0.f, slope1 = 0.f;
-    int u = lo / p.tiles_per_unit, j = lo - u * p.tiles_per_unit;
-    bool fresh = true;  // the next tile starts a segment (the share's part of one unit)
-    int seg_first = j;
-    for (int x = lo; x < hi; ++x) {
-      const int b = u / p.heads_k, hk = u - b * p.heads_k;
-      if (fresh) {
-        fresh = false;
-        seg_first = j;
-        // Q rows of the unit -> swizzled shared memory; rows past the last one are zero.
-        consumers_sync();  // the previous unit's Q has been read
-        for (int c = tid; c < Cfg::kRows * A * 8; c += kConsumers * 32) {
-          const int r = c / (A * 8), ch = c - r * (A * 8);
-          uint4 w = make_uint4(0, 0, 0, 0);
-          if (r < p.rows && ch * 8 < p.head_dim) {
-            const int q = r / p.group, h = hk * p.group + (r - q * p.group);
-            w = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.q_ptr) + b * p.q_batch_stride +
-                                                q * p.q_row_stride + h * p.q_head_stride + ch * 8);
-          }
-          *reinterpret_cast<uint4*>(smem + Cfg::kQOff + (ch / 8) * (Cfg::kRows * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = w;
-        }
-        consumers_sync();
-        if constexpr (A <= 2) {
-#pragma unroll
-          for (int ks = 0; ks < D / 16; ++ks) q_frag(ks, qf[ks]);
-        }
-        if (has_alibi) {
-          const float* al = p.alibi + b * p.alibi_batch_stride + hk * p.group;
-          slope0 = r0 < p.rows ? al[r0 - q0 * p.group] * 1.4426950408889634f : 0.f;
-          slope1 = r1 < p.rows ? al[r1 - q1 * p.group] * 1.4426950408889634f : 0.f;
-        }
-        m0 = m1 = -INFINITY;
-        l0 = l1 = 0.f;
-#pragma unroll
-        for (int i = 0; i < kOT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-      }
-      // ---- scores of this warp's keys
-      float s[kNT][4];
-#pragma unroll
-      for (int i = 0; i < kNT; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
-      mbar_wait(&full[slot], phase, ctl, kWaitDecode + 2);
-      __syncwarp();
-      {
-        const uint32_t kb = s_base + slot * Cfg::kSlotBytes + k_row;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          uint32_t qa[4];
-          if constexpr (A <= 2) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) qa[e] = qf[ks][e];
-          } else {
-            q_frag(ks, qa);
-          }
-#pragma unroll
-          for (int i = 0; i < kNT; i += 2) {
-            uint32_t kf[4];
-            ldsm4(kb + (ks / 4) * (kTile * 128) + i * (8 * 128) + ((((ks % 4) * 2 + (lm & 1)) ^ lr) << 4), kf);
-            mma16816<BF16>(s[i], qa, kf[0], kf[1]);
-            mma16816<BF16>(s[i + 1], qa, kf[2], kf[3]);
-          }
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[slot]);
+    auto next_slot = [&]() {
       if (++slot == Cfg::kSlots) {
         slot = 0;
         phase ^= 1;
       }
-      // ---- transform and mask: scores into the log2 domain
-      const int col0 = (p.tile_lo + j) * kTile + kg * kKeys + 2 * t4;
-      if (p.softcap > 0.f) {
-#pragma unroll
-        for (int i = 0; i < kNT; ++i)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float y;
-            asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(s[i][e] * inv_cap));
-            s[i][e] = cap_l2 * y;
-          }
-      } else {
-#pragma unroll
-        for (int i = 0; i < kNT; ++i)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) s[i][e] *= p.scale_log2;
+    };
+    int u = lo / p.tiles_per_unit, j = lo - u * p.tiles_per_unit;
+    // A segment: the share's part of one unit, tiles [seg_first, seg_end) of it.
+    for (int x = lo; x < hi;) {
+      const int b = u / p.heads_k, hk = u - b * p.heads_k;
+      const int seg_first = j, seg_end = min(p.tiles_per_unit, j + hi - x);
+      x += seg_end - seg_first;
+      // Q rows of the unit -> swizzled shared memory; rows past the last one are zero.
+      consumers_sync();  // the previous unit's Q has been read
+      for (int c = tid; c < Cfg::kRows * A * 8; c += kConsumers * 32) {
+        const int r = c / (A * 8), ch = c - r * (A * 8);
+        uint4 w = make_uint4(0, 0, 0, 0);
+        if (r < p.rows && ch * 8 < p.head_dim) {
+          const int q = r / p.group, h = hk * p.group + (r - q * p.group);
+          w = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.q_ptr) + b * p.q_batch_stride +
+                                              q * p.q_row_stride + h * p.q_head_stride + ch * 8);
+        }
+        *reinterpret_cast<uint4*>(smem + Cfg::kQOff + (ch / 8) * (Cfg::kRows * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = w;
       }
+      consumers_sync();
+      uint32_t qf[A <= 2 ? D / 16 : 1][4];  // Q fragments stay in registers up to head dim 128
+      if constexpr (A <= 2) {
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) q_frag(ks, qf[ks]);
+      }
+      float slope0 = 0.f, slope1 = 0.f;
       if (has_alibi) {
-#pragma unroll
-        for (int i = 0; i < kNT; ++i)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int col = col0 + i * 8 + (e & 1);
-            const float sl = (e & 2) ? slope1 : slope0;
-            s[i][e] += p.causal_alibi ? sl * static_cast<float>(col)
-                                      : -sl * fabsf(static_cast<float>(((e & 2) ? q1 : q0) + p.off - col));
-          }
+        const float* al = p.alibi + b * p.alibi_batch_stride + hk * p.group;
+        slope0 = r0 < p.rows ? al[r0 - q0 * p.group] * 1.4426950408889634f : 0.f;
+        slope1 = r1 < p.rows ? al[r1 - q1 * p.group] * 1.4426950408889634f : 0.f;
       }
-      const int tile_col = (p.tile_lo + j) * kTile;
-      // Only the tiles at the ends of the rows' key ranges have anything to mask.
-      if (tile_col + kTile > p.full_hi || tile_col < p.full_lo) {
-        int hi0 = p.seqlen_k, hi1 = p.seqlen_k, lo0 = 0, lo1 = 0;
-        if (p.window_right >= 0) {
-          hi0 = min(hi0, q0 + p.off + p.window_right + 1);
-          hi1 = min(hi1, q1 + p.off + p.window_right + 1);
-        }
-        if (p.window_left >= 0) {
-          lo0 = q0 + p.off - p.window_left;
-          lo1 = q1 + p.off - p.window_left;
-        }
+      float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+      float o[kOT][4];
 #pragma unroll
-        for (int i = 0; i < kNT; ++i)
+      for (int i = 0; i < kOT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+      for (; j < seg_end; ++j) {
+        // ---- scores of this warp's keys
+        float s[kNT][4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int col = col0 + i * 8 + (e & 1);
-            if (col >= ((e & 2) ? hi1 : hi0) || col < ((e & 2) ? lo1 : lo0)) s[i][e] = -INFINITY;
-          }
-      }
-      // ---- row maxima over the four lanes of a row, rescale
-      float x0 = -INFINITY, x1 = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < kNT; ++i) {
-        x0 = max3(x0, s[i][0], s[i][1]);
-        x1 = max3(x1, s[i][2], s[i][3]);
-      }
-#pragma unroll
-      for (int d = 1; d < 4; d <<= 1) {
-        x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, d));
-        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, d));
-      }
-      const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
-      if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
-        const float a0 = part_scale(m0, n0), a1 = part_scale(m1, n1);
-        l0 *= a0;
-        l1 *= a1;
-#pragma unroll
-        for (int i = 0; i < kOT; ++i) {
-          o[i][0] *= a0;
-          o[i][1] *= a0;
-          o[i][2] *= a1;
-          o[i][3] *= a1;
-        }
-        m0 = n0;
-        m1 = n1;
-      }
-      const float b0 = m0 == -INFINITY ? 0.f : m0, b1 = m1 == -INFINITY ? 0.f : m1;
-      uint32_t pf[kNT][2];
-#pragma unroll
-      for (int i = 0; i < kNT; ++i) {
-        const float e0 = ex2(s[i][0] - b0), e1 = ex2(s[i][1] - b0), e2 = ex2(s[i][2] - b1), e3 = ex2(s[i][3] - b1);
-        l0 += e0 + e1;
-        l1 += e2 + e3;
-        pf[i][0] = pack2<BF16>(e0, e1);
-        pf[i][1] = pack2<BF16>(e2, e3);
-      }
-      // ---- O += P V
-      mbar_wait(&full[slot], phase, ctl, kWaitDecode + 3);
-      __syncwarp();
-      {
-        const uint32_t vb = s_base + slot * Cfg::kSlotBytes + v_row;
-#pragma unroll
-        for (int kk = 0; kk < kNT / 2; ++kk) {
-          const uint32_t pa[4] = {pf[2 * kk][0], pf[2 * kk][1], pf[2 * kk + 1][0], pf[2 * kk + 1][1]};
-#pragma unroll
-          for (int i = 0; i < kOT; i += 2) {
-            uint32_t vf[4];
-            ldsm4_trans(vb + (i / 8) * (kTile * 128) + kk * (16 * 128) + ((((i % 8) + (lm >> 1)) ^ lr) << 4), vf);
-            mma16816<BF16>(o[i], pa, vf[0], vf[1]);
-            mma16816<BF16>(o[i + 1], pa, vf[2], vf[3]);
-          }
-        }
-      }
-      __syncwarp();
-      const bool seg_end = (j + 1 == p.tiles_per_unit) || (x + 1 == hi);
-      if (seg_end) {
-        // ---- the consumers' parts of this segment become one: the last V slot, still held, is the scratch space.
-        l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-        l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-        l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-        l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-        if (t4 == 0) {
-          float* st = s_stat + warp * 32;
-          st[g] = m0;
-          st[8 + g] = m1;
-          st[16 + g] = l0;
-          st[24 + g] = l1;
-        }
-        consumers_sync();
-        float t0 = -INFINITY, t1 = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < kGroups; ++w) {
-          t0 = fmaxf(t0, s_stat[(w * MT + mt) * 32 + g]);
-          t1 = fmaxf(t1, s_stat[(w * MT + mt) * 32 + 8 + g]);
-        }
-        float ls0 = 0.f, ls1 = 0.f;
-#pragma unroll
-        for (int w = 0; w < kGroups; ++w) {
-          const float* st = s_stat + (w * MT + mt) * 32;
-          ls0 += st[16 + g] * part_scale(st[g], t0);
-          ls1 += st[24 + g] * part_scale(st[8 + g], t1);
-        }
+        for (int i = 0; i < kNT; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+        mbar_wait(&full[slot], phase, ctl, kWaitDecode + 2);
+        __syncwarp();
         {
-          const float a0 = part_scale(m0, t0), a1 = part_scale(m1, t1);
+          const uint32_t kb = s_base + slot * Cfg::kSlotBytes + k_row;
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks) {
+            uint32_t qa[4];
+            if constexpr (A <= 2) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) qa[e] = qf[ks][e];
+            } else {
+              q_frag(ks, qa);
+            }
+#pragma unroll
+            for (int i = 0; i < kNT; i += 2) {
+              uint32_t kf[4];
+              ldsm4(kb + (ks / 4) * (kTile * 128) + i * (8 * 128) + ((((ks % 4) * 2 + (lm & 1)) ^ lr) << 4), kf);
+              mma16816<BF16>(s[i], qa, kf[0], kf[1]);
+              mma16816<BF16>(s[i + 1], qa, kf[2], kf[3]);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[slot]);
+        next_slot();
+        // ---- transform and mask: scores into the log2 domain
+        const int col0 = (p.tile_lo + j) * kTile + kg * kKeys + 2 * t4;
+        if (p.softcap > 0.f) {
+#pragma unroll
+          for (int i = 0; i < kNT; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float y;
+              asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(s[i][e] * inv_cap));
+              s[i][e] = cap_l2 * y;
+            }
+        } else {
+#pragma unroll
+          for (int i = 0; i < kNT; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[i][e] *= p.scale_log2;
+        }
+        if (has_alibi) {
+#pragma unroll
+          for (int i = 0; i < kNT; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int col = col0 + i * 8 + (e & 1);
+              const float sl = (e & 2) ? slope1 : slope0;
+              s[i][e] += p.causal_alibi ? sl * static_cast<float>(col)
+                                        : -sl * fabsf(static_cast<float>(((e & 2) ? q1 : q0) + p.off - col));
+            }
+        }
+        const int tile_col = (p.tile_lo + j) * kTile;
+        // Only the tiles at the ends of the rows' key ranges have anything to mask.
+        if (tile_col + kTile > p.full_hi || tile_col < p.full_lo) {
+          int hi0 = p.seqlen_k, hi1 = p.seqlen_k, lo0 = 0, lo1 = 0;
+          if (p.window_right >= 0) {
+            hi0 = min(hi0, q0 + p.off + p.window_right + 1);
+            hi1 = min(hi1, q1 + p.off + p.window_right + 1);
+          }
+          if (p.window_left >= 0) {
+            lo0 = q0 + p.off - p.window_left;
+            lo1 = q1 + p.off - p.window_left;
+          }
+#pragma unroll
+          for (int i = 0; i < kNT; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int col = col0 + i * 8 + (e & 1);
+              if (col >= ((e & 2) ? hi1 : hi0) || col < ((e & 2) ? lo1 : lo0)) s[i][e] = -INFINITY;
+            }
+        }
+        // ---- row maxima over the four lanes of a row, rescale
+        float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < kNT; ++i) {
+          x0 = max3(x0, s[i][0], s[i][1]);
+          x1 = max3(x1, s[i][2], s[i][3]);
+        }
+#pragma unroll
+        for (int d = 1; d < 4; d <<= 1) {
+          x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, d));
+          x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, d));
+        }
+        const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+        if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
+          const float a0 = part_scale(m0, n0), a1 = part_scale(m1, n1);
+          l0 *= a0;
+          l1 *= a1;
 #pragma unroll
           for (int i = 0; i < kOT; ++i) {
             o[i][0] *= a0;
@@ -368,153 +306,239 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
             o[i][2] *= a1;
             o[i][3] *= a1;
           }
+          m0 = n0;
+          m1 = n1;
         }
-        float4* scratch = reinterpret_cast<float4*>(smem + slot * Cfg::kSlotBytes);
+        const float b0 = m0 == -INFINITY ? 0.f : m0, b1 = m1 == -INFINITY ? 0.f : m1;
+        uint32_t pf[kNT][2];
 #pragma unroll
-        for (int half = kGroups / 2; half >= 1; half /= 2) {
-          // 4 x 16 rows x D fp32 = one slot: half x MT <= 4 regions of one warp's fragments each
-          if (kg >= half && kg < 2 * half) {
-            float4* dst = scratch + ((kg - half) * MT + mt) * (kOT * 32) + lane;
-#pragma unroll
-            for (int i = 0; i < kOT; ++i) dst[i * 32] = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
-          }
-          consumers_sync();
-          if (kg < half) {
-            const float4* src = scratch + (kg * MT + mt) * (kOT * 32) + lane;
-#pragma unroll
-            for (int i = 0; i < kOT; ++i) {
-              const float4 w = src[i * 32];
-              o[i][0] += w.x;
-              o[i][1] += w.y;
-              o[i][2] += w.z;
-              o[i][3] += w.w;
-            }
-          }
-          consumers_sync();
+        for (int i = 0; i < kNT; ++i) {
+          const float e0 = ex2(s[i][0] - b0), e1 = ex2(s[i][1] - b0), e2 = ex2(s[i][2] - b1), e3 = ex2(s[i][3] - b1);
+          l0 += e0 + e1;
+          l1 += e2 + e3;
+          pf[i][0] = pack2<BF16>(e0, e1);
+          pf[i][1] = pack2<BF16>(e2, e3);
         }
-        // ---- out, or a partial result
-        auto store_pair = [&](int r, int i, float a, float c) {
-          if (r < p.rows && i * 8 < p.head_dim) {
-            const int q = r / p.group, h = hk * p.group + (r - q * p.group);
-            *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.o_ptr) + b * p.o_batch_stride + q * p.o_row_stride +
-                                         h * p.o_head_stride + i * 8 + 2 * t4) = pack2<BF16>(a, c);
-          }
-        };
-        auto store_lse = [&](int r, float m, float l) {
-          if (r < p.rows) {
-            const int q = r / p.group, h = hk * p.group + (r - q * p.group);
-            p.lse_ptr[b * p.lse_batch_stride + h * p.lse_head_stride + q] = l > 0.f ? (m + lg2(l)) * 0.6931471805599453f : INFINITY;
-          }
-        };
-        const bool whole = seg_first == 0 && j + 1 == p.tiles_per_unit;
-        if (whole) {
-          if (kg == 0) {
-            const float i0 = ls0 > 0.f ? 1.f / ls0 : 0.f, i1 = ls1 > 0.f ? 1.f / ls1 : 0.f;
+        // ---- O += P V
+        mbar_wait(&full[slot], phase, ctl, kWaitDecode + 3);
+        __syncwarp();
+        {
+          const uint32_t vb = s_base + slot * Cfg::kSlotBytes + v_row;
 #pragma unroll
-            for (int i = 0; i < kOT; ++i) {
-              store_pair(r0, i, o[i][0] * i0, o[i][1] * i0);
-              store_pair(r1, i, o[i][2] * i1, o[i][3] * i1);
-            }
-            if (t4 == 0) {
-              store_lse(r0, t0, ls0);
-              store_lse(r1, t1, ls1);
-            }
-          }
-        } else {
-          // Slot 2c holds a segment that began before this share, 2c + 1 one that began in it. Layout of a slot: the
-          // fragments of the MT row tiles, then m and l of the rows.
-          constexpr int kPart = Cfg::kRows * (D + 2);  // floats
-          float* part = p.partials + (2 * static_cast<int64_t>(blockIdx.x) + (seg_first == 0 ? 1 : 0)) * kPart;
-          if (kg == 0) {
-            float4* dst = reinterpret_cast<float4*>(part) + mt * (kOT * 32) + lane;
+          for (int kk = 0; kk < kNT / 2; ++kk) {
+            const uint32_t pa[4] = {pf[2 * kk][0], pf[2 * kk][1], pf[2 * kk + 1][0], pf[2 * kk + 1][1]};
 #pragma unroll
-            for (int i = 0; i < kOT; ++i) __stcg(dst + i * 32, make_float4(o[i][0], o[i][1], o[i][2], o[i][3]));
-            if (t4 == 0) {
-              float* st = part + Cfg::kRows * D;
-              __stcg(st + r0, t0);
-              __stcg(st + r1, t1);
-              __stcg(st + Cfg::kRows + r0, ls0);
-              __stcg(st + Cfg::kRows + r1, ls1);
-            }
-            __threadfence();
-          }
-          // CTAs whose shares touch this unit: the owners of its first and its last tile.
-          const int64_t g64 = gridDim.x;
-          const int64_t first_tile = static_cast<int64_t>(u) * p.tiles_per_unit;
-          const int c_first = static_cast<int>(((first_tile + 1) * g64 + n_tiles - 1) / n_tiles - 1);
-          const int c_last = static_cast<int>(((first_tile + p.tiles_per_unit) * g64 + n_tiles - 1) / n_tiles - 1);
-          consumers_sync();
-          if (tid == 0) {
-            // Counter of the unit, tagged with the launch: a word of another launch (or of other use of the memory)
-            // counts as zero. The last one to come resets it, so a replayed graph finds no trace of its last run.
-            unsigned long long* ctr = p.counters + c_first;
-            const unsigned long long tag = p.launch_tag << 16;
-            unsigned long long seen = *reinterpret_cast<volatile unsigned long long*>(ctr), assumed, next;
-            bool last;
-            do {
-              assumed = seen;
-              const unsigned long long n = (assumed & ~0xffffull) == tag ? (assumed & 0xffffull) + 1 : 1;
-              last = n == static_cast<unsigned long long>(c_last - c_first + 1);
-              next = last ? 0ull : (tag | n);
-              seen = atomicCAS(ctr, assumed, next);
-            } while (seen != assumed);
-            __threadfence();
-            *s_last = last ? 1 : 0;
-          }
-          consumers_sync();
-          if (*s_last) {
-            // All consumers add the parts up: warp (mt, kg) takes every kGroups-th output column tile of row tile mt.
-            auto part_of = [&](int c) { return p.partials + (2 * static_cast<int64_t>(c) + (c == c_first ? 1 : 0)) * kPart; };
-            float mm0 = -INFINITY, mm1 = -INFINITY;
-            for (int c = c_first; c <= c_last; ++c) {
-              const float* st = part_of(c) + Cfg::kRows * D;
-              mm0 = fmaxf(mm0, __ldcg(st + r0));
-              mm1 = fmaxf(mm1, __ldcg(st + r1));
-            }
-            constexpr int kMine = kOT / kGroups;
-            float acc[kMine][4];
-#pragma unroll
-            for (int i = 0; i < kMine; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-            float sum0 = 0.f, sum1 = 0.f;
-            for (int c = c_first; c <= c_last; ++c) {
-              const float* pp = part_of(c);
-              const float* st = pp + Cfg::kRows * D;
-              const float f0 = part_scale(__ldcg(st + r0), mm0), f1 = part_scale(__ldcg(st + r1), mm1);
-              sum0 += f0 * __ldcg(st + Cfg::kRows + r0);
-              sum1 += f1 * __ldcg(st + Cfg::kRows + r1);
-              const float4* src = reinterpret_cast<const float4*>(pp) + mt * (kOT * 32) + lane;
-#pragma unroll
-              for (int i = 0; i < kMine; ++i) {
-                const float4 w = __ldcg(src + (kg * kMine + i) * 32);
-                acc[i][0] += f0 * w.x;
-                acc[i][1] += f0 * w.y;
-                acc[i][2] += f1 * w.z;
-                acc[i][3] += f1 * w.w;
-              }
-            }
-            const float i0 = sum0 > 0.f ? 1.f / sum0 : 0.f, i1 = sum1 > 0.f ? 1.f / sum1 : 0.f;
-#pragma unroll
-            for (int i = 0; i < kMine; ++i) {
-              store_pair(r0, kg * kMine + i, acc[i][0] * i0, acc[i][1] * i0);
-              store_pair(r1, kg * kMine + i, acc[i][2] * i1, acc[i][3] * i1);
-            }
-            if (kg == 0 && t4 == 0) {
-              store_lse(r0, mm0, sum0);
-              store_lse(r1, mm1, sum1);
+            for (int i = 0; i < kOT; i += 2) {
+              uint32_t vf[4];
+              ldsm4_trans(vb + (i / 8) * (kTile * 128) + kk * (16 * 128) + ((((i % 8) + (lm >> 1)) ^ lr) << 4), vf);
+              mma16816<BF16>(o[i], pa, vf[0], vf[1]);
+              mma16816<BF16>(o[i + 1], pa, vf[2], vf[3]);
             }
           }
         }
-        fresh = true;
+        __syncwarp();
+        if (j + 1 < seg_end) {  // the last V slot stays held
+          if (lane == 0) mbar_arrive(&empty[slot]);
+          next_slot();
+        }
       }
-      // The V slot goes back to the loader (as the scratch space it was written by the generic proxy).
-      if (seg_end) fence_proxy_async_smem();
+      // ---- the consumers' parts of this segment become one: the last V slot, still held, is the scratch space.
+      l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+      l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+      if (t4 == 0) {
+        float* st = s_stat + warp * 32;
+        st[g] = m0;
+        st[8 + g] = m1;
+        st[16 + g] = l0;
+        st[24 + g] = l1;
+      }
+      consumers_sync();
+      float t0 = -INFINITY, t1 = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < kGroups; ++w) {
+        t0 = fmaxf(t0, s_stat[(w * MT + mt) * 32 + g]);
+        t1 = fmaxf(t1, s_stat[(w * MT + mt) * 32 + 8 + g]);
+      }
+      float ls0 = 0.f, ls1 = 0.f;
+#pragma unroll
+      for (int w = 0; w < kGroups; ++w) {
+        const float* st = s_stat + (w * MT + mt) * 32;
+        ls0 += st[16 + g] * part_scale(st[g], t0);
+        ls1 += st[24 + g] * part_scale(st[8 + g], t1);
+      }
+      {
+        const float a0 = part_scale(m0, t0), a1 = part_scale(m1, t1);
+#pragma unroll
+        for (int i = 0; i < kOT; ++i) {
+          o[i][0] *= a0;
+          o[i][1] *= a0;
+          o[i][2] *= a1;
+          o[i][3] *= a1;
+        }
+      }
+      // Half of the key groups leave their fragments, the other half adds its own on top, then every warp sums its
+      // share of the columns over what is left: two barriers, and the rest of the segment's end is spread over
+      // all warps. 4 x 16 rows x D fp32 = one slot.
+      float4* scratch = reinterpret_cast<float4*>(smem + slot * Cfg::kSlotBytes);
+      constexpr int kHalf = kGroups / 2;
+      float4* mine = scratch + ((kg % kHalf) * MT + mt) * (kOT * 32) + lane;
+      if (kg >= kHalf) {
+#pragma unroll
+        for (int i = 0; i < kOT; ++i) mine[i * 32] = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+      }
+      consumers_sync();
+      if (kg < kHalf) {
+#pragma unroll
+        for (int i = 0; i < kOT; ++i) {
+          const float4 w = mine[i * 32];
+          mine[i * 32] = make_float4(o[i][0] + w.x, o[i][1] + w.y, o[i][2] + w.z, o[i][3] + w.w);
+        }
+      }
+      consumers_sync();
+      constexpr int kMine = kOT / kGroups;  // column tiles of this warp: kg * kMine + i
+      float4 part_o[kMine];
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) {
+        const float4* src = scratch + mt * (kOT * 32) + (kg * kMine + i) * 32 + lane;
+        part_o[i] = src[0];
+#pragma unroll
+        for (int w = 1; w < kHalf; ++w) {
+          const float4 t = src[w * MT * (kOT * 32)];
+          part_o[i].x += t.x;
+          part_o[i].y += t.y;
+          part_o[i].z += t.z;
+          part_o[i].w += t.w;
+        }
+      }
+      // ---- out, or a partial result
+      auto store_pair = [&](int r, int i, float a, float c) {
+        if (r < p.rows && i * 8 < p.head_dim) {
+          const int q = r / p.group, h = hk * p.group + (r - q * p.group);
+          *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.o_ptr) + b * p.o_batch_stride + q * p.o_row_stride +
+                                       h * p.o_head_stride + i * 8 + 2 * t4) = pack2<BF16>(a, c);
+        }
+      };
+      auto store_lse = [&](int r, float m, float l) {
+        if (r < p.rows) {
+          const int q = r / p.group, h = hk * p.group + (r - q * p.group);
+          p.lse_ptr[b * p.lse_batch_stride + h * p.lse_head_stride + q] = l > 0.f ? (m + lg2(l)) * 0.6931471805599453f : INFINITY;
+        }
+      };
+      const bool whole = seg_first == 0 && seg_end == p.tiles_per_unit;
+      if (whole) {
+        const float i0 = ls0 > 0.f ? 1.f / ls0 : 0.f, i1 = ls1 > 0.f ? 1.f / ls1 : 0.f;
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+          store_pair(r0, kg * kMine + i, part_o[i].x * i0, part_o[i].y * i0);
+          store_pair(r1, kg * kMine + i, part_o[i].z * i1, part_o[i].w * i1);
+        }
+        if (kg == 0 && t4 == 0) {
+          store_lse(r0, t0, ls0);
+          store_lse(r1, t1, ls1);
+        }
+      } else {
+        // Slot 2c holds a segment that began before this share, 2c + 1 one that began in it. Layout of a slot: O
+        // [row][column], then m and l of the rows; rows past the last one are neither written nor read.
+        constexpr int kPart = Cfg::kRows * (D + 2);  // floats
+        float* part = p.partials + (2 * static_cast<int64_t>(blockIdx.x) + (seg_first == 0 ? 1 : 0)) * kPart;
+        float2* dst = reinterpret_cast<float2*>(part + r0 * D + 2 * t4);
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+          if (r0 < p.rows) __stcg(dst + (kg * kMine + i) * 4, make_float2(part_o[i].x, part_o[i].y));
+          if (r1 < p.rows) __stcg(dst + 4 * D + (kg * kMine + i) * 4, make_float2(part_o[i].z, part_o[i].w));
+        }
+        if (kg == 0 && t4 == 0) {
+          float* st = part + Cfg::kRows * D;
+          __stcg(st + r0, t0);
+          __stcg(st + r1, t1);
+          __stcg(st + Cfg::kRows + r0, ls0);
+          __stcg(st + Cfg::kRows + r1, ls1);
+        }
+        __threadfence();
+        // CTAs whose shares touch this unit: the owners of its first and its last tile.
+        const int64_t g64 = gridDim.x;
+        const int64_t first_tile = static_cast<int64_t>(u) * p.tiles_per_unit;
+        const int c_first = static_cast<int>(((first_tile + 1) * g64 + n_tiles - 1) / n_tiles - 1);
+        const int c_last = static_cast<int>(((first_tile + p.tiles_per_unit) * g64 + n_tiles - 1) / n_tiles - 1);
+        auto part_index = [&](int c) { return 2 * c + (c == c_first ? 1 : 0); };
+        consumers_sync();
+        if (warp == 0) {
+          // One flag per part, set to the launch's number once the part is in memory: a flag left over from another
+          // launch, or from other use of the memory, is not set. Whoever sees all of a unit's flags set merges. The
+          // last to set one does (store, fence, load); two may, and then both write the same bits. A counter
+          // in place of the flags would need clearing, or a compare-and-swap that 19 CTAs queue up for (0.5 us each).
+          volatile unsigned long long* flags = p.flags;
+          if (lane == 0) flags[part_index(blockIdx.x)] = p.launch_tag;
+          __syncwarp();
+          asm volatile("fence.sc.gpu;" ::: "memory");
+          bool all = true;
+          for (int c = c_first + lane; c <= c_last; c += 32) all = all && flags[part_index(c)] == p.launch_tag;
+          all = __all_sync(0xffffffffu, all);
+          asm volatile("fence.acq_rel.gpu;" ::: "memory");
+          if (all) {
+            // A replayed graph launches with the same number: it has to find the flags clear.
+            for (int c = c_first + lane; c <= c_last; c += 32) flags[part_index(c)] = 0;
+          }
+          if (lane == 0) *s_last = all ? 1 : 0;
+        }
+        consumers_sync();
+        if (*s_last) {
+          // All consumers add the parts up: the rows' maxima and sums go to shared memory, then a thread takes four
+          // columns of a row at a time, with the loads of eight parts issued together: each is an L2 round trip.
+          auto part_of = [&](int c) { return p.partials + part_index(c) * static_cast<int64_t>(kPart); };
+          const int n_parts = c_last - c_first + 1;
+          float* sm = reinterpret_cast<float*>(scratch);
+          float* sl = sm + n_parts * Cfg::kRows;
+          for (int i = tid; i < n_parts * Cfg::kRows; i += kConsumers * 32) {
+            const int r = i % Cfg::kRows;
+            if (r < p.rows) {
+              const float* st = part_of(c_first + i / Cfg::kRows) + Cfg::kRows * D + r;
+              sm[i] = __ldcg(st);
+              sl[i] = __ldcg(st + Cfg::kRows);
+            }
+          }
+          consumers_sync();
+          for (int i = tid; i < p.rows * (D / 4); i += kConsumers * 32) {
+            const int r = i / (D / 4), col = i % (D / 4) * 4;
+            constexpr int kBatch = 8;
+            float m = -INFINITY, l = 0.f;
+            for (int c = 0; c < n_parts; ++c) m = fmaxf(m, sm[c * Cfg::kRows + r]);
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = 0; c < n_parts; c += kBatch) {
+              float4 w[kBatch];
+#pragma unroll
+              for (int e = 0; e < kBatch; ++e)
+                if (c + e < n_parts) w[e] = __ldcg(reinterpret_cast<const float4*>(part_of(c_first + c + e) + r * D + col));
+#pragma unroll
+              for (int e = 0; e < kBatch; ++e)
+                if (c + e < n_parts) {
+                  const float f = part_scale(sm[(c + e) * Cfg::kRows + r], m);
+                  l += f * sl[(c + e) * Cfg::kRows + r];
+                  acc.x += f * w[e].x;
+                  acc.y += f * w[e].y;
+                  acc.z += f * w[e].z;
+                  acc.w += f * w[e].w;
+                }
+            }
+            if (col < p.head_dim) {
+              const float inv = l > 0.f ? 1.f / l : 0.f;
+              const int q = r / p.group, h = hk * p.group + (r - q * p.group);
+              *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.o_ptr) + b * p.o_batch_stride + q * p.o_row_stride +
+                                        h * p.o_head_stride + col) =
+                  make_uint2(pack2<BF16>(acc.x * inv, acc.y * inv), pack2<BF16>(acc.z * inv, acc.w * inv));
+              if (col == 0) store_lse(r, m, l);
+            }
+          }
+        }
+      }
+      // The V slot goes back to the loader; as the scratch space it was written by the generic proxy.
+      fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[slot]);
-      if (++slot == Cfg::kSlots) {
-        slot = 0;
-        phase ^= 1;
-      }
-      if (++j == p.tiles_per_unit) {
+      next_slot();
+      if (j == p.tiles_per_unit) {
         j = 0;
         ++u;
       }

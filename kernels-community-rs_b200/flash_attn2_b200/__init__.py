@@ -17,7 +17,7 @@ def __getattr__(name):
         interface = importlib.import_module(__name__ + ".interface")
         if name == "interface":
             return interface
-        if name == "ops":
-            return interface.ops
-        return getattr(interface, name)
+        value = interface.ops if name == "ops" else getattr(interface, name)
+        globals()[name] = value  # the next use finds it without coming here
+        return value
     raise AttributeError(name)

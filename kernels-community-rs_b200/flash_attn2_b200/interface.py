@@ -1,17 +1,35 @@
 """Python surface of the operators, mirroring the reference package for the paths this library
 builds (flash-attn2-rs/tvm-ffi-ext/flash_attn2_rs/flash_attn_interface.py): the same function
 names, argument meaning, return lists and error behaviour for `fwd_explicit`, `fwd`, `bwd`,
-`varlen_fwd`, `varlen_bwd`, `flash_attn_func` and `flash_attn_varlen_func`. Every call goes through
-the tvm-ffi operators in `_ops`; there is no CPU implementation (CPU tensors raise
-NotImplementedError like the reference's CPU dispatch does).
+`varlen_fwd`, `varlen_bwd`, `flash_attn_func` and `flash_attn_varlen_func`. Plain dense calls (torch tensors in a
+layout the kernels address, no supplied outputs) go through the native module `_fa2_torch` (csrc/torch_calls.cc), which
+answers None for anything else; every other call, and every call that has to fail, goes through the tvm-ffi
+operators in `_ops`. There is no CPU implementation (CPU tensors raise NotImplementedError like the reference's CPU
+dispatch does).
 """
 from __future__ import annotations
 
+import importlib.machinery
+import importlib.util
 import operator
+from pathlib import Path
 
 import torch
 
 from ._ops import ops
+
+
+def _load_native():
+    path = Path(__file__).resolve().parent.parent / "lib" / "_fa2_torch.so"
+    if not path.exists():
+        raise ImportError(f"{path} is missing: build it with `python kernels-community-rs_b200/build.py`")
+    loader = importlib.machinery.ExtensionFileLoader("_fa2_torch", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fa2_torch", loader))
+    loader.exec_module(module)
+    return module
+
+
+_native = _load_native()
 
 
 def _torch_tensors(values):
@@ -60,6 +78,10 @@ def fwd_explicit(*args):
 def fwd(q, k, v, out=None, alibi_slopes=None, p_dropout=0.0, softmax_scale=None, is_causal=False,
         window_size_left=-1, window_size_right=-1, softcap=0.0, return_softmax=False, gen=None):
     """Returns [output, LSE, probabilities (empty), RNG state (unused)]."""
+    if out is None and return_softmax is False and type(p_dropout) is float and p_dropout == 0.0:
+        values = _native.fwd(q, k, v, softmax_scale, is_causal, window_size_left, window_size_right, softcap, alibi_slopes)
+        if values is not None:
+            return values
     _require_cuda("fwd", q, k, v, out, alibi_slopes)
     p = _float_arg(p_dropout, "p_dropout")
     scale = None if softmax_scale is None else _float_arg(softmax_scale, "softmax_scale")
@@ -97,6 +119,11 @@ def bwd(dout, q, k, v, out, softmax_lse, dq=None, dk=None, dv=None, alibi_slopes
         softmax_scale=None, is_causal=False, window_size_left=-1, window_size_right=-1, softcap=0.0,
         deterministic=False, gen=None, rng_state=None):
     """Returns [dQ, dK, dV, softmax_d] (softmax_d = rowsum(dO * O), padded to 128 rows)."""
+    if dq is None and dk is None and dv is None and type(p_dropout) is float and p_dropout == 0.0:
+        values = _native.bwd(dout, q, k, v, out, softmax_lse, softmax_scale, is_causal, window_size_left, window_size_right,
+                             softcap, alibi_slopes, deterministic)
+        if values is not None:
+            return values
     _require_cuda("bwd", dout, q, k, v, out, softmax_lse, dq, dk, dv)
     p = _float_arg(p_dropout, "p_dropout")
     scale = None if softmax_scale is None else _float_arg(softmax_scale, "softmax_scale")
@@ -219,6 +246,10 @@ def flash_attn_func(q, k, v, dropout_p=0.0, softmax_scale=None, causal=False, wi
     _no_dropout(dropout_p)
     if return_attn_probs:
         raise RuntimeError("return_attn_probs requires dropout, which is not built in the sm_100a library")
+    left, right = window_size
+    out = _native.attention(q, k, v, softmax_scale, causal, left, right, softcap, alibi_slopes, deterministic)
+    if out is not None:
+        return out
     return _DenseAttention.apply(q, k, v, softmax_scale, causal, tuple(window_size), softcap, alibi_slopes, deterministic)
 
 

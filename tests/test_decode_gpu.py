@@ -53,7 +53,7 @@ def test_few_query_rows(shape, opt, dtype):
 
 
 def test_workspace_contents_do_not_matter_and_graph_replays():
-    """Counters left over from anything else count as zero, and a captured call can be replayed."""
+    """Flags left over from anything else count as clear, and a captured call can be replayed."""
     import flash_attn2_b200 as fa2
 
     q, k, v = (t.cuda() for t in make_qkv(6, 1, 16, 4, 1, 5000, 128, torch.bfloat16))
