@@ -133,10 +133,10 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   return ti;
 }
 
-// FANCY: softcap or ALiBi in use; PACKED: cu_seqlens batches. Both are compile-time so that the plain dense
+// MODE: what is done to the scores; PACKED: cu_seqlens batches. Both are compile-time so that the plain dense
 // kernel carries none of their code: at 156 KB the all-in-one kernel missed the SM's instruction cache on a
 // quarter of its fetches and ran 6-9 % slower than the 62 KB one.
-template <int D, bool BF16, bool FANCY, bool PACKED>
+template <int D, bool BF16, int MODE, bool PACKED>
 __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = BwdCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -466,7 +466,9 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         v = p.delta[ti.bq * p.delta_batch_stride + hq * p.delta_head_stride + ti.q_row0 + ti.b * p.delta_seq_pad + q];
       return v;
     };
-    constexpr bool fancy = FANCY;
+    constexpr bool fancy = MODE == kScoreAny;
+    const float inv_cap1 = MODE == kScoreSoftcap ? p.scale / p.softcap : 0.f;
+    const float cap1 = p.softcap * kLog2e;
     Walk w{0, 0};
     float stat_next = n_iter > 0 ? load_stat(w) : 0.f;
     for (int it = 0; it < n_iter; ++it) {
@@ -499,14 +501,46 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         if (kpos >= ti.sk) c_hi = -1;
       }
       float pr[64];
-      if (!fancy) {
+      if constexpr (MODE == kScoreSoftcap) {
+        // P = exp2(cap tanh - lse); dS takes P times the derivative of the cap, 1 - tanh^2.
 #pragma unroll
         for (int i = 0; i < 64; i += 4) {
           const float4 l4 = lse4[i / 4];
-          pr[i] = ex2(fmaf(__uint_as_float(sr[i]), p.scale_log2, -l4.x));
-          pr[i + 1] = ex2(fmaf(__uint_as_float(sr[i + 1]), p.scale_log2, -l4.y));
-          pr[i + 2] = ex2(fmaf(__uint_as_float(sr[i + 2]), p.scale_log2, -l4.z));
-          pr[i + 3] = ex2(fmaf(__uint_as_float(sr[i + 3]), p.scale_log2, -l4.w));
+          const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+          float pp[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float t = tanh_approx(__uint_as_float(sr[i + e]) * inv_cap1);
+            pp[e] = ex2(fmaf(t, cap1, -l[e]));
+            if (need_mask && (i + e < c_lo || i + e >= c_hi)) pp[e] = 0.f;
+            pr[i + e] = pp[e] * fmaf(-t, t, 1.f);
+          }
+          sr[i / 2] = pack2<BF16>(pp[0], pp[1]);
+          sr[i / 2 + 1] = pack2<BF16>(pp[2], pp[3]);
+        }
+      } else if (!fancy) {
+        // The bias of a key is the same for all queries in the causal form of ALiBi.
+        float slope1 = 0.f, bias1 = 0.f;
+        if constexpr (MODE == kScoreAlibi) {
+          slope1 = p.alibi[ti.b * p.alibi_batch_stride + ti.hk * p.group + g_cur] * kLog2e;
+          bias1 = slope1 * static_cast<float>(kpos);
+          if (!p.causal_alibi) {
+            const float dist = static_cast<float>(qbase + ti.off - kpos);
+            bias1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 64; ++i)
+              sr[i] = __float_as_uint(fmaf(-slope1, fabsf(dist + static_cast<float>(i)), __uint_as_float(sr[i]) * p.scale_log2));
+          }
+        }
+        auto bias_minus = [&](float l) { return MODE == kScoreAlibi ? bias1 - l : -l; };
+        const float mul1 = MODE == kScoreAlibi && !p.causal_alibi ? 1.f : p.scale_log2;
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) {
+          const float4 l4 = lse4[i / 4];
+          pr[i] = ex2(fmaf(__uint_as_float(sr[i]), mul1, bias_minus(l4.x)));
+          pr[i + 1] = ex2(fmaf(__uint_as_float(sr[i + 1]), mul1, bias_minus(l4.y)));
+          pr[i + 2] = ex2(fmaf(__uint_as_float(sr[i + 2]), mul1, bias_minus(l4.z)));
+          pr[i + 3] = ex2(fmaf(__uint_as_float(sr[i + 3]), mul1, bias_minus(l4.w)));
         }
         if (need_mask) {
 #pragma unroll
@@ -758,7 +792,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-template <int D, bool BF16, bool FANCY, bool PACKED>
+template <int D, bool BF16, int MODE, bool PACKED>
 cudaError_t launch_one(const BwdParams& p, int num_ctas, cudaStream_t stream) {
   using Cfg = BwdCfg<D>;
   static bool configured[64] = {};
@@ -766,29 +800,33 @@ cudaError_t launch_one(const BwdParams& p, int num_ctas, cudaStream_t stream) {
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     cudaError_t e =
-        cudaFuncSetAttribute(bwd_kernel<D, BF16, FANCY, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(bwd_kernel<D, BF16, MODE, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  bwd_kernel<D, BF16, FANCY, PACKED><<<num_ctas, kThreads, Cfg::kSmemBytes, stream>>>(p);
+  bwd_kernel<D, BF16, MODE, PACKED><<<num_ctas, kThreads, Cfg::kSmemBytes, stream>>>(p);
   return cudaGetLastError();
 }
 
 template <int D, bool BF16>
-cudaError_t pick_features(const BwdParams& p, bool fancy, bool packed, int num_ctas, cudaStream_t stream) {
-  if (fancy) {
-    return packed ? launch_one<D, BF16, true, true>(p, num_ctas, stream)
-                  : launch_one<D, BF16, true, false>(p, num_ctas, stream);
+cudaError_t pick_features(const BwdParams& p, int mode, bool packed, int num_ctas, cudaStream_t stream) {
+  if (packed) {
+    return mode != kScorePlain ? launch_one<D, BF16, kScoreAny, true>(p, num_ctas, stream)
+                               : launch_one<D, BF16, kScorePlain, true>(p, num_ctas, stream);
   }
-  return packed ? launch_one<D, BF16, false, true>(p, num_ctas, stream)
-                : launch_one<D, BF16, false, false>(p, num_ctas, stream);
+  switch (mode) {
+    case kScorePlain: return launch_one<D, BF16, kScorePlain, false>(p, num_ctas, stream);
+    case kScoreSoftcap: return launch_one<D, BF16, kScoreSoftcap, false>(p, num_ctas, stream);
+    case kScoreAlibi: return launch_one<D, BF16, kScoreAlibi, false>(p, num_ctas, stream);
+    default: return launch_one<D, BF16, kScoreAny, false>(p, num_ctas, stream);
+  }
 }
 
 template <int D>
-cudaError_t pick_dtype(const BwdParams& p, bool bf16, bool fancy, bool packed, int num_ctas, cudaStream_t stream) {
-  return bf16 ? pick_features<D, true>(p, fancy, packed, num_ctas, stream)
-              : pick_features<D, false>(p, fancy, packed, num_ctas, stream);
+cudaError_t pick_dtype(const BwdParams& p, bool bf16, int mode, bool packed, int num_ctas, cudaStream_t stream) {
+  return bf16 ? pick_features<D, true>(p, mode, packed, num_ctas, stream)
+              : pick_features<D, false>(p, mode, packed, num_ctas, stream);
 }
 
 }  // namespace
@@ -797,10 +835,10 @@ cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int /*num_sm
   const int num_ctas = p.num_nblk * p.batch * p.heads_k;
   if (num_ctas <= 0) return cudaSuccess;
   if (head_dim <= 0 || head_dim > 128) return cudaErrorInvalidValue;
-  const bool fancy = (p.softcap > 0.f) || (p.alibi != nullptr);
+  const int mode = (p.softcap > 0.f ? kScoreSoftcap : 0) | (p.alibi != nullptr ? kScoreAlibi : 0);
   const bool packed = p.cu_q != nullptr;
-  return head_dim > 64 ? pick_dtype<128>(p, bf16, fancy, packed, num_ctas, stream)
-                       : pick_dtype<64>(p, bf16, fancy, packed, num_ctas, stream);
+  return head_dim > 64 ? pick_dtype<128>(p, bf16, mode, packed, num_ctas, stream)
+                       : pick_dtype<64>(p, bf16, mode, packed, num_ctas, stream);
 }
 
 }  // namespace fa2

@@ -5,6 +5,11 @@
 
 namespace fa2 {
 
+// What happens to a score besides the scale, as a template argument of the kernels for head dims up to 128: one
+// transform alone has code of its own, without a test per score for the other one. kScoreAny takes everything
+// (both transforms; in the forward also a negative scale without a transform) and is what packed batches use.
+enum ScoreMode : int { kScorePlain = 0, kScoreSoftcap = 1, kScoreAlibi = 2, kScoreAny = 3 };
+
 // Dense and packed (varlen) forward; head_dim is a multiple of 8 up to 128 (kernels for D = 64 and 128).
 cudaError_t launch_fwd(const FwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream);
 

@@ -203,10 +203,10 @@ __device__ __forceinline__ float tanh_approx(float x) {
   return y;
 }
 
-// FANCY: softcap, ALiBi or a negative scale in use; PACKED: cu_seqlens batches. Both are compile-time so that the
+// MODE: what is done to the scores; PACKED: cu_seqlens batches. Both are compile-time so that the
 // plain dense kernel carries none of their code and stays within reach of the SM's instruction cache: without the
 // score transforms the kernel is a third smaller and ran 3-4 % faster.
-template <int D, bool BF16, bool FANCY, bool PACKED>
+template <int D, bool BF16, int MODE, bool PACKED>
 __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
   using Cfg = FwdCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -293,7 +293,10 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
       const uint32_t addr = p_row + (c >> 3) * (kBlockM * 128) + ((static_cast<uint32_t>(c & 7) << 4) ^ p_swz);
       asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
     };
-    constexpr bool fancy = FANCY;
+    constexpr bool fancy = MODE == kScoreAny;
+    // What turns the (transformed) scores into the log2 domain.
+    const float mul = MODE == kScoreSoftcap ? p.softcap * 1.4426950408889634f : MODE == kScoreAlibi ? 1.f : p.scale_log2;
+    const float inv_cap = MODE == kScoreSoftcap ? p.scale / p.softcap : 0.f;
     uint32_t n_sfull = 0, n_pv = 0, n_store = 0, n_first = 0;
     for (int t = blockIdx.x; t - static_cast<int>(blockIdx.x) < p.num_tiles; t += gridDim.x) {
       const Tile ti = get_tile(p, ld, t);
@@ -304,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
       const int ne_s = s ? ti.ne[1] : ti.ne[0];
       float m = -INFINITY, l = 0.f;
       float slope = 0.f;
-      if (p.alibi != nullptr) slope = p.alibi[ti.b * p.alibi_batch_stride + ti.h] * 1.4426950408889634f;
+      if ((MODE == kScoreAlibi || MODE == kScoreAny) && p.alibi != nullptr) slope = p.alibi[ti.b * p.alibi_batch_stride + ti.h] * 1.4426950408889634f;
       bool ok = true;
       for (int j = nb_s; j < ne_s; ++j) {
         if (!warp_wait(&s_full[s], n_sfull & 1, ctl, kWaitSoftmaxSFull)) { ok = false; break; }
@@ -329,6 +332,31 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         if (!fancy) {
           // ---- fast path (also for tiles that touch a mask boundary: masked scores become -inf first):
           // row max with 3-input max, then the O rescale decision
+          if constexpr (MODE == kScoreSoftcap) {
+            // tanh is monotonic: everything that follows is the plain path with the cap as its scale.
+#pragma unroll
+            for (int i = 0; i < kBlockN; ++i) sr[i] = __float_as_uint(tanh_approx(__uint_as_float(sr[i]) * inv_cap));
+          }
+          if constexpr (MODE == kScoreAlibi) {
+            if (p.causal_alibi) {
+              const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), s2 = pack_f32x2(slope, slope);
+              const float base = slope * static_cast<float>(col0);
+              const uint64_t b2 = pack_f32x2(base, base);
+#pragma unroll
+              for (int i = 0; i < kBlockN; i += 2) {
+                const uint64_t bias = fma2(pack_f32x2(static_cast<float>(i), static_cast<float>(i + 1)), s2, b2);
+                float a, b;
+                unpack_f32x2(fma2(pack_f32x2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, bias), a, b);
+                sr[i] = __float_as_uint(a);
+                sr[i + 1] = __float_as_uint(b);
+              }
+            } else {
+              const float dist = static_cast<float>(row + ti.off - col0);
+#pragma unroll
+              for (int i = 0; i < kBlockN; ++i)
+                sr[i] = __float_as_uint(fmaf(-slope, fabsf(dist - static_cast<float>(i)), __uint_as_float(sr[i]) * p.scale_log2));
+            }
+          }
           if (need_mask) {
             int hi = ti.sk;
             if (p.window_right >= 0) hi = min(hi, row + ti.off + p.window_right + 1);
@@ -353,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
           }
           mx0 = max3(mx0, __uint_as_float(sr[kBlockN - 4]), __uint_as_float(sr[kBlockN - 3]));
           mx1 = max3(mx1, __uint_as_float(sr[kBlockN - 2]), __uint_as_float(sr[kBlockN - 1]));
-          const float m_new = fmaxf(m, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2);
+          const float m_new = fmaxf(m, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * mul);
           grow = (m_new - m) > kRescaleThreshold;
           if (grow) {
             alpha = ex2(m - m_new);
@@ -445,7 +473,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         }
         if (!fancy) {
           // ---- fast path: x = s * c - m with packed FMAs, exp2 on the MUFU unit, packed row-sum accumulation.
-          const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2);
+          const uint64_t c2 = pack_f32x2(mul, mul);
           // A row that has seen no key yet has m = -inf and only -inf scores: keep x = -inf (not NaN).
           const float neg_m = (m == -INFINITY) ? 0.f : -m;
           const uint64_t nm2 = pack_f32x2(neg_m, neg_m);
@@ -791,7 +819,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
 }
 
-template <int D, bool BF16, bool FANCY, bool PACKED>
+template <int D, bool BF16, int MODE, bool PACKED>
 cudaError_t launch_one(const FwdParams& p, int num_sms, cudaStream_t stream) {
   using Cfg = FwdCfg<D>;
   static bool configured[64] = {};
@@ -799,30 +827,34 @@ cudaError_t launch_one(const FwdParams& p, int num_sms, cudaStream_t stream) {
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     cudaError_t e =
-        cudaFuncSetAttribute(fwd_kernel<D, BF16, FANCY, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(fwd_kernel<D, BF16, MODE, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   const int grid = p.num_tiles < num_sms ? p.num_tiles : num_sms;
-  fwd_kernel<D, BF16, FANCY, PACKED><<<grid, kThreads, Cfg::kSmemBytes, stream>>>(p);
+  fwd_kernel<D, BF16, MODE, PACKED><<<grid, kThreads, Cfg::kSmemBytes, stream>>>(p);
   return cudaGetLastError();
 }
 
 template <int D, bool BF16>
-cudaError_t pick_features(const FwdParams& p, bool fancy, bool packed, int num_sms, cudaStream_t stream) {
-  if (fancy) {
-    return packed ? launch_one<D, BF16, true, true>(p, num_sms, stream)
-                  : launch_one<D, BF16, true, false>(p, num_sms, stream);
+cudaError_t pick_features(const FwdParams& p, int mode, bool packed, int num_sms, cudaStream_t stream) {
+  if (packed) {
+    return mode != kScorePlain ? launch_one<D, BF16, kScoreAny, true>(p, num_sms, stream)
+                               : launch_one<D, BF16, kScorePlain, true>(p, num_sms, stream);
   }
-  return packed ? launch_one<D, BF16, false, true>(p, num_sms, stream)
-                : launch_one<D, BF16, false, false>(p, num_sms, stream);
+  switch (mode) {
+    case kScorePlain: return launch_one<D, BF16, kScorePlain, false>(p, num_sms, stream);
+    case kScoreSoftcap: return launch_one<D, BF16, kScoreSoftcap, false>(p, num_sms, stream);
+    case kScoreAlibi: return launch_one<D, BF16, kScoreAlibi, false>(p, num_sms, stream);
+    default: return launch_one<D, BF16, kScoreAny, false>(p, num_sms, stream);
+  }
 }
 
 template <int D>
-cudaError_t pick_dtype(const FwdParams& p, bool bf16, bool fancy, bool packed, int num_sms, cudaStream_t stream) {
-  return bf16 ? pick_features<D, true>(p, fancy, packed, num_sms, stream)
-              : pick_features<D, false>(p, fancy, packed, num_sms, stream);
+cudaError_t pick_dtype(const FwdParams& p, bool bf16, int mode, bool packed, int num_sms, cudaStream_t stream) {
+  return bf16 ? pick_features<D, true>(p, mode, packed, num_sms, stream)
+              : pick_features<D, false>(p, mode, packed, num_sms, stream);
 }
 
 }  // namespace
@@ -831,10 +863,11 @@ cudaError_t launch_fwd(const FwdParams& p, int head_dim, bool bf16, int num_sms,
   if (p.num_tiles <= 0) return cudaSuccess;
   // Head dims below the kernel's D ride on TMA: loads past the real head dim read zeros, stores are clipped.
   if (head_dim <= 0 || head_dim > 128) return cudaErrorInvalidValue;
-  const bool fancy = (p.softcap > 0.f) || (p.alibi != nullptr) || (p.scale_log2 < 0.f);
+  int mode = (p.softcap > 0.f ? kScoreSoftcap : 0) | (p.alibi != nullptr ? kScoreAlibi : 0);
+  if (mode == kScorePlain && p.scale_log2 < 0.f) mode = kScoreAny;  // the plain path scales the row maximum
   const bool packed = p.cu_q != nullptr;
-  return head_dim > 64 ? pick_dtype<128>(p, bf16, fancy, packed, num_sms, stream)
-                       : pick_dtype<64>(p, bf16, fancy, packed, num_sms, stream);
+  return head_dim > 64 ? pick_dtype<128>(p, bf16, mode, packed, num_sms, stream)
+                       : pick_dtype<64>(p, bf16, mode, packed, num_sms, stream);
 }
 
 }  // namespace fa2
