@@ -101,11 +101,12 @@ FA2_API int fa2_bwd_preprocess(const fa2_bwd_preprocess_args* args, void* stream
 /* Backward: dQ, dK, dV from Q, K, V, dO, LSE and delta. dQ is accumulated in fp32 in
  * `dq_accum` (fa2_bwd_workspace_bytes() bytes, 16-byte aligned, need not be cleared) and
  * converted to the 16-bit dQ at the end. `which` selects outputs: bit 0 = dQ, bit 1 = dK and dV.
- * The workspace is the accumulator (B*Sq*H*D floats, rounded up to 256 bytes) followed by one 32-bit
- * turn counter per 32 query rows of every (batch, head). With them a dQ-only call (which = 1, the
- * deterministic bwd_dq of the reference) adds the key blocks' contributions in a fixed order, so dQ
- * is bit-reproducible; a workspace that only holds the accumulator is accepted too (arrival order).
- * dK and dV never use atomics and are always bit-reproducible. Head dims above 128 always add dQ in
+ * A dense dQ-only call (which = 1, the deterministic bwd_dq of the reference) up to head dim 128 has a
+ * kernel of its own that sums dQ in key order, so dQ is bit-reproducible; it needs no workspace. Elsewhere
+ * the workspace is the accumulator (B*Sq*H*D floats, rounded up to 256 bytes) followed by one 32-bit
+ * turn counter per 32 query rows of every (batch, head): with them a packed dQ-only call adds the key
+ * blocks' contributions in a fixed order; a workspace that only holds the accumulator is accepted too
+ * (arrival order). dK and dV never use atomics and are always bit-reproducible. Head dims above 128 always add dQ in
  * arrival order. A dQ-only call (which = 1) may pass dk = dv = NULL, a dK/dV-only call dq = dq_accum = NULL.
  * Replaces backward_component + the `backward` and `backward_kv` kernels
  * (flash-attn2-rs/src/host/backward.rs:14-566, src/device/backward/dq.rs:12-302,438-576,

@@ -472,6 +472,56 @@ int64_t bwd_turn_counters(const fa2_bwd_args* a) {
   return static_cast<int64_t>(a->batch) * a->heads * ((a->seqlen_q + 127) / 128) * 4;
 }
 
+// A dQ-only call for dense tensors has a kernel of its own up to head dim 128 and needs no accumulator.
+bool dq_kernel_takes(const fa2_bwd_args* a) { return a->which == 1 && a->cu_seqlens_q == nullptr && a->head_dim <= 128; }
+
+int bwd_dq(const fa2_bwd_args* a, Runtime* rt, cudaStream_t stream) {
+  fa2::DqParams p;
+  memset(&p, 0, sizeof(p));
+  const int d = a->head_dim;
+  const int64_t hd = static_cast<int64_t>(a->heads) * d;
+  int rc;
+  if ((rc = make_map(&p.tm_q, a->q, a->dtype, 2, d, a->heads, a->seqlen_q, a->batch, a->q_stride[2], a->q_stride[1],
+                     a->q_stride[0], 64, 128, "q")) != FA2_OK) return rc;
+  if ((rc = make_map(&p.tm_do, a->dout, a->dtype, 2, d, a->heads, a->seqlen_q, a->batch, a->do_stride[2], a->do_stride[1],
+                     a->do_stride[0], 64, 128, "dout")) != FA2_OK) return rc;
+  if ((rc = make_map(&p.tm_k, a->k, a->dtype, 2, d, a->heads_k, a->seqlen_k, a->batch, a->k_stride[2], a->k_stride[1],
+                     a->k_stride[0], 64, 128, "k")) != FA2_OK) return rc;
+  if ((rc = make_map(&p.tm_v, a->v, a->dtype, 2, d, a->heads_k, a->seqlen_k, a->batch, a->v_stride[2], a->v_stride[1],
+                     a->v_stride[0], 64, 128, "v")) != FA2_OK) return rc;
+  if ((rc = make_map(&p.tm_dq, a->dq, a->dtype, 2, d, a->heads, a->seqlen_q, a->batch, d, hd, a->seqlen_q * hd, 64, 128,
+                     "dq")) != FA2_OK) return rc;
+  const int64_t sq_pad = (a->seqlen_q + 127) / 128 * 128;
+  p.lse = a->lse;
+  p.delta = a->delta;
+  p.alibi = a->alibi_slopes;
+  p.alibi_batch_stride = a->alibi_batch_stride;
+  p.lse_head_stride = a->seqlen_q;
+  p.lse_batch_stride = static_cast<int64_t>(a->heads) * a->seqlen_q;
+  p.delta_head_stride = sq_pad;
+  p.delta_batch_stride = static_cast<int64_t>(a->heads) * sq_pad;
+  p.batch = a->batch;
+  p.heads = a->heads;
+  p.group = a->heads / a->heads_k;
+  p.seqlen_q = a->seqlen_q;
+  p.seqlen_k = a->seqlen_k;
+  p.num_mblk = (a->seqlen_q + 127) / 128;
+  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
+  p.window_left = w.left;
+  p.window_right = w.right;
+  p.causal_alibi = w.causal_alibi;
+  p.scale = a->softmax_scale;
+  p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
+  p.softcap = a->softcap > 0.f ? a->softcap : 0.f;
+  p.head_dim = d;
+  p.status = rt->status;
+  if (a->ev_kernel_start != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_start), stream);
+  const cudaError_t e = fa2::launch_bwd_dq(p, a->dtype == FA2_BF16, stream);
+  if (a->ev_kernel_stop != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_stop), stream);
+  if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "backward launch failed: %s", cudaGetErrorString(e));
+  return FA2_OK;
+}
+
 int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
   if (a == nullptr) return fail(FA2_E_VALUE, "args is null");
   if (a->dtype != FA2_F16 && a->dtype != FA2_BF16) return fail(FA2_E_TYPE, "q, k, v must be float16 or bfloat16");
@@ -506,7 +556,11 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
     }
     return FA2_OK;
   }
-  if (want_dq) {
+  const bool dq_alone = dq_kernel_takes(a);
+  if (dq_alone) {
+    if (a->dq == nullptr) return fail(FA2_E_VALUE, "dq must be non-null");
+    if (reinterpret_cast<uintptr_t>(a->dq) % 16) return fail(FA2_E_VALUE, "dq must be 16-byte aligned");
+  } else if (want_dq) {
     if (a->dq == nullptr || a->dq_accum == nullptr) return fail(FA2_E_VALUE, "dq and dq_accum must be non-null");
     if (a->dq_accum_bytes < n_dq * 4) return fail(FA2_E_VALUE, "dq_accum is smaller than fa2_bwd_workspace_bytes()");
     if (reinterpret_cast<uintptr_t>(a->dq_accum) % 16 || reinterpret_cast<uintptr_t>(a->dq) % 16)
@@ -522,6 +576,7 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
   if ((rc = check_layout(a->dout, a->do_stride + so, ns, "dout")) != FA2_OK) return rc;
   if (want_dkv && (reinterpret_cast<uintptr_t>(a->dk) % 16 || reinterpret_cast<uintptr_t>(a->dv) % 16))
     return fail(FA2_E_VALUE, "dk and dv must be 16-byte aligned");
+  if (dq_alone) return bwd_dq(a, rt, stream);
 
   fa2::BwdParams p;
   memset(&p, 0, sizeof(p));
@@ -785,7 +840,7 @@ extern "C" {
 int fa2_bwd_preprocess(const fa2_bwd_preprocess_args* args, void* stream) { return bwd_preprocess_impl(args, stream); }
 
 int64_t fa2_bwd_workspace_bytes(const fa2_bwd_args* args) {
-  if (args == nullptr || (args->which & 1) == 0) return 0;
+  if (args == nullptr || (args->which & 1) == 0 || dq_kernel_takes(args)) return 0;
   // The fp32 accumulator, then (used by dQ-only calls) one turn counter per 32 query rows of every
   // (batch, head) for the ordered accumulation.
   return bwd_accum_bytes(args) + bwd_turn_counters(args) * 4;

@@ -31,6 +31,9 @@ cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int num_sms,
 // 64 rows; p.tm_q and p.tm_do carry boxes of 64 rows, dQ goes through p.dq_acc, dK and dV through p.dk_ptr / p.dv_ptr.
 cudaError_t launch_bwd_wide(const BwdParams& p, int head_dim, bool bf16, cudaStream_t stream);
 
+// dQ alone, dense, head_dim a multiple of 8 up to 128: summed in key order, written as 16-bit.
+cudaError_t launch_bwd_dq(const DqParams& p, bool bf16, cudaStream_t stream);
+
 // delta = rowsum(dO * O) into the padded layouts (dense [B,H,Sq_pad], packed [H,total_q+128*B]).
 cudaError_t launch_bwd_preprocess(const PreprocessParams& p, cudaStream_t stream);
 

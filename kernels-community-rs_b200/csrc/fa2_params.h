@@ -21,6 +21,7 @@ enum WaitSite : int {
   kWaitEpiPvDone = 42,
   kWaitBwd = 50,
   kWaitDecode = 80,
+  kWaitBwdDq = 90,
 };
 
 struct FwdParams {
@@ -111,6 +112,23 @@ struct BwdParams {
   // That kernel reads V row by row from global memory (it keeps V in TMEM): element strides of [batch, row, head].
   const void* v_ptr;
   int64_t v_batch_stride, v_row_stride, v_head_stride;
+};
+
+// dQ alone, dense, head dims up to 128 (bwd_dq_sm100.cu).
+struct DqParams {
+  CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_dq;  // box (64, 1, 128, 1)
+  const float* lse;
+  const float* delta;
+  const float* alibi;
+  int64_t lse_head_stride, lse_batch_stride;
+  int64_t delta_head_stride, delta_batch_stride;
+  int alibi_batch_stride, causal_alibi;
+  int batch, heads, group, seqlen_q, seqlen_k;
+  int num_mblk;                         // ceil(seqlen_q / 128)
+  int window_left, window_right;
+  float scale, scale_log2, softcap;
+  int head_dim;
+  int* status;
 };
 
 struct PreprocessParams {

@@ -1,0 +1,45 @@
+"""GPU parity of the dQ-only backward call (dense, head dims up to 128) against the CPU oracle: tile edges, ragged
+lengths, masks, score transforms, head groups, rows without keys; and the same bits from every run."""
+import pytest
+import torch
+
+from tests._cases import BWD_TOL, alibi_slopes, make_qkv
+
+pytestmark = pytest.mark.gpu
+
+# (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim), options
+CASES = [
+    ((1, 1, 1, 1, 1, 8), {}),
+    ((2, 4, 2, 128, 128, 128), dict(causal=True)),
+    ((1, 4, 1, 129, 127, 64), {}),
+    ((1, 4, 4, 777, 777, 128), dict(causal=True)),
+    ((1, 2, 2, 100, 1409, 96), dict(causal=True)),
+    ((1, 2, 2, 640, 200, 128), dict(causal=True)),                      # rows without keys
+    ((1, 4, 2, 500, 900, 64), dict(window_left=130, window_right=70)),
+    ((1, 2, 1, 300, 300, 128), dict(causal=True, softcap=15.0)),
+    ((1, 4, 2, 300, 420, 64), dict(causal=True, alibi=True)),
+    ((1, 4, 2, 300, 420, 128), dict(alibi=True)),
+    ((1, 2, 2, 260, 260, 128), dict(causal=True, softcap=20.0, alibi=True)),
+]
+
+
+@pytest.mark.parametrize("shape,opt", CASES, ids=[str(c[0]) for c in CASES])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
+def test_dq_alone(shape, opt, dtype):
+    from flash_attn2_b200 import cabi_ops as ops
+    from oracle.attention_oracle import attention_backward
+
+    b, h, hk, sq, sk, d = shape
+    opt = dict(opt)
+    q, k, v, do = make_qkv(11, b, h, hk, sq, sk, d, dtype, with_do=True)
+    slopes = alibi_slopes(h) if opt.pop("alibi", False) else None
+    gpu = dict(alibi_slopes=None if slopes is None else slopes.cuda(), **opt)
+    qc, kc, vc, doc = q.cuda(), k.cuda(), v.cuda(), do.cuda()
+    out, lse = ops.fwd(qc, kc, vc, **gpu)
+    delta = ops.bwd_preprocess(doc, out)
+    dq = ops.bwd(qc, kc, vc, doc, lse, delta, which=1, **gpu)[0]
+    assert ops.device_status() == 0
+    ref = attention_backward(q, k, v, do, out=out.float().cpu(), lse=lse.cpu(), alibi_slopes=slopes, **opt)[0]
+    torch.testing.assert_close(dq.float().cpu(), ref, **BWD_TOL[dtype])
+    for _ in range(2):
+        assert torch.equal(ops.bwd(qc, kc, vc, doc, lse, delta, which=1, **gpu)[0], dq)
