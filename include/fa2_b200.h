@@ -143,6 +143,15 @@ typedef struct fa2_bwd_args {
   const float* alibi_slopes;
   int32_t alibi_batch_stride;
   float softcap;
+  /* With `out` (the forward's output) the call computes delta itself, into the memory `delta` points to,
+   * and clears the accumulator in the same pass: one kernel instead of fa2_bwd_preprocess and a fill.
+   * NULL: `delta` is an input. */
+  const void* out;
+  int64_t o_stride[3];
+  /* 1: several CTAs may share a key block when there are too few of them for the GPU (dense, head dims up to 128);
+   * the workspace then has room for their fp32 parts. dK and dV are the same bits every time either way, but not the
+   * same with and without. */
+  int32_t share_key_blocks;
 } fa2_bwd_args;
 FA2_API int64_t fa2_bwd_workspace_bytes(const fa2_bwd_args* args);
 FA2_API int fa2_bwd(const fa2_bwd_args* args, void* stream);

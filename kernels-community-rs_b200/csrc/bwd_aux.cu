@@ -2,7 +2,7 @@
 //   * delta = rowsum(dO * O) in fp32, written into the padded layouts the reference uses
 //     (flash-attn2-rs/src/device/backward/reduce.rs:40-108, src/device/varlen/backward.rs:53-132);
 //   * the final dQ = 16-bit(scale * fp32 accumulator) conversion
-//     (same shape as the reference's backward_dq_merge, reduce.rs:164-197).
+//     (same shape as the reference's backward_dq_merge, reduce.rs:164-197), and the sum of split key blocks' parts.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include "fa2_params.h"
@@ -76,6 +76,10 @@ __global__ void __launch_bounds__(256) preprocess_kernel(const PreprocessParams 
       y[r] = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.out) + bq * p.o_batch_stride +
                                             row * p.o_row_stride + h * p.o_head_stride)[lane];
     }
+    if (p.zero_acc != nullptr && live && lane < chunks) {
+      float4* z = reinterpret_cast<float4*>(p.zero_acc + ((static_cast<int64_t>(b) * p.seqlen_q + s) * p.heads + h) * p.head_dim) + 2 * lane;
+      z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     if (++h == p.heads) {
       h = 0;
       if (++s == p.seqlen_pad) {
@@ -101,27 +105,58 @@ __global__ void __launch_bounds__(256) preprocess_kernel(const PreprocessParams 
 }
 
 template <bool BF16>
-__global__ void __launch_bounds__(256) dq_convert_kernel(const float4* __restrict__ src, uint4* __restrict__ dst,
-                                                         int64_t n8, float scale) {
-  // From the end of the accumulator to its start: the backward kernel walks the heads in ascending order, so
-  // what it touched last (and the L2 still holds) sits at the end.
-  for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < n8;
-       j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t i = n8 - 1 - j;
-    const float4 a = src[2 * i], b = src[2 * i + 1];
-    uint4 w;
-    if constexpr (BF16) {
-      __nv_bfloat162 t0 = __floats2bfloat162_rn(a.x * scale, a.y * scale), t1 = __floats2bfloat162_rn(a.z * scale, a.w * scale);
-      __nv_bfloat162 t2 = __floats2bfloat162_rn(b.x * scale, b.y * scale), t3 = __floats2bfloat162_rn(b.z * scale, b.w * scale);
-      w = make_uint4(*reinterpret_cast<uint32_t*>(&t0), *reinterpret_cast<uint32_t*>(&t1),
-                     *reinterpret_cast<uint32_t*>(&t2), *reinterpret_cast<uint32_t*>(&t3));
-    } else {
-      __half2 t0 = __floats2half2_rn(a.x * scale, a.y * scale), t1 = __floats2half2_rn(a.z * scale, a.w * scale);
-      __half2 t2 = __floats2half2_rn(b.x * scale, b.y * scale), t3 = __floats2half2_rn(b.z * scale, b.w * scale);
-      w = make_uint4(*reinterpret_cast<uint32_t*>(&t0), *reinterpret_cast<uint32_t*>(&t1),
-                     *reinterpret_cast<uint32_t*>(&t2), *reinterpret_cast<uint32_t*>(&t3));
+__device__ __forceinline__ uint4 pack8(const float4 a, const float4 b, float scale) {
+  uint4 w;
+  if constexpr (BF16) {
+    __nv_bfloat162 t0 = __floats2bfloat162_rn(a.x * scale, a.y * scale), t1 = __floats2bfloat162_rn(a.z * scale, a.w * scale);
+    __nv_bfloat162 t2 = __floats2bfloat162_rn(b.x * scale, b.y * scale), t3 = __floats2bfloat162_rn(b.z * scale, b.w * scale);
+    w = make_uint4(*reinterpret_cast<uint32_t*>(&t0), *reinterpret_cast<uint32_t*>(&t1),
+                   *reinterpret_cast<uint32_t*>(&t2), *reinterpret_cast<uint32_t*>(&t3));
+  } else {
+    __half2 t0 = __floats2half2_rn(a.x * scale, a.y * scale), t1 = __floats2half2_rn(a.z * scale, a.w * scale);
+    __half2 t2 = __floats2half2_rn(b.x * scale, b.y * scale), t3 = __floats2half2_rn(b.z * scale, b.w * scale);
+    w = make_uint4(*reinterpret_cast<uint32_t*>(&t0), *reinterpret_cast<uint32_t*>(&t1),
+                   *reinterpret_cast<uint32_t*>(&t2), *reinterpret_cast<uint32_t*>(&t3));
+  }
+  return w;
+}
+
+// Bound by memory: the accumulator is read and dQ written once. blockIdx.y 0: dQ; 1: the parts of split key blocks.
+template <bool BF16>
+__global__ void __launch_bounds__(256) finish_kernel(const __grid_constant__ FinishParams p) {
+  const int64_t first = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  if (blockIdx.y == 0) {
+    if (p.dq_acc == nullptr) return;
+    const float4* src = reinterpret_cast<const float4*>(p.dq_acc);
+    uint4* dst = static_cast<uint4*>(p.dq);
+    const int64_t n8 = p.n_dq / 8;
+    // From the end of the accumulator to its start: the backward kernel walks the heads in ascending order, so
+    // what it touched last (and the L2 still holds) sits at the end.
+    for (int64_t j = first; j < n8; j += step) {
+      const int64_t i = n8 - 1 - j;
+      dst[i] = pack8<BF16>(src[2 * i], src[2 * i + 1], p.scale);
     }
-    dst[i] = w;
+  } else {
+    // Parts are summed in the order of the walk, so dK and dV come out the same every time.
+    const int per_row = p.row_elems / 8;
+    const int64_t n8 = static_cast<int64_t>(p.batch) * p.rows * per_row;
+    for (int64_t i = first; i < n8; i += step) {
+      const int row = static_cast<int>((i / per_row) % p.rows), nb = row / 128;
+      const int parts = p.part_start[nb + 1] - p.part_start[nb];
+      if (parts < 2) continue;  // the main kernel has written it
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        const float4* src = reinterpret_cast<const float4*>(which ? p.dv_part : p.dk_part) + 2 * i;
+        float4 a = src[0], b = src[1];
+        for (int e = 1; e < parts; ++e) {
+          const float4 c = src[e * (p.part_stride / 4)], d = src[e * (p.part_stride / 4) + 1];
+          a = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w + c.w);
+          b = make_float4(b.x + d.x, b.y + d.y, b.z + d.z, b.w + d.w);
+        }
+        static_cast<uint4*>(which ? p.dv : p.dk)[i] = pack8<BF16>(a, b, which ? 1.f : p.scale);
+      }
+    }
   }
 }
 
@@ -200,13 +235,14 @@ cudaError_t launch_copy_rows(const void* src, void* dst, int64_t n0, int64_t n1,
   return cudaGetLastError();
 }
 
-cudaError_t launch_dq_convert(const float* src, void* dst, int64_t n, float scale, bool bf16, cudaStream_t stream) {
-  const int64_t n8 = n / 8;
-  if (n8 == 0) return cudaSuccess;
-  const int64_t want = (n8 + 255) / 256;
-  const unsigned grid = static_cast<unsigned>(want < 148 * 16 ? want : 148 * 16);
-  if (bf16) dq_convert_kernel<true><<<grid, 256, 0, stream>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<uint4*>(dst), n8, scale);
-  else dq_convert_kernel<false><<<grid, 256, 0, stream>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<uint4*>(dst), n8, scale);
+cudaError_t launch_bwd_finish(const FinishParams& p, cudaStream_t stream) {
+  const int64_t n_dq = p.dq_acc != nullptr ? p.n_dq / 8 : 0;
+  const int64_t n_dkv = p.dk_part != nullptr ? static_cast<int64_t>(p.batch) * p.rows * (p.row_elems / 8) : 0;
+  const int64_t want = ((n_dq > n_dkv ? n_dq : n_dkv) + 255) / 256;
+  if (want == 0) return cudaSuccess;
+  const dim3 grid(static_cast<unsigned>(want < 148 * 16 ? want : 148 * 16), n_dkv > 0 ? 2 : 1);
+  if (p.bf16) finish_kernel<true><<<grid, 256, 0, stream>>>(p);
+  else finish_kernel<false><<<grid, 256, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

@@ -64,6 +64,8 @@ struct KvTile {
   int b, hk, n0;
   int sq, sk, q_row0, k_row0, bq, off;
   int m_start, n_m, n_iter;
+  int g0, mi0;         // where the walk over (query head, query block) starts
+  int part, parts;     // which part of a split key block this CTA is
   bool valid;
 };
 
@@ -103,8 +105,26 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   // dQ accumulator stay in L2 while the 16-odd CTAs that add into it run side by side. With a
   // causal mask the first key blocks see the most query rows, so each head starts with its
   // heaviest CTAs.
-  const int bh = t / p.num_nblk;
-  int nblk = t - bh * p.num_nblk;
+  int bh, nblk;
+  ti.part = 0;
+  ti.parts = 1;
+  if (p.dk_part != nullptr) {
+    // The parts of all key blocks of a head, block by block.
+    bh = t / p.items_per_head;
+    const int i = t - bh * p.items_per_head;
+    int lo = 0, hi = p.num_nblk;  // part_start[lo] <= i < part_start[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (p.part_start[mid] <= i) lo = mid;
+      else hi = mid;
+    }
+    nblk = lo;
+    ti.part = i - p.part_start[lo];
+    ti.parts = p.part_start[lo + 1] - p.part_start[lo];
+  } else {
+    bh = t / p.num_nblk;
+    nblk = t - bh * p.num_nblk;
+  }
   // Ordered dQ accumulation waits for the higher key blocks of the same head. CTAs start in grid order, so
   // there the highest key block comes first: a CTA only ever waits for CTAs that were started before it,
   // whatever the number of key blocks and of resident CTAs.
@@ -130,6 +150,13 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   ti.valid = ti.n0 < ti.sk;
   q_block_range(p, ti.sq, ti.sk, ti.n0, ti.m_start, ti.n_m);
   ti.n_iter = ti.n_m * p.group;
+  ti.g0 = ti.mi0 = 0;
+  if (ti.parts > 1) {
+    const int first = ti.n_iter * ti.part / ti.parts;
+    ti.n_iter = ti.n_iter * (ti.part + 1) / ti.parts - first;
+    ti.g0 = first / ti.n_m;
+    ti.mi0 = first - ti.g0 * ti.n_m;
+  }
   return ti;
 }
 
@@ -209,8 +236,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     // The first loads go out before the rest of the CTA is set up (TMEM allocation, the block-wide
     // barrier): their latency is the longest item of a CTA's start.
     if (ti.n_iter > 0) {
-      const int hq0 = ti.hk * p.group;
-      const int m00 = ti.m_start * kBlk;
+      const int hq0 = ti.hk * p.group + ti.g0;
+      const int m00 = (ti.m_start + ti.mi0) * kBlk;
       mbar_expect_tx(kv_full, Cfg::kTileBytes);
       mbar_expect_tx(v_full, Cfg::kTileBytes);
       mbar_expect_tx(&q_full[0], Cfg::kTileBytes);
@@ -243,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       // ---------------------------------------------------------------- loader
       // K, V and the first Q / dO tiles were requested during set-up.
       bool ok = true;
-      Walk w{0, 0};
+      Walk w{ti.g0, ti.mi0};
       for (int it = 1; it < n_iter && ok; ++it) {
         w = walk_next(w, ti.n_m);
         const int hq = ti.hk * p.group + w.g;
@@ -319,12 +346,12 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       bool ok = n_iter > 0;
       if (ok) ok = mbar_wait(kv_full, 0, ctl, kWaitBwd + 3);
       if (ok && packed && ti.n0 + kBlk > ti.sk) ok = mbar_wait(kv_fixed, 0, ctl, kWaitBwd + 20);
-      if (ok) ok = q_ready(0, 0, 0, kWaitBwd + 4);  // iteration 0 is query block m_start
+      if (ok) ok = q_ready(ti.mi0, 0, 0, kWaitBwd + 4);
       if (ok) {
         tc_fence_after();
         kmajor_pair(tmem + Cfg::kTmemS, k_kmaj, q_kmaj);
         mma_commit(s_full);
-        ok = do_ready(0, 0, 0, kWaitBwd + 5);
+        ok = do_ready(ti.mi0, 0, 0, kWaitBwd + 5);
         if (ok) ok = mbar_wait(v_full, 0, ctl, kWaitBwd + 3);
       }
       if (ok) {
@@ -332,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj);
         mma_commit(dp_full);
       }
-      Walk wn{0, 0};  // position of iteration it + 1
+      Walk wn{ti.g0, ti.mi0};  // position of iteration it + 1
       for (int it = 0; it < n_iter && ok; ++it) {
         wn = walk_next(wn, ti.n_m);
         const uint32_t st = it & 1;
@@ -422,7 +449,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           publish(kv_fixed);
         }
       }
-      Walk w{0, 0};
+      Walk w{ti.g0, ti.mi0};
       for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
         const int first = ti.sq - (ti.m_start + w.mi) * kBlk;
         const uint32_t st = it & 1, ph = (it >> 1) & 1;
@@ -469,7 +496,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     constexpr bool fancy = MODE == kScoreAny;
     const float inv_cap1 = MODE == kScoreSoftcap ? p.scale / p.softcap : 0.f;
     const float cap1 = p.softcap * kLog2e;
-    Walk w{0, 0};
+    Walk w{ti.g0, ti.mi0};
     float stat_next = n_iter > 0 ? load_stat(w) : 0.f;
     for (int it = 0; it < n_iter; ++it) {
       const int m0 = (ti.m_start + w.mi) * kBlk;
@@ -637,28 +664,43 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
 #pragma unroll
           for (int i = 0; i < D; ++i) acc[i] = 0;
         }
+        if (!PACKED && ti.parts > 1) {
+          // A part of a split key block: fp32, 32 bytes (a whole sector) per store.
+          if (kpos < ti.sk) {
+            float* row = (wg == 0 ? p.dk_part : p.dv_part) + ti.part * p.part_stride + ti.bq * p.dkv_batch_stride +
+                         static_cast<int64_t>(kpos) * p.dkv_row_stride + ti.hk * p.dkv_head_stride;
 #pragma unroll
-        for (int c = 0; c < D / 8; ++c) {  // 16-byte chunks of the row
-          uint4 w;
-          w.x = pack2<BF16>(__uint_as_float(acc[8 * c]) * mul, __uint_as_float(acc[8 * c + 1]) * mul);
-          w.y = pack2<BF16>(__uint_as_float(acc[8 * c + 2]) * mul, __uint_as_float(acc[8 * c + 3]) * mul);
-          w.z = pack2<BF16>(__uint_as_float(acc[8 * c + 4]) * mul, __uint_as_float(acc[8 * c + 5]) * mul);
-          w.w = pack2<BF16>(__uint_as_float(acc[8 * c + 6]) * mul, __uint_as_float(acc[8 * c + 7]) * mul);
-          if (tma_store) {
-            *reinterpret_cast<uint4*>(stage + (c / 8) * (kBlk * 128) + key_in * 128 + (((c & 7) ^ (key_in & 7)) << 4)) = w;
-          } else if (kpos < ti.sk && c * 8 < p.head_dim) {
-            *reinterpret_cast<uint4*>(grow + c * 8) = w;
+            for (int c = 0; c < D / 8; ++c)
+              if (c * 8 < p.head_dim)
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(row + 8 * c), "r"(acc[8 * c]),
+                             "r"(acc[8 * c + 1]), "r"(acc[8 * c + 2]), "r"(acc[8 * c + 3]), "r"(acc[8 * c + 4]),
+                             "r"(acc[8 * c + 5]), "r"(acc[8 * c + 6]), "r"(acc[8 * c + 7])
+                             : "memory");
           }
-        }
-        if (tma_store) {
-          fence_proxy_async_smem();
-          mbar_arrive(&epi_full[wg]);
-          if ((ct & 127) == 0 && mbar_wait(&epi_full[wg], 0, ctl, kWaitBwd + 16)) {
+        } else {
 #pragma unroll
-            for (int a = 0; a < Cfg::kAtoms; ++a)
-              if (a * 64 < p.head_dim) tma_store_4d(tm, stage + a * (kBlk * 128), a * 64, ti.hk, ti.k_row0 + ti.n0, ti.bq);
-            tma_commit_group();
-            tma_wait_group_read<0>();  // the staging tile must outlive the copy's reads, not its writes
+          for (int c = 0; c < D / 8; ++c) {  // 16-byte chunks of the row
+            uint4 w;
+            w.x = pack2<BF16>(__uint_as_float(acc[8 * c]) * mul, __uint_as_float(acc[8 * c + 1]) * mul);
+            w.y = pack2<BF16>(__uint_as_float(acc[8 * c + 2]) * mul, __uint_as_float(acc[8 * c + 3]) * mul);
+            w.z = pack2<BF16>(__uint_as_float(acc[8 * c + 4]) * mul, __uint_as_float(acc[8 * c + 5]) * mul);
+            w.w = pack2<BF16>(__uint_as_float(acc[8 * c + 6]) * mul, __uint_as_float(acc[8 * c + 7]) * mul);
+            if (tma_store) {
+              *reinterpret_cast<uint4*>(stage + (c / 8) * (kBlk * 128) + key_in * 128 + (((c & 7) ^ (key_in & 7)) << 4)) = w;
+            } else if (kpos < ti.sk && c * 8 < p.head_dim) {
+              *reinterpret_cast<uint4*>(grow + c * 8) = w;
+            }
+          }
+          if (tma_store) {
+            fence_proxy_async_smem();
+            mbar_arrive(&epi_full[wg]);
+            if ((ct & 127) == 0 && mbar_wait(&epi_full[wg], 0, ctl, kWaitBwd + 16)) {
+#pragma unroll
+              for (int a = 0; a < Cfg::kAtoms; ++a)
+                if (a * 64 < p.head_dim) tma_store_4d(tm, stage + a * (kBlk * 128), a * 64, ti.hk, ti.k_row0 + ti.n0, ti.bq);
+              tma_commit_group();
+              tma_wait_group_read<0>();  // the staging tile must outlive the copy's reads, not its writes
+            }
           }
         }
       }
@@ -673,7 +715,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     const uint32_t t_dq = tmem + lane_addr + Cfg::kTmemDP;
     if (want_dq) {
       bool ok = true;
-      Walk w{0, 0};
+      Walk w{ti.g0, ti.mi0};
       for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
         const int hq = ti.hk * p.group + w.g;
         const int m0 = (ti.m_start + w.mi) * kBlk;
@@ -832,7 +874,7 @@ cudaError_t pick_dtype(const BwdParams& p, bool bf16, int mode, bool packed, int
 }  // namespace
 
 cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int /*num_sms*/, cudaStream_t stream) {
-  const int num_ctas = p.num_nblk * p.batch * p.heads_k;
+  const int num_ctas = (p.dk_part != nullptr ? p.items_per_head : p.num_nblk) * p.batch * p.heads_k;
   if (num_ctas <= 0) return cudaSuccess;
   if (head_dim <= 0 || head_dim > 128) return cudaErrorInvalidValue;
   const int mode = (p.softcap > 0.f ? kScoreSoftcap : 0) | (p.alibi != nullptr ? kScoreAlibi : 0);

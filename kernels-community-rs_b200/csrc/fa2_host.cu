@@ -132,7 +132,9 @@ class DeviceScope {
       device_ = attr.device;
     else
       cudaGetLastError();  // an unknown pointer is not an error of this call
-    if (device_ != prev_) cudaSetDevice(device_);
+    // Also when it is current already: a thread that has made no runtime call yet (autograd's) has no context bound,
+    // and the driver's tensor-map encoder needs one.
+    cudaSetDevice(device_);
   }
   ~DeviceScope() {
     if (device_ != prev_) cudaSetDevice(prev_);
@@ -409,7 +411,7 @@ int fwd_common(const fa2_fwd_args* a, void* stream_v, bool packed) {
   return FA2_OK;
 }
 
-int bwd_preprocess_impl(const fa2_bwd_preprocess_args* a, void* stream_v) {
+int preprocess_launch(const fa2_bwd_preprocess_args* a, float* zero_acc, void* stream_v) {
   if (a == nullptr) return fail(FA2_E_VALUE, "args is null");
   if (a->dtype != FA2_F16 && a->dtype != FA2_BF16) return fail(FA2_E_TYPE, "dout and out must be float16 or bfloat16");
   const int d = a->head_dim;
@@ -427,6 +429,7 @@ int bwd_preprocess_impl(const fa2_bwd_preprocess_args* a, void* stream_v) {
   if ((rc = check_layout(a->out, a->o_stride + (packed ? 1 : 0), ns, "out")) != FA2_OK) return rc;
   fa2::PreprocessParams p;
   memset(&p, 0, sizeof(p));
+  p.zero_acc = zero_acc;
   p.dout = a->dout;
   p.out = a->out;
   p.delta = a->delta;
@@ -457,6 +460,8 @@ int bwd_preprocess_impl(const fa2_bwd_preprocess_args* a, void* stream_v) {
   return FA2_OK;
 }
 
+int bwd_preprocess_impl(const fa2_bwd_preprocess_args* a, void* stream_v) { return preprocess_launch(a, nullptr, stream_v); }
+
 int64_t bwd_rows(const fa2_bwd_args* a) {
   return a->cu_seqlens_q != nullptr ? static_cast<int64_t>(a->total_q)
                                     : static_cast<int64_t>(a->batch) * a->seqlen_q;
@@ -467,9 +472,77 @@ int64_t bwd_accum_bytes(const fa2_bwd_args* a) {
   return (bwd_rows(a) * a->heads * a->head_dim * 4 + 255) / 256 * 256;
 }
 
+// What a call with dQ keeps in front of the parts of split key blocks.
+int64_t bwd_dq_bytes(const fa2_bwd_args* a);
+
 // One counter per (batch, head, 128-row query block, 32-row slab of a drain warp).
 int64_t bwd_turn_counters(const fa2_bwd_args* a) {
   return static_cast<int64_t>(a->batch) * a->heads * ((a->seqlen_q + 127) / 128) * 4;
+}
+
+// ---- key blocks shared by several CTAs (bwd_sm100.cu: part_start). A CTA owns 128 keys of one kv head and walks the
+// query blocks of all the group's heads; with few (batch, kv head, key block) triples most SMs would have nothing
+// to do, or wait for the CTA with the longest walk.
+struct BwdSplit {
+  int items_per_head = 0;      // 0: not split
+  int64_t part_elems = 0;      // elements of one slot (= elements of dK)
+  int max_parts = 1;
+  uint16_t start[fa2::kMaxSplitBlocks + 1];
+  int64_t bytes() const { return items_per_head > 0 ? 2 * max_parts * ((part_elems * 4 + 255) / 256 * 256) : 0; }
+};
+void plan_bwd_split(const fa2_bwd_args* a, int sm_count, BwdSplit* out) {
+  const int nblk = (a->seqlen_k + 127) / 128;
+  const int64_t units = static_cast<int64_t>(a->batch) * a->heads_k;
+  if (!a->share_key_blocks || a->cu_seqlens_q != nullptr || a->head_dim > 128 || (a->which & 2) == 0 || a->seqlen_q <= 0 || a->seqlen_k <= 0 ||
+      nblk > fa2::kMaxSplitBlocks || units * nblk > 2 * sm_count)
+    return;
+  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
+  const int64_t off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q, group = a->heads / a->heads_k;
+  int64_t n[fa2::kMaxSplitBlocks], most = 0, total = 0, least = INT64_MAX;
+  for (int i = 0; i < nblk; ++i) {
+    const int64_t n0 = i * 128LL, n_last = std::min<int64_t>(n0 + 127, a->seqlen_k - 1);
+    int64_t lo = 0, hi = a->seqlen_q;
+    if (w.right >= 0) lo = std::max<int64_t>(0, n0 - off - w.right);
+    if (w.left >= 0) hi = std::min<int64_t>(hi, n_last - off + w.left + 1);
+    n[i] = hi > lo ? ((hi + 127) / 128 - lo / 128) * group : 0;
+    most = std::max(most, n[i]);
+    least = std::min(least, n[i]);
+    total += n[i];
+  }
+  // Costs in cycles, from clock stamps: an iteration of the walk, a CTA's start and end, and per byte of the parts
+  // (written and read once each at the memory's rate). The same split for calls with and without dQ: dK and dV are the
+  // same bits in both.
+  const double t_it = a->head_dim > 64 ? 4300 : 3000, t_cta = 8500;
+  const int64_t dkv = static_cast<int64_t>(a->batch) * a->seqlen_k * a->heads_k * a->head_dim;
+  const double base_cost = 4000, part_cost = dkv * 16.0 / 3400;
+  auto cost = [&](double items, double longest, double all, bool even) {
+    if (items <= sm_count) return longest;
+    if (even) return std::ceil(items / sm_count) * longest;
+    return std::max(longest, all / sm_count + longest / 2);
+  };
+  double best = cost(static_cast<double>(units * nblk), most * t_it + t_cta, units * (total * t_it + nblk * t_cta), least == most);
+  int best_parts = 1;
+  for (int parts = 2; parts <= 8 && parts <= most; ++parts) {
+    const int64_t len = (most + parts - 1) / parts;
+    int64_t items = 0;
+    for (int i = 0; i < nblk; ++i) items += std::max<int64_t>(1, (n[i] + len - 1) / len);
+    const double c = cost(static_cast<double>(units * items), len * t_it + t_cta, units * (total * t_it + items * t_cta), true) +
+                     base_cost + part_cost * parts;
+    if (c < 0.95 * best) {
+      best = c;
+      best_parts = parts;
+    }
+  }
+  if (best_parts == 1) return;
+  const int64_t len = (most + best_parts - 1) / best_parts;
+  out->start[0] = 0;
+  for (int i = 0; i < nblk; ++i) {
+    const int64_t parts = std::max<int64_t>(1, (n[i] + len - 1) / len);
+    out->max_parts = std::max<int>(out->max_parts, static_cast<int>(parts));
+    out->start[i + 1] = static_cast<uint16_t>(out->start[i] + parts);
+  }
+  out->items_per_head = out->start[nblk];
+  out->part_elems = dkv;
 }
 
 // A dQ-only call for dense tensors has a kernel of its own up to head dim 128 and needs no accumulator.
@@ -515,11 +588,32 @@ int bwd_dq(const fa2_bwd_args* a, Runtime* rt, cudaStream_t stream) {
   p.softcap = a->softcap > 0.f ? a->softcap : 0.f;
   p.head_dim = d;
   p.status = rt->status;
+  if (a->out != nullptr) {
+    fa2_bwd_preprocess_args pre;
+    memset(&pre, 0, sizeof(pre));
+    pre.dout = a->dout;
+    pre.out = a->out;
+    pre.delta = const_cast<float*>(a->delta);
+    pre.dtype = a->dtype;
+    pre.batch = a->batch;
+    pre.seqlen_q = a->seqlen_q;
+    pre.heads = a->heads;
+    pre.head_dim = d;
+    memcpy(pre.do_stride, a->do_stride, sizeof(pre.do_stride));
+    memcpy(pre.o_stride, a->o_stride, sizeof(pre.o_stride));
+    if ((rc = preprocess_launch(&pre, nullptr, stream)) != FA2_OK) return rc;
+  }
   if (a->ev_kernel_start != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_start), stream);
   const cudaError_t e = fa2::launch_bwd_dq(p, a->dtype == FA2_BF16, stream);
   if (a->ev_kernel_stop != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_stop), stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "backward launch failed: %s", cudaGetErrorString(e));
   return FA2_OK;
+}
+
+int64_t bwd_dq_bytes(const fa2_bwd_args* a) {
+  if ((a->which & 1) == 0 || dq_kernel_takes(a)) return 0;
+  // The fp32 accumulator, then (used by dQ-only calls) the turn counters of the ordered accumulation.
+  return (bwd_accum_bytes(a) + bwd_turn_counters(a) * 4 + 255) / 256 * 256;
 }
 
 int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
@@ -657,8 +751,49 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
   const bool ordered = !wide && a->which == 1 && a->dq_accum_bytes >= acc_bytes + n_turn * 4;
   p.dq_turn = ordered ? reinterpret_cast<int*>(static_cast<char*>(a->dq_accum) + acc_bytes) : nullptr;
   p.num_mblk_q = (a->seqlen_q + 127) / 128;
-  if (want_dq && (e = cudaMemsetAsync(a->dq_accum, 0, ordered ? acc_bytes + n_turn * 4 : n_dq * 4, stream)) != cudaSuccess)
+  // With `out` the delta preprocess is part of this call and clears the accumulator on its way.
+  const bool fused_pre = a->out != nullptr && !packed && !ordered;
+  if (a->out != nullptr) {
+    fa2_bwd_preprocess_args pre;
+    memset(&pre, 0, sizeof(pre));
+    pre.dout = a->dout;
+    pre.out = a->out;
+    pre.delta = const_cast<float*>(a->delta);
+    pre.dtype = a->dtype;
+    pre.batch = a->batch;
+    pre.seqlen_q = a->seqlen_q;
+    pre.heads = a->heads;
+    pre.head_dim = d;
+    memcpy(pre.do_stride, a->do_stride, sizeof(pre.do_stride));
+    memcpy(pre.o_stride, a->o_stride, sizeof(pre.o_stride));
+    pre.cu_seqlens_q = a->cu_seqlens_q;
+    pre.total_q = a->total_q;
+    if ((rc = preprocess_launch(&pre, fused_pre && want_dq ? static_cast<float*>(a->dq_accum) : nullptr, stream)) != FA2_OK) return rc;
+  }
+  if (want_dq && !fused_pre &&
+      (e = cudaMemsetAsync(a->dq_accum, 0, ordered ? acc_bytes + n_turn * 4 : n_dq * 4, stream)) != cudaSuccess)
     return fail(FA2_E_RUNTIME, "memset failed: %s", cudaGetErrorString(e));
+  fa2::FinishParams fin;
+  fin.dk_part = nullptr;
+  BwdSplit split;
+  plan_bwd_split(a, rt->sm_count, &split);
+  const int64_t before = bwd_dq_bytes(a);
+  if (split.items_per_head > 0 && a->dq_accum != nullptr && a->dq_accum_bytes >= before + split.bytes()) {
+    p.dk_part = reinterpret_cast<float*>(static_cast<char*>(a->dq_accum) + before);
+    p.part_stride = (split.part_elems * 4 + 255) / 256 * 64;
+    p.dv_part = p.dk_part + split.max_parts * p.part_stride;
+    p.items_per_head = split.items_per_head;
+    memcpy(p.part_start, split.start, sizeof(split.start));
+    fin.dk_part = p.dk_part;
+    fin.dv_part = p.dv_part;
+    fin.dk = a->dk;
+    fin.dv = a->dv;
+    fin.part_stride = p.part_stride;
+    fin.batch = a->batch;
+    fin.rows = a->seqlen_k;
+    fin.row_elems = a->heads_k * d;
+    memcpy(fin.part_start, split.start, sizeof(split.start));
+  }
   if (a->ev_kernel_start != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_start), stream);
   p.head_dim = d;
   p.dq_acc = static_cast<float*>(a->dq_accum);
@@ -671,9 +806,13 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
            : fa2::launch_bwd(p, d, a->dtype == FA2_BF16, rt->sm_count, stream);
   if (a->ev_kernel_stop != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_stop), stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "backward launch failed: %s", cudaGetErrorString(e));
-  if (want_dq && (e = fa2::launch_dq_convert(static_cast<const float*>(a->dq_accum), a->dq, n_dq, a->softmax_scale,
-                                             a->dtype == FA2_BF16, stream)) != cudaSuccess)
-    return fail(FA2_E_RUNTIME, "dq convert launch failed: %s", cudaGetErrorString(e));
+  fin.dq_acc = want_dq ? static_cast<const float*>(a->dq_accum) : nullptr;
+  fin.dq = a->dq;
+  fin.n_dq = n_dq;
+  fin.scale = a->softmax_scale;
+  fin.bf16 = a->dtype == FA2_BF16;
+  if ((e = fa2::launch_bwd_finish(fin, stream)) != cudaSuccess)
+    return fail(FA2_E_RUNTIME, "conversion launch failed: %s", cudaGetErrorString(e));
   return FA2_OK;
 }
 
@@ -828,7 +967,14 @@ int bwd_static_impl(const fa2_bwd_args* a, void* stream_v) {
   p.head_dim = d;
   if ((e = fa2::launch_bwd(p, d, a->dtype == FA2_BF16, rt->sm_count, stream)) != cudaSuccess)
     return fail(FA2_E_RUNTIME, "backward launch failed: %s", cudaGetErrorString(e));
-  if ((e = fa2::launch_dq_convert(rt->accum, a->dq, n_dq, a->softmax_scale, a->dtype == FA2_BF16, stream)) != cudaSuccess)
+  fa2::FinishParams fin;
+  fin.dk_part = nullptr;
+  fin.dq_acc = rt->accum;
+  fin.dq = a->dq;
+  fin.n_dq = n_dq;
+  fin.scale = a->softmax_scale;
+  fin.bf16 = a->dtype == FA2_BF16;
+  if ((e = fa2::launch_bwd_finish(fin, stream)) != cudaSuccess)
     return fail(FA2_E_RUNTIME, "dq convert launch failed: %s", cudaGetErrorString(e));
   return FA2_OK;
 }
@@ -840,10 +986,16 @@ extern "C" {
 int fa2_bwd_preprocess(const fa2_bwd_preprocess_args* args, void* stream) { return bwd_preprocess_impl(args, stream); }
 
 int64_t fa2_bwd_workspace_bytes(const fa2_bwd_args* args) {
-  if (args == nullptr || (args->which & 1) == 0 || dq_kernel_takes(args)) return 0;
-  // The fp32 accumulator, then (used by dQ-only calls) one turn counter per 32 query rows of every
-  // (batch, head) for the ordered accumulation.
-  return bwd_accum_bytes(args) + bwd_turn_counters(args) * 4;
+  if (args == nullptr || args->heads_k <= 0 || args->heads <= 0 || args->heads % args->heads_k != 0 || args->batch <= 0) return 0;
+  int64_t bytes = bwd_dq_bytes(args);
+  if ((args->which & 2) != 0 && args->cu_seqlens_q == nullptr && args->head_dim <= 128) {
+    const DeviceScope scope(args->q);
+    Runtime* rt = nullptr;
+    BwdSplit split;
+    if (get_runtime(scope.device(), &rt) == FA2_OK) plan_bwd_split(args, rt->sm_count, &split);
+    bytes += split.bytes();
+  }
+  return bytes;
 }
 
 int fa2_bwd(const fa2_bwd_args* args, void* stream) { return bwd_impl(args, stream); }

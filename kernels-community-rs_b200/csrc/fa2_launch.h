@@ -40,7 +40,7 @@ cudaError_t launch_bwd_preprocess(const PreprocessParams& p, cudaStream_t stream
 // Copy of a 16-bit [n0, n1, n2, d] tensor (unit last stride) between two layouts given by their outer element strides.
 cudaError_t launch_copy_rows(const void* src, void* dst, int64_t n0, int64_t n1, int64_t n2, int64_t d,
                              const int64_t src_strides[3], const int64_t dst_strides[3], cudaStream_t stream);
-// dst(16-bit) = src(fp32) * scale over n elements (n a multiple of 8).
-cudaError_t launch_dq_convert(const float* src, void* dst, int64_t n, float scale, bool bf16, cudaStream_t stream);
+// The conversions after the main backward kernel, in one launch.
+cudaError_t launch_bwd_finish(const FinishParams& p, cudaStream_t stream);
 
 }  // namespace fa2

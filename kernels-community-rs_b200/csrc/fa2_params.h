@@ -73,6 +73,8 @@ struct DecodeParams {
   int* status;
 };
 
+constexpr int kMaxSplitBlocks = 160;   // a grid of more key blocks fills the GPU by itself
+
 struct BwdParams {
   CUtensorMap tm_q, tm_k, tm_v, tm_do;  // 16-bit inputs, box (64, 1, 128, 1)
   CUtensorMap tm_dk, tm_dv;             // 16-bit outputs, box (64, 1, 128, 1)
@@ -99,6 +101,14 @@ struct BwdParams {
   int causal_alibi;                     // bias = slope * key index instead of -slope * |distance|
   float softcap;                        // scores = softcap * tanh(raw * scale / softcap)
   int head_dim;                         // real head dim (<= the kernel's D; columns beyond it are padding)
+  // Split key blocks (null = none): the walk over (query head, query block) of key block n is shared by
+  // part_start[n + 1] - part_start[n] CTAs, each of which leaves its fp32 dK and dV in a slot of its own,
+  // dk_part + part * part_stride in the layout of dK; a block with one part is written as usual.
+  float* dk_part;
+  float* dv_part;
+  int64_t part_stride;                  // elements
+  int items_per_head;                   // part_start[num_nblk]
+  uint16_t part_start[kMaxSplitBlocks + 1];
   // Ordered dQ accumulation (null = arrival order). dq_turn[((batch * heads + head) * num_mblk_q + query
   // block) * 4 + drain warp] counts the key blocks whose adds into those 32 rows have landed; it is
   // zero at launch. A CTA adds only when the count equals the number of higher key blocks that add into the
@@ -131,7 +141,25 @@ struct DqParams {
   int* status;
 };
 
+// What is left after the main backward kernel: dQ = 16-bit(scale * accumulator), and the sum of the parts of split key
+// blocks, dK (scaled) and dV as 16-bit.
+struct FinishParams {
+  const float* dq_acc;                  // null: no dQ
+  void* dq;
+  int64_t n_dq;                         // elements, a multiple of 8
+  const float* dk_part;                 // null: no split key blocks
+  const float* dv_part;
+  void* dk;
+  void* dv;
+  int64_t part_stride;
+  int batch, rows, row_elems;           // dK and dV are [batch][rows][row_elems]
+  float scale;
+  int bf16;
+  uint16_t part_start[kMaxSplitBlocks + 1];
+};
+
 struct PreprocessParams {
+  float* zero_acc;                      // dense: clears the fp32 [batch, seqlen_q, heads, head_dim] accumulator too (or null)
   const void* dout;
   const void* out;
   float* delta;

@@ -143,19 +143,6 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
   const auto dt = q.scalar_type();
   Gradients g;
   g.delta = empty({qs[0], qs[2], (qs[1] + 127) / 128 * 128}, at::kFloat, q.device());
-  fa2_bwd_preprocess_args p{};
-  p.dout = dout.data_ptr();
-  p.out = out.data_ptr();
-  p.delta = static_cast<float*>(g.delta.data_ptr());
-  p.dtype = dt == at::kBFloat16 ? FA2_BF16 : FA2_F16;
-  p.batch = static_cast<int32_t>(qs[0]);
-  p.seqlen_q = static_cast<int32_t>(qs[1]);
-  p.heads = static_cast<int32_t>(qs[2]);
-  p.head_dim = static_cast<int32_t>(qs[3]);
-  strides_of(dout, p.do_stride);
-  strides_of(out, p.o_stride);
-  check(fa2_bwd_preprocess(&p, stream));
-
   g.dq = empty(qs, dt, q.device());
   g.dk = empty(ks, dt, q.device());
   g.dv = empty(ks, dt, q.device());
@@ -169,13 +156,13 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
   a.dq = g.dq.data_ptr();
   a.dk = g.dk.data_ptr();
   a.dv = g.dv.data_ptr();
-  a.dtype = p.dtype;
-  a.batch = p.batch;
-  a.seqlen_q = p.seqlen_q;
+  a.dtype = dt == at::kBFloat16 ? FA2_BF16 : FA2_F16;
+  a.batch = static_cast<int32_t>(qs[0]);
+  a.seqlen_q = static_cast<int32_t>(qs[1]);
   a.seqlen_k = static_cast<int32_t>(ks[1]);
-  a.heads = p.heads;
+  a.heads = static_cast<int32_t>(qs[2]);
   a.heads_k = static_cast<int32_t>(ks[2]);
-  a.head_dim = p.head_dim;
+  a.head_dim = static_cast<int32_t>(qs[3]);
   strides_of(q, a.q_stride);
   strides_of(k, a.k_stride);
   strides_of(v, a.v_stride);
@@ -189,6 +176,9 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
   a.causal = effective_causal(o, qs[1]);
   a.window_left = static_cast<int32_t>(o.left);
   a.window_right = static_cast<int32_t>(o.right);
+  a.out = out.data_ptr();  // the first call computes delta
+  strides_of(out, a.o_stride);
+  a.share_key_blocks = 1;
   // Bit-reproducible gradients come from the two separate calls: dQ in a fixed order, then dK and dV.
   const int calls[2] = {deterministic ? 1 : 3, deterministic ? 2 : 0};
   for (const int which : calls) {
@@ -202,6 +192,7 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
       a.dq_accum = workspace.data_ptr();
     }
     check(fa2_bwd(&a, stream));
+    a.out = nullptr;
   }
   return g;
 }

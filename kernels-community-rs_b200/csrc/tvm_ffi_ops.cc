@@ -426,6 +426,7 @@ Any bwd_impl(const AnyView* args, int32_t n, int which) {
   a.window_left = static_cast<int32_t>(wl);
   a.window_right = static_cast<int32_t>(wr);
   a.which = which;
+  a.share_key_blocks = 1;
   // Gradients are allocated like the inputs (backward.rs:199-204); the fp32 dQ accumulator is a
   // workspace tensor from the same stream-ordered allocator.
   // Only what the call returns is allocated (bwd_dq: dQ; bwd_dkv: dK and dV).

@@ -56,6 +56,7 @@ class BwdArgs(C.Structure):
         ("total_q", C.c_int32), ("total_k", C.c_int32),
         ("ev_kernel_start", C.c_void_p), ("ev_kernel_stop", C.c_void_p),
         ("alibi_slopes", C.c_void_p), ("alibi_batch_stride", C.c_int32), ("softcap", C.c_float),
+        ("out", C.c_void_p), ("o_stride", C.c_int64 * 3), ("share_key_blocks", C.c_int32),
     ]
 
 

@@ -43,3 +43,36 @@ def test_dq_alone(shape, opt, dtype):
     torch.testing.assert_close(dq.float().cpu(), ref, **BWD_TOL[dtype])
     for _ in range(2):
         assert torch.equal(ops.bwd(qc, kc, vc, doc, lse, delta, which=1, **gpu)[0], dq)
+
+
+# (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim), options: key blocks whose walk several CTAs share
+SPLIT_CASES = [
+    ((1, 4, 1, 777, 777, 128), dict(causal=True)),
+    ((1, 1, 1, 2000, 130, 64), {}),
+    ((2, 8, 2, 513, 513, 96), dict(causal=True, window_left=200)),
+    ((1, 2, 2, 1025, 1000, 128), {}),
+    ((1, 8, 1, 300, 1100, 64), dict(causal=True, softcap=20.0)),
+]
+
+
+@pytest.mark.parametrize("shape,opt", SPLIT_CASES, ids=[str(c[0]) for c in SPLIT_CASES])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["f16", "bf16"])
+@pytest.mark.parametrize("deterministic", [False, True], ids=["all", "pair"])
+def test_split_key_blocks(shape, opt, dtype, deterministic):
+    """Through `bwd`, whose first launch computes delta and clears the accumulator as well."""
+    import flash_attn2_b200 as fa2
+    from oracle.attention_oracle import attention_backward
+
+    b, h, hk, sq, sk, d = shape
+    q, k, v, do = make_qkv(12, b, h, hk, sq, sk, d, dtype, with_do=True)
+    qc, kc, vc, doc = q.cuda(), k.cuda(), v.cuda(), do.cuda()
+    args = dict(is_causal=opt.get("causal", False), window_size_left=opt.get("window_left", -1), softcap=opt.get("softcap", 0.0))
+    out, lse = fa2.fwd(qc, kc, vc, **args)[:2]
+    got = fa2.bwd(doc, qc, kc, vc, out, lse, deterministic=deterministic, **args)
+    ref = attention_backward(q, k, v, do, out=out.float().cpu(), lse=lse.cpu(), **opt)
+    for name, g, r in zip(("dq", "dk", "dv"), got, ref):
+        torch.testing.assert_close(g.float().cpu(), r, msg=lambda m, n=name: f"{n}: {m}", **BWD_TOL[dtype])
+    torch.testing.assert_close(got[3].cpu(), ref[3], atol=2e-5, rtol=1e-5)
+    again = fa2.bwd(doc, qc, kc, vc, out, lse, deterministic=deterministic, **args)
+    assert torch.equal(again[1], got[1]) and torch.equal(again[2], got[2])
+    assert fa2.cabi_ops.device_status() == 0
