@@ -12,17 +12,26 @@
 //   P^T   = exp2(S^T c - lse)     compute warps, written back over S^T as 16-bit
 //   dV_c += P^T dO_c              TMEM x smem (dO as an MN-major operand)
 //   dS^T  = P^T (dP^T - delta)    compute warps -> swizzled smem [128 keys x 64 q]
-//   dK_c += dS^T Q_c              smem x smem (Q as an MN-major operand)
 //   dQ_c^T = K_c^T dS^T           smem x smem, both MN-major -> TMEM [128 d x 64 q] over the dP^T columns; the
-//                                 compute warps transpose it into the retired Q stage (one d column per thread,
-//                                 [64 q x 32 d] fp32 per warp) and add it into the fp32 dQ accumulator with one
-//                                 cp.reduce.async.bulk per warp (64 plain reductions per thread took 3500 cycles
-//                                 an iteration and set its pace)
+//                                 drain warps transpose it into a staging buffer (one d column per thread, two
+//                                 pieces of [32 q x 32 d] fp32 per warp) and add it into the fp32 dQ accumulator
+//                                 with cp.reduce.async.bulk (64 plain reductions per thread took 3500 cycles)
+//   dK_c += dS^T Q_c              smem x smem (Q as an MN-major operand)
 //
 // TMEM columns: dK_c [0,128) dV_c [128,256) S^T/P^T [256,320) dP^T/dQ_c^T [320,384) V [384,512).
-// Shared memory: K whole (64 KB), two stages of a Q and a dO tile of 64 rows (32 KB each), dS^T (16 KB).
-// Warps: 0-3 compute (one key row per thread; one d row per thread for dQ^T), 4 loader, 5 MMA issuer,
-// 6 fixer (packed batches: clears the rows of K, Q and dO tiles that lie past the end of the sequence).
+// Shared memory: K whole (64 KB), two stages of a Q and a dO tile of 64 rows (32 KB each), dS^T (16 KB),
+// dQ staging (16 KB).
+// Warps: 0-7 compute (two warpgroups, 32 query columns each, one key row per thread), 8-11 dQ drain (one d row of
+// dQ^T per thread), 12 loader, 13 MMA issuer, 14 fixer (packed batches: clears the rows of K, Q and dO tiles that lie
+// past the end of the sequence).
+//
+// What bounds it: an iteration's MMAs take about 2700 cycles (those with N = 64 cost up to 54 instead of 32 each), and
+// the chain S^T -> P^T -> dV, dS^T -> dQ, dK around them. One warpgroup that did P^T, dS^T and the drain in turn, with the
+// next S^T issued behind dK and dQ, took 6500 cycles an iteration (its share of a CTA's start and end included). Two
+// warpgroups halve both steps of the chain, the drain runs beside the next iteration's P^T, and S^T is issued right
+// behind dV, the last reader of P^T: 5900. The drain has a staging buffer of its own, so the Q stage goes back to the
+// loader when dK has read it and not when the reductions have: 4800. Kernel at B4 H16/8 S2048 D256 causal bf16:
+// 833 -> 754 -> 610 us.
 //
 // Stands in, for these head dims, for the reference kernels `backward` and `backward_kv`
 // (flash-attn2-rs/src/device/backward/dq.rs:12-302, dkv.rs:15-266, common.rs:121-152) and their packed
@@ -37,10 +46,12 @@ namespace {
 
 constexpr int kBK = 128;  // keys per CTA
 constexpr int kBQ = 64;   // query rows per iteration
-constexpr int kBWThreads = 256;
-constexpr int kBWLoadWarp = 4;
-constexpr int kBWMmaWarp = 5;
-constexpr int kBWFixWarp = 6;
+constexpr int kBWThreads = 512;
+constexpr int kBWCompute = 256;  // threads of the compute warps
+constexpr int kBWDrainWarp = 8;  // the first of four
+constexpr int kBWLoadWarp = 12;
+constexpr int kBWMmaWarp = 13;
+constexpr int kBWFixWarp = 14;
 constexpr float kBWLog2e = 1.4426950408889634f;
 
 struct BwdWideCfg {
@@ -52,7 +63,9 @@ struct BwdWideCfg {
   static constexpr int kQOff = kMaxAtoms * kAtomK;        // 2 stages
   static constexpr int kDOOff = kQOff + 2 * kStageBytes;  // 2 stages
   static constexpr int kDSOff = kDOOff + 2 * kStageBytes; // [128 keys x 64 q] 16-bit, one atom
-  static constexpr int kBarOff = kDSOff + kAtomK;
+  static constexpr int kDQOff = kDSOff + kAtomK;          // dQ staging: [32 q x 32 d] fp32 per drain warp
+  static constexpr int kDQPiece = 32 * 128;
+  static constexpr int kBarOff = kDQOff + 4 * kDQPiece;
   static constexpr int kNumBars = 23;
   static constexpr int kMiscOff = (kBarOff + kNumBars * 8 + 15) / 16 * 16;
   static constexpr int kStatOff = kMiscOff + 32;   // lse / delta: [2 buffers][2][64] fp32
@@ -144,7 +157,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   uint64_t* k_full = bars + 0;
   uint64_t* q_full = bars + 1;     // [2]
   uint64_t* do_full = bars + 3;    // [2]
-  uint64_t* q_free = bars + 5;     // [2] S^T and dK have read the Q stage and the dQ reductions staged in it have left
+  uint64_t* q_free = bars + 5;     // [2] S^T and dK, the readers of the Q stage, have completed
   uint64_t* do_free = bars + 7;    // [2] dP^T and dV, the readers of the dO stage, have completed
   uint64_t* s_full = bars + 9;
   uint64_t* p_full = bars + 10;
@@ -180,20 +193,20 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
     for (int st = 0; st < 2; ++st) {
       mbar_init(&q_full[st], 1);
       mbar_init(&do_full[st], 1);
-      mbar_init(&q_free[st], 5);  // the dK commit and the four compute warps
+      mbar_init(&q_free[st], 1);
       mbar_init(&do_free[st], 1);
       mbar_init(&q_fixed[st], 1);
       mbar_init(&do_fixed[st], 1);
     }
     mbar_init(s_full, 1);
-    mbar_init(p_full, kBK);
+    mbar_init(p_full, kBWCompute);
     mbar_init(dp_full, 1);
-    mbar_init(ds_full, kBK);
+    mbar_init(ds_full, kBWCompute);
     mbar_init(dq_full, 1);
     mbar_init(dq_free, kBK);
     mbar_init(dkv_done, 1);
-    mbar_init(stat_full, kBK);
-    mbar_init(v_ready, kBK);
+    mbar_init(stat_full, kBWCompute);
+    mbar_init(v_ready, kBWCompute);
     mbar_init(k_fixed, 1);
     mbar_fence_init();
   }
@@ -211,24 +224,26 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp < 4) {
+  if (warp < kBWDrainWarp) {
     // ------------------------------------------------------------------ compute
-    const int key_in = tid;
+    const int wg = warp >> 2;                    // query columns [32 wg, 32 wg + 32)
+    const int key_in = (warp & 3) * 32 + lane;
     const int kpos = ti.n0 + key_in;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
-    const uint32_t t_s = tmem + lane_addr + Cfg::kTmemS;
-    const uint32_t t_dp = tmem + lane_addr + Cfg::kTmemDP;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t t_s = tmem + lane_addr + Cfg::kTmemS + wg * 32;
+    const uint32_t t_dp = tmem + lane_addr + Cfg::kTmemDP + wg * 32;
     bool ok = true;
     if (n_iter > 0) {
       // V of this key row goes from global memory into TMEM as the 16-bit A operand of dP^T: column c holds the
-      // elements 2c and 2c + 1, which is the row's own memory layout. Rows past the sequence and columns past the
-      // head dim are zero.
+      // elements 2c and 2c + 1, which is the row's own memory layout; each warpgroup takes half of the row. Rows past
+      // the sequence and columns past the head dim are zero.
       const uint4* vrow = reinterpret_cast<const uint4*>(
           reinterpret_cast<const uint16_t*>(p.v_ptr) + ti.bq * p.v_batch_stride +
           static_cast<int64_t>(ti.k_row0 + kpos) * p.v_row_stride + ti.hk * p.v_head_stride);
       const int chunks = (kpos < ti.sk) ? p.head_dim / 8 : 0;
 #pragma unroll
-      for (int part = 0; part < 4; ++part) {
+      for (int half_part = 0; half_part < 2; ++half_part) {
+        const int part = wg * 2 + half_part;
         uint32_t vr[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -245,8 +260,8 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       tc_fence_before();
       mbar_arrive(v_ready);
     }
-    // LSE (log2 domain) and delta of one query block: thread t < 64 loads LSE of row t, the others delta of
-    // row t - 64; rows past the sequence give P = 0. The value for iteration it + 1 is requested while
+    // LSE (log2 domain) and delta of one query block: thread t < 64 loads LSE of row t, thread t < 128 delta
+    // of row t - 64; rows past the sequence give P = 0. The value for iteration it + 1 is requested while
     // iteration it computes.
     auto load_stat = [&](WWalk w) -> float {
       const int hq = ti.hk * p.group + w.g;
@@ -257,7 +272,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
         return v;
       }
       float v = 0.f;
-      if (q < ti.sq)
+      if (tid < 2 * kBQ && q < ti.sq)
         v = p.delta[ti.bq * p.delta_batch_stride + hq * p.delta_head_stride + ti.q_row0 + ti.b * p.delta_seq_pad + q];
       return v;
     };
@@ -268,53 +283,55 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
     float stat_next = n_iter > 0 ? load_stat(w) : 0.f;
     for (int it = 0; it < n_iter; ++it) {
       const int m0 = (ti.m_start + w.mi) * kBQ;
-      const int hq = ti.hk * p.group + w.g;
+      const int g_cur = w.g;
       w = wwalk_next(w, ti.n_m);
       float* stat = s_stat + (it & 1) * (2 * kBQ);
-      stat[tid] = stat_next;
+      if (tid < 2 * kBQ) stat[tid] = stat_next;
       if (it + 1 < n_iter) stat_next = load_stat(w);
       mbar_arrive(stat_full);
       const bool stat_ok = mbar_wait(stat_full, it & 1, ctl, kWaitBwd + 15);  // voted on with s_full below
-      if (it > 0) {
-        // The reductions of the previous iteration have read their staging area by now: its Q stage goes back
-        // to the loader.
-        if (lane == 0) {
-          tma_wait_group_read<0>();
-          mbar_arrive(&q_free[(it - 1) & 1]);
-        }
-        __syncwarp();
-      }
-      const float* lse_s = stat;
-      const float* dl_s = stat + kBQ;
+      const float4* lse4 = reinterpret_cast<const float4*>(stat + wg * 32);
+      const float4* dl4 = reinterpret_cast<const float4*>(stat + kBQ + wg * 32);
 
       // ---- phase A: P^T = exp2(S^T c - lse)
       if (!__all_sync(0xffffffffu, mbar_wait(s_full, it & 1, ctl, kWaitBwd + 11) && stat_ok)) { ok = false; break; }
       tc_fence_after();
-      uint32_t sr[kBQ];
+      uint32_t sr[32];
       tmem_ld32(t_s, sr);
-      tmem_ld32(t_s + 32, sr + 32);
       tmem_wait_ld();
-      // Columns [c_lo, c_hi) of this key row are visible.
-      int c_lo = 0, c_hi = kBQ;
-      if (p.window_right >= 0) c_lo = kpos - ti.off - p.window_right - m0;
-      if (p.window_left >= 0) c_hi = kpos - ti.off + p.window_left + 1 - m0;
-      if (kpos >= ti.sk) c_hi = -1;
-      const float slope = (p.alibi != nullptr) ? p.alibi[ti.b * p.alibi_batch_stride + hq] * kBWLog2e : 0.f;
-      float pr[kBQ];  // P times the derivative of the score transform: what goes on to dS
+      // Bit i of `keep`: column i of this warpgroup's 32 is visible to the key row.
+      const int qbase = m0 + wg * 32;
+      bool need_mask = ti.n0 + kBK > ti.sk;
+      if (p.window_right >= 0) need_mask |= ti.n0 + kBK - 1 > m0 + ti.off + p.window_right;
+      if (p.window_left >= 0) need_mask |= ti.n0 < m0 + kBQ - 1 + ti.off - p.window_left;
+      uint32_t keep = 0xffffffffu;
+      if (need_mask) {
+        int c_lo = 0, c_hi = 32;
+        if (p.window_right >= 0) c_lo = kpos - ti.off - p.window_right - qbase;
+        if (p.window_left >= 0) c_hi = kpos - ti.off + p.window_left + 1 - qbase;
+        keep = kpos < ti.sk ? bit_range(c_lo, c_hi) : 0u;
+      }
+      float pr[32];  // P times the derivative of the score transform: what goes on to dS
       if (!fancy) {
 #pragma unroll
-        for (int i = 0; i < kBQ; i += 2) {
-          float pv0 = ex2(fmaf(__uint_as_float(sr[i]), p.scale_log2, -lse_s[i]));
-          float pv1 = ex2(fmaf(__uint_as_float(sr[i + 1]), p.scale_log2, -lse_s[i + 1]));
-          if (i < c_lo || i >= c_hi) pv0 = 0.f;
-          if (i + 1 < c_lo || i + 1 >= c_hi) pv1 = 0.f;
-          pr[i] = pv0;
-          pr[i + 1] = pv1;
-          sr[i / 2] = pack2<BF16>(pv0, pv1);
+        for (int i = 0; i < 32; i += 4) {
+          const float4 l4 = lse4[i / 4];
+          pr[i] = ex2(fmaf(__uint_as_float(sr[i]), p.scale_log2, -l4.x));
+          pr[i + 1] = ex2(fmaf(__uint_as_float(sr[i + 1]), p.scale_log2, -l4.y));
+          pr[i + 2] = ex2(fmaf(__uint_as_float(sr[i + 2]), p.scale_log2, -l4.z));
+          pr[i + 3] = ex2(fmaf(__uint_as_float(sr[i + 3]), p.scale_log2, -l4.w));
         }
-      } else {
+        if (need_mask) {
 #pragma unroll
-        for (int i = 0; i < kBQ; i += 2) {
+          for (int i = 0; i < 32; ++i)
+            if (!(keep & (1u << i))) pr[i] = 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sr[i] = pack2<BF16>(pr[2 * i], pr[2 * i + 1]);
+      } else {
+        const float slope = (p.alibi != nullptr) ? p.alibi[ti.b * p.alibi_batch_stride + ti.hk * p.group + g_cur] * kBWLog2e : 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
           float pp[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
@@ -329,16 +346,17 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
             }
             if (p.alibi != nullptr)
               x += p.causal_alibi ? slope * static_cast<float>(kpos)
-                                  : -slope * fabsf(static_cast<float>(m0 + i + e + ti.off - kpos));
-            float pv = ex2(x - lse_s[i + e]);
-            if (i + e < c_lo || i + e >= c_hi) pv = 0.f;
+                                  : -slope * fabsf(static_cast<float>(qbase + i + e + ti.off - kpos));
+            float pv = ex2(x - reinterpret_cast<const float*>(lse4)[i + e]);
+            if (!(keep & (1u << (i + e)))) pv = 0.f;
             pp[e] = pv;
             pr[i + e] = pv * deriv;
           }
           sr[i / 2] = pack2<BF16>(pp[0], pp[1]);
         }
       }
-      tmem_st32(t_s, sr);
+      // Each warpgroup writes P^T into the columns that it has read itself: 16 of them, at S^T + 0 and S^T + 32.
+      tmem_st16(t_s, sr);
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(p_full);
@@ -347,102 +365,101 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       if (!warp_wait(dp_full, it & 1, ctl, kWaitBwd + 12)) { ok = false; break; }
       tc_fence_after();
       tmem_ld32(t_dp, sr);
-      tmem_ld32(t_dp + 32, sr + 32);
       tmem_wait_ld();
       tc_fence_before();
-      // The dS^T buffer is free: dq_full (or q_free) of the previous iteration has been seen in phase C.
+      // The dS^T buffer is free: dp_full was committed behind the products that read the previous one.
       uint8_t* ds_row = s_ds + key_in * 128;
 #pragma unroll
-      for (int c = 0; c < kBQ / 8; ++c) {
+      for (int c = 0; c < 4; ++c) {
+        const float4 d0 = dl4[2 * c], d1 = dl4[2 * c + 1];
         const int i = c * 8;
         uint4 wv;
-        wv.x = pack2<BF16>(pr[i] * (__uint_as_float(sr[i]) - dl_s[i]), pr[i + 1] * (__uint_as_float(sr[i + 1]) - dl_s[i + 1]));
-        wv.y = pack2<BF16>(pr[i + 2] * (__uint_as_float(sr[i + 2]) - dl_s[i + 2]), pr[i + 3] * (__uint_as_float(sr[i + 3]) - dl_s[i + 3]));
-        wv.z = pack2<BF16>(pr[i + 4] * (__uint_as_float(sr[i + 4]) - dl_s[i + 4]), pr[i + 5] * (__uint_as_float(sr[i + 5]) - dl_s[i + 5]));
-        wv.w = pack2<BF16>(pr[i + 6] * (__uint_as_float(sr[i + 6]) - dl_s[i + 6]), pr[i + 7] * (__uint_as_float(sr[i + 7]) - dl_s[i + 7]));
-        *reinterpret_cast<uint4*>(ds_row + ((c ^ (key_in & 7)) << 4)) = wv;
+        wv.x = pack2<BF16>(pr[i] * (__uint_as_float(sr[i]) - d0.x), pr[i + 1] * (__uint_as_float(sr[i + 1]) - d0.y));
+        wv.y = pack2<BF16>(pr[i + 2] * (__uint_as_float(sr[i + 2]) - d0.z), pr[i + 3] * (__uint_as_float(sr[i + 3]) - d0.w));
+        wv.z = pack2<BF16>(pr[i + 4] * (__uint_as_float(sr[i + 4]) - d1.x), pr[i + 5] * (__uint_as_float(sr[i + 5]) - d1.y));
+        wv.w = pack2<BF16>(pr[i + 6] * (__uint_as_float(sr[i + 6]) - d1.z), pr[i + 7] * (__uint_as_float(sr[i + 7]) - d1.w));
+        *reinterpret_cast<uint4*>(ds_row + (((wg * 4 + c) ^ (key_in & 7)) << 4)) = wv;
       }
       fence_proxy_async_smem();
       mbar_arrive(ds_full);
-
-      // ---- phase C: this half of dQ^T [128 d x 64 q] (in the dP^T columns) into the fp32 accumulator: every
-      // thread holds one d column; a warp writes its [64 q x 32 d] block, rows of 128 bytes with the 16-byte
-      // chunks swizzled as the tensor map expects, into the Q stage that dK has finished with, and one bulk
-      // reduce-add takes it from there. dq_full also tells that dK has read dS^T.
-      if (!warp_wait(dq_full, it & 1, ctl, kWaitBwd + 14)) { ok = false; break; }
-      if (want_dq) {
+    }
+    // ---- epilogue, 32 columns at a time, straight to global memory: warpgroup 0 writes this half of dK (scaled),
+    // warpgroup 1 this half of dV. A dQ-only call still sees the last commits land before the CTA ends.
+    if (ok && n_iter > 0) ok = warp_wait(dkv_done, 0, ctl, kWaitBwd + 13);
+    if (ok && (p.which & 2) != 0) {
+      tc_fence_after();
+      const float mul = (wg == 0) ? p.scale : 1.f;
+      uint16_t* grow = reinterpret_cast<uint16_t*>(wg == 0 ? p.dk_ptr : p.dv_ptr) + ti.bq * p.dkv_batch_stride +
+                       static_cast<int64_t>(ti.k_row0 + kpos) * p.dkv_row_stride + ti.hk * p.dkv_head_stride + ti.half * 128;
+      const uint32_t t_acc = tmem + lane_addr + (wg == 0 ? Cfg::kTmemDK : Cfg::kTmemDV);
+      for (int c = 0; c < ncol / 32; ++c) {
+        uint32_t acc[32];
+        if (n_iter > 0) {
+          tmem_ld32(t_acc + c * 32, acc);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[i] = 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint4 wv;
+          wv.x = pack2<BF16>(__uint_as_float(acc[8 * q]) * mul, __uint_as_float(acc[8 * q + 1]) * mul);
+          wv.y = pack2<BF16>(__uint_as_float(acc[8 * q + 2]) * mul, __uint_as_float(acc[8 * q + 3]) * mul);
+          wv.z = pack2<BF16>(__uint_as_float(acc[8 * q + 4]) * mul, __uint_as_float(acc[8 * q + 5]) * mul);
+          wv.w = pack2<BF16>(__uint_as_float(acc[8 * q + 6]) * mul, __uint_as_float(acc[8 * q + 7]) * mul);
+          const int col = c * 32 + q * 8;
+          if (kpos < ti.sk && ti.half * 128 + col < p.head_dim) *reinterpret_cast<uint4*>(grow + col) = wv;
+        }
+      }
+      tc_fence_before();
+    }
+    __syncwarp();
+  } else if (warp < kBWDrainWarp + 4) {
+    // ------------------------------------------------------------------ dQ drain: this half of dQ^T [128 d x 64 q] (in
+    // the dP^T columns) into the fp32 accumulator. Every thread holds one d column; a warp writes its [64 q x 32 d]
+    // block in two pieces of 32 rows, 128 bytes a row with the 16-byte chunks swizzled as the tensor map expects, into
+    // its own staging buffer, and bulk reduce-adds take them from there.
+    if (want_dq) {
+      const int dw = warp - kBWDrainWarp;
+      const uint32_t t_dq = tmem + (static_cast<uint32_t>(dw * 32) << 16) + Cfg::kTmemDP;
+      const int d0 = ti.half * 128 + dw * 32;
+      uint8_t* buf = smem + Cfg::kDQOff + dw * Cfg::kDQPiece;
+      const uint32_t col_byte = static_cast<uint32_t>(lane & 3) * 4;
+      const uint32_t chunk = static_cast<uint32_t>(lane >> 2);
+      WWalk w{0, 0};
+      for (int it = 0; it < n_iter; ++it, w = wwalk_next(w, ti.n_m)) {
+        const int m0 = (ti.m_start + w.mi) * kBQ;
+        if (!warp_wait(dq_full, it & 1, ctl, kWaitBwd + 14)) break;
         tc_fence_after();
-        tmem_ld32(t_dp, sr);
-        tmem_ld32(t_dp + 32, sr + 32);
+        uint32_t acc[kBQ];
+        tmem_ld32(t_dq, acc);
+        tmem_ld32(t_dq + 32, acc + 32);
         tmem_wait_ld();
         tc_fence_before();
         mbar_arrive(dq_free);
-        // Rows past the sequence (the 64-row box reaches the next sequence of a packed batch) add exact zeros.
-        const int rows = min(kBQ, ti.sq - m0);
-        uint8_t* buf = s_q + (it & 1) * Cfg::kStageBytes + warp * (kBQ * 128);
-        const uint32_t col_byte = static_cast<uint32_t>(lane & 3) * 4;
-        const uint32_t chunk = static_cast<uint32_t>(lane >> 2);
+        if (d0 >= p.head_dim) continue;
+        // Packed batches: the box may reach into the next sequence, whose rows get exact zeros.
+        const int rows = PACKED ? ti.sq - m0 : kBQ;
 #pragma unroll
-        for (int i = 0; i < kBQ; ++i)
-          *reinterpret_cast<uint32_t*>(buf + i * 128 + ((chunk ^ (i & 7)) << 4) + col_byte) = (i < rows) ? sr[i] : 0u;
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          const int d0 = ti.half * 128 + warp * 32;
-          if (d0 < p.head_dim) tma_reduce_add_4d(&p.tm_dqa, buf, d0, hq, ti.q_row0 + m0, ti.bq);
-          tma_commit_group();
-        }
-        __syncwarp();
-      }
-    }
-    if (n_iter > 0) {
-      // The last iteration's reductions: see them read their staging area before the CTA may end.
-      if (lane == 0) {
-        tma_wait_group_read<0>();
-        mbar_arrive(&q_free[(n_iter - 1) & 1]);
-      }
-      __syncwarp();
-    }
-    // ---- epilogue: this half of dK (scaled) and of dV, 32 columns at a time, straight to global memory
-    if (ok && (p.which & 2) != 0) {
-      bool done = true;
-      if (n_iter > 0) done = warp_wait(dkv_done, 0, ctl, kWaitBwd + 13);
-      if (done) {
-        tc_fence_after();
-        const int64_t row_off = ti.bq * p.dkv_batch_stride + static_cast<int64_t>(ti.k_row0 + kpos) * p.dkv_row_stride +
-                                ti.hk * p.dkv_head_stride + ti.half * 128;
-        for (int o = 0; o < 2; ++o) {
-          const float mul = (o == 0) ? p.scale : 1.f;
-          uint16_t* grow = reinterpret_cast<uint16_t*>(o == 0 ? p.dk_ptr : p.dv_ptr) + row_off;
-          const uint32_t t_acc = tmem + lane_addr + (o == 0 ? Cfg::kTmemDK : Cfg::kTmemDV);
-          for (int c = 0; c < ncol / 32; ++c) {
-            uint32_t acc[32];
-            if (n_iter > 0) {
-              tmem_ld32(t_acc + c * 32, acc);
-              tmem_wait_ld();
-            } else {
+        for (int piece = 0; piece < 2; ++piece) {
+          if (lane == 0) tma_wait_group_read<0>();  // the previous piece has been read out of the buffer
+          __syncwarp();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) acc[i] = 0u;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 wv;
-              wv.x = pack2<BF16>(__uint_as_float(acc[8 * q]) * mul, __uint_as_float(acc[8 * q + 1]) * mul);
-              wv.y = pack2<BF16>(__uint_as_float(acc[8 * q + 2]) * mul, __uint_as_float(acc[8 * q + 3]) * mul);
-              wv.z = pack2<BF16>(__uint_as_float(acc[8 * q + 4]) * mul, __uint_as_float(acc[8 * q + 5]) * mul);
-              wv.w = pack2<BF16>(__uint_as_float(acc[8 * q + 6]) * mul, __uint_as_float(acc[8 * q + 7]) * mul);
-              const int col = c * 32 + q * 8;
-              if (kpos < ti.sk && ti.half * 128 + col < p.head_dim) *reinterpret_cast<uint4*>(grow + col) = wv;
-            }
+          for (int i = 0; i < 32; ++i)
+            *reinterpret_cast<uint32_t*>(buf + i * 128 + ((chunk ^ (i & 7)) << 4) + col_byte) =
+                (piece * 32 + i < rows) ? acc[piece * 32 + i] : 0u;
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_4d(&p.tm_dqa, buf, d0, ti.hk * p.group + w.g, ti.q_row0 + m0 + piece * 32, ti.bq);
+            tma_commit_group();
           }
         }
-        tc_fence_before();
       }
-    } else if (ok && n_iter > 0) {
-      // dQ-only call: still see the last commits land before the CTA ends.
-      warp_wait(dkv_done, 0, ctl, kWaitBwd + 13);
+      if (lane == 0) tma_wait_group_read<0>();
+      __syncwarp();
     }
-    __syncwarp();
   } else if (warp == kBWLoadWarp) {
     if (n_iter > 0 && elect_one()) {
       // ---------------------------------------------------------------- loader
@@ -455,17 +472,19 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
         const int m0 = (ti.m_start + w.mi) * kBQ;
         const int st = it & 1;
         const uint32_t ph = (it >> 1) & 1;
-        // A stage is free once the MMAs of its previous use that read it have completed.
-        ok = mbar_wait(&q_free[st], ph ^ 1, ctl, kWaitBwd + 1);
-        if (!ok) break;
-        mbar_expect_tx(&q_full[st], atoms * Cfg::kAtomQ);
-        for (int a = 0; a < atoms; ++a)
-          tma_load_4d(s_q + st * Cfg::kStageBytes + a * Cfg::kAtomQ, &p.tm_q, &q_full[st], a * 64, hq, ti.q_row0 + m0, ti.bq);
-        ok = mbar_wait(&do_free[st], ph ^ 1, ctl, kWaitBwd + 2);
-        if (!ok) break;
-        mbar_expect_tx(&do_full[st], atoms * Cfg::kAtomQ);
-        for (int a = 0; a < atoms; ++a)
-          tma_load_4d(s_do + st * Cfg::kStageBytes + a * Cfg::kAtomQ, &p.tm_do, &do_full[st], a * 64, hq, ti.q_row0 + m0, ti.bq);
+        // A stage is free once the MMAs of its previous use that read it have completed; that of dO is first. At
+        // the start S^T waits for Q.
+#pragma unroll
+        for (int x = 0; x < 2 && ok; ++x) {
+          const bool load_q = (x == 0) == (it == 0);
+          ok = load_q ? mbar_wait(&q_free[st], ph ^ 1, ctl, kWaitBwd + 1) : mbar_wait(&do_free[st], ph ^ 1, ctl, kWaitBwd + 2);
+          if (!ok) break;
+          uint64_t* full = load_q ? &q_full[st] : &do_full[st];
+          uint8_t* dst = (load_q ? s_q : s_do) + st * Cfg::kStageBytes;
+          mbar_expect_tx(full, atoms * Cfg::kAtomQ);
+          for (int a = 0; a < atoms; ++a)
+            tma_load_4d(dst + a * Cfg::kAtomQ, load_q ? &p.tm_q : &p.tm_do, full, a * 64, hq, ti.q_row0 + m0, ti.bq);
+        }
       }
       // The loader leaves last: the commits on the free barriers of each stage's last use have landed.
       for (int st = 0; st < 2 && ok; ++st) {
@@ -597,23 +616,39 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       const uint32_t nph = ((it + 1) >> 1) & 1;  // phase of the stage barriers of iteration it + 1
       const bool has_next = it + 1 < n_iter;
       const uint32_t acc = it > 0 ? 1u : 0u;
-      // dV_c += P^T dO_c (P^T: 32 packed columns at S^T; 16 query rows of dO are 2048 bytes)
+      // dV_c += P^T dO_c (P^T: two runs of 16 packed columns at S^T + 0 and S^T + 32; 16 query rows of dO are 2048 bytes)
       ok = mbar_wait(p_full, it & 1, ctl, kWaitBwd + 6);
       if (!ok) break;
       tc_fence_after();
       {
         const uint64_t b = do_mn + st * kStage16;
         static_for<kBQ / 16>([&](auto ks) {
-          mma_ts_o<ks.value * 8, ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv,
-                                                         ks.value > 0 ? 1u : acc);
+          mma_ts_o<(ks.value / 2) * 32 + (ks.value % 2) * 8, ks.value * (2048 >> 4)>(
+              tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv, ks.value > 0 ? 1u : acc);
         });
       }
       mma_commit(&do_free[st]);
-      // dK_c += dS^T Q_c, then dQ_c^T = K_c^T dS^T over the 128 keys into the dP^T columns (the compute warps
-      // have read dP^T). They go before the next S^T: the compute warps wait for dQ^T next.
+      // S^T of the next iteration right behind dV, the last reader of P^T: its scores are there when the compute
+      // warps come out of phase B.
+      if (has_next) {
+        ok = q_ready(wn.mi, st ^ 1, nph, kWaitBwd + 8);
+        if (!ok) break;
+        tc_fence_after();
+        issue_st(q_kmaj + (st ^ 1) * kStage16);
+        mma_commit(s_full);
+      }
+      // dQ_c^T = K_c^T dS^T over the 128 keys into the dP^T columns (the compute warps have read dP^T), then
+      // dK_c += dS^T Q_c, under which the drain warps take dQ^T out of TMEM.
       ok = mbar_wait(ds_full, it & 1, ctl, kWaitBwd + 7);
       if (!ok) break;
       tc_fence_after();
+      if (want_dq) {
+        static_for<kBK / 16>([&](auto ks) {
+          mma_ss_o<ks.value * (2048 >> 4), ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDP, k_mn, ds_mn, idesc_dq,
+                                                                    ks.value > 0 ? 1u : 0u);
+        });
+        mma_commit(dq_full);
+      }
       {
         const uint64_t b = q_mn + st * kStage16;
         static_for<kBQ / 16>([&](auto ks) {
@@ -621,21 +656,8 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
         });
       }
       mma_commit(&q_free[st]);
-      if (want_dq) {
-        static_for<kBK / 16>([&](auto ks) {
-          mma_ss_o<ks.value * (2048 >> 4), ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDP, k_mn, ds_mn, idesc_dq,
-                                                                    ks.value > 0 ? 1u : 0u);
-        });
-      }
-      mma_commit(dq_full);
+      // dP^T of the next iteration, once dQ^T has left the columns.
       if (has_next) {
-        // S^T of the next iteration (dV, the last reader of P^T, was issued above), then its dP^T once dQ^T has
-        // left the columns.
-        ok = q_ready(wn.mi, st ^ 1, nph, kWaitBwd + 8);
-        if (!ok) break;
-        tc_fence_after();
-        issue_st(q_kmaj + (st ^ 1) * kStage16);
-        mma_commit(s_full);
         ok = do_ready(wn.mi, st ^ 1, nph, kWaitBwd + 9);
         if (ok && want_dq) ok = mbar_wait(dq_free, it & 1, ctl, kWaitBwd + 10);
         if (!ok) break;

@@ -696,8 +696,8 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
     p.tm_dv = p.tm_v;
   }
   if (want_dq) {
-    // one reduce-add box: 32 columns of 32 query rows (64 on the kernel for head dims above 128)
-    if ((rc = make_map(&p.tm_dqa, a->dq_accum, 2, 4, d, a->heads, rows_q, nbatch, d, hd, rows_q * hd, 32, wide ? 64 : 32,
+    // one reduce-add box: 32 columns of 32 query rows
+    if ((rc = make_map(&p.tm_dqa, a->dq_accum, 2, 4, d, a->heads, rows_q, nbatch, d, hd, rows_q * hd, 32, 32,
                        "dq_accum")) != FA2_OK) return rc;
   } else {
     p.tm_dqa = p.tm_q;

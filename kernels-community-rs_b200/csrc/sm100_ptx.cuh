@@ -310,6 +310,15 @@ __device__ __forceinline__ void reg_dealloc() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+// Bits [lo, hi) of a 32-bit word; either end may lie outside [0, 32). PTX shifts by 32 or more give zero.
+// Masks go through such words: a test of a constant bit per score is cheaper than two comparisons.
+__device__ __forceinline__ uint32_t bit_range(int lo, int hi) {
+  uint32_t from_lo, from_hi;
+  asm("shl.b32 %0, %1, %2;" : "=r"(from_lo) : "r"(0xffffffffu), "r"(max(lo, 0)));
+  asm("shl.b32 %0, %1, %2;" : "=r"(from_hi) : "r"(0xffffffffu), "r"(max(hi, 0)));
+  return from_lo & ~from_hi;
+}
+
 // ---------------------------------------------------------------- math
 __device__ __forceinline__ float ex2(float x) {
   float y;
