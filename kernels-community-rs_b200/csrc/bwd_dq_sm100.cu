@@ -174,9 +174,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_kernel(const __grid_consta
         if (p.window_left >= 0) lo = row + off - p.window_left;
         hi -= col0;
         lo -= col0;
-#pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (i < lo || i >= hi) pr[i] = 0.f;
+        fill_outside<64>(pr, lo, hi, 0.f);
       }
       if (!warp_wait(dp_full, it & 1, ctl, kWaitBwdDq + 2)) { ok = false; break; }
       tc_fence_after();

@@ -570,9 +570,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           pr[i + 3] = ex2(fmaf(__uint_as_float(sr[i + 3]), mul1, bias_minus(l4.w)));
         }
         if (need_mask) {
-#pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (i < c_lo || i >= c_hi) pr[i] = 0.f;
+          fill_outside<64>(pr, c_lo, c_hi, 0.f);
         }
 #pragma unroll
         for (int i = 0; i < 32; ++i) sr[i] = pack2<BF16>(pr[2 * i], pr[2 * i + 1]);

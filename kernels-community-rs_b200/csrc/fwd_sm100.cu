@@ -364,9 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
             if (p.window_left >= 0) lo = row + ti.off - p.window_left;
             hi -= col0;
             lo -= col0;
-#pragma unroll
-            for (int i = 0; i < kBlockN; ++i)
-              if (i < lo || i >= hi) sr[i] = __float_as_uint(-INFINITY);
+            fill_outside<kBlockN>(sr, lo, hi, 0xff800000u);  // -inf
           }
           float mx0 = max3(__uint_as_float(sr[0]), __uint_as_float(sr[1]), __uint_as_float(sr[2]));
           float mx1 = max3(__uint_as_float(sr[3]), __uint_as_float(sr[4]), __uint_as_float(sr[5]));
@@ -413,9 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
             if (p.window_left >= 0) lo = row + ti.off - p.window_left;
             hi -= col0;
             lo -= col0;
-  #pragma unroll
-            for (int i = 0; i < kBlockN; ++i)
-              if (i < lo || i >= hi) sr[i] = __float_as_uint(-INFINITY);
+            fill_outside<kBlockN>(sr, lo, hi, 0xff800000u);
           }
           float mx0 = __uint_as_float(sr[0]), mx1 = __uint_as_float(sr[1]);
           float mx2 = __uint_as_float(sr[2]), mx3 = __uint_as_float(sr[3]);

@@ -255,11 +255,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
         if (p.window_left >= 0) lo = row + ti.off - p.window_left;
         hi -= col0;
         lo -= col0;
-        if (lo > 0 || hi < kWN) {
-#pragma unroll
-          for (int c = 0; c < kWN; ++c)
-            if (c < lo || c >= hi) sr[c] = __float_as_uint(-INFINITY);
-        }
+        if (lo > 0 || hi < kWN) fill_outside<kWN>(sr, lo, hi, 0xff800000u);  // -inf
       }
       float mx0 = __uint_as_float(sr[0]), mx1 = __uint_as_float(sr[1]);
       float mx2 = __uint_as_float(sr[2]), mx3 = __uint_as_float(sr[3]);

@@ -311,12 +311,24 @@ __device__ __forceinline__ void reg_dealloc() {
 }
 
 // Bits [lo, hi) of a 32-bit word; either end may lie outside [0, 32). PTX shifts by 32 or more give zero.
-// Masks go through such words: a test of a constant bit per score is cheaper than two comparisons.
 __device__ __forceinline__ uint32_t bit_range(int lo, int hi) {
   uint32_t from_lo, from_hi;
   asm("shl.b32 %0, %1, %2;" : "=r"(from_lo) : "r"(0xffffffffu), "r"(max(lo, 0)));
   asm("shl.b32 %0, %1, %2;" : "=r"(from_hi) : "r"(0xffffffffu), "r"(max(hi, 0)));
   return from_lo & ~from_hi;
+}
+// v[i] = fill for every i outside [lo, hi). The tests go through words of 32 bits: one constant bit per element in
+// place of two comparisons.
+template <int N, typename T>
+__device__ __forceinline__ void fill_outside(T* v, int lo, int hi, T fill) {
+  static_assert(N % 32 == 0, "whole words");
+#pragma unroll
+  for (int c = 0; c < N; c += 32) {
+    const uint32_t keep = bit_range(lo - c, hi - c);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (!(keep & (1u << i))) v[c + i] = fill;
+  }
 }
 
 // ---------------------------------------------------------------- math
