@@ -24,6 +24,8 @@ enum WaitSite : int {
   kWaitBwdDq = 90,
 };
 
+constexpr int kMaxStreamBlocks = 64;   // 256-row query blocks of a head in a forward that shares tiles between CTAs
+
 struct FwdParams {
   CUtensorMap tm_q, tm_k, tm_v, tm_o;  // 4-D maps: (D, heads, rows, batch), box (64, 1, 128, 1)
   void* o_ptr;                         // for the predicated (non-TMA) output path
@@ -45,7 +47,15 @@ struct FwdParams {
   float softcap;                       // 0 = off
   int* status;                         // device status word (0 = ok)
   int head_dim;                         // real head dim (<= the kernel's D; columns beyond it are padding)
+  // Tiles shared between CTAs (null = none): the (work tile, key block) pairs of all heads form one list, which is cut
+  // into equal shares. A share's part of a tile that it does not cover alone goes to slot 2 * CTA (+ 1 if the part has
+  // the tile's first key block): O of [256 rows][D] fp32, unnormalised, then the rows' maxima and sums.
+  float* parts;
+  int stream_grid;                      // CTAs
+  int units_per_head;                   // = block_start[num_mblk]
+  uint16_t block_start[kMaxStreamBlocks + 1];  // units of a head before query block m
 };
+__host__ __device__ constexpr int64_t stream_slot_floats(int d) { return 256 * (static_cast<int64_t>(d) + 2); }
 
 // Forward for few query rows (fwd_decode_sm100.cu). A unit is one (batch, kv head): its rows are the query rows of all
 // the group's heads, row r = query r / group, head r % group.

@@ -97,7 +97,13 @@ struct Tile {
   int jlo, jhi;
   int flip;            // 1: stage 0 takes the upper 128 rows of the block and stage 1 the lower ones
   bool valid;
+  int slot;            // shared tiles: where this part goes, or -1 if it is the whole tile
 };
+
+// Share of CTA c in the list of all (work tile, key block) pairs of a launch with shared tiles.
+__device__ __forceinline__ int stream_bound(const FwdParams& p, int c) {
+  return static_cast<int>(static_cast<int64_t>(p.units_per_head) * p.batch * p.heads * c / p.stream_grid);
+}
 
 // Divisors of the work-list index as fixed-point reciprocals floor(2^40 / d) + 1: an integer division is a long
 // dependent chain, every role walks the list, and the softmax warps do so between two tiles. The quotient is one
@@ -118,6 +124,75 @@ __device__ __forceinline__ int div_small(int n, int d, unsigned long long m) {
   int q = static_cast<int>((static_cast<unsigned long long>(static_cast<unsigned>(n)) * m) >> 40);
   if (q * d > n) --q;  // the reciprocal is rounded up: the estimate can be one too large for d >= 2^16
   return q;
+}
+
+// Key-tile ranges of the two stages of a block and their union.
+__device__ __forceinline__ void key_ranges(const FwdParams& p, Tile& ti) {
+  ti.jlo = 0x7fffffff;
+  ti.jhi = 0;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const int r_lo = ti.m0 + (s ^ ti.flip) * kBlockM;
+    int nb = 0, ne = 0;
+    if (r_lo < ti.sq) {
+      const int r_hi = min(r_lo + kBlockM - 1, ti.sq - 1);
+      int hi_col = ti.sk;
+      if (p.window_right >= 0) hi_col = min(ti.sk, r_hi + ti.off + p.window_right + 1);
+      int lo_col = 0;
+      if (p.window_left >= 0) lo_col = max(0, r_lo + ti.off - p.window_left);
+      if (hi_col > lo_col) {
+        nb = lo_col / kBlockN;
+        ne = (hi_col + kBlockN - 1) / kBlockN;
+      }
+    }
+    ti.nb[s] = nb;
+    ti.ne[s] = ne;
+    if (ne > nb) {
+      ti.jlo = min(ti.jlo, nb);
+      ti.jhi = max(ti.jhi, ne);
+    }
+  }
+  if (ti.jhi == 0) ti.jlo = 0;
+}
+
+// The part of a work tile that starts at position x of the list of a launch with shared tiles; the share ends at
+// `end`. Query blocks of a head are neighbours in the list, and so are the heads of a GQA group: CTAs that run side by
+// side read the same K and V.
+__device__ __forceinline__ Tile get_segment(const FwdParams& p, int x, int end) {
+  Tile ti;
+  const int bh = x / p.units_per_head;
+  const int r = x - bh * p.units_per_head;
+  int lo = 0, hi = p.num_mblk;  // block_start[lo] <= r < block_start[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (p.block_start[mid] <= r) lo = mid;
+    else hi = mid;
+  }
+  ti.b = bh / p.heads;
+  ti.h = bh - ti.b * p.heads;
+  ti.hk = ti.h / p.group;
+  ti.m0 = lo * (2 * kBlockM);
+  ti.q_row0 = 0;
+  ti.k_row0 = 0;
+  ti.sq = p.seqlen_q;
+  ti.sk = p.seqlen_k;
+  ti.bq = ti.b;
+  ti.off = ti.sk - ti.sq;
+  ti.flip = (lo ^ bh) & 1;
+  ti.valid = true;
+  key_ranges(p, ti);
+  const int first = ti.jlo + r - p.block_start[lo];
+  const int last = min(ti.jhi, first + end - x);
+  ti.slot = -1;
+  if (first > ti.jlo || last < ti.jhi) ti.slot = 2 * static_cast<int>(blockIdx.x) + (first == ti.jlo ? 1 : 0);
+  ti.jlo = first;
+  ti.jhi = last;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    ti.nb[s] = max(ti.nb[s], first);
+    ti.ne[s] = max(ti.nb[s], min(ti.ne[s], last));
+  }
+  return ti;
 }
 
 __device__ __forceinline__ Tile get_tile(const FwdParams& p, const volatile ListDiv* ldp, int t) {
@@ -160,31 +235,7 @@ __device__ __forceinline__ Tile get_tile(const FwdParams& p, const volatile List
   }
   ti.off = ti.sk - ti.sq;
   ti.valid = ti.m0 < ti.sq;
-  ti.jlo = 0x7fffffff;
-  ti.jhi = 0;
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const int r_lo = ti.m0 + (s ^ ti.flip) * kBlockM;
-    int nb = 0, ne = 0;
-    if (r_lo < ti.sq) {
-      const int r_hi = min(r_lo + kBlockM - 1, ti.sq - 1);
-      int hi_col = ti.sk;
-      if (p.window_right >= 0) hi_col = min(ti.sk, r_hi + ti.off + p.window_right + 1);
-      int lo_col = 0;
-      if (p.window_left >= 0) lo_col = max(0, r_lo + ti.off - p.window_left);
-      if (hi_col > lo_col) {
-        nb = lo_col / kBlockN;
-        ne = (hi_col + kBlockN - 1) / kBlockN;
-      }
-    }
-    ti.nb[s] = nb;
-    ti.ne[s] = ne;
-    if (ne > nb) {
-      ti.jlo = min(ti.jlo, nb);
-      ti.jhi = max(ti.jhi, ne);
-    }
-  }
-  if (ti.jhi == 0) ti.jlo = 0;
+  key_ranges(p, ti);
   return ti;
 }
 
@@ -206,7 +257,11 @@ __device__ __forceinline__ float tanh_approx(float x) {
 // MODE: what is done to the scores; PACKED: cu_seqlens batches. Both are compile-time so that the
 // plain dense kernel carries none of their code and stays within reach of the SM's instruction cache: without the
 // score transforms the kernel is a third smaller and ran 3-4 % faster.
-template <int D, bool BF16, int MODE, bool PACKED>
+// SHARED: tiles shared between CTAs. With few work tiles the time is that of the longest tile on one SM while others have
+// nothing to do; equal shares of the key blocks cost a part's way through memory and the merge. Causal, bf16: H2 Sq 128
+// Sk 4096 D128 47.4 -> 20.7 us, H8 Sq 500 Sk 4096 65.9 -> 31.2, H32/8 Sq 300 Sk 9001 134 -> 82, H8/2 Sq 2048 Sk 16384
+// 234 -> 127, H32 Sq 1500 Sk 16384 (192 tiles: a second round for 44 of them) 454 -> 392.
+template <int D, bool BF16, int MODE, bool PACKED, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
   using Cfg = FwdCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -239,6 +294,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   const int lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
   volatile ListDiv* ld = reinterpret_cast<volatile ListDiv*>(smem + Cfg::kMiscOff + 16);
+  // Every role walks this CTA's positions of the work list.
+  const int t_first = SHARED ? stream_bound(p, blockIdx.x) : static_cast<int>(blockIdx.x);
+  const int t_end = SHARED ? stream_bound(p, blockIdx.x + 1) : p.num_tiles + static_cast<int>(blockIdx.x);
+  auto tile_at = [&](int t) { return SHARED ? get_segment(p, t, t_end) : get_tile(p, ld, t); };
+  auto step_of = [&](const Tile& ti) { return SHARED ? max(1, ti.jhi - ti.jlo) : static_cast<int>(gridDim.x); };
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -275,6 +335,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (SHARED) asm volatile("griddepcontrol.launch_dependents;");  // the merge waits for this grid before it reads
 
   if (warp < 8) {
     // ------------------------------------------------------------------ softmax + epilogue of stage s
@@ -298,8 +359,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
     const float mul = MODE == kScoreSoftcap ? p.softcap * 1.4426950408889634f : MODE == kScoreAlibi ? 1.f : p.scale_log2;
     const float inv_cap = MODE == kScoreSoftcap ? p.scale / p.softcap : 0.f;
     uint32_t n_sfull = 0, n_pv = 0, n_store = 0, n_first = 0;
-    for (int t = blockIdx.x; t - static_cast<int>(blockIdx.x) < p.num_tiles; t += gridDim.x) {
-      const Tile ti = get_tile(p, ld, t);
+    for (int t = t_first, step; t < t_end; t += step) {
+      const Tile ti = tile_at(t);
+      step = step_of(ti);
       if (!ti.valid) continue;
       const int r_lo = ti.m0 + (s ^ ti.flip) * kBlockM;
       const int row = r_lo + row_in;
@@ -535,6 +597,33 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
       uint16_t* orow = reinterpret_cast<uint16_t*>(p.o_ptr) + ti.bq * p.o_batch_stride +
                        static_cast<int64_t>(ti.q_row0 + row) * p.o_row_stride + ti.h * p.o_head_stride;
       const bool tma_store = !PACKED || (r_lo + kBlockM <= ti.sq);
+      if (SHARED && ti.slot >= 0) {
+        // Part of a shared tile: O as it is, fp32, 32 bytes (a whole sector) per store, and the row's maximum and sum.
+        float* part = p.parts + ti.slot * stream_slot_floats(D);
+        const int prow = (s ^ ti.flip) * kBlockM + row_in;
+        if (ne_s > nb_s) {
+          if (!warp_wait(&pv_done[s], (n_pv - 1) & 1, ctl, kWaitEpiPvDone)) break;
+          tc_fence_after();
+          uint32_t orr[D];
+#pragma unroll
+          for (int c = 0; c < D / 32; ++c) tmem_ld32(t_o + c * 32, orr + c * 32);
+          tmem_wait_ld();
+          tc_fence_before();
+          if (row < ti.sq) {
+            float* dst = part + prow * D;
+#pragma unroll
+            for (int c = 0; c < D / 8; ++c)
+              asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 8 * c), "r"(orr[8 * c]),
+                           "r"(orr[8 * c + 1]), "r"(orr[8 * c + 2]), "r"(orr[8 * c + 3]), "r"(orr[8 * c + 4]),
+                           "r"(orr[8 * c + 5]), "r"(orr[8 * c + 6]), "r"(orr[8 * c + 7])
+                           : "memory");
+          }
+        }
+        mbar_arrive(&o_free[s]);
+        *reinterpret_cast<float2*>(part + 256 * D + 2 * prow) = make_float2(m, l);
+        __syncwarp();
+        continue;
+      }
       if (ne_s > nb_s) {
         const float inv_l = (l > 0.f) ? 1.f / l : 0.f;  // before the wait: the reciprocal queues behind the other stage's exp2 stream
         if (!warp_wait(&pv_done[s], (n_pv - 1) & 1, ctl, kWaitEpiPvDone)) break;
@@ -623,8 +712,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         }
         return true;
       };
-      for (int t = blockIdx.x; t - static_cast<int>(blockIdx.x) < p.num_tiles && ok; t += gridDim.x) {
-        const Tile ti = get_tile(p, ld, t);
+      for (int t = t_first, step; t < t_end && ok; t += step) {
+        const Tile ti = tile_at(t);
+        step = step_of(ti);
         if (!ti.valid) continue;
         auto load_q = [&](int s) -> bool {
           if (ti.ne[s] <= ti.nb[s]) return true;
@@ -669,7 +759,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
       if (PACKED) {
         uint32_t slot = 0, ring_phase = 0;
         bool ok = true;
-        auto step = [&](int first_stray) -> bool {
+        auto fix_tile = [&](int first_stray) -> bool {
           if (!__all_sync(0xffffffffu, mbar_wait(&kv_full[slot], ring_phase, ctl, kWaitMmaKVFull))) return false;
           if (first_stray < kBlockN) {
             uint8_t* tile = s_kv + slot * Cfg::kTileBytes;
@@ -689,13 +779,14 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
           }
           return true;
         };
-        for (int t = blockIdx.x; t - static_cast<int>(blockIdx.x) < p.num_tiles && ok; t += gridDim.x) {
-          const Tile ti = get_tile(p, ld, t);
+        for (int t = t_first, step; t < t_end && ok; t += step) {
+          const Tile ti = tile_at(t);
+          step = step_of(ti);
           if (!ti.valid) continue;
-          if (ti.jlo < ti.jhi) ok = step(kBlockN);
+          if (ti.jlo < ti.jhi) ok = fix_tile(kBlockN);
           for (int j = ti.jlo; j < ti.jhi && ok; ++j) {
-            if (j + 1 < ti.jhi) ok = step(kBlockN);
-            if (ok) ok = step(ragged_row<PACKED>(ti.sk, j));
+            if (j + 1 < ti.jhi) ok = fix_tile(kBlockN);
+            if (ok) ok = fix_tile(ragged_row<PACKED>(ti.sk, j));
           }
         }
       }
@@ -732,8 +823,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
           ring_phase ^= 1;
         }
       };
-      for (int t = blockIdx.x; t - static_cast<int>(blockIdx.x) < p.num_tiles && ok; t += gridDim.x) {
-        const Tile ti = get_tile(p, ld, t);
+      for (int t = t_first, step; t < t_end && ok; t += step) {
+        const Tile ti = tile_at(t);
+        step = step_of(ti);
         if (!ti.valid) continue;
         const int nb = s ? ti.nb[1] : ti.nb[0], ne = s ? ti.ne[1] : ti.ne[0];
         bool q_ready = false;
@@ -815,7 +907,91 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
 }
 
-template <int D, bool BF16, int MODE, bool PACKED>
+// The parts of shared tiles become rows of the output: D / 4 lanes per row, 4 columns a lane, kMergeSteps rows per lane
+// group. Bound by the latency of the loads (the L2 still holds most parts), so all of a thread's loads for four parts
+// are issued before the first is used: with one row per warp and the maxima in a pass of their own a call at B1 H16
+// Sq 2048 Sk 4096 D64 causal took 70.1 us, now 61.8. Launched while the forward kernel runs: what is before the wait
+// overlaps it.
+constexpr int kMergeSteps = 4;
+template <int D>
+constexpr int kMergeRows = 8 * kMergeSteps * (128 / D);  // rows of a block
+template <int D, bool BF16>
+__global__ void __launch_bounds__(256) merge_parts_kernel(const __grid_constant__ FwdParams p) {
+  constexpr int kLanes = D / 4, kGroups = 256 / kLanes;
+  const int tile = blockIdx.x / (256 / kMergeRows<D>);
+  const int bh = tile / p.num_mblk, mb = tile - bh * p.num_mblk;
+  const int64_t total = static_cast<int64_t>(p.units_per_head) * p.batch * p.heads, g = p.stream_grid;
+  // CTAs that own the tile's first and last key block
+  const int64_t u0 = static_cast<int64_t>(bh) * p.units_per_head;
+  const int c_first = static_cast<int>(((u0 + p.block_start[mb] + 1) * g + total - 1) / total - 1);
+  const int c_last = static_cast<int>(((u0 + p.block_start[mb + 1]) * g + total - 1) / total - 1);
+  const int b = bh / p.heads, h = bh - b * p.heads;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (c_first == c_last) return;  // the forward kernel has written it
+  const int col = (threadIdx.x % kLanes) * 4;
+  const int prow0 = (blockIdx.x % (256 / kMergeRows<D>)) * kMergeRows<D> + threadIdx.x / kLanes;
+  auto part_of = [&](int c) { return p.parts + (2 * c + (c == c_first ? 1 : 0)) * stream_slot_floats(D); };
+  float m[kMergeSteps], l[kMergeSteps];
+  float4 acc[kMergeSteps];
+#pragma unroll
+  for (int r = 0; r < kMergeSteps; ++r) {
+    m[r] = -INFINITY;
+    l[r] = 0.f;
+    acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  constexpr int kBatch = 4;
+  for (int c0 = c_first; c0 <= c_last; c0 += kBatch) {
+    float2 st[kMergeSteps][kBatch];
+    float4 o[kMergeSteps][kBatch];
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e) {
+      const float* part = part_of(min(c0 + e, c_last));
+#pragma unroll
+      for (int r = 0; r < kMergeSteps; ++r) {
+        const int prow = prow0 + r * kGroups;
+        st[r][e] = __ldcg(reinterpret_cast<const float2*>(part + 256 * D) + prow);
+        o[r][e] = __ldcg(reinterpret_cast<const float4*>(part + prow * D + col));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kMergeSteps; ++r) {
+      float m_new = m[r];
+#pragma unroll
+      for (int e = 0; e < kBatch; ++e)
+        if (c0 + e <= c_last) m_new = fmaxf(m_new, st[r][e].x);
+      if (m_new == -INFINITY) continue;
+      const float f = ex2(m[r] - m_new);
+      m[r] = m_new;
+      l[r] *= f;
+      acc[r] = make_float4(acc[r].x * f, acc[r].y * f, acc[r].z * f, acc[r].w * f);
+#pragma unroll
+      for (int e = 0; e < kBatch; ++e) {
+        // A part without a visible key (m = -inf) has left no O.
+        if (c0 + e > c_last || st[r][e].x == -INFINITY) continue;
+        const float w = ex2(st[r][e].x - m_new);
+        l[r] += w * st[r][e].y;
+        acc[r].x += w * o[r][e].x;
+        acc[r].y += w * o[r][e].y;
+        acc[r].z += w * o[r][e].z;
+        acc[r].w += w * o[r][e].w;
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kMergeSteps; ++r) {
+    const int row = mb * 256 + prow0 + r * kGroups;
+    if (row >= p.seqlen_q) continue;
+    const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
+    if (col < p.head_dim)
+      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.o_ptr) + b * p.o_batch_stride + row * p.o_row_stride +
+                                h * p.o_head_stride + col) =
+          make_uint2(pack2<BF16>(acc[r].x * inv, acc[r].y * inv), pack2<BF16>(acc[r].z * inv, acc[r].w * inv));
+    if (col == 0)
+      p.lse_ptr[b * p.lse_batch_stride + h * p.lse_head_stride + row] = l[r] > 0.f ? (m[r] + lg2(l[r])) * 0.6931471805599453f : INFINITY;
+  }
+}
+
+template <int D, bool BF16, int MODE, bool PACKED, bool SHARED = false>
 cudaError_t launch_one(const FwdParams& p, int num_sms, cudaStream_t stream) {
   using Cfg = FwdCfg<D>;
   static bool configured[64] = {};
@@ -823,13 +999,26 @@ cudaError_t launch_one(const FwdParams& p, int num_sms, cudaStream_t stream) {
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     cudaError_t e =
-        cudaFuncSetAttribute(fwd_kernel<D, BF16, MODE, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(fwd_kernel<D, BF16, MODE, PACKED, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const int grid = p.num_tiles < num_sms ? p.num_tiles : num_sms;
-  fwd_kernel<D, BF16, MODE, PACKED><<<grid, kThreads, Cfg::kSmemBytes, stream>>>(p);
+  const int grid = SHARED ? p.stream_grid : p.num_tiles < num_sms ? p.num_tiles : num_sms;
+  fwd_kernel<D, BF16, MODE, PACKED, SHARED><<<grid, kThreads, Cfg::kSmemBytes, stream>>>(p);
+  if (SHARED) {
+    cudaLaunchAttribute early[1] = {};
+    early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(p.num_tiles * (256 / kMergeRows<D>)));
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cfg.attrs = early;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, merge_parts_kernel<D, BF16>, p);
+    if (e != cudaSuccess) return e;
+  }
   return cudaGetLastError();
 }
 
@@ -838,6 +1027,14 @@ cudaError_t pick_features(const FwdParams& p, int mode, bool packed, int num_sms
   if (packed) {
     return mode != kScorePlain ? launch_one<D, BF16, kScoreAny, true>(p, num_sms, stream)
                                : launch_one<D, BF16, kScorePlain, true>(p, num_sms, stream);
+  }
+  if (p.parts != nullptr) {
+    switch (mode) {
+      case kScorePlain: return launch_one<D, BF16, kScorePlain, false, true>(p, num_sms, stream);
+      case kScoreSoftcap: return launch_one<D, BF16, kScoreSoftcap, false, true>(p, num_sms, stream);
+      case kScoreAlibi: return launch_one<D, BF16, kScoreAlibi, false, true>(p, num_sms, stream);
+      default: return launch_one<D, BF16, kScoreAny, false, true>(p, num_sms, stream);
+    }
   }
   switch (mode) {
     case kScorePlain: return launch_one<D, BF16, kScorePlain, false>(p, num_sms, stream);
