@@ -284,7 +284,9 @@ int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, Runtime* rt, cudaStre
 }
 
 // ---- dense forward with few work tiles (fwd_sm100.cu, SHARED): a work tile is 256 query rows of a head, one CTA at a
-// time works on it, and with fewer tiles than SMs (or little more than a whole number of rounds) SMs have nothing to do.
+// time works on it, and with fewer tiles than SMs some have nothing to do. Calls with more tiles are not shared, also
+// where a last, nearly empty round would gain (H32 Sq 1500 Sk 16384, 192 tiles: 454 -> 392 us): there the bits of a head do
+// not depend on how many other heads the call has, which a long-context run that is sharded by heads relies on.
 struct StreamPlan {
   int grid = 0;  // 0: one tile per CTA at a time
   int64_t workspace_bytes = 0;
@@ -294,10 +296,10 @@ void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
   const int64_t mblk = (static_cast<int64_t>(a->seqlen_q) + 255) / 256;
   if (a->head_dim > 128 || mblk <= 0 || mblk > fa2::kMaxStreamBlocks || a->seqlen_k <= 0) return;
   const int64_t heads = static_cast<int64_t>(a->batch) * a->heads, tiles = heads * mblk;
-  if (tiles > 3LL * sm_count) return;  // an incomplete last round weighs little
+  if (tiles > sm_count) return;
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
   const int64_t off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q;
-  int64_t total = 0, longest = 0, shortest = INT64_MAX;
+  int64_t total = 0, longest = 0;
   for (int64_t m = 0; m < mblk; ++m) {
     // Key blocks of the tile: the union over its two 128-row stages, as the kernel walks it.
     int64_t jlo = INT64_MAX, jhi = 0;
@@ -318,7 +320,6 @@ void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
     out->start[m] = static_cast<uint16_t>(total);
     total += jhi - jlo;
     longest = std::max(longest, jhi - jlo);
-    shortest = std::min(shortest, jhi - jlo);
   }
   out->start[mblk] = static_cast<uint16_t>(total);
   const int64_t units = total * heads;
@@ -329,10 +330,7 @@ void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
   const double t_blk = 3300, t_tile = 6000, t_part = 4000, t_merge = 7000;
   const int64_t grid = std::min<int64_t>(sm_count, units / 3);
   if (grid < 2) return;
-  double whole;
-  if (tiles <= sm_count) whole = longest * t_blk + t_tile;
-  else if (shortest == longest) whole = static_cast<double>((tiles + sm_count - 1) / sm_count) * (longest * t_blk + t_tile);
-  else whole = std::max(longest * t_blk + t_tile, (units * t_blk + tiles * t_tile) / sm_count + 0.5 * longest * t_blk);
+  const double whole = longest * t_blk + t_tile;
   const int64_t dim = a->head_dim > 64 ? 128 : 64;
   const int64_t bytes = 2 * grid * fa2::stream_slot_floats(static_cast<int>(dim)) * 4;
   const double shared = static_cast<double>(units) / grid * t_blk + (static_cast<double>(tiles) / grid + 1) * t_tile + t_part +

@@ -260,7 +260,7 @@ __device__ __forceinline__ float tanh_approx(float x) {
 // SHARED: tiles shared between CTAs. With few work tiles the time is that of the longest tile on one SM while others have
 // nothing to do; equal shares of the key blocks cost a part's way through memory and the merge. Causal, bf16: H2 Sq 128
 // Sk 4096 D128 47.4 -> 20.7 us, H8 Sq 500 Sk 4096 65.9 -> 31.2, H32/8 Sq 300 Sk 9001 134 -> 82, H8/2 Sq 2048 Sk 16384
-// 234 -> 127, H32 Sq 1500 Sk 16384 (192 tiles: a second round for 44 of them) 454 -> 392.
+// 234 -> 127.
 template <int D, bool BF16, int MODE, bool PACKED, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
   using Cfg = FwdCfg<D>;
