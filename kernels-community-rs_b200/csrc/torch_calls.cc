@@ -13,6 +13,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pycfunction_helpers.h>
 
 #include <cmath>
@@ -51,6 +52,9 @@ struct Options {
   double softcap = 0.0;
   Tensor alibi;  // undefined: none
 };
+
+// A tracer records the autograd function in Python; the output of a native call would be a constant to it.
+bool transformed() { return torch::jit::tracer::isTracing(); }
 
 // q, k, v and the slopes of a plain dense call.
 bool plain(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o) {
@@ -329,7 +333,7 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Options o;
   bool deterministic;
   if (n != 10 || !tensor_arg(args[0], q) || !tensor_arg(args[1], k) || !tensor_arg(args[2], v) || !options_arg(args + 3, o) ||
-      !bool_arg(args[9], deterministic) || !plain(q, k, v, o))
+      !bool_arg(args[9], deterministic) || transformed() || !plain(q, k, v, o))
     Py_RETURN_NONE;
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
     return THPVariable_Wrap(DenseAttention::apply(q, k, v, o, deterministic));

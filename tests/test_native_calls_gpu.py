@@ -1,0 +1,25 @@
+"""GPU: calls of `flash_attn_func` that the native front (csrc/torch_calls.cc) has to leave to the autograd function in
+Python, or has to take as it does."""
+import pytest
+import torch
+
+from tests._cases import make_qkv
+
+pytestmark = pytest.mark.gpu
+
+
+def _qkv(seed=31, grad=False, seqlen=200, dtype=torch.bfloat16):
+    return [t.cuda().requires_grad_(grad) for t in make_qkv(seed, 2, 4, 2, seqlen, seqlen, 64, dtype)]
+
+
+@pytest.mark.parametrize("grad", [False, True], ids=["plain", "grad"])
+def test_traced_call_follows_its_inputs(grad):
+    """A traced call is recorded; its output is not a constant of the trace."""
+    import flash_attn2_b200 as fa2
+
+    def layer(q, k, v):
+        return fa2.flash_attn_func(q, k, v, causal=True) + q
+
+    traced = torch.jit.trace(layer, _qkv(grad=grad), check_trace=False)
+    other = _qkv(seed=32, grad=grad)
+    assert torch.equal(traced(*other), layer(*other))
