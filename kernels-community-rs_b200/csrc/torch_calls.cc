@@ -53,8 +53,14 @@ struct Options {
   Tensor alibi;  // undefined: none
 };
 
-// A tracer records the autograd function in Python; the output of a native call would be a constant to it.
-bool transformed() { return torch::jit::tracer::isTracing(); }
+// Calls that only the autograd function in Python answers rightly: a tracer records that function (the output of a native
+// call would be a constant to it), and it refuses forward-mode derivatives (a native call would drop them).
+bool transformed(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o) {
+  if (torch::jit::tracer::isTracing()) return true;
+  for (const Tensor* t : {&q, &k, &v, &o.alibi})
+    if (t->defined() && t->_fw_grad(0).defined()) return true;
+  return false;
+}
 
 // q, k, v and the slopes of a plain dense call.
 bool plain(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o) {
@@ -333,7 +339,7 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Options o;
   bool deterministic;
   if (n != 10 || !tensor_arg(args[0], q) || !tensor_arg(args[1], k) || !tensor_arg(args[2], v) || !options_arg(args + 3, o) ||
-      !bool_arg(args[9], deterministic) || transformed() || !plain(q, k, v, o))
+      !bool_arg(args[9], deterministic) || transformed(q, k, v, o) || !plain(q, k, v, o))
     Py_RETURN_NONE;
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
     return THPVariable_Wrap(DenseAttention::apply(q, k, v, o, deterministic));

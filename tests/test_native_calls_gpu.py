@@ -23,3 +23,18 @@ def test_traced_call_follows_its_inputs(grad):
     traced = torch.jit.trace(layer, _qkv(grad=grad), check_trace=False)
     other = _qkv(seed=32, grad=grad)
     assert torch.equal(traced(*other), layer(*other))
+
+
+@pytest.mark.parametrize("which", ["q", "k", "v", "alibi_slopes"])
+@pytest.mark.parametrize("grad", [False, True], ids=["plain", "grad"])
+def test_forward_mode_derivatives_are_refused(which, grad):
+    """There is no forward-mode formula: an error, not an output without a tangent."""
+    import torch.autograd.forward_ad as fwd_ad
+
+    import flash_attn2_b200 as fa2
+
+    args = dict(zip("qkv", _qkv(grad=grad)), alibi_slopes=torch.full((4,), 0.1, device="cuda"))
+    with fwd_ad.dual_level():
+        args[which] = fwd_ad.make_dual(args[which], torch.ones_like(args[which]))
+        with pytest.raises(NotImplementedError, match="jvp"):
+            fa2.flash_attn_func(**args, causal=True)
