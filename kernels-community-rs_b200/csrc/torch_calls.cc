@@ -8,6 +8,7 @@
 // The semantics are those of interface.py's `fwd`, `bwd` and `flash_attn_func`
 // (flash-attn2-rs/tvm-ffi-ext/flash_attn2_rs/flash_attn_interface.py in the reference).
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -54,9 +55,11 @@ struct Options {
 };
 
 // Calls that only the autograd function in Python answers rightly: a tracer records that function (the output of a native
-// call would be a constant to it), and it refuses forward-mode derivatives (a native call would drop them).
+// call would be a constant to it), and it refuses function transforms and forward-mode derivatives (a native call would
+// hand their wrappers' storage to the kernels, or drop them).
 bool transformed(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o) {
-  if (torch::jit::tracer::isTracing()) return true;
+  if (torch::jit::tracer::isTracing() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+    return true;
   for (const Tensor* t : {&q, &k, &v, &o.alibi})
     if (t->defined() && t->_fw_grad(0).defined()) return true;
   return false;

@@ -38,3 +38,18 @@ def test_forward_mode_derivatives_are_refused(which, grad):
         args[which] = fwd_ad.make_dual(args[which], torch.ones_like(args[which]))
         with pytest.raises(NotImplementedError, match="jvp"):
             fa2.flash_attn_func(**args, causal=True)
+
+
+def test_functorch_transforms_are_refused():
+    """The autograd function has no rules for them, whichever tensor of the call is transformed."""
+    import flash_attn2_b200 as fa2
+
+    q, k, v = _qkv()
+    weight = torch.randn(3, device="cuda")
+    calls = [lambda: torch.func.vmap(lambda w: fa2.flash_attn_func(q, k, v) * w)(weight),
+             lambda: torch.func.vmap(lambda x: fa2.flash_attn_func(x, k, v))(torch.stack([q, q])),
+             lambda: torch.func.grad(lambda w: (fa2.flash_attn_func(q, k, v).float() * w).sum())(weight[0]),
+             lambda: torch.func.jvp(lambda x: fa2.flash_attn_func(x, k, v), (q,), (q,))]
+    for call in calls:
+        with pytest.raises(RuntimeError, match="setup_context"):
+            call()
