@@ -56,13 +56,13 @@ struct Options {
 
 // Calls that only the autograd function in Python answers rightly: a tracer records that function (the output of a native
 // call would be a constant to it), and it refuses function transforms and forward-mode derivatives (a native call would
-// hand their wrappers' storage to the kernels, or drop them).
+// hand their wrappers' storage to the kernels, or drop them). Slopes that require grad are inputs of it, too.
 bool transformed(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o) {
   if (torch::jit::tracer::isTracing() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
     return true;
   for (const Tensor* t : {&q, &k, &v, &o.alibi})
     if (t->defined() && t->_fw_grad(0).defined()) return true;
-  return false;
+  return at::GradMode::is_enabled() && o.alibi.defined() && o.alibi.requires_grad();
 }
 
 // q, k, v and the slopes of a plain dense call.

@@ -53,3 +53,15 @@ def test_functorch_transforms_are_refused():
     for call in calls:
         with pytest.raises(RuntimeError, match="setup_context"):
             call()
+
+
+def test_slopes_that_require_grad_keep_the_graph():
+    """The slopes get no gradient, but the output belongs to the graph as for any other differentiable input."""
+    import flash_attn2_b200 as fa2
+
+    q, k, v = _qkv()
+    slopes = torch.full((4,), 0.1, device="cuda", requires_grad=True)
+    out = fa2.flash_attn_func(q, k, v, causal=True, alibi_slopes=slopes)
+    assert out.requires_grad
+    out.sum().backward()
+    assert slopes.grad is None
