@@ -54,11 +54,14 @@ struct Options {
   Tensor alibi;  // undefined: none
 };
 
+// The trace of an autograd function holds what its forward does, down to an operation that made the output.
+bool tracing() { return torch::jit::tracer::isTracing(); }
+
 // Calls that only the autograd function in Python answers rightly: a tracer records that function (the output of a native
 // call would be a constant to it), and it refuses function transforms and forward-mode derivatives (a native call would
 // hand their wrappers' storage to the kernels, or drop them). Slopes that require grad are inputs of it, too.
 bool transformed(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o) {
-  if (torch::jit::tracer::isTracing() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+  if (tracing() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
     return true;
   for (const Tensor* t : {&q, &k, &v, &o.alibi})
     if (t->defined() && t->_fw_grad(0).defined()) return true;
@@ -310,7 +313,7 @@ PyObject* py_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Tensor q, k, v;
   Options o;
   if (n != 9 || !tensor_arg(args[0], q) || !tensor_arg(args[1], k) || !tensor_arg(args[2], v) || !options_arg(args + 3, o) ||
-      !plain(q, k, v, o))
+      tracing() || !plain(q, k, v, o))
     Py_RETURN_NONE;
   Tensor out, lse;
   forward(q, k, v, o, out, lse);
