@@ -40,6 +40,11 @@ bool addressable(const Tensor& t) {
   return true;
 }
 
+// `t`, or a copy that the kernels can address.
+Tensor laid_out(const Tensor& t) {
+  return t.is_cuda() && t.layout() == c10::kStrided && t.dim() == 4 && !addressable(t) ? t.clone(at::MemoryFormat::Contiguous) : t;
+}
+
 void strides_of(const Tensor& t, int64_t out[3]) {
   const auto sh = t.sizes(), st = t.strides();
   for (int i = 0; i < 3; ++i) out[i] = sh[i] > 1 ? st[i] : 0;  // the stride of a size-1 dimension is never used
@@ -253,10 +258,11 @@ class DenseAttention : public torch::autograd::Function<DenseAttention> {
     o.right = d["right"].toInt();
     o.softcap = d["softcap"].toDouble();
     if (const auto it = d.find("alibi"); it != d.end()) o.alibi = it->second.toTensor();
-    Tensor dout = grads[0].contiguous();
-    if (reinterpret_cast<uintptr_t>(dout.data_ptr()) % 16 != 0) dout = dout.clone();
-    TORCH_CHECK(plain_backward(dout, saved[0], saved[3], saved[4]), "dout must match q's shape, dtype and device");
-    Gradients g = ::backward(dout, saved[0], saved[1], saved[2], saved[3], saved[4], o, d["deterministic"].toBool());
+    // What saved-tensor hooks hand back is checked and laid out anew like any argument.
+    const Tensor dout = laid_out(grads[0].contiguous()), q = laid_out(saved[0]), k = laid_out(saved[1]), v = laid_out(saved[2]),
+                 out = laid_out(saved[3]), &lse = saved[4];
+    TORCH_CHECK(plain(q, k, v, o) && plain_backward(dout, q, out, lse), "dout and the saved tensors must match the forward's shapes, dtypes and device");
+    Gradients g = ::backward(dout, q, k, v, out, lse, o, d["deterministic"].toBool());
     return {g.dq, g.dk, g.dv, Tensor(), Tensor()};
   }
 };

@@ -65,3 +65,40 @@ def test_slopes_that_require_grad_keep_the_graph():
     assert out.requires_grad
     out.sum().backward()
     assert slopes.grad is None
+
+
+def _through_hooks(unpack):
+    """Gradients of a call whose saved tensors come back through `unpack`, and of the call without hooks."""
+    import flash_attn2_b200 as fa2
+
+    q, k, v = _qkv(grad=True)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().clone(), unpack):
+        out = fa2.flash_attn_func(q, k, v, causal=True, deterministic=True)
+    want = torch.autograd.grad(fa2.flash_attn_func(q, k, v, causal=True, deterministic=True), (q, k, v), torch.ones_like(out))
+    return torch.autograd.grad(out, (q, k, v), torch.ones_like(out)), want
+
+
+def _odd_offset(t):
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    return buf[1:].view(t.shape).copy_(t)
+
+
+def _odd_stride(t):
+    buf = torch.empty(*t.shape[:-1], t.shape[-1] + 1, dtype=t.dtype, device=t.device)
+    return buf[..., :t.shape[-1]].copy_(t)
+
+
+@pytest.mark.parametrize("layout", [_odd_offset, _odd_stride], ids=["offset", "stride"])
+def test_saved_tensors_may_come_back_in_another_layout(layout):
+    got, want = _through_hooks(lambda t: layout(t) if t.dim() == 4 else t)
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
+
+
+@pytest.mark.parametrize("rank,change", [(4, torch.Tensor.cpu), (4, torch.Tensor.float), (4, lambda t: t[:, 1:]),
+                                         (3, torch.Tensor.cpu), (3, torch.Tensor.half), (3, lambda t: t[:, 1:])],
+                         ids=["cpu", "type", "shape", "lse-cpu", "lse-type", "lse-shape"])
+def test_saved_tensors_that_do_not_match_are_refused(rank, change):
+    """An error before any launch."""
+    with pytest.raises(RuntimeError):
+        _through_hooks(lambda t: change(t) if t.dim() == rank else t)
