@@ -246,11 +246,11 @@ def flash_attn_func(q, k, v, dropout_p=0.0, softmax_scale=None, causal=False, wi
     _no_dropout(dropout_p)
     if return_attn_probs:
         raise RuntimeError("return_attn_probs requires dropout, which is not built in the sm_100a library")
-    left, right = window_size
-    out = _native.attention(q, k, v, softmax_scale, causal, left, right, softcap, alibi_slopes, deterministic)
+    window_size = tuple(window_size)
+    out = _native.attention(q, k, v, softmax_scale, causal, window_size[0], window_size[1], softcap, alibi_slopes, deterministic)
     if out is not None:
         return out
-    return _DenseAttention.apply(q, k, v, softmax_scale, causal, tuple(window_size), softcap, alibi_slopes, deterministic)
+    return _DenseAttention.apply(q, k, v, softmax_scale, causal, window_size, softcap, alibi_slopes, deterministic)
 
 
 def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, dropout_p=0.0,

@@ -102,3 +102,14 @@ def test_saved_tensors_that_do_not_match_are_refused(rank, change):
     """An error before any launch."""
     with pytest.raises(RuntimeError):
         _through_hooks(lambda t: change(t) if t.dim() == rank else t)
+
+
+@pytest.mark.parametrize("window", [[5, 3], (5, 3, 9)], ids=["list", "longer"])
+def test_window_forms(window):
+    """Any sequence: its first two elements count. An iterator serves a call that falls back to Python as well."""
+    import flash_attn2_b200 as fa2
+
+    q, k, v = _qkv()
+    want = fa2.flash_attn_func(q, k, v, window_size=(5, 3))
+    assert torch.equal(fa2.flash_attn_func(q, k, v, window_size=window), want)
+    assert torch.equal(fa2.flash_attn_func(_odd_offset(q), k, v, window_size=iter(window)), want)
