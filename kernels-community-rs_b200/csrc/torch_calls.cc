@@ -305,6 +305,13 @@ bool options_arg(PyObject* const* a, Options& o) {
          (a[5] == Py_None || tensor_arg(a[5], o.alibi));
 }
 
+// Allocations and launches can block (a full launch queue, a cudaMalloc): other Python threads run meanwhile. Saved-tensor
+// hooks take the lock for themselves.
+struct WithoutPython {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~WithoutPython() { PyEval_RestoreThread(state); }
+};
+
 PyObject* list_of(std::initializer_list<Tensor> ts) {
   PyObject* list = PyList_New(static_cast<Py_ssize_t>(ts.size()));
   Py_ssize_t i = 0;
@@ -321,9 +328,14 @@ PyObject* py_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 9 || !tensor_arg(args[0], q) || !tensor_arg(args[1], k) || !tensor_arg(args[2], v) || !options_arg(args + 3, o) ||
       tracing() || !plain(q, k, v, o))
     Py_RETURN_NONE;
-  Tensor out, lse;
-  forward(q, k, v, o, out, lse);
-  return list_of({out, lse, empty({0}, q.scalar_type(), q.device()), empty({2}, at::kLong, q.device())});
+  Tensor out, lse, probabilities, state;
+  {
+    const WithoutPython unlocked;
+    forward(q, k, v, o, out, lse);
+    probabilities = empty({0}, q.scalar_type(), q.device());
+    state = empty({2}, at::kLong, q.device());
+  }
+  return list_of({out, lse, probabilities, state});
   END_HANDLE_TH_ERRORS
 }
 
@@ -338,7 +350,11 @@ PyObject* py_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
       !tensor_arg(args[4], out) || !tensor_arg(args[5], lse) || !options_arg(args + 6, o) || !bool_arg(args[12], deterministic) ||
       !plain(q, k, v, o) || !plain_backward(dout, q, out, lse))
     Py_RETURN_NONE;
-  const Gradients g = backward(dout, q, k, v, out, lse, o, deterministic);
+  Gradients g;
+  {
+    const WithoutPython unlocked;
+    g = backward(dout, q, k, v, out, lse, o, deterministic);
+  }
   return list_of({g.dq, g.dk, g.dv, g.delta});
   END_HANDLE_TH_ERRORS
 }
@@ -353,10 +369,14 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 10 || !tensor_arg(args[0], q) || !tensor_arg(args[1], k) || !tensor_arg(args[2], v) || !options_arg(args + 3, o) ||
       !bool_arg(args[9], deterministic) || transformed(q, k, v, o) || !plain(q, k, v, o))
     Py_RETURN_NONE;
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
-    return THPVariable_Wrap(DenseAttention::apply(q, k, v, o, deterministic));
   Tensor out, lse;
-  forward(q, k, v, o, out, lse);
+  {
+    const WithoutPython unlocked;
+    if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
+      out = DenseAttention::apply(q, k, v, o, deterministic);
+    else
+      forward(q, k, v, o, out, lse);
+  }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }

@@ -1,5 +1,8 @@
 """GPU: calls of `flash_attn_func` that the native front (csrc/torch_calls.cc) has to leave to the autograd function in
 Python, or has to take as it does."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -113,3 +116,37 @@ def test_window_forms(window):
     want = fa2.flash_attn_func(q, k, v, window_size=(5, 3))
     assert torch.equal(fa2.flash_attn_func(q, k, v, window_size=window), want)
     assert torch.equal(fa2.flash_attn_func(_odd_offset(q), k, v, window_size=iter(window)), want)
+
+
+@pytest.mark.parametrize("call", ["fwd", "bwd", "attention", "attention-grad"])
+def test_other_threads_run_while_a_call_waits(call):
+    """The GPU is busy and the launch queue full, so the calls block; a thread that wants to run every millisecond can."""
+    import flash_attn2_b200 as fa2
+
+    q, k, v = _qkv(seqlen=64, grad=call == "attention-grad")
+    out, lse = (t.detach() for t in fa2.fwd(q, k, v)[:2])
+    calls = {"fwd": lambda: fa2.fwd(q, k, v), "bwd": lambda: fa2.bwd(out, q, k, v, out, lse)}
+    once = calls.get(call, lambda: fa2.flash_attn_func(q, k, v))
+    once()
+    torch.cuda.synchronize()
+    gaps, done = [], threading.Event()
+
+    def ticks():
+        last = time.perf_counter()
+        while not done.wait(0.001):
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    ticker = threading.Thread(target=ticks)
+    ticker.start()
+    torch.cuda._sleep(1_000_000_000)  # half a second
+    start = time.perf_counter()
+    for _ in range(1500):
+        once()
+    blocked = time.perf_counter() - start
+    done.set()
+    ticker.join()
+    torch.cuda.synchronize()
+    assert blocked > 0.2, "the queue never filled: nothing was tested"
+    assert max(gaps) < 0.1
