@@ -61,20 +61,22 @@ typedef struct fa2_fwd_args {
   const int32_t* cu_seqlens_k;
   int32_t total_q, total_k;
   int32_t zero_tensors; /* packed mode: clear out (0) and LSE (-inf) first, as the reference's flag does */
-  /* Optional scratch memory of fa2_fwd_workspace_bytes() bytes, 256-byte aligned, contents irrelevant. With it a
-   * call whose (batch, head) work does not fill the GPU is split along the keys as well. May be NULL. */
-  void* workspace;
-  int64_t workspace_bytes;
 } fa2_fwd_args;
 
-/* Bytes of scratch memory the dense forward can use for these arguments (0: none); reads the shapes, the window
- * and the pointers' device only. */
-FA2_API int64_t fa2_fwd_workspace_bytes(const fa2_fwd_args* args);
-
-/* Dense forward. Replaces launch_forward + flash_attn_fwd of the reference
+/* Dense forward. The bits of a head do not depend on the batch and the other heads of the call. Replaces launch_forward + flash_attn_fwd of the reference
  * (flash-attn2-rs/src/host/forward/mod.rs:449-813, src/device/forward/dense.rs:472-590).
  * Empty Sk gives O = 0 and LSE = +inf (forward/mod.rs:548-582). */
 FA2_API int fa2_fwd(const fa2_fwd_args* args, void* stream);
+
+/* The same with scratch memory: a call with few query rows, or whose (batch, head) work does not fill the GPU, is split
+ * along the keys as well. How, and with it the order of its sums, follows from the sizes of the whole call; a call repeats
+ * itself bit for bit. `workspace` is 256-byte aligned, its contents are irrelevant; without it, or with less than
+ * fa2_fwd_workspace_bytes() bytes of it, the call does with what needs none. */
+FA2_API int fa2_fwd_with_workspace(const fa2_fwd_args* args, void* workspace, int64_t workspace_bytes, void* stream);
+
+/* Bytes of scratch memory that call can use for these arguments (0: none); reads the shapes, the window and the
+ * pointers' device only. */
+FA2_API int64_t fa2_fwd_workspace_bytes(const fa2_fwd_args* args);
 
 /* Packed variable-length forward driven by cu_seqlens on the device, no host read of the
  * metadata. Replaces varlen_fwd (flash-attn2-rs/src/host/varlen/mod.rs:21-630,
@@ -143,6 +145,13 @@ typedef struct fa2_bwd_args {
   const float* alibi_slopes;
   int32_t alibi_batch_stride;
   float softcap;
+} fa2_bwd_args;
+FA2_API int64_t fa2_bwd_workspace_bytes(const fa2_bwd_args* args);
+FA2_API int fa2_bwd(const fa2_bwd_args* args, void* stream);
+
+/* What a backward call can do besides. */
+typedef struct fa2_bwd_options {
+  int64_t size; /* sizeof(fa2_bwd_options) */
   /* With `out` (the forward's output) the call computes delta itself, into the memory `delta` points to,
    * and clears the accumulator in the same pass: one kernel instead of fa2_bwd_preprocess and a fill.
    * NULL: `delta` is an input. */
@@ -152,9 +161,9 @@ typedef struct fa2_bwd_args {
    * the workspace then has room for their fp32 parts. dK and dV are the same bits every time either way, but not the
    * same with and without. */
   int32_t share_key_blocks;
-} fa2_bwd_args;
-FA2_API int64_t fa2_bwd_workspace_bytes(const fa2_bwd_args* args);
-FA2_API int fa2_bwd(const fa2_bwd_args* args, void* stream);
+} fa2_bwd_options;
+FA2_API int64_t fa2_bwd_workspace_bytes_with_options(const fa2_bwd_args* args, const fa2_bwd_options* options);
+FA2_API int fa2_bwd_with_options(const fa2_bwd_args* args, const fa2_bwd_options* options, void* stream);
 
 /* Views the kernels cannot address (base not 16-byte aligned, or an outer stride that is not a
  * multiple of 8 elements) are copied into a packed tensor first, as prepare_attention_tensor does

@@ -183,6 +183,13 @@ __global__ void fill_f32_kernel(float* dst, int64_t n, float value) {
   if (i < n) dst[i] = value;
 }
 
+// Scratch memory of a forward call that may be split along the keys.
+struct Scratch {
+  void* ptr;
+  int64_t bytes;
+  bool holds(int64_t need) const { return ptr != nullptr && bytes >= need && reinterpret_cast<uintptr_t>(ptr) % 256 == 0; }
+};
+
 // ---- dense forward with few query rows per kv head (fwd_decode_sm100.cu)
 struct DecodePlan {
   int rows = 0;            // query rows per kv head; 0: the path does not take this call
@@ -227,7 +234,7 @@ DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
   return d;
 }
 
-int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, Runtime* rt, cudaStream_t stream) {
+int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, const Scratch& scratch, Runtime* rt, cudaStream_t stream) {
   fa2::DecodeParams p;
   memset(&p, 0, sizeof(p));
   int rc;
@@ -268,15 +275,14 @@ int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, Runtime* rt, cudaStre
   p.head_dim = a->head_dim;
   p.status = rt->status;
   int grid = d.whole_grid;
-  if (d.split && a->workspace != nullptr && a->workspace_bytes >= d.workspace_bytes &&
-      reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0) {
+  if (d.split && scratch.holds(d.workspace_bytes)) {
     grid = d.grid;
     // The flags in the workspace are set to this number, so their old contents do not matter.
     static std::atomic<unsigned long long> launches{static_cast<unsigned long long>(
         std::chrono::steady_clock::now().time_since_epoch().count())};
     p.launch_tag = (launches.fetch_add(1) + 1) | (1ull << 63);  // never the cleared value
-    p.flags = static_cast<unsigned long long*>(a->workspace);
-    p.partials = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + d.flag_bytes);
+    p.flags = static_cast<unsigned long long*>(scratch.ptr);
+    p.partials = reinterpret_cast<float*>(static_cast<char*>(scratch.ptr) + d.flag_bytes);
   }
   const cudaError_t e = fa2::launch_fwd_decode(p, grid, a->dtype == FA2_BF16, stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "forward launch failed: %s", cudaGetErrorString(e));
@@ -340,7 +346,8 @@ void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
   out->workspace_bytes = (bytes + 255) / 256 * 256;
 }
 
-int fwd_common(const fa2_fwd_args* a, void* stream_v, bool packed) {
+// `scratch`: null where the work is not split along the keys (packed batches, fa2_fwd).
+int fwd_common(const fa2_fwd_args* a, const Scratch* scratch, void* stream_v, bool packed) {
   if (a == nullptr) return fail(FA2_E_VALUE, "args is null");
   if (a->dtype != FA2_F16 && a->dtype != FA2_BF16) return fail(FA2_E_TYPE, "q, k, v must be float16 or bfloat16");
   const int d = a->head_dim;
@@ -422,9 +429,9 @@ int fwd_common(const fa2_fwd_args* a, void* stream_v, bool packed) {
   if ((rc = check_layout(a->v, vs, ns, "v")) != FA2_OK) return rc;
   if ((rc = check_layout(a->out, os, ns, "out")) != FA2_OK) return rc;
 
-  if (!packed) {
+  if (scratch != nullptr) {
     const DecodePlan plan = decode_plan(a, rt->sm_count);
-    if (plan.rows > 0) return fwd_decode(a, plan, rt, stream);
+    if (plan.rows > 0) return fwd_decode(a, plan, *scratch, rt, stream);
   }
   if ((rc = make_map(&p.tm_q, a->q, a->dtype, 2, d, a->heads, rows_q, nbatch, a->q_stride[2], a->q_stride[1],
                      a->q_stride[0], 64, 128, "q")) != FA2_OK)
@@ -461,11 +468,11 @@ int fwd_common(const fa2_fwd_args* a, void* stream_v, bool packed) {
   p.softcap = a->softcap > 0.f ? a->softcap : 0.f;
   p.status = rt->status;
 
-  if (!packed && a->workspace != nullptr && reinterpret_cast<uintptr_t>(a->workspace) % 256 == 0) {
+  if (scratch != nullptr) {
     StreamPlan plan;
     plan_stream(a, rt->sm_count, &plan);
-    if (plan.grid > 0 && a->workspace_bytes >= plan.workspace_bytes) {
-      p.parts = static_cast<float*>(a->workspace);
+    if (plan.grid > 0 && scratch->holds(plan.workspace_bytes)) {
+      p.parts = static_cast<float*>(scratch->ptr);
       p.stream_grid = plan.grid;
       p.units_per_head = plan.start[p.num_mblk];
       memcpy(p.block_start, plan.start, sizeof(plan.start));
@@ -557,10 +564,10 @@ struct BwdSplit {
   uint16_t start[fa2::kMaxSplitBlocks + 1];
   int64_t bytes() const { return items_per_head > 0 ? 2 * max_parts * ((part_elems * 4 + 255) / 256 * 256) : 0; }
 };
-void plan_bwd_split(const fa2_bwd_args* a, int sm_count, BwdSplit* out) {
+void plan_bwd_split(const fa2_bwd_args* a, bool share, int sm_count, BwdSplit* out) {
   const int nblk = (a->seqlen_k + 127) / 128;
   const int64_t units = static_cast<int64_t>(a->batch) * a->heads_k;
-  if (!a->share_key_blocks || a->cu_seqlens_q != nullptr || a->head_dim > 128 || (a->which & 2) == 0 || a->seqlen_q <= 0 || a->seqlen_k <= 0 ||
+  if (!share || a->cu_seqlens_q != nullptr || a->head_dim > 128 || (a->which & 2) == 0 || a->seqlen_q <= 0 || a->seqlen_k <= 0 ||
       nblk > fa2::kMaxSplitBlocks || units * nblk > 2 * sm_count)
     return;
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
@@ -615,7 +622,7 @@ void plan_bwd_split(const fa2_bwd_args* a, int sm_count, BwdSplit* out) {
 // A dQ-only call for dense tensors has a kernel of its own up to head dim 128 and needs no accumulator.
 bool dq_kernel_takes(const fa2_bwd_args* a) { return a->which == 1 && a->cu_seqlens_q == nullptr && a->head_dim <= 128; }
 
-int bwd_dq(const fa2_bwd_args* a, Runtime* rt, cudaStream_t stream) {
+int bwd_dq(const fa2_bwd_args* a, const fa2_bwd_options& opt, Runtime* rt, cudaStream_t stream) {
   fa2::DqParams p;
   memset(&p, 0, sizeof(p));
   const int d = a->head_dim;
@@ -655,11 +662,11 @@ int bwd_dq(const fa2_bwd_args* a, Runtime* rt, cudaStream_t stream) {
   p.softcap = a->softcap > 0.f ? a->softcap : 0.f;
   p.head_dim = d;
   p.status = rt->status;
-  if (a->out != nullptr) {
+  if (opt.out != nullptr) {
     fa2_bwd_preprocess_args pre;
     memset(&pre, 0, sizeof(pre));
     pre.dout = a->dout;
-    pre.out = a->out;
+    pre.out = opt.out;
     pre.delta = const_cast<float*>(a->delta);
     pre.dtype = a->dtype;
     pre.batch = a->batch;
@@ -667,7 +674,7 @@ int bwd_dq(const fa2_bwd_args* a, Runtime* rt, cudaStream_t stream) {
     pre.heads = a->heads;
     pre.head_dim = d;
     memcpy(pre.do_stride, a->do_stride, sizeof(pre.do_stride));
-    memcpy(pre.o_stride, a->o_stride, sizeof(pre.o_stride));
+    memcpy(pre.o_stride, opt.o_stride, sizeof(pre.o_stride));
     if ((rc = preprocess_launch(&pre, nullptr, stream)) != FA2_OK) return rc;
   }
   if (a->ev_kernel_start != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_start), stream);
@@ -683,7 +690,7 @@ int64_t bwd_dq_bytes(const fa2_bwd_args* a) {
   return (bwd_accum_bytes(a) + bwd_turn_counters(a) * 4 + 255) / 256 * 256;
 }
 
-int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
+int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) {
   if (a == nullptr) return fail(FA2_E_VALUE, "args is null");
   if (a->dtype != FA2_F16 && a->dtype != FA2_BF16) return fail(FA2_E_TYPE, "q, k, v must be float16 or bfloat16");
   const bool packed = a->cu_seqlens_q != nullptr;
@@ -737,7 +744,7 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
   if ((rc = check_layout(a->dout, a->do_stride + so, ns, "dout")) != FA2_OK) return rc;
   if (want_dkv && (reinterpret_cast<uintptr_t>(a->dk) % 16 || reinterpret_cast<uintptr_t>(a->dv) % 16))
     return fail(FA2_E_VALUE, "dk and dv must be 16-byte aligned");
-  if (dq_alone) return bwd_dq(a, rt, stream);
+  if (dq_alone) return bwd_dq(a, opt, rt, stream);
 
   fa2::BwdParams p;
   memset(&p, 0, sizeof(p));
@@ -819,12 +826,12 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
   p.dq_turn = ordered ? reinterpret_cast<int*>(static_cast<char*>(a->dq_accum) + acc_bytes) : nullptr;
   p.num_mblk_q = (a->seqlen_q + 127) / 128;
   // With `out` the delta preprocess is part of this call and clears the accumulator on its way.
-  const bool fused_pre = a->out != nullptr && !packed && !ordered;
-  if (a->out != nullptr) {
+  const bool fused_pre = opt.out != nullptr && !packed && !ordered;
+  if (opt.out != nullptr) {
     fa2_bwd_preprocess_args pre;
     memset(&pre, 0, sizeof(pre));
     pre.dout = a->dout;
-    pre.out = a->out;
+    pre.out = opt.out;
     pre.delta = const_cast<float*>(a->delta);
     pre.dtype = a->dtype;
     pre.batch = a->batch;
@@ -832,7 +839,7 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
     pre.heads = a->heads;
     pre.head_dim = d;
     memcpy(pre.do_stride, a->do_stride, sizeof(pre.do_stride));
-    memcpy(pre.o_stride, a->o_stride, sizeof(pre.o_stride));
+    memcpy(pre.o_stride, opt.o_stride, sizeof(pre.o_stride));
     pre.cu_seqlens_q = a->cu_seqlens_q;
     pre.total_q = a->total_q;
     if ((rc = preprocess_launch(&pre, fused_pre && want_dq ? static_cast<float*>(a->dq_accum) : nullptr, stream)) != FA2_OK) return rc;
@@ -843,7 +850,7 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
   fa2::FinishParams fin;
   fin.dk_part = nullptr;
   BwdSplit split;
-  plan_bwd_split(a, rt->sm_count, &split);
+  plan_bwd_split(a, opt.share_key_blocks != 0, rt->sm_count, &split);
   const int64_t before = bwd_dq_bytes(a);
   if (split.items_per_head > 0 && a->dq_accum != nullptr && a->dq_accum_bytes >= before + split.bytes()) {
     p.dk_part = reinterpret_cast<float*>(static_cast<char*>(a->dq_accum) + before);
@@ -880,6 +887,29 @@ int bwd_impl(const fa2_bwd_args* a, void* stream_v) {
   fin.bf16 = a->dtype == FA2_BF16;
   if ((e = fa2::launch_bwd_finish(fin, stream)) != cudaSuccess)
     return fail(FA2_E_RUNTIME, "conversion launch failed: %s", cudaGetErrorString(e));
+  return FA2_OK;
+}
+
+int64_t bwd_workspace_bytes(const fa2_bwd_args* args, const fa2_bwd_options& opt) {
+  if (args == nullptr || args->heads_k <= 0 || args->heads <= 0 || args->heads % args->heads_k != 0 || args->batch <= 0) return 0;
+  int64_t bytes = bwd_dq_bytes(args);
+  if (opt.share_key_blocks != 0 && (args->which & 2) != 0 && args->cu_seqlens_q == nullptr && args->head_dim <= 128) {
+    const DeviceScope scope(args->q);
+    Runtime* rt = nullptr;
+    BwdSplit split;
+    if (get_runtime(scope.device(), &rt) == FA2_OK) plan_bwd_split(args, true, rt->sm_count, &split);
+    bytes += split.bytes();
+  }
+  return bytes;
+}
+
+// A caller's options, whose size says which of them it knows.
+int read_options(const fa2_bwd_options* options, fa2_bwd_options* out) {
+  *out = {};
+  if (options == nullptr) return FA2_OK;
+  if (options->size < static_cast<int64_t>(sizeof(options->size)) || options->size > static_cast<int64_t>(sizeof(*options)))
+    return fail(FA2_E_VALUE, "fa2_bwd_options: size %lld is not one that this library knows", static_cast<long long>(options->size));
+  memcpy(out, options, static_cast<size_t>(options->size));
   return FA2_OK;
 }
 
@@ -1053,20 +1083,25 @@ extern "C" {
 int fa2_bwd_preprocess(const fa2_bwd_preprocess_args* args, void* stream) { return bwd_preprocess_impl(args, stream); }
 
 int64_t fa2_bwd_workspace_bytes(const fa2_bwd_args* args) {
-  if (args == nullptr || args->heads_k <= 0 || args->heads <= 0 || args->heads % args->heads_k != 0 || args->batch <= 0) return 0;
-  int64_t bytes = bwd_dq_bytes(args);
-  if ((args->which & 2) != 0 && args->cu_seqlens_q == nullptr && args->head_dim <= 128) {
-    const DeviceScope scope(args->q);
-    Runtime* rt = nullptr;
-    BwdSplit split;
-    if (get_runtime(scope.device(), &rt) == FA2_OK) plan_bwd_split(args, rt->sm_count, &split);
-    bytes += split.bytes();
-  }
-  return bytes;
+  const fa2_bwd_options none = {};
+  return bwd_workspace_bytes(args, none);
 }
 
-int fa2_bwd(const fa2_bwd_args* args, void* stream) { return bwd_impl(args, stream); }
+int64_t fa2_bwd_workspace_bytes_with_options(const fa2_bwd_args* args, const fa2_bwd_options* options) {
+  fa2_bwd_options opt;
+  return read_options(options, &opt) == FA2_OK ? bwd_workspace_bytes(args, opt) : 0;
+}
 
+int fa2_bwd(const fa2_bwd_args* args, void* stream) {
+  const fa2_bwd_options none = {};
+  return bwd_impl(args, none, stream);
+}
+
+int fa2_bwd_with_options(const fa2_bwd_args* args, const fa2_bwd_options* options, void* stream) {
+  fa2_bwd_options opt;
+  const int rc = read_options(options, &opt);
+  return rc != FA2_OK ? rc : bwd_impl(args, opt, stream);
+}
 int fa2_layout_is_addressable(const void* ptr, const int64_t* outer_strides, int32_t n_outer) {
   if (ptr == nullptr || reinterpret_cast<uintptr_t>(ptr) % 16 != 0) return 0;
   for (int i = 0; i < n_outer; ++i)
@@ -1137,9 +1172,14 @@ int64_t fa2_fwd_workspace_bytes(const fa2_fwd_args* args) {
   return plan.workspace_bytes;
 }
 
-int fa2_fwd(const fa2_fwd_args* args, void* stream) { return fwd_common(args, stream, false); }
+int fa2_fwd(const fa2_fwd_args* args, void* stream) { return fwd_common(args, nullptr, stream, false); }
 
-int fa2_varlen_fwd(const fa2_fwd_args* args, void* stream) { return fwd_common(args, stream, true); }
+int fa2_fwd_with_workspace(const fa2_fwd_args* args, void* workspace, int64_t workspace_bytes, void* stream) {
+  const Scratch scratch{workspace, workspace_bytes};
+  return fwd_common(args, &scratch, stream, false);
+}
+
+int fa2_varlen_fwd(const fa2_fwd_args* args, void* stream) { return fwd_common(args, nullptr, stream, true); }
 
 const char* fa2_last_error(void) { return g_error; }
 

@@ -144,12 +144,9 @@ void forward(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o
   a.window_right = static_cast<int32_t>(o.right);
   a.softcap = static_cast<float>(o.softcap);
   Tensor workspace;
-  if (const int64_t need = fa2_fwd_workspace_bytes(&a); need > 0) {
-    workspace = empty({need}, at::kByte, q.device());
-    a.workspace = workspace.data_ptr();
-    a.workspace_bytes = need;
-  }
-  check(fa2_fwd(&a, c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
+  const int64_t need = fa2_fwd_workspace_bytes(&a);
+  if (need > 0) workspace = empty({need}, at::kByte, q.device());
+  check(fa2_fwd_with_workspace(&a, need > 0 ? workspace.data_ptr() : nullptr, need, c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
 }
 
 struct Gradients {
@@ -197,9 +194,11 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
   a.causal = effective_causal(o, qs[1]);
   a.window_left = static_cast<int32_t>(o.left);
   a.window_right = static_cast<int32_t>(o.right);
-  a.out = out.data_ptr();  // the first call computes delta
-  strides_of(out, a.o_stride);
-  a.share_key_blocks = 1;
+  fa2_bwd_options opt{};
+  opt.size = sizeof(opt);
+  opt.out = out.data_ptr();  // the first call computes delta
+  strides_of(out, opt.o_stride);
+  opt.share_key_blocks = 1;
   // Bit-reproducible gradients come from the two separate calls: dQ in a fixed order, then dK and dV.
   const int calls[2] = {deterministic ? 1 : 3, deterministic ? 2 : 0};
   for (const int which : calls) {
@@ -207,13 +206,13 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
     a.which = which;
     Tensor workspace;
     a.dq_accum = nullptr;
-    a.dq_accum_bytes = fa2_bwd_workspace_bytes(&a);
+    a.dq_accum_bytes = fa2_bwd_workspace_bytes_with_options(&a, &opt);
     if (a.dq_accum_bytes > 0) {
       workspace = empty({a.dq_accum_bytes}, at::kByte, q.device());
       a.dq_accum = workspace.data_ptr();
     }
-    check(fa2_bwd(&a, stream));
-    a.out = nullptr;
+    check(fa2_bwd_with_options(&a, &opt, stream));
+    opt.out = nullptr;
   }
   return g;
 }

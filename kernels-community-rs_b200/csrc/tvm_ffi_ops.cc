@@ -306,12 +306,8 @@ Any fwd_impl(const AnyView* args, int32_t n, bool lse_only) {
   a.softcap = static_cast<float>(softcap);
   Optional<Tensor> workspace;
   const int64_t need = fa2_fwd_workspace_bytes(&a);
-  if (need > 0) {
-    workspace = alloc({need / 4}, kF32, dev);
-    a.workspace = workspace.value().data_ptr();
-    a.workspace_bytes = need;
-  }
-  check(fa2_fwd(&a, stream_of(dev)));
+  if (need > 0) workspace = alloc({need / 4}, kF32, dev);
+  check(fa2_fwd_with_workspace(&a, need > 0 ? workspace.value().data_ptr() : nullptr, need, stream_of(dev)));
   if (copy_out) {
     const Tensor& o = supplied.value();
     const int64_t shape4[4] = {b, sq, h, d};
@@ -426,7 +422,9 @@ Any bwd_impl(const AnyView* args, int32_t n, int which) {
   a.window_left = static_cast<int32_t>(wl);
   a.window_right = static_cast<int32_t>(wr);
   a.which = which;
-  a.share_key_blocks = 1;
+  fa2_bwd_options opt{};
+  opt.size = sizeof(opt);
+  opt.share_key_blocks = 1;
   // Gradients are allocated like the inputs (backward.rs:199-204); the fp32 dQ accumulator is a
   // workspace tensor from the same stream-ordered allocator.
   // Only what the call returns is allocated (bwd_dq: dQ; bwd_dkv: dK and dV).
@@ -442,13 +440,13 @@ Any bwd_impl(const AnyView* args, int32_t n, int which) {
     a.dv = dv.value().data_ptr();
   }
   Optional<Tensor> accum;
-  const int64_t ws = fa2_bwd_workspace_bytes(&a);
+  const int64_t ws = fa2_bwd_workspace_bytes_with_options(&a, &opt);
   if (ws > 0) {
     accum = alloc({ws / 4}, kF32, dev);
     a.dq_accum = accum.value().data_ptr();
     a.dq_accum_bytes = ws;
   }
-  check(fa2_bwd(&a, stream_of(dev)));
+  check(fa2_bwd_with_options(&a, &opt, stream_of(dev)));
   if (which == 1) return Any(dq.value());
   if (which == 2) return Any(Array<Tensor>{dk.value(), dv.value()});
   return Any(Array<Tensor>{dq.value(), dk.value(), dv.value()});

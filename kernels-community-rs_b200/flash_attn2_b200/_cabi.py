@@ -27,7 +27,6 @@ class FwdArgs(C.Structure):
         ("window_left", C.c_int32), ("window_right", C.c_int32), ("softcap", C.c_float),
         ("cu_seqlens_q", C.c_void_p), ("cu_seqlens_k", C.c_void_p),
         ("total_q", C.c_int32), ("total_k", C.c_int32), ("zero_tensors", C.c_int32),
-        ("workspace", C.c_void_p), ("workspace_bytes", C.c_int64),
     ]
 
 
@@ -56,13 +55,19 @@ class BwdArgs(C.Structure):
         ("total_q", C.c_int32), ("total_k", C.c_int32),
         ("ev_kernel_start", C.c_void_p), ("ev_kernel_stop", C.c_void_p),
         ("alibi_slopes", C.c_void_p), ("alibi_batch_stride", C.c_int32), ("softcap", C.c_float),
-        ("out", C.c_void_p), ("o_stride", C.c_int64 * 3), ("share_key_blocks", C.c_int32),
+    ]
+
+
+class BwdOptions(C.Structure):
+    _fields_ = [
+        ("size", C.c_int64), ("out", C.c_void_p), ("o_stride", C.c_int64 * 3), ("share_key_blocks", C.c_int32),
     ]
 
 
 # Every symbol include/fa2_b200.h declares; the CPU test suite checks that the library exports them.
 EXPORTS = (
-    "fa2_fwd", "fa2_fwd_workspace_bytes", "fa2_varlen_fwd", "fa2_bwd_preprocess", "fa2_bwd_workspace_bytes", "fa2_bwd",
+    "fa2_fwd", "fa2_fwd_with_workspace", "fa2_fwd_workspace_bytes", "fa2_varlen_fwd", "fa2_bwd_preprocess",
+    "fa2_bwd_workspace_bytes", "fa2_bwd", "fa2_bwd_workspace_bytes_with_options", "fa2_bwd_with_options",
     "fa2_bwd_static", "fa2_bwd_static_status", "fa2_layout_is_addressable", "fa2_pack_16bit", "fa2_copy_16bit",
     "fa2_last_error", "fa2_device_status", "fa2_sm_count",
 )
@@ -83,6 +88,8 @@ def load() -> C.CDLL:
         for name in ("fa2_fwd", "fa2_varlen_fwd"):
             getattr(lib, name).argtypes = [C.POINTER(FwdArgs), C.c_void_p]
             getattr(lib, name).restype = C.c_int
+        lib.fa2_fwd_with_workspace.argtypes = [C.POINTER(FwdArgs), C.c_void_p, C.c_int64, C.c_void_p]
+        lib.fa2_fwd_with_workspace.restype = C.c_int
         lib.fa2_fwd_workspace_bytes.argtypes = [C.POINTER(FwdArgs)]
         lib.fa2_fwd_workspace_bytes.restype = C.c_int64
         if hasattr(lib, "fa2_bwd_preprocess"):
@@ -92,6 +99,10 @@ def load() -> C.CDLL:
             lib.fa2_bwd.restype = C.c_int
             lib.fa2_bwd_workspace_bytes.argtypes = [C.POINTER(BwdArgs)]
             lib.fa2_bwd_workspace_bytes.restype = C.c_int64
+            lib.fa2_bwd_with_options.argtypes = [C.POINTER(BwdArgs), C.POINTER(BwdOptions), C.c_void_p]
+            lib.fa2_bwd_with_options.restype = C.c_int
+            lib.fa2_bwd_workspace_bytes_with_options.argtypes = [C.POINTER(BwdArgs), C.POINTER(BwdOptions)]
+            lib.fa2_bwd_workspace_bytes_with_options.restype = C.c_int64
         if hasattr(lib, "fa2_bwd_static"):
             lib.fa2_bwd_static.argtypes = [C.POINTER(BwdArgs), C.c_void_p]
             lib.fa2_bwd_static.restype = C.c_int

@@ -92,10 +92,8 @@ def fwd(q, k, v, *, out=None, alibi_slopes=None, softmax_scale=None, causal=Fals
     a.softcap = float(softcap)
     with torch.cuda.device(q.device):
         need = lib.fa2_fwd_workspace_bytes(C.byref(a))
-        if need > 0:
-            workspace = _alloc((need // 4,), torch.float32, q.device)
-            a.workspace, a.workspace_bytes = workspace.data_ptr(), need
-        _cabi.check(lib.fa2_fwd(C.byref(a), _stream(q)))
+        workspace = _alloc((need // 4,), torch.float32, q.device) if need > 0 else None
+        _cabi.check(lib.fa2_fwd_with_workspace(C.byref(a), None if workspace is None else workspace.data_ptr(), need, _stream(q)))
     return out, lse
 
 

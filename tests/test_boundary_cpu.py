@@ -76,3 +76,53 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_cabi, "LIB_PATH", tmp_path / "libfa2_b200.so")
     with pytest.raises(RuntimeError, match="no CPU fallback"):
         _cabi.load()
+
+
+def _header_fields(struct):
+    """(name, array length) of a struct's fields, from the header."""
+    header = re.sub(r"/\*.*?\*/", "", (ROOT / "include" / "fa2_b200.h").read_text(), flags=re.S)
+    body = re.search(r"typedef struct %s \{(.*?)\} %s;" % (struct, struct), header, flags=re.S).group(1)
+    names = [n for decl in body.split(";") if decl.strip() for n in decl.rsplit("*", 1)[-1].split(",")]
+    return [(re.search(r"(\w+)\s*(?:\[\d+\])?\s*$", n).group(1), re.findall(r"\[(\d+)\]", n)) for n in names]
+
+
+def test_argument_structs_do_not_change_size(built_libs):
+    """A host binds these by layout: a field more would be read behind what an older host passes. What a call can do
+    besides goes into calls of its own and into fa2_bwd_options, which says its size."""
+    from flash_attn2_b200 import _cabi
+
+    assert ctypes.sizeof(_cabi.FwdArgs) == 232
+    assert ctypes.sizeof(_cabi.BwdPreprocessArgs) == 112
+    assert ctypes.sizeof(_cabi.BwdArgs) == 296
+    assert _header_fields("fa2_fwd_args")[-1][0] == "zero_tensors" and _header_fields("fa2_bwd_args")[-1][0] == "softcap"
+
+
+@pytest.mark.parametrize("struct,mirror", [("fa2_fwd_args", "FwdArgs"), ("fa2_bwd_preprocess_args", "BwdPreprocessArgs"),
+                                           ("fa2_bwd_args", "BwdArgs"), ("fa2_bwd_options", "BwdOptions")])
+def test_ctypes_mirrors_have_the_fields_of_the_header(struct, mirror):
+    from flash_attn2_b200 import _cabi
+
+    got = [(n, [str(t._length_)] if hasattr(t, "_length_") else []) for n, t in getattr(_cabi, mirror)._fields_]
+    assert got == _header_fields(struct)
+
+
+def test_integration_guide_shows_the_header():
+    """The guide's Rust mirror has the header's fields in the header's order, and names only functions that exist."""
+    guide = (ROOT / "INTEGRATION.md").read_text()
+    body = re.search(r"pub struct Fa2FwdArgs \{(.*?)\n\}", guide, flags=re.S).group(1)
+    assert [(n, re.findall(r"\[i64; (\d+)\]", t)) for n, t in re.findall(r"pub (\w+): ([^,]*(?:\[[^\]]*\])?)", body)] == \
+        _header_fields("fa2_fwd_args")
+    header = (ROOT / "include" / "fa2_b200.h").read_text()
+    bound = re.findall(r"\bfn (fa2_\w+)\(", guide)
+    assert {"fa2_fwd", "fa2_fwd_with_workspace", "fa2_fwd_workspace_bytes", "fa2_bwd", "fa2_bwd_with_options"} <= set(bound)
+    for name in set(re.findall(r"\bfa2_(?:fwd|bwd|varlen)\w*", guide)) - {"fa2_fwd_args", "fa2_bwd_args", "fa2_bwd_preprocess_args", "fa2_bwd_options"}:
+        assert re.search(r"\b%s\s*\(" % name, header), name
+
+
+def test_backward_options_of_an_unknown_size_are_refused(built_libs):
+    from flash_attn2_b200 import _cabi
+
+    lib = _cabi.load()
+    opt = _cabi.BwdOptions(size=ctypes.sizeof(_cabi.BwdOptions) + 8)
+    assert lib.fa2_bwd_with_options(ctypes.byref(_cabi.BwdArgs()), ctypes.byref(opt), None) == -1
+    assert b"size" in lib.fa2_last_error()
