@@ -158,7 +158,7 @@ typedef struct fa2_bwd_options {
   const void* out;
   int64_t o_stride[3];
   /* 1: several CTAs may share a key block when there are too few of them for the GPU (dense, head dims up to 128);
-   * the workspace then has room for their fp32 parts. dK and dV are the same bits every time either way, but not the
+   * the workspace then has room for their fp32 parts. They are shared only in a workspace that is 256-byte aligned. dK and dV are the same bits every time either way, but not the
    * same with and without. */
   int32_t share_key_blocks;
 } fa2_bwd_options;

@@ -4,10 +4,10 @@
 // the paths this library implements.
 #include "../../include/fa2_b200.h"
 #include "fa2_launch.h"
+#include "fa2_plan.h"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
-#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <climits>
@@ -18,6 +18,16 @@
 #include <mutex>
 
 namespace {
+
+using fa2::BwdSplit;
+using fa2::DecodePlan;
+using fa2::decode_plan;
+using fa2::normalise_windows;
+using fa2::plan_bwd_split;
+using fa2::plan_stream;
+using fa2::Scratch;
+using fa2::StreamPlan;
+using fa2::Windows;
 
 thread_local char g_error[512] = "";
 
@@ -147,23 +157,6 @@ class DeviceScope {
   int prev_ = 0, device_ = 0;
 };
 
-struct Windows {
-  int left, right, causal_alibi;
-};
-// Window normalisation of the reference (forward/mod.rs:310-328, backward.rs:134-149): clamp
-// sides that cover every key to "open", causal means right = 0.
-Windows normalise_windows(int64_t wl, int64_t wr, bool causal, int64_t seqlen_k, bool causal_first) {
-  if (causal_first && causal) wr = 0;
-  if (wl >= seqlen_k) wl = -1;
-  if (wr >= seqlen_k) wr = -1;
-  if (causal) wr = 0;
-  Windows w;
-  w.causal_alibi = (wl < 0 && wr == 0) ? 1 : 0;
-  w.left = wl < 0 ? -1 : static_cast<int>(wl);
-  w.right = wr < 0 ? -1 : static_cast<int>(wr);
-  return w;
-}
-
 __global__ void fill_empty_kernel(uint16_t* out, float* lse, int64_t rows, int heads, int d, int64_t o_row_stride,
                                   int64_t o_head_stride, int64_t o_batch_stride, int64_t rows_per_batch,
                                   int64_t lse_head_stride, int64_t lse_batch_stride, float lse_value) {
@@ -181,57 +174,6 @@ __global__ void fill_empty_kernel(uint16_t* out, float* lse, int64_t rows, int h
 __global__ void fill_f32_kernel(float* dst, int64_t n, float value) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i < n) dst[i] = value;
-}
-
-// Scratch memory of a forward call that may be split along the keys.
-struct Scratch {
-  void* ptr;
-  int64_t bytes;
-  bool holds(int64_t need) const { return ptr != nullptr && bytes >= need && reinterpret_cast<uintptr_t>(ptr) % 256 == 0; }
-};
-
-// ---- dense forward with few query rows per kv head (fwd_decode_sm100.cu)
-struct DecodePlan {
-  int rows = 0;            // query rows per kv head; 0: the path does not take this call
-  int tile_lo = 0, tiles = 0;
-  int grid = 0, whole_grid = 0;  // CTAs with a workspace, and without one
-  bool split = false;            // some unit is shared by CTAs (needs the workspace)
-  int64_t flag_bytes = 0, workspace_bytes = 0;
-};
-DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
-  DecodePlan d;
-  const int64_t rows = static_cast<int64_t>(a->seqlen_q) * (a->heads / a->heads_k);
-  if (rows <= 0 || rows > fa2::kDecodeMaxRows || a->seqlen_k <= 0) return d;
-  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
-  const int64_t off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q;
-  int64_t lo = 0, hi = a->seqlen_k;
-  if (w.left >= 0) lo = std::max<int64_t>(0, off - w.left);
-  if (w.right >= 0) hi = std::min<int64_t>(hi, a->seqlen_q - 1 + off + w.right + 1);
-  if (hi <= lo) return d;  // no row sees a key
-  d.rows = static_cast<int>(rows);
-  d.tile_lo = static_cast<int>(lo / 128);
-  d.tiles = static_cast<int>((hi + 127) / 128) - d.tile_lo;
-  const int64_t units = static_cast<int64_t>(a->batch) * a->heads_k, n = units * d.tiles, sms = sm_count;
-  // Whole units per CTA, as evenly as that goes: what happens without a workspace.
-  const int64_t per_cta = (units + sms - 1) / sms;
-  d.whole_grid = d.grid = static_cast<int>((units + per_cta - 1) / per_cta);
-  // Splitting units over CTAs costs about 5 us at the end (parts to memory, flags, merge), as much as a CTA takes for
-  // four tiles of its own. Few units: each is cut into as many equal parts as the SMs allow and leave three tiles; at
-  // most 24, because one CTA merges them. More units than SMs: equal shares of the whole list when the last,
-  // incomplete round of whole units would take more than five tiles longer.
-  if (units <= sms) {
-    const int64_t parts = std::min<int64_t>({sms / units, 24, d.tiles / 3});
-    if (parts > 1) d.grid = static_cast<int>(units * parts);
-  } else if (per_cta * d.tiles - n / sms > 5) {
-    d.grid = sm_count;
-  }
-  d.split = d.grid != d.whole_grid || (units > sms && d.grid == sm_count && units % sms != 0);
-  if (d.split) {
-    const int64_t dim = (a->head_dim + 63) / 64 * 64;
-    d.flag_bytes = (2 * static_cast<int64_t>(d.grid) * 8 + 255) / 256 * 256;
-    d.workspace_bytes = d.flag_bytes + 2 * static_cast<int64_t>(d.grid) * 16 * fa2::decode_row_tiles(d.rows) * (dim + 2) * 4;
-  }
-  return d;
 }
 
 int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, const Scratch& scratch, Runtime* rt, cudaStream_t stream) {
@@ -287,63 +229,6 @@ int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, const Scratch& scratc
   const cudaError_t e = fa2::launch_fwd_decode(p, grid, a->dtype == FA2_BF16, stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "forward launch failed: %s", cudaGetErrorString(e));
   return FA2_OK;
-}
-
-// ---- dense forward with few work tiles (fwd_sm100.cu, SHARED): a work tile is 256 query rows of a head, one CTA at a
-// time works on it, and with fewer tiles than SMs some have nothing to do. Calls with more tiles are not shared, also
-// where a last, nearly empty round would gain (H32 Sq 1500 Sk 16384, 192 tiles: 454 -> 392 us): there the bits of a head do
-// not depend on how many other heads the call has, which a long-context run that is sharded by heads relies on.
-struct StreamPlan {
-  int grid = 0;  // 0: one tile per CTA at a time
-  int64_t workspace_bytes = 0;
-  uint16_t start[fa2::kMaxStreamBlocks + 1];
-};
-void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
-  const int64_t mblk = (static_cast<int64_t>(a->seqlen_q) + 255) / 256;
-  if (a->head_dim > 128 || mblk <= 0 || mblk > fa2::kMaxStreamBlocks || a->seqlen_k <= 0) return;
-  const int64_t heads = static_cast<int64_t>(a->batch) * a->heads, tiles = heads * mblk;
-  if (tiles > sm_count) return;
-  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
-  const int64_t off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q;
-  int64_t total = 0, longest = 0;
-  for (int64_t m = 0; m < mblk; ++m) {
-    // Key blocks of the tile: the union over its two 128-row stages, as the kernel walks it.
-    int64_t jlo = INT64_MAX, jhi = 0;
-    for (int s = 0; s < 2; ++s) {
-      const int64_t r_lo = m * 256 + s * 128;
-      if (r_lo >= a->seqlen_q) break;
-      const int64_t r_hi = std::min<int64_t>(r_lo + 127, a->seqlen_q - 1);
-      int64_t hi = a->seqlen_k, lo = 0;
-      if (w.right >= 0) hi = std::min(hi, r_hi + off + w.right + 1);
-      if (w.left >= 0) lo = std::max<int64_t>(0, r_lo + off - w.left);
-      if (hi > lo) {
-        jlo = std::min(jlo, lo / 128);
-        jhi = std::max(jhi, (hi + 127) / 128);
-      }
-    }
-    if (jhi <= jlo) return;  // a tile without keys is in no share
-    if (total + jhi - jlo > UINT16_MAX) return;
-    out->start[m] = static_cast<uint16_t>(total);
-    total += jhi - jlo;
-    longest = std::max(longest, jhi - jlo);
-  }
-  out->start[mblk] = static_cast<uint16_t>(total);
-  const int64_t units = total * heads;
-  if (units > INT32_MAX / 2) return;
-  // Costs in cycles: a key block, a tile's start and end, a part's way to memory, and the merge (a launch, and the parts
-  // read back); at least three key blocks per CTA. With these a call that is shared is faster or equal from 4 tiles
-  // (H4 Sq 128 Sk 1024 D64: 17.0 -> 16.5 us) to 128 (H8 S4096: 66.7 -> 65.6).
-  const double t_blk = 3300, t_tile = 6000, t_part = 4000, t_merge = 7000;
-  const int64_t grid = std::min<int64_t>(sm_count, units / 3);
-  if (grid < 2) return;
-  const double whole = longest * t_blk + t_tile;
-  const int64_t dim = a->head_dim > 64 ? 128 : 64;
-  const int64_t bytes = 2 * grid * fa2::stream_slot_floats(static_cast<int>(dim)) * 4;
-  const double shared = static_cast<double>(units) / grid * t_blk + (static_cast<double>(tiles) / grid + 1) * t_tile + t_part +
-                        t_merge + static_cast<double>(std::min<int64_t>(grid, tiles) + grid) / (2.0 * grid) * bytes / 3000;
-  if (shared > 0.92 * whole) return;
-  out->grid = static_cast<int>(grid);
-  out->workspace_bytes = (bytes + 255) / 256 * 256;
 }
 
 // `scratch`: null where the work is not split along the keys (packed batches, fa2_fwd).
@@ -552,71 +437,6 @@ int64_t bwd_dq_bytes(const fa2_bwd_args* a);
 // One counter per (batch, head, 128-row query block, 32-row slab of a drain warp).
 int64_t bwd_turn_counters(const fa2_bwd_args* a) {
   return static_cast<int64_t>(a->batch) * a->heads * ((a->seqlen_q + 127) / 128) * 4;
-}
-
-// ---- key blocks shared by several CTAs (bwd_sm100.cu: part_start). A CTA owns 128 keys of one kv head and walks the
-// query blocks of all the group's heads; with few (batch, kv head, key block) triples most SMs would have nothing
-// to do, or wait for the CTA with the longest walk.
-struct BwdSplit {
-  int items_per_head = 0;      // 0: not split
-  int64_t part_elems = 0;      // elements of one slot (= elements of dK)
-  int max_parts = 1;
-  uint16_t start[fa2::kMaxSplitBlocks + 1];
-  int64_t bytes() const { return items_per_head > 0 ? 2 * max_parts * ((part_elems * 4 + 255) / 256 * 256) : 0; }
-};
-void plan_bwd_split(const fa2_bwd_args* a, bool share, int sm_count, BwdSplit* out) {
-  const int nblk = (a->seqlen_k + 127) / 128;
-  const int64_t units = static_cast<int64_t>(a->batch) * a->heads_k;
-  if (!share || a->cu_seqlens_q != nullptr || a->head_dim > 128 || (a->which & 2) == 0 || a->seqlen_q <= 0 || a->seqlen_k <= 0 ||
-      nblk > fa2::kMaxSplitBlocks || units * nblk > 2 * sm_count)
-    return;
-  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
-  const int64_t off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q, group = a->heads / a->heads_k;
-  int64_t n[fa2::kMaxSplitBlocks], most = 0, total = 0, least = INT64_MAX;
-  for (int i = 0; i < nblk; ++i) {
-    const int64_t n0 = i * 128LL, n_last = std::min<int64_t>(n0 + 127, a->seqlen_k - 1);
-    int64_t lo = 0, hi = a->seqlen_q;
-    if (w.right >= 0) lo = std::max<int64_t>(0, n0 - off - w.right);
-    if (w.left >= 0) hi = std::min<int64_t>(hi, n_last - off + w.left + 1);
-    n[i] = hi > lo ? ((hi + 127) / 128 - lo / 128) * group : 0;
-    most = std::max(most, n[i]);
-    least = std::min(least, n[i]);
-    total += n[i];
-  }
-  // Costs in cycles, from clock stamps: an iteration of the walk, a CTA's start and end, and per byte of the parts
-  // (written and read once each at the memory's rate). The same split for calls with and without dQ: dK and dV are the
-  // same bits in both.
-  const double t_it = a->head_dim > 64 ? 4300 : 3000, t_cta = 8500;
-  const int64_t dkv = static_cast<int64_t>(a->batch) * a->seqlen_k * a->heads_k * a->head_dim;
-  const double base_cost = 4000, part_cost = dkv * 16.0 / 3400;
-  auto cost = [&](double items, double longest, double all, bool even) {
-    if (items <= sm_count) return longest;
-    if (even) return std::ceil(items / sm_count) * longest;
-    return std::max(longest, all / sm_count + longest / 2);
-  };
-  double best = cost(static_cast<double>(units * nblk), most * t_it + t_cta, units * (total * t_it + nblk * t_cta), least == most);
-  int best_parts = 1;
-  for (int parts = 2; parts <= 8 && parts <= most; ++parts) {
-    const int64_t len = (most + parts - 1) / parts;
-    int64_t items = 0;
-    for (int i = 0; i < nblk; ++i) items += std::max<int64_t>(1, (n[i] + len - 1) / len);
-    const double c = cost(static_cast<double>(units * items), len * t_it + t_cta, units * (total * t_it + items * t_cta), true) +
-                     base_cost + part_cost * parts;
-    if (c < 0.95 * best) {
-      best = c;
-      best_parts = parts;
-    }
-  }
-  if (best_parts == 1) return;
-  const int64_t len = (most + best_parts - 1) / best_parts;
-  out->start[0] = 0;
-  for (int i = 0; i < nblk; ++i) {
-    const int64_t parts = std::max<int64_t>(1, (n[i] + len - 1) / len);
-    out->max_parts = std::max<int>(out->max_parts, static_cast<int>(parts));
-    out->start[i + 1] = static_cast<uint16_t>(out->start[i] + parts);
-  }
-  out->items_per_head = out->start[nblk];
-  out->part_elems = dkv;
 }
 
 // A dQ-only call for dense tensors has a kernel of its own up to head dim 128 and needs no accumulator.
@@ -852,7 +672,7 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   BwdSplit split;
   plan_bwd_split(a, opt.share_key_blocks != 0, rt->sm_count, &split);
   const int64_t before = bwd_dq_bytes(a);
-  if (split.items_per_head > 0 && a->dq_accum != nullptr && a->dq_accum_bytes >= before + split.bytes()) {
+  if (split.fits(a->dq_accum, a->dq_accum_bytes, before)) {
     p.dk_part = reinterpret_cast<float*>(static_cast<char*>(a->dq_accum) + before);
     p.part_stride = (split.part_elems * 4 + 255) / 256 * 64;
     p.dv_part = p.dk_part + split.max_parts * p.part_stride;

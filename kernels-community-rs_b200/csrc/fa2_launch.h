@@ -20,7 +20,6 @@ cudaError_t launch_fwd_wide(const FwdParams& p, int head_dim, bool bf16, cudaStr
 // Dense forward with at most kDecodeMaxRows query rows per kv head, head_dim a multiple of 8 up to 256; `grid` CTAs
 // share the tile list evenly. The workspace behind p.partials and p.flags holds 2 * grid partial results of
 // 16 * decode_row_tiles(rows) rows x (D + 2) floats (D: head_dim rounded up to 64) and as many 8-byte flags.
-int decode_row_tiles(int rows);
 cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, cudaStream_t stream);
 
 // dQ / dK / dV for head_dim a multiple of 8 up to 128; the fp32 dQ accumulator behind p.tm_dqa (and the turn

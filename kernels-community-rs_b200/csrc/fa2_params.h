@@ -60,6 +60,7 @@ __host__ __device__ constexpr int64_t stream_slot_floats(int d) { return 256 * (
 // Forward for few query rows (fwd_decode_sm100.cu). A unit is one (batch, kv head): its rows are the query rows of all
 // the group's heads, row r = query r / group, head r % group.
 constexpr int kDecodeMaxRows = 64;
+constexpr int decode_row_tiles(int rows) { return rows <= 16 ? 1 : rows <= 32 ? 2 : 4; }  // 16-row tiles of a unit's kernel
 struct DecodeParams {
   CUtensorMap tm_k, tm_v;              // box (64, 1, 128, 1)
   const void* q_ptr;

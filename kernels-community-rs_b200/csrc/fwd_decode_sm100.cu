@@ -586,8 +586,6 @@ cudaError_t pick_dim(const DecodeParams& p, int grid, cudaStream_t stream) {
 
 }  // namespace
 
-int decode_row_tiles(int rows) { return rows <= 16 ? 1 : rows <= 32 ? 2 : 4; }
-
 cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, cudaStream_t stream) {
   if (p.rows <= 0 || p.rows > kDecodeMaxRows || p.head_dim <= 0 || p.head_dim > 256 || grid <= 0) return cudaErrorInvalidValue;
   return bf16 ? pick_dim<true>(p, grid, stream) : pick_dim<false>(p, grid, stream);
