@@ -42,6 +42,46 @@ struct DecodePlan {
   bool split = false;            // some unit is shared by CTAs (needs the workspace)
   int64_t flag_bytes = 0, workspace_bytes = 0;
 };
+
+// Is the few-row kernel the faster one for a call that it can take? Its consumers do mma.sync on 16, 32 or 64 rows, so a
+// key tile costs it more the more rows there are, and a unit's end (parts of eight warps become one) costs it more than
+// the general kernel's; it wins where the general kernels read K and V once per query head of a group, or leave SMs idle.
+// Both times are estimated in us: a launch, then per CTA its units and its key tiles, or K and V at the memory's rate, then
+// the merge of parts. Constants fitted to 5200 measured calls (1 to 64 rows, groups of 1 to 64, 1 to 1000 units, 64 to 16384
+// keys, D 64 to 256, both ways each): median error 3-9 %, hence the margin. With the rule 27 of these calls are more than 5 %
+// slower than the other way (up to 1.3 times, single heads' worth of work that the shared tiles finish sooner), without it
+// 1354 (up to 2.6 times): B64 H8 Sq 64 Sk 64 D128 35 us against 17, B5 H8 Sq 64 Sk 384 D256 25 against 13.
+inline bool few_rows_win(const fa2_fwd_args* a, const DecodePlan& d, int64_t keys, int64_t sms) {
+  struct Cost { double launch, unit, tile, merge; };
+  static constexpr Cost kFew[4][3] = {{{4.5, 1.85, 0.62, 2.9}, {3.9, 2.4, 0.87, 4.7}, {3.4, 3.4, 1.42, 6.3}},
+                                      {{3.65, 2.7, 0.94, 3.9}, {3.2, 4.0, 1.52, 5.9}, {3.0, 6.0, 2.1, 9.4}},
+                                      {{3.1, 3.85, 1.33, 4.2}, {2.5, 5.7, 2.27, 7.45}, {2.4, 8.95, 3.0, 12.4}},
+                                      {{3.25, 4.5, 1.69, 3.6}, {2.7, 6.8, 2.73, 8.4}, {1.2, 11.3, 4.27, 16.2}}};
+  static constexpr Cost kGeneral[4] = {{6.4, 1.2, 1.16, 6.1}, {6.75, 1.17, 1.28, 8.55}, {3.0, 3.75, 1.76, 0}, {2.6, 4.3, 1.8, 0}};
+  const int atoms = (a->head_dim - 1) / 64, row_tiles = decode_row_tiles(d.rows);
+  const Cost& f = kFew[atoms][row_tiles == 4 ? 2 : row_tiles - 1];
+  const Cost& g = kGeneral[atoms];
+  const double units = static_cast<double>(a->batch) * a->heads_k, heads = static_cast<double>(a->batch) * a->heads;
+  const double memory = units * keys * a->head_dim * 4 / 5.9e6;
+  // the longest share: its tiles, and the units that it ends in
+  double tiles, ends;
+  if (d.split) {
+    tiles = std::ceil(units * d.tiles / d.grid);
+    ends = units <= sms ? 1 : units / d.grid + 1;
+  } else {
+    ends = std::ceil(units / d.grid);
+    tiles = ends * d.tiles;
+  }
+  const double few = f.launch + std::max(ends * f.unit + tiles * f.tile, memory) + (d.split ? f.merge : 0);
+  // One work tile per head; head dims up to 128 may share it between CTAs (plan_stream).
+  const double blocks = a->head_dim <= 128 ? d.tiles : (keys + 63) / 64 / 2.0;
+  double general = std::ceil(heads / sms) * (g.unit + blocks * g.tile);
+  const double shares = std::min<double>(sms, std::floor(heads * d.tiles / 3));
+  if (a->head_dim <= 128 && heads <= sms && shares >= 2)
+    general = std::min(general, heads * d.tiles / shares * g.tile + (heads / shares + 1) * g.unit + g.merge);
+  return few < 0.95 * (g.launch + std::max(general, memory));
+}
+
 inline DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
   DecodePlan d;
   const int64_t rows = static_cast<int64_t>(a->seqlen_q) * (a->heads / a->heads_k);
@@ -70,6 +110,7 @@ inline DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
     d.grid = sm_count;
   }
   d.split = d.grid != d.whole_grid || (units > sms && d.grid == sm_count && units % sms != 0);
+  if (!few_rows_win(a, d, hi - lo, sms)) return DecodePlan{};
   if (d.split) {
     const int64_t dim = (a->head_dim + 63) / 64 * 64;
     d.flag_bytes = (2 * static_cast<int64_t>(d.grid) * 8 + 255) / 256 * 256;

@@ -19,6 +19,9 @@ int bwd_shares(const fa2_bwd_args* a, int sms, uint64_t address, int64_t short_b
   if (s.items_per_head == 0) return -1;
   return s.fits(reinterpret_cast<const void*>(address), 512 + s.bytes() - short_by, 512);
 }
+// query rows that the few-row kernel takes at a time (0: it does not take the call)
+int few_rows(const fa2_fwd_args* a, int sms) { return fa2::decode_plan(a, sms).rows; }
+int64_t few_rows_workspace(const fa2_fwd_args* a, int sms) { return fa2::decode_plan(a, sms).workspace_bytes; }
 }
 '''
 
@@ -29,7 +32,16 @@ def plans(tmp_path_factory):
     (d / "shim.cc").write_text(SHIM)
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{ROOT / 'kernels-community-rs_b200' / 'csrc'}",
                     "-I/usr/local/cuda/include", str(d / "shim.cc"), "-o", str(d / "shim.so")], check=True)
-    return ctypes.CDLL(str(d / "shim.so"))
+    lib = ctypes.CDLL(str(d / "shim.so"))
+    lib.few_rows_workspace.restype = ctypes.c_int64
+    return lib
+
+
+def _fwd_args(b, h, hk, sq, sk, d, **kw):
+    from flash_attn2_b200 import _cabi
+
+    return _cabi.FwdArgs(**{**dict(batch=b, heads=h, heads_k=hk, seqlen_q=sq, seqlen_k=sk, head_dim=d, window_left=-1,
+                                   window_right=-1), **kw})
 
 
 def _bwd_args(b, h, hk, sq, sk, d, which=3):
@@ -47,3 +59,22 @@ def test_key_blocks_are_shared_in_an_aligned_workspace_only(plans, which, offset
     assert plans.bwd_shares(ctypes.byref(args), SMS, ctypes.c_uint64((1 << 40) + offset), ctypes.c_int64(0)) == shares
     assert plans.bwd_shares(ctypes.byref(args), SMS, ctypes.c_uint64((1 << 40) + offset), ctypes.c_int64(1)) == 0
     assert plans.bwd_shares(ctypes.byref(args), SMS, ctypes.c_uint64(0), ctypes.c_int64(0)) == 0
+
+
+# Shapes (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim) timed both ways; us general, few-row kernel.
+SLOWER = [((64, 8, 8, 64, 64, 128), (17, 35)), ((64, 8, 8, 33, 384, 128), (29, 56)), ((64, 8, 8, 64, 1024, 256), (103, 176)),
+          ((5, 8, 8, 64, 384, 256), (13, 25)), ((1, 74, 74, 48, 384, 192), (13, 21)), ((64, 8, 8, 24, 64, 128), (17, 25)),
+          ((64, 8, 8, 33, 384, 64), (25, 33))]
+FASTER = [((1, 32, 8, 1, 8192, 128), (86, 16)), ((32, 32, 8, 1, 4093, 128), (316, 91)), ((5, 8, 8, 1, 4096, 128), (33, 19)),
+          ((2, 64, 8, 8, 4096, 128), (49, 34)), ((64, 8, 8, 1, 2048, 64), (87, 68)), ((5, 64, 8, 8, 1024, 256), (58, 43)),
+          ((2, 8, 8, 32, 4096, 192), (62, 29))]
+
+
+@pytest.mark.parametrize("shape,us", SLOWER + FASTER, ids=[str(s) for s, _ in SLOWER + FASTER])
+def test_the_few_row_kernel_takes_what_it_is_faster_for(plans, shape, us):
+    b, h, hk, sq, sk, d = shape
+    taken = plans.few_rows(ctypes.byref(_fwd_args(*shape)), SMS)
+    assert taken == (sq * h // hk if us[1] < us[0] else 0)
+    # a window leaves fewer key tiles; a mask that hides every key is not for it
+    assert plans.few_rows(ctypes.byref(_fwd_args(b, h, hk, sq, 128, d, causal=1, window_left=3)), SMS) in (0, sq * h // hk)
+    assert plans.few_rows(ctypes.byref(_fwd_args(b, h, hk, 65, sk, d)), SMS) == 0
