@@ -161,16 +161,20 @@ inline void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
   const int64_t units = total * heads;
   if (units > INT32_MAX / 2) return;
   // Costs in cycles: a key block, a tile's start and end, a part's way to memory, and the merge (a launch, and the parts
-  // read back); at least three key blocks per CTA. With these a call that is shared is faster or equal from 4 tiles
-  // (H4 Sq 128 Sk 1024 D64: 17.0 -> 16.5 us) to 128 (H8 S4096: 66.7 -> 65.6).
-  const double t_blk = 3300, t_tile = 6000, t_part = 4000, t_merge = 7000;
+  // written and read back, which at D128 hits memory and not the L2); at least three key blocks per CTA. Checked on 1384
+  // calls timed with and without sharing (2 to 148 tiles, Sq 65 to 4000, Sk 384 to 9000, masks): of the 231 that D64
+  // shares none is slower for it, of the 180 that D128 shares two are by more than 2 % (3 %); the best are 5 times as
+  // fast. H4 Sq 128 Sk 9000 D64 94 -> 23 us, H20 Sq 512 Sk 4096 D128 66 -> 46. With the constants of D64 26 more calls of D128
+  // were shared, among them H12 Sq 2000 Sk 2048 causal (39 -> 45) and H50 Sq 512 Sk 4096 causal (70 -> 79).
+  const bool d128 = a->head_dim > 64;
+  const double t_blk = d128 && a->seqlen_q <= 128 ? 2150 : 3300, t_tile = 6000, t_part = 4000, t_merge = 7000;
+  const double part_rate = d128 ? 1400 : 3000;  // bytes a cycle
   const int64_t grid = std::min<int64_t>(sm_count, units / 3);
   if (grid < 2) return;
   const double whole = longest * t_blk + t_tile;
-  const int64_t dim = a->head_dim > 64 ? 128 : 64;
-  const int64_t bytes = 2 * grid * stream_slot_floats(static_cast<int>(dim)) * 4;
+  const int64_t bytes = 2 * grid * stream_slot_floats(d128 ? 128 : 64) * 4;
   const double shared = static_cast<double>(units) / grid * t_blk + (static_cast<double>(tiles) / grid + 1) * t_tile + t_part +
-                        t_merge + static_cast<double>(std::min<int64_t>(grid, tiles) + grid) / (2.0 * grid) * bytes / 3000;
+                        t_merge + static_cast<double>(std::min<int64_t>(grid, tiles) + grid) / (2.0 * grid) * bytes / part_rate;
   if (shared > 0.92 * whole) return;
   out->grid = static_cast<int>(grid);
   out->workspace_bytes = (bytes + 255) / 256 * 256;

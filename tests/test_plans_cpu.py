@@ -21,6 +21,11 @@ int bwd_shares(const fa2_bwd_args* a, int sms, uint64_t address, int64_t short_b
 }
 // query rows that the few-row kernel takes at a time (0: it does not take the call)
 int few_rows(const fa2_fwd_args* a, int sms) { return fa2::decode_plan(a, sms).rows; }
+int shared_tiles(const fa2_fwd_args* a, int sms) {  // CTAs that share the call's work tiles, 0: none are shared
+  fa2::StreamPlan p;
+  fa2::plan_stream(a, sms, &p);
+  return p.grid;
+}
 int64_t few_rows_workspace(const fa2_fwd_args* a, int sms) { return fa2::decode_plan(a, sms).workspace_bytes; }
 }
 '''
@@ -78,3 +83,16 @@ def test_the_few_row_kernel_takes_what_it_is_faster_for(plans, shape, us):
     # a window leaves fewer key tiles; a mask that hides every key is not for it
     assert plans.few_rows(ctypes.byref(_fwd_args(b, h, hk, sq, 128, d, causal=1, window_left=3)), SMS) in (0, sq * h // hk)
     assert plans.few_rows(ctypes.byref(_fwd_args(b, h, hk, 65, sk, d)), SMS) == 0
+
+
+# Shapes (heads, seqlen_q, seqlen_k, head_dim, causal) timed with and without sharing.
+NOT_SHARED = [(12, 2000, 2048, 128, 1), (12, 2000, 4096, 128, 0), (50, 512, 4096, 128, 1), (18, 1000, 2048, 128, 1),
+              (6, 4000, 4096, 128, 0), (9, 4000, 4096, 128, 1), (100, 65, 9000, 128, 0), (100, 128, 9000, 128, 0)]
+SHARED = [(4, 128, 9000, 64, 0), (4, 256, 9000, 128, 0), (20, 512, 4096, 128, 0), (40, 128, 9000, 128, 1), (74, 128, 2048, 64, 0)]
+
+
+@pytest.mark.parametrize("shape", NOT_SHARED + SHARED, ids=str)
+def test_tiles_are_shared_where_that_is_faster(plans, shape):
+    h, sq, sk, d, causal = shape
+    got = plans.shared_tiles(ctypes.byref(_fwd_args(1, h, h, sq, sk, d, causal=causal)), SMS)
+    assert (got > 0) == (shape in SHARED)
