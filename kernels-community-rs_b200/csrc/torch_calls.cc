@@ -29,6 +29,16 @@ Tensor empty(at::IntArrayRef shape, c10::ScalarType type, c10::Device dev) {
   return Tensor(at::detail::empty_cuda(shape, type, dev, std::nullopt));
 }
 
+// Scratch memory that a call can do without: undefined when there is none left (the call then takes more time, and sums
+// in another order).
+Tensor scratch(int64_t bytes, c10::Device dev) {
+  try {
+    return empty({bytes}, at::kByte, dev);
+  } catch (const c10::OutOfMemoryError&) {
+    return Tensor();
+  }
+}
+
 // The kernels address a tensor by TMA: 16-byte aligned base, unit last stride, outer strides multiples of 8 elements
 // (of dimensions longer than 1).
 bool addressable(const Tensor& t) {
@@ -145,8 +155,8 @@ void forward(const Tensor& q, const Tensor& k, const Tensor& v, const Options& o
   a.softcap = static_cast<float>(o.softcap);
   Tensor workspace;
   const int64_t need = fa2_fwd_workspace_bytes(&a);
-  if (need > 0) workspace = empty({need}, at::kByte, q.device());
-  check(fa2_fwd_with_workspace(&a, need > 0 ? workspace.data_ptr() : nullptr, need, c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
+  if (need > 0) workspace = scratch(need, q.device());
+  check(fa2_fwd_with_workspace(&a, workspace.defined() ? workspace.data_ptr() : nullptr, need, c10::cuda::getCurrentCUDAStream(q.device().index()).stream()));
 }
 
 struct Gradients {
@@ -208,7 +218,13 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
     a.dq_accum = nullptr;
     a.dq_accum_bytes = fa2_bwd_workspace_bytes_with_options(&a, &opt);
     if (a.dq_accum_bytes > 0) {
-      workspace = empty({a.dq_accum_bytes}, at::kByte, q.device());
+      // The parts of shared key blocks can be done without, but not in calls whose bits are to be the same every time.
+      if (!deterministic) workspace = scratch(a.dq_accum_bytes, q.device());
+      if (!workspace.defined()) {
+        opt.share_key_blocks = deterministic;
+        a.dq_accum_bytes = fa2_bwd_workspace_bytes_with_options(&a, &opt);
+        workspace = empty({a.dq_accum_bytes}, at::kByte, q.device());
+      }
       a.dq_accum = workspace.data_ptr();
     }
     check(fa2_bwd_with_options(&a, &opt, stream));

@@ -91,6 +91,17 @@ Tensor alloc(std::initializer_list<int64_t> shape, DLDataType dtype, DLDevice de
   return Tensor::FromEnvAlloc(TVMFFIEnvTensorAlloc, tvm::ffi::ShapeView(s.data(), s.size()), dtype, dev);
 }
 
+// Scratch memory that a call can do without: none when there is none left (the call then takes more time, and sums in
+// another order).
+Optional<Tensor> scratch(int64_t bytes, DLDevice dev) {
+  try {
+    return alloc({bytes / 4}, kF32, dev);
+  } catch (const tvm::ffi::Error& e) {
+    if (e.kind() != "MemoryError") throw;
+    return Optional<Tensor>();
+  }
+}
+
 void* stream_of(DLDevice dev) { return TVMFFIEnvGetStream(dev.device_type, dev.device_id); }
 
 bool is_contiguous(const Tensor& t) {
@@ -306,8 +317,8 @@ Any fwd_impl(const AnyView* args, int32_t n, bool lse_only) {
   a.softcap = static_cast<float>(softcap);
   Optional<Tensor> workspace;
   const int64_t need = fa2_fwd_workspace_bytes(&a);
-  if (need > 0) workspace = alloc({need / 4}, kF32, dev);
-  check(fa2_fwd_with_workspace(&a, need > 0 ? workspace.value().data_ptr() : nullptr, need, stream_of(dev)));
+  if (need > 0) workspace = scratch(need, dev);
+  check(fa2_fwd_with_workspace(&a, workspace.has_value() ? workspace.value().data_ptr() : nullptr, need, stream_of(dev)));
   if (copy_out) {
     const Tensor& o = supplied.value();
     const int64_t shape4[4] = {b, sq, h, d};
@@ -440,9 +451,15 @@ Any bwd_impl(const AnyView* args, int32_t n, int which) {
     a.dv = dv.value().data_ptr();
   }
   Optional<Tensor> accum;
-  const int64_t ws = fa2_bwd_workspace_bytes_with_options(&a, &opt);
+  int64_t ws = fa2_bwd_workspace_bytes_with_options(&a, &opt);
   if (ws > 0) {
-    accum = alloc({ws / 4}, kF32, dev);
+    // bwd_dq and bwd_dkv are the pair whose bits are the same every time: there the parts of shared key blocks stay.
+    if (which == 3) accum = scratch(ws, dev);
+    if (!accum.has_value()) {
+      opt.share_key_blocks = which != 3;
+      ws = fa2_bwd_workspace_bytes_with_options(&a, &opt);
+      accum = alloc({ws / 4}, kF32, dev);
+    }
     a.dq_accum = accum.value().data_ptr();
     a.dq_accum_bytes = ws;
   }

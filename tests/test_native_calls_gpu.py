@@ -150,3 +150,63 @@ def test_other_threads_run_while_a_call_waits(call):
     torch.cuda.synchronize()
     assert blocked > 0.2, "the queue never filled: nothing was tested"
     assert max(gaps) < 0.1
+
+
+class _LittleMemory:
+    """Within it the allocator has nothing left but pieces of these sizes."""
+
+    def __init__(self, *spare):
+        self.spare = spare
+
+    def __enter__(self):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
+        keep, self.held = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in self.spare], []
+        for size in (1 << 21, 1 << 18, 1 << 12, 1 << 9):
+            try:
+                while True:
+                    self.held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                pass
+        del keep
+
+    def __exit__(self, *exc):
+        self.held.clear()
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+@pytest.mark.parametrize("shape", [(1, 32, 8, 1, 8192), (1, 4, 4, 200, 8192)], ids=["few-rows", "shared-tiles"])
+@pytest.mark.parametrize("route", ["native", "operator"])
+def test_forward_without_room_for_scratch(shape, route):
+    """A call whose outputs fit runs; the scratch memory is for speed."""
+    import flash_attn2_b200 as fa2
+
+    b, h, hk, sq, sk = shape
+    q, k, v = [t.cuda() for t in make_qkv(33, b, h, hk, sq, sk, 128, torch.bfloat16)]
+    out = torch.empty_like(q)
+    call = (lambda: fa2.fwd(q, k, v)) if route == "native" else (lambda: fa2.fwd(q, k, v, out=out))
+    want = [t.clone() for t in call()[:2]]
+    with _LittleMemory(1 << 20):
+        with pytest.raises(torch.OutOfMemoryError):
+            torch.empty(3 << 20, dtype=torch.uint8, device="cuda")
+        got = call()[:2]
+        torch.cuda.synchronize()
+    torch.testing.assert_close(got[0], want[0], atol=1e-2, rtol=1e-2)
+    torch.testing.assert_close(got[1], want[1], atol=1e-4, rtol=1e-4)
+
+
+def test_backward_without_room_for_parts():
+    """The accumulator of dQ fits, the parts of shared key blocks do not."""
+    import flash_attn2_b200 as fa2
+
+    q, k, v, do = [t.cuda() for t in make_qkv(34, 1, 1, 1, 4096, 2048, 64, torch.bfloat16, with_do=True)]
+    out, lse = fa2.fwd(q, k, v)[:2]
+    want = [t.clone() for t in fa2.bwd(do, q, k, v, out, lse)]
+    # dQ, dK, dV and delta take small pieces, the accumulator a little more than 1 MB, the parts 8 MB.
+    with _LittleMemory(1 << 19, 1 << 19, 1 << 19, 5 << 20):
+        got = fa2.bwd(do, q, k, v, out, lse)
+        torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        torch.testing.assert_close(g, w, atol=2e-2, rtol=2e-2)
