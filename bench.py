@@ -163,7 +163,7 @@ def run_long_context(ops, dev, rank, world, timed, steps):
     state = {}
 
     def fwd():
-        state["o"], state["lse"] = ops.fwd(q, k, v, causal=True)
+        state["o"], state["lse"] = ops.fwd(q, k, v, causal=True, split=False)  # the bits of the unsharded run
 
     def bwd():
         delta = ops.bwd_preprocess(do, state["o"])
@@ -186,7 +186,7 @@ def run_long_context(ops, dev, rank, world, timed, steps):
     else:
         gathered = {n: t for n, (t, _) in shards.items()}
     if rank == 0:
-        o, lse = ops.fwd(*full[:3], causal=True)
+        o, lse = ops.fwd(*full[:3], causal=True, split=False)
         delta = ops.bwd_preprocess(full[3], o)
         ref = dict(zip(("dq", "dk", "dv"), ops.bwd(*full, lse, delta, causal=True)), out=o, lse=lse)
         verify = {}

@@ -121,8 +121,9 @@ inline DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
 
 // ---- dense forward with few work tiles (fwd_sm100.cu, SHARED): a work tile is 256 query rows of a head, one CTA at a
 // time works on it, and with fewer tiles than SMs some have nothing to do. Calls with more tiles are not shared, also
-// where a last, nearly empty round would gain (H32 Sq 1500 Sk 16384, 192 tiles: 454 -> 392 us): there the bits of a head do
-// not depend on how many other heads the call has, which a long-context run that is sharded by heads relies on.
+// where a last, nearly empty round would gain (H32 Sq 1500 Sk 16384, 192 tiles: 454 -> 392 us): sharing makes the bits of a
+// head depend on how many tiles the call has. A caller that needs them independent for any size leaves the scratch memory
+// out (fa2_fwd).
 struct StreamPlan {
   int grid = 0;  // 0: one tile per CTA at a time
   int64_t workspace_bytes = 0;

@@ -49,8 +49,12 @@ def _check_last_stride(name, t):
 
 
 def fwd(q, k, v, *, out=None, alibi_slopes=None, softmax_scale=None, causal=False, window_left=-1,
-        window_right=-1, softcap=0.0):
-    """Dense forward: returns (out [B,Sq,H,D], lse fp32 [B,H,Sq])."""
+        window_right=-1, softcap=0.0, split=True):
+    """Dense forward: returns (out [B,Sq,H,D], lse fp32 [B,H,Sq]).
+
+    `split`: a call that does not fill the GPU may be split along the keys, by a rule on the sizes of the whole call.
+    Without it the bits of a head do not depend on the batch and the other heads: a run sharded by batch or heads
+    gives the bits of the unsharded one, for any number of shards."""
     _require_cuda(q, k, v, out, alibi_slopes)
     lib = _cabi.load()
     if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
@@ -91,9 +95,12 @@ def fwd(q, k, v, *, out=None, alibi_slopes=None, softmax_scale=None, causal=Fals
     a.window_left, a.window_right = int(window_left), int(window_right)
     a.softcap = float(softcap)
     with torch.cuda.device(q.device):
-        need = lib.fa2_fwd_workspace_bytes(C.byref(a))
-        workspace = _alloc((need // 4,), torch.float32, q.device) if need > 0 else None
-        _cabi.check(lib.fa2_fwd_with_workspace(C.byref(a), None if workspace is None else workspace.data_ptr(), need, _stream(q)))
+        if split:
+            need = lib.fa2_fwd_workspace_bytes(C.byref(a))
+            workspace = _alloc((need // 4,), torch.float32, q.device) if need > 0 else None
+            _cabi.check(lib.fa2_fwd_with_workspace(C.byref(a), None if workspace is None else workspace.data_ptr(), need, _stream(q)))
+        else:
+            _cabi.check(lib.fa2_fwd(C.byref(a), _stream(q)))
     return out, lse
 
 
@@ -178,10 +185,12 @@ def bwd_preprocess(dout, out, *, cu_seqlens_q=None, max_seqlen_q=None):
 
 def bwd(q, k, v, dout, lse, delta, *, softmax_scale=None, causal=False, window_left=-1, window_right=-1,
         which=3, cu_seqlens_q=None, cu_seqlens_k=None, max_seqlen_q=None, max_seqlen_k=None, dq_accum=None,
-        kernel_events=None, alibi_slopes=None, softcap=0.0):
+        kernel_events=None, alibi_slopes=None, softcap=0.0, share_key_blocks=False):
     """dQ, dK, dV (input dtype, contiguous). `which`: bit 0 = dQ, bit 1 = dK and dV.
 
-    `kernel_events`: optional pair of torch.cuda.Event recorded around the main kernel only."""
+    `kernel_events`: optional pair of torch.cuda.Event recorded around the main kernel only.
+    `share_key_blocks`: with few key blocks several CTAs share one, by a rule on the sizes of the whole call. Without it
+    the bits of dK and dV of a head do not depend on the batch and the other heads."""
     _require_cuda(q, k, v, dout, lse, delta)
     lib = _cabi.load()
     if k.dtype != q.dtype or v.dtype != q.dtype or dout.dtype != q.dtype:
@@ -235,11 +244,12 @@ def bwd(q, k, v, dout, lse, delta, *, softmax_scale=None, causal=False, window_l
             raise ValueError("alibi_slopes must be [H] or [B, H]")
         a.alibi_slopes = alibi_slopes.data_ptr()
     a.softcap = float(softcap)
-    need = lib.fa2_bwd_workspace_bytes(C.byref(a))
+    opt = _cabi.BwdOptions(size=C.sizeof(_cabi.BwdOptions), share_key_blocks=int(share_key_blocks))
+    need = lib.fa2_bwd_workspace_bytes_with_options(C.byref(a), C.byref(opt))
     if need > 0:
         if dq_accum is None:
             dq_accum = _alloc((need // 4,), torch.float32, q.device)
         a.dq_accum, a.dq_accum_bytes = dq_accum.data_ptr(), dq_accum.numel() * 4
     with torch.cuda.device(q.device):
-        _cabi.check(lib.fa2_bwd(C.byref(a), _stream(q)))
+        _cabi.check(lib.fa2_bwd_with_options(C.byref(a), C.byref(opt), _stream(q)))
     return dq, dk, dv

@@ -20,6 +20,34 @@ def _inputs():
     return [torch.randn(1, S, H, D, generator=g).to(torch.bfloat16) for _ in range(4)]  # q, k, v, dO
 
 
+# (heads, heads_k, seqlen_q, seqlen_k, head_dim) and the shard's kv heads: few rows, few tiles, few key blocks, the wide kernels
+SHARDS = [((64, 16, 1, 5000, 128), slice(3, 4)), ((40, 40, 300, 3000, 128), slice(7, 9)), ((32, 8, 600, 600, 64), slice(2, 3)),
+          ((16, 16, 200, 900, 192), slice(15, 16)), ((8, 8, 33, 2000, 256), slice(0, 2))]
+
+
+@pytest.mark.parametrize("shape,shard", SHARDS, ids=[str(s) for s, _ in SHARDS])
+def test_bits_of_a_head_do_not_depend_on_the_other_heads(shape, shard):
+    """With `split=False`, and in the backward without shared key blocks, for any shard."""
+    from flash_attn2_b200 import cabi_ops as ops
+    from tests._cases import make_qkv
+
+    h, hk, sq, sk, d = shape
+    q, k, v, do = [t.cuda() for t in make_qkv(41, 2, h, hk, sq, sk, d, torch.bfloat16, with_do=True)]
+    heads = slice(shard.start * (h // hk), shard.stop * (h // hk))
+    part = [q[1:, :, heads], k[1:, :, shard], v[1:, :, shard], do[1:, :, heads]]
+    out, lse = ops.fwd(q, k, v, causal=True, split=False)
+    o, l = ops.fwd(*part[:3], causal=True, split=False)
+    assert torch.equal(o, out[1:, :, heads]) and torch.equal(l, lse[1:, heads])
+    delta, dl = ops.bwd_preprocess(do, out), ops.bwd_preprocess(part[3], o)
+    dk, dv = ops.bwd(q, k, v, do, lse, delta, causal=True, which=2)[1:]
+    dk1, dv1 = ops.bwd(*part, l, dl, causal=True, which=2)[1:]
+    assert torch.equal(dk1, dk[1:, :, shard]) and torch.equal(dv1, dv[1:, :, shard])
+    if d <= 128:
+        dq = ops.bwd(q, k, v, do, lse, delta, causal=True, which=1)[0]
+        assert torch.equal(ops.bwd(*part, l, dl, causal=True, which=1)[0], dq[1:, :, heads])
+    assert ops.device_status() == 0
+
+
 def test_long_context_forward_backward_and_head_shards():
     from flash_attn2_b200 import cabi_ops as ops
     from flash_attn2_b200.sharding import shard_heads
