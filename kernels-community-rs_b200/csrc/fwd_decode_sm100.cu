@@ -456,7 +456,6 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
           __stcg(st + Cfg::kRows + r0, ls0);
           __stcg(st + Cfg::kRows + r1, ls1);
         }
-        __threadfence();
         // CTAs whose shares touch this unit: the owners of its first and its last tile.
         const int64_t g64 = gridDim.x;
         const int64_t first_tile = static_cast<int64_t>(u) * p.tiles_per_unit;
@@ -470,7 +469,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
           // last to set one does (store, fence, load); two may, and then both write the same bits. A counter
           // in place of the flags would need clearing, or a compare-and-swap that 19 CTAs queue up for (0.5 us each).
           volatile unsigned long long* flags = p.flags;
-          if (lane == 0) flags[part_index(blockIdx.x)] = p.launch_tag;
+          // All warps' stores come before the barrier; this thread's fence behind it makes them the flag's predecessors.
+          if (lane == 0) {
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            flags[part_index(blockIdx.x)] = p.launch_tag;
+          }
           __syncwarp();
           asm volatile("fence.sc.gpu;" ::: "memory");
           bool all = true;
