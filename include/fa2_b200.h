@@ -105,9 +105,9 @@ FA2_API int fa2_bwd_preprocess(const fa2_bwd_preprocess_args* args, void* stream
  * converted to the 16-bit dQ at the end. `which` selects outputs: bit 0 = dQ, bit 1 = dK and dV.
  * A dense dQ-only call (which = 1, the deterministic bwd_dq of the reference) up to head dim 128 has a
  * kernel of its own that sums dQ in key order, so dQ is bit-reproducible; it needs no workspace. Elsewhere
- * the workspace is the accumulator (B*Sq*H*D floats, rounded up to 256 bytes) followed by one 32-bit
- * turn counter per 32 query rows of every (batch, head): with them a packed dQ-only call adds the key
- * blocks' contributions in a fixed order; a workspace that only holds the accumulator is accepted too
+ * the workspace is the accumulator (B*Sq*H*D floats, rounded up to 256 bytes), for a packed dQ-only call up to
+ * head dim 128 followed by one 32-bit turn counter per 32 query rows of every (batch, head): with them it adds the
+ * key blocks' contributions in a fixed order; a workspace that only holds the accumulator is accepted too
  * (arrival order). dK and dV never use atomics and are always bit-reproducible. Head dims above 128 always add dQ in
  * arrival order. A dQ-only call (which = 1) may pass dk = dv = NULL, a dK/dV-only call dq = dq_accum = NULL.
  * Replaces backward_component + the `backward` and `backward_kv` kernels

@@ -209,7 +209,9 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   const KvTile ti = get_kv_tile(p, blockIdx.x);
   if (!ti.valid) return;
   const bool want_dq = (p.which & 1) != 0;
-  const bool want_dkv = (p.which & 2) != 0;  // a dQ-only call skips the dV and dK GEMMs (their commits still hand the stages back)
+  // A dQ-only call skips the dV and dK GEMMs (their commits still hand the stages back). Only packed ones come here: dense
+  // ones have bwd_dq_sm100.cu.
+  const bool want_dkv = !PACKED || (p.which & 2) != 0;
 
   // Descriptor fetches start first: they are the head of the latency chain of the first loads.
   if (warp == 2 && lane == 0) {
@@ -745,7 +747,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         static_assert(kHalf * Cfg::kPieceBytes <= Cfg::kTileBytes, "half of the dQ tile fits one stage");
         uint8_t* stage_do = s_do + st * Cfg::kTileBytes + (warp & 3) * (kHalf * kWarpPiece);
         int* turn = nullptr;
-        if (p.dq_turn != nullptr) {
+        if (PACKED && p.dq_turn != nullptr) {
           // Ordered mode: the key blocks that add into these rows take their turns in descending order,
           // which is the order in which they get there under a causal or sliding-window mask (a higher key
           // block starts at a later query block). This block's turn is the number of higher key blocks

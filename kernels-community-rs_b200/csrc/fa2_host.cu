@@ -435,7 +435,9 @@ int64_t bwd_accum_bytes(const fa2_bwd_args* a) {
 int64_t bwd_dq_bytes(const fa2_bwd_args* a);
 
 // One counter per (batch, head, 128-row query block, 32-row slab of a drain warp).
+// Packed dQ-only calls up to head dim 128 use them.
 int64_t bwd_turn_counters(const fa2_bwd_args* a) {
+  if (a->which != 1 || a->cu_seqlens_q == nullptr || a->head_dim > 128) return 0;
   return static_cast<int64_t>(a->batch) * a->heads * ((a->seqlen_q + 127) / 128) * 4;
 }
 
@@ -506,7 +508,7 @@ int bwd_dq(const fa2_bwd_args* a, const fa2_bwd_options& opt, Runtime* rt, cudaS
 
 int64_t bwd_dq_bytes(const fa2_bwd_args* a) {
   if ((a->which & 1) == 0 || dq_kernel_takes(a)) return 0;
-  // The fp32 accumulator, then (used by dQ-only calls) the turn counters of the ordered accumulation.
+  // The fp32 accumulator, then the turn counters of the ordered accumulation where there is one.
   return (bwd_accum_bytes(a) + bwd_turn_counters(a) * 4 + 255) / 256 * 256;
 }
 
@@ -642,7 +644,7 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   // registers in key order) accumulates in a fixed key-block order when the workspace holds the
   // turn counters; otherwise, and in the combined call, the adds land in arrival order.
   const int64_t acc_bytes = bwd_accum_bytes(a), n_turn = bwd_turn_counters(a);
-  const bool ordered = !wide && a->which == 1 && a->dq_accum_bytes >= acc_bytes + n_turn * 4;
+  const bool ordered = n_turn > 0 && a->dq_accum_bytes >= acc_bytes + n_turn * 4;
   p.dq_turn = ordered ? reinterpret_cast<int*>(static_cast<char*>(a->dq_accum) + acc_bytes) : nullptr;
   p.num_mblk_q = (a->seqlen_q + 127) / 128;
   // With `out` the delta preprocess is part of this call and clears the accumulator on its way.

@@ -126,3 +126,22 @@ def test_backward_options_of_an_unknown_size_are_refused(built_libs):
     opt = _cabi.BwdOptions(size=ctypes.sizeof(_cabi.BwdOptions) + 8)
     assert lib.fa2_bwd_with_options(ctypes.byref(_cabi.BwdArgs()), ctypes.byref(opt), None) == -1
     assert b"size" in lib.fa2_last_error()
+
+
+def test_workspace_holds_turn_counters_only_where_they_are_used(built_libs):
+    """Behind the fp32 accumulator of dQ, for packed dQ-only calls up to head dim 128."""
+    from flash_attn2_b200 import _cabi
+
+    lib = _cabi.load()
+    shape = dict(batch=2, seqlen_q=256, seqlen_k=256, heads=4, heads_k=2, window_left=-1, window_right=-1)
+
+    def need(which, d, packed):
+        args = _cabi.BwdArgs(which=which, head_dim=d, **shape, **(dict(cu_seqlens_q=8, cu_seqlens_k=8, total_q=512, total_k=512)
+                                                                  if packed else {}))
+        return lib.fa2_bwd_workspace_bytes(ctypes.byref(args))
+
+    for d in (64, 128, 256):
+        accum = 2 * 256 * 4 * d * 4
+        assert need(3, d, False) == need(3, d, True) == accum and need(2, d, False) == need(2, d, True) == 0
+        assert need(1, d, False) == (0 if d <= 128 else accum)
+        assert need(1, d, True) == accum + (2 * 4 * 2 * 4 * 4 if d <= 128 else 0)

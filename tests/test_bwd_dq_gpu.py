@@ -76,3 +76,28 @@ def test_split_key_blocks(shape, opt, dtype, deterministic):
     again = fa2.bwd(doc, qc, kc, vc, out, lse, deterministic=deterministic, **args)
     assert torch.equal(again[1], got[1]) and torch.equal(again[2], got[2])
     assert fa2.cabi_ops.device_status() == 0
+
+
+@pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_packed_dq_alone_is_ordered(causal, head_dim):
+    """A packed dQ-only call adds the key blocks' contributions in a fixed order when the workspace holds the turn counters:
+    the same bits from every run, empty and ragged sequences and head groups included."""
+    from flash_attn2_b200 import cabi_ops as ops
+    from oracle.attention_oracle import varlen_backward
+
+    lengths = [300, 1, 0, 641, 128, 77]
+    g = torch.Generator().manual_seed(13)
+    total, cu = sum(lengths), torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32)
+    q, do = (torch.randn(total, 4, head_dim, generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(total, 2, head_dim, generator=g).bfloat16() for _ in range(2))
+    qc, kc, vc, doc, cc = (t.cuda() for t in (q, k, v, do, cu))
+    out, lse = ops.varlen_fwd(qc, kc, vc, cc, cc, 641, 641, causal=causal)
+    delta = ops.bwd_preprocess(doc, out, cu_seqlens_q=cc, max_seqlen_q=641)
+    runs = [ops.bwd(qc, kc, vc, doc, lse, delta, which=1, causal=causal, cu_seqlens_q=cc, cu_seqlens_k=cc, max_seqlen_q=641,
+                    max_seqlen_k=641)[0] for _ in range(4)]
+    assert ops.device_status() == 0
+    ref = varlen_backward(q, k, v, do, cu, cu, out=out.float().cpu(), lse=lse.cpu(), causal=causal)[0]
+    torch.testing.assert_close(runs[0].float().cpu(), ref, **BWD_TOL[torch.bfloat16])
+    for again in runs[1:]:
+        assert torch.equal(again, runs[0])
