@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
     mbar_init(dq_free, kBK);
     mbar_init(dkv_done, 1);
     mbar_init(stat_full, kBWCompute);
-    mbar_init(v_ready, kBWCompute);
+    mbar_init(v_ready, kBK);
     mbar_init(k_fixed, 1);
     mbar_fence_init();
   }
@@ -233,17 +233,18 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
     const uint32_t t_s = tmem + lane_addr + Cfg::kTmemS + wg * 32;
     const uint32_t t_dp = tmem + lane_addr + Cfg::kTmemDP + wg * 32;
     bool ok = true;
-    if (n_iter > 0) {
+    if (n_iter > 0 && wg == 0) {
       // V of this key row goes from global memory into TMEM as the 16-bit A operand of dP^T: column c holds the
-      // elements 2c and 2c + 1, which is the row's own memory layout; each warpgroup takes half of the row. Rows past
-      // the sequence and columns past the head dim are zero.
+      // elements 2c and 2c + 1, which is the row's own memory layout. Rows past the sequence and columns past the head
+      // dim are zero. One warpgroup does it: the 16-byte loads of a row's 128-byte lines rely on the L1, which has room for
+      // the lines of 128 rows beside this much shared memory, not for twice as many. With half a row per warpgroup a
+      // backward call with one query block (H148 Sq 64 Sk 1000 D256) took 221 us, now 199.
       const uint4* vrow = reinterpret_cast<const uint4*>(
           reinterpret_cast<const uint16_t*>(p.v_ptr) + ti.bq * p.v_batch_stride +
           static_cast<int64_t>(ti.k_row0 + kpos) * p.v_row_stride + ti.hk * p.v_head_stride);
       const int chunks = (kpos < ti.sk) ? p.head_dim / 8 : 0;
 #pragma unroll
-      for (int half_part = 0; half_part < 2; ++half_part) {
-        const int part = wg * 2 + half_part;
+      for (int part = 0; part < 4; ++part) {
         uint32_t vr[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
