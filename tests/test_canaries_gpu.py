@@ -77,3 +77,33 @@ def test_packed_outputs_stay_inside_their_buffers(d, monkeypatch):
             max_seqlen_k=max(lengths), causal=True)
     assert ops.device_status() == 0
     can.check()
+
+
+# Calls that use scratch memory: (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim). Few rows (a unit in parts, equal shares of
+# the whole list), shared tiles, shared key blocks; ragged everywhere.
+SCRATCH = [((1, 32, 8, 1, 8191, 128), "fwd"), ((19, 16, 8, 1, 2501, 64), "fwd"), ((2, 64, 8, 8, 4099, 128), "fwd"),
+           ((1, 8, 8, 33, 6001, 192), "fwd"), ((1, 3, 1, 290, 3333, 128), "fwd"), ((1, 40, 40, 150, 3001, 72), "fwd"),
+           ((1, 4, 1, 777, 777, 128), "bwd"), ((1, 1, 1, 2001, 2003, 64), "bwd"), ((2, 8, 2, 513, 515, 96), "bwd")]
+
+
+@pytest.mark.parametrize("shape,uses", SCRATCH, ids=[f"{s[1]}-b{s[0][0]}-h{s[0][1]}/{s[0][2]}-sq{s[0][3]}-sk{s[0][4]}-d{s[0][5]}" for s in SCRATCH])
+def test_scratch_memory_stays_inside_its_buffer(shape, uses, monkeypatch):
+    from flash_attn2_b200 import cabi_ops as ops
+    from tests._cases import make_qkv
+
+    b, h, hk, sq, sk, d = shape
+    q, k, v, do = [t.cuda() for t in make_qkv(23, b, h, hk, sq, sk, d, torch.bfloat16, with_do=True)]
+    can = Canaries()
+    monkeypatch.setattr(ops, "_alloc", can.alloc)
+    out, lse = ops.fwd(q, k, v, causal=True)
+    if uses == "fwd":
+        assert len(can.buffers) == 3, "out, LSE and the scratch memory"
+    if uses == "bwd":
+        delta = ops.bwd_preprocess(do, out)
+        for which in (2, 3):
+            before, accum = len(can.buffers), (q.numel() * 4 + 255) // 256 * 256 if which == 3 else 0
+            ops.bwd(q, k, v, do, lse, delta, causal=True, which=which, share_key_blocks=True)
+            workspace = can.buffers[before + 3]  # behind dQ, dK and dV
+            assert workspace.numel() * 4 - 8 * PAD > accum, "the case shares no key blocks"
+    assert ops.device_status() == 0
+    can.check()

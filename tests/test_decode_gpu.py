@@ -1,10 +1,13 @@
 """GPU parity of the forward for few query rows (at most 64 per kv head) against the CPU oracle: edges of the 16-row
 and 128-key tiles, shares that end inside a unit, masks, score transforms, every head-dim bucket, cache views."""
+import ctypes
+
 import pytest
 import torch
 
 from tests._cases import alibi_slopes, make_qkv
 from tests.test_fwd_gpu import _check
+from tests.test_plans_cpu import SMS, _fwd_args, plans  # noqa: F401 (a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +73,62 @@ def test_workspace_contents_do_not_matter_and_graph_replays():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+# Shapes that the few-row kernel takes, and whether parts of units are shared (units = batch x kv heads).
+ROUTED = [
+    ((40, 8, 4, 1, 3000, 64), {}, True),                                  # more units than SMs: equal shares of the whole list,
+    ((19, 16, 8, 4, 2500, 128), dict(causal=True), True),                 # each ending one unit and starting another
+    ((21, 16, 8, 2, 3300, 192), dict(causal=True), True),
+    ((20, 8, 8, 1, 2600, 256), dict(softcap=15.0), True),
+    ((19, 16, 8, 4, 4000, 128), dict(causal=True, window_left=3000, alibi=True), True),
+    ((1, 24, 1, 1, 3000, 128), {}, True),                                 # 17 to 32 rows
+    ((1, 4, 4, 17, 5000, 256), dict(causal=True), True),
+    ((1, 64, 1, 1, 5000, 64), {}, True),                                  # 33 to 64 rows, every head-dim bucket
+    ((2, 64, 8, 8, 4096, 128), dict(causal=True), True),
+    ((1, 8, 8, 33, 6000, 192), dict(causal=True, window_left=5000), True),
+    ((4, 128, 16, 8, 1030, 256), dict(causal=True), True),
+    ((3, 64, 2, 2, 260, 64), dict(causal=True), False),                   # whole units
+]
+
+
+@pytest.mark.parametrize("shape,opt,shared", ROUTED, ids=[str(c[0]) for c in ROUTED])
+def test_routed_shapes(shape, opt, shared, plans):
+    """The plan is the one that the case is about; then the comparison above."""
+    args = ctypes.byref(_fwd_args(*shape, **{k: int(v) for k, v in opt.items() if k in ("causal", "window_left")}))
+    assert plans.few_rows(args, SMS) == shape[1] // shape[2] * shape[3]
+    assert (plans.few_rows_workspace(args, SMS) > 0) == shared
+    test_few_query_rows(shape, opt, torch.bfloat16)
+
+
+def test_workspace_contents_are_irrelevant():
+    """One buffer for calls of different shapes, and after it was filled with anything: the same bits as from a buffer of
+    their own."""
+    import ctypes as C
+
+    from flash_attn2_b200 import _cabi
+
+    lib = _cabi.load()
+    buf = torch.zeros(16 << 20, dtype=torch.uint8, device="cuda")
+
+    def call(shape, prepare):
+        b, h, hk, sq, sk, d = shape
+        q, k, v = (t.cuda() for t in make_qkv(9, b, h, hk, sq, sk, d, torch.bfloat16))
+        out, lse = torch.empty_like(q), torch.empty(b, h, sq, device="cuda")
+        a = _fwd_args(*shape, causal=1, q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), out=out.data_ptr(), lse=lse.data_ptr(),
+                      dtype=_cabi.FA2_BF16, softmax_scale=d ** -0.5)
+        for name, t in (("q", q), ("k", k), ("v", v), ("o", out)):
+            setattr(a, name + "_stride", (C.c_int64 * 3)(*t.stride()[:3]))
+        need = lib.fa2_fwd_workspace_bytes(C.byref(a))
+        assert 0 < need <= buf.numel()
+        prepare(need)
+        _cabi.check(lib.fa2_fwd_with_workspace(C.byref(a), buf.data_ptr(), need, torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        return out, lse
+
+    shapes = [(1, 16, 4, 1, 5000, 128), (19, 16, 8, 1, 2500, 64), (1, 16, 4, 1, 3000, 128), (1, 2, 2, 200, 3000, 64)]
+    want = [call(s, lambda n: buf.zero_()) for s in shapes]
+    for prepare in (lambda n: None, lambda n: buf.fill_(0xFF), lambda n: buf[:n].random_(0, 256), lambda n: buf.fill_(1)):
+        for s, (out, lse) in zip(shapes, want):
+            o, l = call(s, prepare)
+            assert torch.equal(o, out) and torch.equal(l, lse)

@@ -6,7 +6,7 @@ import time
 import pytest
 import torch
 
-from tests._cases import make_qkv
+from tests._cases import BWD_TOL, FWD_TOL, alibi_slopes, make_qkv
 
 pytestmark = pytest.mark.gpu
 
@@ -150,6 +150,97 @@ def test_other_threads_run_while_a_call_waits(call):
     torch.cuda.synchronize()
     assert blocked > 0.2, "the queue never filled: nothing was tested"
     assert max(gaps) < 0.1
+
+
+# (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim), options of flash_attn_func
+GRADIENTS = [
+    ((2, 4, 2, 150, 150, 64), dict()),
+    ((2, 4, 2, 150, 220, 64), dict(causal=True, softmax_scale=0.2)),
+    ((1, 4, 4, 300, 300, 128), dict(causal=True, softcap=15.0)),
+    ((1, 4, 2, 260, 300, 96), dict(window_size=(70, 30))),
+    ((2, 4, 4, 200, 200, 64), dict(causal=True, window_size=(50, 0), deterministic=True)),
+    ((2, 4, 2, 130, 190, 128), dict(causal=True, alibi="heads")),
+    ((2, 4, 2, 130, 190, 64), dict(alibi="batch", softcap=20.0)),
+    ((2, 4, 2, 130, 190, 64), dict(causal=True, alibi="batch", deterministic=True)),
+    ((1, 4, 2, 200, 200, 192), dict(causal=True, softcap=30.0, softmax_scale=0.1)),
+    ((1, 4, 2, 150, 200, 256), dict(alibi="heads", window_size=(100, -1))),
+    ((1, 4, 1, 1, 300, 128), dict(causal=True)),                      # one query sees every key
+    ((1, 4, 1, 1, 300, 128), dict(causal=True, alibi="heads")),       # ... and with slopes its position matters
+]
+
+
+@pytest.mark.parametrize("shape,opt", GRADIENTS, ids=[f"{s}-{'-'.join(o)}" for s, o in GRADIENTS])
+@pytest.mark.parametrize("upstream", ["plain", "strided", "expanded"])
+def test_gradients_follow_every_option(shape, opt, upstream):
+    """Output and gradients of `flash_attn_func` against the CPU oracle; q, k and v may be views of one projection, the
+    gradient that arrives may be laid out in any way."""
+    import flash_attn2_b200 as fa2
+    from oracle.attention_oracle import attention_backward, attention_forward
+
+    b, h, hk, sq, sk, d = shape
+    opt, dtype = dict(opt), torch.bfloat16
+    q, k, v, do = make_qkv(35, b, h, hk, sq, sk, d, dtype, with_do=True)
+    if h == hk and sq == sk:
+        fused = torch.stack([q, k, v], 2).cuda()
+        qc, kc, vc = (t.detach().requires_grad_() for t in fused.unbind(2))
+        assert not qc.is_contiguous()
+    else:
+        qc, kc, vc = (t.cuda().requires_grad_() for t in (q, k, v))
+    slopes, which = None, opt.pop("alibi", None)
+    if which:
+        slopes = alibi_slopes(h) if which == "heads" else torch.stack([alibi_slopes(h) * (1 + i) for i in range(b)])
+    if upstream == "expanded":
+        do = do[:, :1, :, :1].expand(b, sq, h, d)
+        arrives = do[:, :1, :, :1].cuda().expand(b, sq, h, d)
+    else:
+        arrives = do.cuda() if upstream == "plain" else do.transpose(1, 2).contiguous().cuda().transpose(1, 2)
+    out = fa2.flash_attn_func(qc, kc, vc, alibi_slopes=None if slopes is None else slopes.cuda(), **opt)
+    grads = torch.autograd.grad(out, (qc, kc, vc), arrives)
+    left, right = opt.pop("window_size", (-1, -1))
+    opt.pop("deterministic", None)
+    if sq == 1 and slopes is None:
+        opt["causal"] = False
+    ref = dict(opt, alibi_slopes=slopes, window_left=left, window_right=right)
+    o_ref, lse_ref = attention_forward(q, k, v, **ref)
+    torch.testing.assert_close(out.detach().float().cpu(), o_ref, atol=FWD_TOL[dtype]["atol"], rtol=FWD_TOL[dtype]["rtol"])
+    want = attention_backward(q, k, v, do.contiguous(), out=out.detach().float().cpu(), lse=lse_ref, **ref)
+    for name, g, r in zip(("dq", "dk", "dv"), grads, want):
+        torch.testing.assert_close(g.float().cpu(), r, msg=lambda m, n=name: f"{n}: {m}", **BWD_TOL[dtype])
+    assert fa2.cabi_ops.device_status() == 0
+
+
+@pytest.mark.parametrize("opt", [dict(), dict(is_causal=True, softcap=15.0), dict(window_size_left=60, window_size_right=10, softmax_scale=0.2)],
+                         ids=["plain", "softcap", "window"])
+def test_native_and_operator_route_agree(opt):
+    """A supplied output takes the operator library: the same bits, on a side stream and from another thread as well."""
+    import flash_attn2_b200 as fa2
+
+    q, k, v = _qkv()
+    dout = torch.ones_like(q)
+    out = torch.empty_like(q)
+    want = fa2.fwd(q, k, v, out=out, **opt)
+    want_grads = fa2.bwd(dout, q, k, v, want[0], want[1], dk=torch.empty_like(k), **opt)
+    got = []
+
+    def call():
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            o, l = fa2.fwd(q, k, v, **opt)[:2]
+            got.append((o, l, fa2.bwd(dout, q, k, v, o, l, **opt)))
+        stream.synchronize()
+
+    torch.cuda.synchronize()
+    call()
+    threads = [threading.Thread(target=call) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(got) == 3
+    for o, l, grads in got:
+        assert torch.equal(o, want[0]) and torch.equal(l, want[1])
+        assert torch.equal(grads[1], want_grads[1]) and torch.equal(grads[2], want_grads[2]) and torch.equal(grads[3], want_grads[3])
+        torch.testing.assert_close(grads[0], want_grads[0], atol=2e-2, rtol=2e-2)  # fp32 adds land in arrival order
 
 
 class _LittleMemory:
