@@ -58,7 +58,7 @@ def build_kernels(verbose: bool = False) -> Path:
                     cmd.insert(1, "-Xptxas=-v")
                 jobs.append(cmd)
             objs.append(str(o))
-        # one nvcc per translation unit, side by side: every kernel file holds 16 instantiations
+        # one nvcc per translation unit, side by side: every kernel file holds 16 to 40 instantiations
         if jobs:
             with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 1)) as pool:
                 list(pool.map(_run, jobs))
