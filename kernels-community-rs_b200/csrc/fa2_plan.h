@@ -85,7 +85,7 @@ inline bool few_rows_win(const fa2_fwd_args* a, const DecodePlan& d, int64_t key
 inline DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
   DecodePlan d;
   const int64_t rows = static_cast<int64_t>(a->seqlen_q) * (a->heads / a->heads_k);
-  if (rows <= 0 || rows > kDecodeMaxRows || a->seqlen_k <= 0) return d;
+  if (rows <= 0 || rows > kDecodeMaxRows || a->seqlen_k <= 0 || a->head_dim <= 0 || a->head_dim > 256) return d;
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
   const int64_t off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q;
   int64_t lo = 0, hi = a->seqlen_k;

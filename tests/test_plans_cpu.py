@@ -85,6 +85,16 @@ def test_the_few_row_kernel_takes_what_it_is_faster_for(plans, shape, us):
     assert plans.few_rows(ctypes.byref(_fwd_args(b, h, hk, 65, sk, d)), SMS) == 0
 
 
+@pytest.mark.parametrize("head_dim", [257, 264, 1024, 0, -8])
+def test_head_dims_outside_the_range_have_no_plan(plans, head_dim):
+    """Scratch memory is asked for before a call is checked."""
+    for sq in (1, 300):
+        args = _fwd_args(1, 8, 2, sq, 4000, head_dim)
+        assert plans.few_rows(ctypes.byref(args), SMS) == 0 and plans.few_rows_workspace(ctypes.byref(args), SMS) == 0
+        if head_dim > 0:
+            assert plans.shared_tiles(ctypes.byref(args), SMS) == 0
+
+
 # Shapes (heads, seqlen_q, seqlen_k, head_dim, causal) timed with and without sharing.
 NOT_SHARED = [(12, 2000, 2048, 128, 1), (12, 2000, 4096, 128, 0), (50, 512, 4096, 128, 1), (18, 1000, 2048, 128, 1),
               (6, 4000, 4096, 128, 0), (9, 4000, 4096, 128, 1), (100, 65, 9000, 128, 0), (100, 128, 9000, 128, 0)]
