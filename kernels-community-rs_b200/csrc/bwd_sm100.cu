@@ -47,16 +47,24 @@ struct BwdCfg {
   static constexpr int kKOff = 0;
   static constexpr int kVOff = kTileBytes;
   static constexpr int kQOff = 2 * kTileBytes;     // 2 stages
-  static constexpr int kDOOff = 4 * kTileBytes;    // 2 stages; a retired stage doubles as dQ staging
-  static constexpr int kDSOff = 6 * kTileBytes;    // [128 keys x 128 q] 16-bit
+  // The dQ pieces have staging buffers of their own. While they went through the retired dO stage (two stages at either
+  // head dim), dO came back to the loader only after the reductions had read it, two thirds of an iteration late. At
+  // D = 128 the staging takes the place of the second dO stage: one is enough, because dV, its last reader, is issued
+  // most of an iteration before the next dP^T. Forward and backward together, causal bf16: B16 H16 S2048 1413 -> 1392 us,
+  // B1 H32 S16384 7933 -> 7742.
+  static constexpr int kDOStages = D == 128 ? 1 : 2;
+  static constexpr int kDOOff = 4 * kTileBytes;
+  static constexpr int kDSOff = kDOOff + kDOStages * kTileBytes;  // [128 keys x 128 q] 16-bit
   static constexpr int kDSBytes = kBlk * kBlk * 2;
-  static constexpr int kBarOff = kDSOff + kDSBytes;
+  static constexpr int kPieceBytes = kBlk * 128;   // dQ staging piece: [128 rows x 32 fp32]
+  static constexpr int kPieces = 2;                // staging buffers: 4 KB per drain warp and piece
+  static constexpr int kDQOff = kDSOff + kDSBytes;
+  static constexpr int kBarOff = kDQOff + kPieces * kPieceBytes;
   static constexpr int kNumBars = 28;
   static constexpr int kMiscOff = (kBarOff + kNumBars * 8 + 15) / 16 * 16;  // what follows is read as float4
   static constexpr int kStatOff = kMiscOff + 32;       // lse / delta: [2 buffers][2][128] fp32
   static constexpr int kSmemBytes = kStatOff + 2 * 2 * kBlk * 4;  // the dynamic window must start 1024-aligned
   static_assert(kStatOff % 16 == 0, "lse / delta are read as float4");
-  static constexpr int kPieceBytes = kBlk * 128;       // dQ staging piece: [128 rows x 32 fp32]
   static constexpr uint32_t kTmemDK = 0, kTmemDV = D, kTmemS = 256, kTmemDP = 384;
 };
 
@@ -181,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   uint64_t* q_full = bars + 1;    // [2]
   uint64_t* q_empty = bars + 3;   // [2]
   uint64_t* do_full = bars + 5;   // [2]
-  uint64_t* do_empty = bars + 7;  // [2] dV has read the stage and the dQ drain is done staging in it
+  uint64_t* do_empty = bars + 7;  // [2] dV has read the stage (and, in packed batches, the fixer has seen it)
   uint64_t* s_full = bars + 9;
   uint64_t* p_full = bars + 10;
   uint64_t* dp_full = bars + 11;
@@ -227,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       uint32_t count = 1;
       if (lane == 10 || lane == 12 || lane == 16) count = 256;            // p_full, ds_full, stat_full
       if (lane == 14 || lane == 18 || lane == 19 || lane == 20) count = kBlk;  // dq_free, stage_full, epi_full[2]
-      if ((lane == 7 || lane == 8) && want_dq) count = 5;  // do_empty: the dV commit and, with dQ, the four drain warps
+      if (PACKED && (lane == 7 || lane == 8)) count = 2;  // do_empty: the dV commit and the fixer
       mbar_init(bars + lane, count);
     }
     if (lane == 0) *abort_flag = 0;
@@ -286,12 +294,13 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         for (int a = 0; a < Cfg::kAtoms; ++a)
           tma_load_4d(s_q + st * Cfg::kTileBytes + a * (kBlk * 128), &p.tm_q, &q_full[st], a * 64, hq,
                       ti.q_row0 + m0, ti.bq);
-        ok = mbar_wait(&do_empty[st], ph ^ 1, ctl, kWaitBwd + 2);
+        const int dst = it % Cfg::kDOStages;
+        ok = mbar_wait(&do_empty[dst], ((it / Cfg::kDOStages) & 1) ^ 1, ctl, kWaitBwd + 2);
         if (!ok) break;
-        mbar_expect_tx(&do_full[st], Cfg::kTileBytes);
+        mbar_expect_tx(&do_full[dst], Cfg::kTileBytes);
 #pragma unroll
         for (int a = 0; a < Cfg::kAtoms; ++a)
-          tma_load_4d(s_do + st * Cfg::kTileBytes + a * (kBlk * 128), &p.tm_do, &do_full[st], a * 64, hq,
+          tma_load_4d(s_do + dst * Cfg::kTileBytes + a * (kBlk * 128), &p.tm_do, &do_full[dst], a * 64, hq,
                       ti.q_row0 + m0, ti.bq);
       }
       if (!ok) {
@@ -365,7 +374,9 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       for (int it = 0; it < n_iter && ok; ++it) {
         wn = walk_next(wn, ti.n_m);
         const uint32_t st = it & 1;
-        const uint32_t nph = ((it + 1) >> 1) & 1;  // phase of the stage barriers of iteration it + 1
+        const uint32_t nph = ((it + 1) >> 1) & 1;  // phase of the Q stage barriers of iteration it + 1
+        const uint32_t dst = it % Cfg::kDOStages, ndst = (it + 1) % Cfg::kDOStages;
+        const uint32_t ndph = ((it + 1) / Cfg::kDOStages) & 1;
         const bool has_next = it + 1 < n_iter;
         const uint32_t acc = it > 0 ? 1u : 0u;
         // dV += P^T dO   (P^T: two 32-column halves at S + 0 and S + 64)
@@ -373,13 +384,13 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         if (!ok) break;
         tc_fence_after();
         if (want_dkv) {
-          const uint64_t b = do_mn + st * kTile16;
+          const uint64_t b = do_mn + dst * kTile16;
           static_for<kBlk / 16>([&](auto ks) {
             mma_ts_o<(ks.value / 4) * 64 + (ks.value % 4) * 8, ks.value * (2048 >> 4)>(
                 tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv, ks.value > 0 ? 1u : acc);
           });
         }
-        mma_commit(&do_empty[st]);
+        mma_commit(&do_empty[dst]);
         if (!has_next) mma_commit(dv_done);  // dV is final: its epilogue runs beside the last dQ and dK GEMMs
         // S^T of the next iteration right behind dV, the last reader of P^T: the scores are there when the
         // compute warps come out of phase B.
@@ -412,11 +423,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         mma_commit(&q_empty[st]);
         // dP^T of the next iteration, once the dQ tile has left TMEM
         if (has_next) {
-          ok = do_ready(wn.mi, st ^ 1, nph, kWaitBwd + 9);
+          ok = do_ready(wn.mi, ndst, ndph, kWaitBwd + 9);
           if (ok && want_dq) ok = mbar_wait(dq_free, it & 1, ctl, kWaitBwd + 10);
           if (!ok) break;
           tc_fence_after();
-          kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj + (st ^ 1) * kTile16);
+          kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj + ndst * kTile16);
           mma_commit(dp_full);
         }
       }
@@ -460,11 +471,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           clear_rows(s_q + st * Cfg::kTileBytes, first);
           publish(&q_fixed[st]);
         }
-        ok = ok && __all_sync(0xffffffffu, mbar_wait(&do_full[st], ph, ctl, kWaitBwd + 5));
+        const uint32_t dst = it % Cfg::kDOStages;
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(&do_full[dst], (it / Cfg::kDOStages) & 1, ctl, kWaitBwd + 5));
         if (ok && first < kBlk) {
-          clear_rows(s_do + st * Cfg::kTileBytes, first);
-          publish(&do_fixed[st]);
+          clear_rows(s_do + dst * Cfg::kTileBytes, first);
+          publish(&do_fixed[dst]);
         }
+        // The stage is not refilled before this warp has seen it: its waits go by phase parity.
+        if (ok && lane == 0) mbar_arrive(&do_empty[dst]);
+        __syncwarp();
       }
     }
   } else if (warp < 12) {
@@ -708,8 +723,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   } else {
     // ------------------------------------------------------------------ dQ drain
     // The whole 128 x D fp32 tile goes to registers at once so that the dP^T / dQ columns are free
-    // for the next iteration right away; it then leaves through the dO stage and the Q stage this
-    // iteration has retired as cp.reduce.async.bulk adds into the accumulator.
+    // for the next iteration right away; it then leaves through a staging area of the drain's own
+    // as cp.reduce.async.bulk adds into the accumulator.
     reg_alloc<kDrainRegs>();
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t t_dq = tmem + lane_addr + Cfg::kTmemDP;
@@ -719,7 +734,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
         const int hq = ti.hk * p.group + w.g;
         const int m0 = (ti.m_start + w.mi) * kBlk;
-        const uint32_t st = it & 1;
         if (!warp_wait(dq_full, it & 1, ctl, kWaitBwd + 14)) break;
         tc_fence_after();
         uint32_t acc[D];
@@ -735,17 +749,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
 #pragma unroll
           for (int i = 0; i < D; ++i) acc[i] = 0u;
         }
-        // Each warp drains its own 32 rows in pieces of 32 fp32 columns (4 KB). The reduce engine is bound by
-        // the latency of the L2 adds, not by bandwidth: with only the dO stage as staging (half of the tile in
-        // flight) a tile took 4000-4800 cycles and paced the whole loop. The first half of the pieces goes
-        // through the warp's share of the retired dO stage at once, the second half through its share of the
-        // Q stage as soon as dK has read it, so the whole tile is in flight together. Nothing but the warp
-        // itself has to be synchronised.
-        constexpr int kPieces = D / 32;
-        constexpr int kHalf = kPieces / 2;              // pieces per staging area
+        // Each warp drains its own 32 rows in pieces of 32 fp32 columns (4 KB) that roll through two buffers of its
+        // own, also from one tile to the next. Nothing but the warp itself has to be synchronised.
         constexpr int kWarpPiece = Cfg::kPieceBytes / 4;
-        static_assert(kHalf * Cfg::kPieceBytes <= Cfg::kTileBytes, "half of the dQ tile fits one stage");
-        uint8_t* stage_do = s_do + st * Cfg::kTileBytes + (warp & 3) * (kHalf * kWarpPiece);
+        uint8_t* stage = smem + Cfg::kDQOff + (warp & 3) * (Cfg::kPieces * kWarpPiece);
         int* turn = nullptr;
         if (PACKED && p.dq_turn != nullptr) {
           // Ordered mode: the key blocks that add into these rows take their turns in descending order,
@@ -785,13 +792,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           if (!ok) break;
         }
 #pragma unroll
-        for (int k = 0; k < kPieces; ++k) {
-          // dO stage only: piece k reuses the buffer of piece k - kHalf once its reduce has read it
-          if (k >= kHalf) {
-            if (lane == 0) tma_wait_group_read<kHalf - 1>();
-            __syncwarp();
-          }
-          uint8_t* buf = stage_do + (k % kHalf) * kWarpPiece;
+        for (int k = 0; k < D / 32; ++k) {
+          // The buffer is free once the reduce of the piece two before this one has read it.
+          if (lane == 0) tma_wait_group_read<Cfg::kPieces - 1>();
+          __syncwarp();
+          uint8_t* buf = stage + (k % Cfg::kPieces) * kWarpPiece;
           uint8_t* rowp = buf + lane * 128;
 #pragma unroll
           for (int c = 0; c < 8; ++c)
@@ -805,17 +810,12 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           }
         }
         if (!ok) break;
-        // Hand both stages back to the loader once the reduces have read them.
-        if (lane == 0) {
-          tma_wait_group_read<0>();
-          mbar_arrive(&do_empty[st]);
-          if (turn != nullptr) {
-            // The adds have to be in memory before the next key block may start on these rows.
-            tma_wait_group<0>();
-            asm volatile("fence.proxy.async.global;" ::: "memory");
-            __threadfence();
-            atomicAdd(turn, 1);
-          }
+        if (turn != nullptr && lane == 0) {
+          // The adds have to be in memory before the next key block may start on these rows.
+          tma_wait_group<0>();
+          asm volatile("fence.proxy.async.global;" ::: "memory");
+          __threadfence();
+          atomicAdd(turn, 1);
         }
       }
       if (lane == 0) tma_wait_group_read<0>();
