@@ -14,7 +14,7 @@
 //
 // Three products per tile pair, 1536 tensor cycles at D = 128; the exponentials take 1024 MUFU cycles next to them.
 // Warps: 0-7 compute, 8 loader (TMA ring of five tiles: K(0) V(0) K(1) V(1) ...), 9 MMA issuer.
-// CTAs of one head are adjacent in the grid, heaviest first, so the head's K and V stay in L2.
+// The CTAs of a group of heads are listed together, heaviest first (bwd_dq_head_group), so the group's K and V stay in L2.
 //
 // Stands in for the reference's register-accumulating dQ kernel (flash-attn2-rs/src/device/backward/dq.rs:12-302).
 #include "sm100_ptx.cuh"
@@ -75,8 +75,12 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_kernel(const __grid_consta
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
 
-  const int bh = blockIdx.x / p.num_mblk;
-  const int m0 = (p.num_mblk - 1 - (static_cast<int>(blockIdx.x) - bh * p.num_mblk)) * kBlk;
+  const int first_bh = static_cast<int>(blockIdx.x) / (p.head_group * p.num_mblk) * p.head_group;
+  const int n_bh = min(p.head_group, p.batch * p.heads - first_bh);
+  const int in_group = static_cast<int>(blockIdx.x) - first_bh * p.num_mblk;
+  const int m_rev = in_group / n_bh;
+  const int bh = first_bh + in_group - m_rev * n_bh;
+  const int m0 = (p.num_mblk - 1 - m_rev) * kBlk;
   const int b = bh / p.heads, h = bh - b * p.heads, hk = h / p.group;
   const int off = p.seqlen_k - p.seqlen_q;
   // Key blocks [nb, ne) that some row of this block sees.

@@ -109,17 +109,20 @@ __device__ __forceinline__ Walk walk_next(Walk w, int n_m) {
 
 __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   KvTile ti;
-  // Consecutive CTAs walk the key blocks of one (batch, kv head): the head's Q, dO and its fp32
-  // dQ accumulator stay in L2 while the 16-odd CTAs that add into it run side by side. With a
-  // causal mask the first key blocks see the most query rows, so each head starts with its
-  // heaviest CTAs.
-  int bh, nblk;
+  // The key blocks of a group of heads are listed together, the first block of every head, then the second ...: with a
+  // causal mask the first ones see the most query rows, so each group starts with its heaviest CTAs and ends with its
+  // lightest (bwd_head_group: how many heads, and what it gives).
+  const int per_head = p.dk_part != nullptr ? p.items_per_head : p.num_nblk;
+  const int first_bh = t / (p.head_group * per_head) * p.head_group;
+  const int n_bh = min(p.head_group, p.batch * p.heads_k - first_bh);
+  const int in_group = t - first_bh * per_head;
+  const int i = in_group / n_bh;
+  const int bh = first_bh + in_group - i * n_bh;
+  int nblk = i;
   ti.part = 0;
   ti.parts = 1;
   if (p.dk_part != nullptr) {
     // The parts of all key blocks of a head, block by block.
-    bh = t / p.items_per_head;
-    const int i = t - bh * p.items_per_head;
     int lo = 0, hi = p.num_nblk;  // part_start[lo] <= i < part_start[hi]
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
@@ -129,9 +132,6 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
     nblk = lo;
     ti.part = i - p.part_start[lo];
     ti.parts = p.part_start[lo + 1] - p.part_start[lo];
-  } else {
-    bh = t / p.num_nblk;
-    nblk = t - bh * p.num_nblk;
   }
   // Ordered dQ accumulation waits for the higher key blocks of the same head. CTAs start in grid order, so
   // there the highest key block comes first: a CTA only ever waits for CTAs that were started before it,

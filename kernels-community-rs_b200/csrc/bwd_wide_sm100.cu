@@ -99,13 +99,16 @@ __device__ __forceinline__ float bw_tanh(float x) {
 }
 
 // The two halves of a key block are neighbours in the grid (they read the same tiles), and consecutive pairs
-// walk the key blocks of one (batch, kv head), heaviest first under a causal mask.
+// walk the key blocks of a group of heads, heaviest first under a causal mask (bwd_head_group).
 __device__ __forceinline__ WKvTile get_wkv_tile(const BwdParams& p, int t) {
   WKvTile ti;
   ti.half = t & 1;
   t >>= 1;
-  const int bh = t / p.num_nblk;
-  const int nblk = t - bh * p.num_nblk;
+  const int first_bh = t / (p.head_group * p.num_nblk) * p.head_group;
+  const int n_bh = min(p.head_group, p.batch * p.heads_k - first_bh);
+  const int in_group = t - first_bh * p.num_nblk;
+  const int nblk = in_group / n_bh;
+  const int bh = first_bh + in_group - nblk * n_bh;
   ti.b = bh / p.heads_k;
   ti.hk = bh - ti.b * p.heads_k;
   ti.n0 = nblk * kBK;

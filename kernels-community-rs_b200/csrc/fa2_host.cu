@@ -478,6 +478,7 @@ int bwd_dq(const fa2_bwd_args* a, const fa2_bwd_options& opt, Runtime* rt, cudaS
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
   p.window_left = w.left;
   p.window_right = w.right;
+  p.head_group = bwd_dq_head_group(a, w);
   p.causal_alibi = w.causal_alibi;
   p.scale = a->softmax_scale;
   p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
@@ -631,6 +632,7 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, packed);
   p.window_left = w.left;
   p.window_right = w.right;
+  p.head_group = bwd_head_group(a, w, rt->sm_count);
   p.which = a->which;
   p.alibi = a->alibi_slopes;
   p.alibi_batch_stride = a->alibi_batch_stride;
@@ -869,6 +871,7 @@ int bwd_static_impl(const fa2_bwd_args* a, void* stream_v) {
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
   p.window_left = w.left;
   p.window_right = w.right;
+  p.head_group = bwd_head_group(a, w, rt->sm_count);
   p.which = 3;
   p.dq_turn = nullptr;
   p.num_mblk_q = (a->seqlen_q + 127) / 128;

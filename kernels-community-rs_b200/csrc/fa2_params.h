@@ -102,6 +102,7 @@ struct BwdParams {
   int delta_seq_pad;                    // 128 in packed mode (sequence b starts at cu_q[b] + 128 b), else 0
   int batch, heads, heads_k, group, seqlen_q, seqlen_k;
   int num_nblk;                         // ceil(seqlen_k / 128)
+  int head_group;                       // (batch, kv head) pairs whose key blocks are listed together, heaviest first
   int window_left, window_right;
   int which;                            // bit 0: dQ, bit 1: dK and dV
   float scale, scale_log2;
@@ -146,6 +147,7 @@ struct DqParams {
   int alibi_batch_stride, causal_alibi;
   int batch, heads, group, seqlen_q, seqlen_k;
   int num_mblk;                         // ceil(seqlen_q / 128)
+  int head_group;                       // (batch, head) pairs whose query blocks are listed together, heaviest first
   int window_left, window_right;
   float scale, scale_log2, softcap;
   int head_dim;

@@ -181,6 +181,38 @@ inline void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
   out->workspace_bytes = (bytes + 255) / 256 * 256;
 }
 
+// ---- order of the backward's CTAs. One CTA walks a key block of a (batch, kv head); CTAs start in grid order, so a call
+// ends with whatever starts last. Under a causal mask the first key block of a head sees every query row and the last one
+// only its own: listed head by head, the last head's long walks start late and most SMs wait for them. So a group of
+// heads lists all first key blocks, then all second ones ...: the call ends with short walks. What the group's CTAs read
+// and add into should stay in the L2 (126 MB), so calls of many CTAs, whose end weighs little, take groups of at most
+// 96 MB (of Q, dO, the accumulator, K and V); with up to four CTAs per SM the end weighs more than the traffic. Forward and
+// backward, causal bf16, head by head -> grouped: B4 H16/4 S2048 softcap 448 -> 347 us, B2 H32/8 S4096 1183 -> 1001,
+// B4 H16 S1000 128 -> 119, B4 H16/8 S2048 D256 885 -> 834, B1 H32 S16384 7444 -> 7358 (in groups of 250 MB 7602).
+// Walks of the same length have no such end, but side by side those of one head add into the same rows at the same time;
+// small groups mix them: B32 H12 S509 D64 232 -> 228 us, B16 H16 S2048 without a mask 2191 -> 2170 (all heads: 2757).
+inline int bwd_head_group(const fa2_bwd_args* a, const Windows& w, int sm_count) {
+  if (a->cu_seqlens_q != nullptr) return 1;
+  const int64_t heads = std::max<int64_t>(static_cast<int64_t>(a->batch) * a->heads_k, 1);
+  const int64_t ctas = heads * ((a->seqlen_k + 127) / 128) * (a->head_dim > 128 ? 2 : 1);
+  const int64_t bytes = (static_cast<int64_t>(a->heads) * a->seqlen_q * 8 + static_cast<int64_t>(a->heads_k) * a->seqlen_k * 4) *
+                        a->head_dim * a->batch;
+  const bool falling = w.right >= 0 && w.left < 0;
+  const int64_t limit = !falling ? 16 << 20 : ctas > 4 * sm_count ? 96 << 20 : 320 << 20;
+  const int64_t groups = std::min(heads, bytes / limit + 1);
+  return static_cast<int>((heads + groups - 1) / groups);
+}
+
+// The same for the kernel that computes dQ alone, one CTA per 128 query rows of a head: K and V of a group, which its CTAs
+// share, take at most 64 MB.
+inline int bwd_dq_head_group(const fa2_bwd_args* a, const Windows& w) {
+  const int64_t heads = std::max<int64_t>(static_cast<int64_t>(a->batch) * a->heads, 1);
+  if (w.right < 0 || w.left >= 0) return 1;
+  const int64_t bytes = static_cast<int64_t>(a->seqlen_k) * a->head_dim * 4 * a->heads_k * a->batch;
+  const int64_t groups = std::min(heads, bytes / (64 << 20) + 1);
+  return static_cast<int>((heads + groups - 1) / groups);
+}
+
 // ---- key blocks shared by several CTAs (bwd_sm100.cu: part_start). A CTA owns 128 keys of one kv head and walks the
 // query blocks of all the group's heads; with few (batch, kv head, key block) triples most SMs would have nothing
 // to do, or wait for the CTA with the longest walk.
@@ -225,7 +257,9 @@ inline void plan_bwd_split(const fa2_bwd_args* a, bool share, int sm_count, BwdS
   auto cost = [&](double items, double longest, double all, bool even) {
     if (items <= sm_count) return longest;
     if (even) return std::ceil(items / sm_count) * longest;
-    return std::max(longest, all / sm_count + longest / 2);
+    // Walks of all heads in one list, heaviest first, leave little idle at the end; with a head after the other the last
+    // head's long walks start late.
+    return std::max(longest, all / sm_count + (bwd_head_group(a, w, sm_count) >= units ? t_cta : longest / 2));
   };
   double best = cost(static_cast<double>(units * nblk), most * t_it + t_cta, units * (total * t_it + nblk * t_cta), least == most);
   int best_parts = 1;
