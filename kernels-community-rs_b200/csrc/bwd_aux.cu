@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 #include "fa2_params.h"
 #include "fa2_launch.h"
+#include "sm100_ptx.cuh"
 
 namespace fa2 {
 
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(256) preprocess_kernel(const PreprocessParams 
   const IDX bs0 = (any ? gid0 : 0) / static_cast<IDX>(p.heads);
   int s = static_cast<int>(bs0 % static_cast<IDX>(p.seqlen_pad));
   int b = static_cast<int>(bs0 / static_cast<IDX>(p.seqlen_pad));
+  early_trigger();
   // No thread leaves before the shuffles below: a warp holds 32 / LANES groups, some of which may lie past
   // the end.
 #pragma unroll
@@ -136,12 +138,14 @@ __device__ __forceinline__ void convert_dq(const float4* __restrict__ src, uint4
 template <bool BF16>
 __global__ void __launch_bounds__(256) dq_convert_kernel(const float4* __restrict__ src, uint4* __restrict__ dst, int64_t n8,
                                                          float scale) {
+  early_trigger();
   convert_dq<BF16>(src, dst, n8, scale);
 }
 
 // The same with split key blocks: blockIdx.y 0 is dQ, 1 the parts.
 template <bool BF16>
 __global__ void __launch_bounds__(256) finish_kernel(const __grid_constant__ FinishParams p) {
+  early_trigger();
   if (blockIdx.y == 0) {
     if (p.dq_acc != nullptr) convert_dq<BF16>(reinterpret_cast<const float4*>(p.dq_acc), static_cast<uint4*>(p.dq), p.n_dq / 8, p.scale);
   } else {

@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_kernel(const __grid_consta
   using Cfg = DqCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
+    early_wait();
     if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, kWaitNone + 1);
     return;
   }
@@ -116,8 +117,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_kernel(const __grid_consta
     tma_prefetch_desc(&p.tm_v);
   }
   tc_fence_before();
+  early_wait();
   __syncthreads();
   tc_fence_after();
+  early_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp < 8) {
@@ -343,8 +346,7 @@ cudaError_t launch_one(const DqParams& p, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  bwd_dq_kernel<D, BF16, MODE><<<p.num_mblk * p.batch * p.heads, kThreads, Cfg::kSmemBytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(bwd_dq_kernel<D, BF16, MODE>, dim3(p.num_mblk * p.batch * p.heads), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int D, bool BF16>

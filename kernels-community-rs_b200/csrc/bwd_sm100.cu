@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   using Cfg = BwdCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
+    early_wait();
     if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, kWaitNone + 1);
     return;
   }
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
+  if (PACKED) early_wait();  // the sequences' offsets are in global memory
   const KvTile ti = get_kv_tile(p, blockIdx.x);
   if (!ti.valid) return;
   const bool want_dq = (p.which & 1) != 0;
@@ -245,6 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   if (tid == 0) {
     // The first loads go out before the rest of the CTA is set up (TMEM allocation, the block-wide
     // barrier): their latency is the longest item of a CTA's start.
+    early_wait();
     if (ti.n_iter > 0) {
       const int hq0 = ti.hk * p.group + ti.g0;
       const int m00 = (ti.m_start + ti.mi0) * kBlk;
@@ -269,8 +272,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     tmem_relinquish();
   }
   tc_fence_before();
+  early_wait();
   __syncthreads();
   tc_fence_after();
+  early_trigger();
   const uint32_t tmem = *tmem_slot;
   const int n_iter = ti.n_iter;
 
@@ -847,8 +852,7 @@ cudaError_t launch_one(const BwdParams& p, int num_ctas, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  bwd_kernel<D, BF16, MODE, PACKED><<<num_ctas, kThreads, Cfg::kSmemBytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(bwd_kernel<D, BF16, MODE, PACKED>, dim3(num_ctas), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int D, bool BF16>

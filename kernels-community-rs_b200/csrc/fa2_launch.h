@@ -10,6 +10,24 @@ namespace fa2 {
 // (both transforms; in the forward also a negative scale without a transform) and is what packed batches use.
 enum ScoreMode : int { kScorePlain = 0, kScoreSoftcap = 1, kScoreAlibi = 2, kScoreAny = 3 };
 
+// Launches a kernel that calls early_wait: it may start while the kernel before it in the stream ends.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem_bytes, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute early[1] = {};
+  early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = stream;
+  cfg.attrs = early;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 // Dense and packed (varlen) forward; head_dim is a multiple of 8 up to 128 (kernels for D = 64 and 128).
 cudaError_t launch_fwd(const FwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream);
 

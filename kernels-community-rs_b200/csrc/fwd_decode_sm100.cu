@@ -111,7 +111,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
     tma_prefetch_desc(&p.tm_k);
     tma_prefetch_desc(&p.tm_v);
   }
+  early_wait();
   __syncthreads();
+  early_trigger();
 
   if (warp >= kConsumers) {
     // ---------------------------------------------------------------- loader
@@ -568,8 +570,7 @@ cudaError_t launch_one(const DecodeParams& p, int grid, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  fwd_decode_kernel<A, MT, BF16><<<grid, kThreads, Cfg::kSmemBytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(fwd_decode_kernel<A, MT, BF16>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int A, bool BF16>

@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
     // 128-byte swizzled tiles need a 1024-byte aligned base; report instead of computing garbage.
+    early_wait();
     if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, kWaitNone + 1);
     return;
   }
@@ -332,10 +333,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
     tma_prefetch_desc(&p.tm_o);
   }
   tc_fence_before();
+  early_wait();
   __syncthreads();
   tc_fence_after();
+  early_trigger();
   const uint32_t tmem = *tmem_slot;
-  if (SHARED) asm volatile("griddepcontrol.launch_dependents;");  // the merge waits for this grid before it reads
 
   if (warp < 8) {
     // ------------------------------------------------------------------ softmax + epilogue of stage s
@@ -926,7 +928,8 @@ __global__ void __launch_bounds__(256) merge_parts_kernel(const __grid_constant_
   const int c_first = static_cast<int>(((u0 + p.block_start[mb] + 1) * g + total - 1) / total - 1);
   const int c_last = static_cast<int>(((u0 + p.block_start[mb + 1]) * g + total - 1) / total - 1);
   const int b = bh / p.heads, h = bh - b * p.heads;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  early_wait();
+  early_trigger();
   if (c_first == c_last) return;  // the forward kernel has written it
   const int col = (threadIdx.x % kLanes) * 4;
   const int prow0 = (blockIdx.x % (256 / kMergeRows<D>)) * kMergeRows<D> + threadIdx.x / kLanes;
@@ -1005,21 +1008,10 @@ cudaError_t launch_one(const FwdParams& p, int num_sms, cudaStream_t stream) {
     configured[dev] = true;
   }
   const int grid = SHARED ? p.stream_grid : p.num_tiles < num_sms ? p.num_tiles : num_sms;
-  fwd_kernel<D, BF16, MODE, PACKED, SHARED><<<grid, kThreads, Cfg::kSmemBytes, stream>>>(p);
-  if (SHARED) {
-    cudaLaunchAttribute early[1] = {};
-    early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(p.num_tiles * (256 / kMergeRows<D>)));
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cfg.attrs = early;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, merge_parts_kernel<D, BF16>, p);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaGetLastError();
+  cudaError_t e = launch_early(fwd_kernel<D, BF16, MODE, PACKED, SHARED>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
+  if (SHARED && e == cudaSuccess)
+    e = launch_early(merge_parts_kernel<D, BF16>, dim3(p.num_tiles * (256 / kMergeRows<D>)), 256, 0, stream, p);
+  return e;
 }
 
 template <int D, bool BF16>

@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
     // 128-byte swizzled tiles need a 1024-byte aligned base; report instead of computing garbage.
+    early_wait();
     if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, kWaitNone + 1);
     return;
   }
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
+  if (PACKED) early_wait();  // the sequences' offsets are in global memory
   const WTile ti = get_wtile(p, blockIdx.x);
   if (!ti.valid) return;
   constexpr int atoms = ATOMS;
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
 
   if (n_tiles == 0) {
     // No key is visible to this block: O = 0, LSE = +inf.
+    early_wait();
     if (tid < kWM && ti.m0 + tid < ti.sq) {
       const int row = ti.m0 + tid;
       uint16_t* orow = reinterpret_cast<uint16_t*>(p.o_ptr) + ti.bq * p.o_batch_stride +
@@ -198,8 +201,10 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
     tma_prefetch_desc(&p.tm_v);
   }
   tc_fence_before();
+  early_wait();
   __syncthreads();
   tc_fence_after();
+  early_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp < 4) {
@@ -513,9 +518,8 @@ cudaError_t launch_wide(const FwdParams& p, cudaStream_t stream) {
   const int64_t blocks = static_cast<int64_t>((p.seqlen_q + kWM - 1) / kWM) * p.batch * p.heads;
   if (blocks <= 0) return cudaSuccess;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>
-      <<<static_cast<unsigned>(blocks), kWThreads, WideCfg::kSmemBytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_early(fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kWThreads,
+                      WideCfg::kSmemBytes, stream, p);
 }
 
 template <bool BF16, int ATOMS>
