@@ -244,10 +244,12 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     mbar_fence_init();
     __syncwarp();
   }
+  // Behind this library's dQ kernel, whose results it does not read, the grid starts beside it and waits at its end instead.
+  const bool beside = !PACKED && p.beside_dq != 0;
   if (tid == 0) {
     // The first loads go out before the rest of the CTA is set up (TMEM allocation, the block-wide
     // barrier): their latency is the longest item of a CTA's start.
-    early_wait();
+    if (!beside) early_wait();
     if (ti.n_iter > 0) {
       const int hq0 = ti.hk * p.group + ti.g0;
       const int m00 = (ti.m_start + ti.mi0) * kBlk;
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     tmem_relinquish();
   }
   tc_fence_before();
-  early_wait();
+  if (!beside) early_wait();
   __syncthreads();
   tc_fence_after();
   early_trigger();
@@ -837,6 +839,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 512);
+  if (beside) early_wait();
 }
 
 template <int D, bool BF16, int MODE, bool PACKED>

@@ -61,6 +61,7 @@ class BwdArgs(C.Structure):
 class BwdOptions(C.Structure):
     _fields_ = [
         ("size", C.c_int64), ("out", C.c_void_p), ("o_stride", C.c_int64 * 3), ("share_key_blocks", C.c_int32),
+        ("reserved", C.c_int32), ("beside_dq", C.c_int64),
     ]
 
 

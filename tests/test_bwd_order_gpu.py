@@ -29,3 +29,22 @@ def test_a_head_gets_the_same_in_any_group(shape, causal):
         if dq is not None:
             assert torch.equal(ops.bwd(*args, causal=causal, which=1)[0], dq[:, :, mine])
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(2, 16, 4, 777, 128), (1, 8, 2, 1500, 64), (3, 4, 4, 130, 96)], ids=str)
+def test_dkdv_beside_dq(shape):
+    """The second call of a bit-reproducible backward runs beside the first one's last CTAs; what follows on the stream
+    (here the next pair, into the same memory, and a copy) waits for both."""
+    import flash_attn2_b200 as fa2
+    from flash_attn2_b200 import cabi_ops as ops
+
+    b, h, hk, s, d = shape
+    q, k, v, do = [t.cuda() for t in make_qkv(6, b, h, hk, s, s, d, torch.bfloat16, with_do=True)]
+    out, lse = fa2.fwd(q, k, v, is_causal=True)[:2]
+    delta = ops.bwd_preprocess(do, out)
+    dq = ops.bwd(q, k, v, do, lse, delta, causal=True, which=1)[0]
+    _, dk, dv = ops.bwd(q, k, v, do, lse, delta, causal=True, which=2, share_key_blocks=True)
+    for _ in range(20):
+        copies = [t.clone() for t in fa2.bwd(do, q, k, v, out, lse, is_causal=True, deterministic=True)[:3]]
+    assert all(torch.equal(a, r) for a, r in zip(copies, (dq, dk, dv)))
+    assert ops.device_status() == 0
