@@ -15,8 +15,20 @@
 //
 // TMEM: dK [0,D) dV [D,2D) S^T/P^T [256,384) dP^T/dQ [384,512).
 // Warps: 0 loader (TMA), 1 MMA issuer, 4-11 compute (two warpgroups, 64 query columns each),
-// 12-15 dQ drain. dK and dV are accumulated over the whole loop in TMEM and written once, so they
+// 12-15 dQ drain, 3 statistics (-LSE and -delta of the next query block into shared memory), 2 fixer (packed batches).
+// dK and dV are accumulated over the whole loop in TMEM and written once, so they
 // need no atomics; the GQA heads are walked serially like the reference kernel does.
+//
+// What bounds it: the compute warps. An iteration takes 3500-4000 cycles against 2560 of MMA at D = 128, 1450 of them P^T
+// and 1000 dS^T. The warps used to fetch LSE and delta themselves, behind a barrier of both warpgroups, and to do that
+// arithmetic one value at a time; with a warp for the statistics and packed instructions forward and backward of B4 H16/4
+// S2048 D128 softcap take 316 instead of 329 us, B16 H16 S2048 causal 1145 instead of 1154.
+//
+// A CTA's start and end cost 9000 cycles, a third of its time where a head has four query blocks. At D = 64 there is shared
+// memory for K and V of two tiles, so a CTA goes on with the tile of a CTA that has not started: K, V, Q and dO of the next
+// tile are loaded beside the end of this one. B32 H12 S509 D64 fp16 223.6 -> 201.0 us, B2 H16 S4096 D64 causal 378 -> 358.
+// At D = 128 K has to wait for the last dQ and nothing is left to stage dK and dV in: B4 H16 S1000 112.8 -> 114.8 us,
+// B4 H16/4 S2048 softcap 340 -> 345, so there a CTA has one tile. Packed batches have one tile per CTA too.
 //
 // Replaces the reference kernels `backward` (dQ) and `backward_kv`
 // (flash-attn2-rs/src/device/backward/dq.rs:12-302,438-576, dkv.rs:15-266,865-1012,
@@ -44,25 +56,29 @@ template <int D>
 struct BwdCfg {
   static constexpr int kAtoms = D / 64;
   static constexpr int kTileBytes = kBlk * D * 2;
+  // K and V of the next tile are loaded beside the end of this one where there is room for two of each.
+  static constexpr int kKVStages = D == 128 ? 1 : 2;
   static constexpr int kKOff = 0;
-  static constexpr int kVOff = kTileBytes;
-  static constexpr int kQOff = 2 * kTileBytes;     // 2 stages
+  static constexpr int kVOff = kKVStages * kTileBytes;
+  static constexpr int kQOff = 2 * kKVStages * kTileBytes;  // 2 stages
   // The dQ pieces have staging buffers of their own. While they went through the retired dO stage (two stages at either
   // head dim), dO came back to the loader only after the reductions had read it, two thirds of an iteration late. At
   // D = 128 the staging takes the place of the second dO stage: one is enough, because dV, its last reader, is issued
   // most of an iteration before the next dP^T. Forward and backward together, causal bf16: B16 H16 S2048 1413 -> 1392 us,
   // B1 H32 S16384 7933 -> 7742.
   static constexpr int kDOStages = D == 128 ? 1 : 2;
-  static constexpr int kDOOff = 4 * kTileBytes;
+  static constexpr int kDOOff = kQOff + 2 * kTileBytes;
   static constexpr int kDSOff = kDOOff + kDOStages * kTileBytes;  // [128 keys x 128 q] 16-bit
   static constexpr int kDSBytes = kBlk * kBlk * 2;
   static constexpr int kPieceBytes = kBlk * 128;   // dQ staging piece: [128 rows x 32 fp32]
   static constexpr int kPieces = 2;                // staging buffers: 4 KB per drain warp and piece
   static constexpr int kDQOff = kDSOff + kDSBytes;
   static constexpr int kBarOff = kDQOff + kPieces * kPieceBytes;
-  static constexpr int kNumBars = 28;
+  static constexpr int kNumBars = 40;
   static constexpr int kMiscOff = (kBarOff + kNumBars * 8 + 15) / 16 * 16;  // what follows is read as float4
-  static constexpr int kStatOff = kMiscOff + 32;       // lse / delta: [2 buffers][2][128] fp32
+  static constexpr int kAnswerOff = kMiscOff + 16;     // what the scheduler answered
+  static constexpr int kNextOff = kMiscOff + 32;       // [2] the CTA's next tile: twelve words
+  static constexpr int kStatOff = kNextOff + 96;       // lse / delta: [2 buffers][2][128] fp32
   static constexpr int kSmemBytes = kStatOff + 2 * 2 * kBlk * 4;  // the dynamic window must start 1024-aligned
   static_assert(kStatOff % 16 == 0, "lse / delta are read as float4");
   static constexpr uint32_t kTmemDK = 0, kTmemDV = D, kTmemS = 256, kTmemDP = 384;
@@ -107,12 +123,13 @@ __device__ __forceinline__ Walk walk_next(Walk w, int n_m) {
   return w;
 }
 
+template <bool PACKED>
 __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   KvTile ti;
   // The key blocks of a group of heads are listed together, the first block of every head, then the second ...: with a
   // causal mask the first ones see the most query rows, so each group starts with its heaviest CTAs and ends with its
   // lightest (bwd_head_group: how many heads, and what it gives).
-  const int per_head = p.dk_part != nullptr ? p.items_per_head : p.num_nblk;
+  const int per_head = !PACKED && p.dk_part != nullptr ? p.items_per_head : p.num_nblk;
   const int first_bh = t / (p.head_group * per_head) * p.head_group;
   const int n_bh = min(p.head_group, p.batch * p.heads_k - first_bh);
   const int in_group = t - first_bh * per_head;
@@ -121,7 +138,7 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   int nblk = i;
   ti.part = 0;
   ti.parts = 1;
-  if (p.dk_part != nullptr) {
+  if (!PACKED && p.dk_part != nullptr) {
     // The parts of all key blocks of a head, block by block.
     int lo = 0, hi = p.num_nblk;  // part_start[lo] <= i < part_start[hi]
     while (hi - lo > 1) {
@@ -136,11 +153,11 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   // Ordered dQ accumulation waits for the higher key blocks of the same head. CTAs start in grid order, so
   // there the highest key block comes first: a CTA only ever waits for CTAs that were started before it,
   // whatever the number of key blocks and of resident CTAs.
-  if (p.dq_turn != nullptr) nblk = p.num_nblk - 1 - nblk;
+  if (PACKED && p.dq_turn != nullptr) nblk = p.num_nblk - 1 - nblk;
   ti.b = bh / p.heads_k;
   ti.hk = bh - ti.b * p.heads_k;
   ti.n0 = nblk * kBlk;
-  if (p.cu_q != nullptr) {
+  if (PACKED) {
     ti.q_row0 = p.cu_q[ti.b];
     ti.sq = p.cu_q[ti.b + 1] - ti.q_row0;
     ti.k_row0 = p.cu_k[ti.b];
@@ -174,6 +191,7 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
 template <int D, bool BF16, int MODE, bool PACKED>
 __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = BwdCfg<D>;
+  constexpr bool kPersistent = D == 64 && !PACKED;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
     early_wait();
@@ -186,27 +204,31 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   uint8_t* s_do = smem + Cfg::kDOOff;
   uint8_t* s_ds = smem + Cfg::kDSOff;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kBarOff);
-  uint64_t* kv_full = bars + 0;    // K has landed (V has a barrier of its own: the first S^T needs only K and Q)
-  uint64_t* q_full = bars + 1;    // [2]
-  uint64_t* q_empty = bars + 3;   // [2]
-  uint64_t* do_full = bars + 5;   // [2]
-  uint64_t* do_empty = bars + 7;  // [2] dV has read the stage (and, in packed batches, the fixer has seen it)
-  uint64_t* s_full = bars + 9;
-  uint64_t* p_full = bars + 10;
-  uint64_t* dp_full = bars + 11;
-  uint64_t* ds_full = bars + 12;
-  uint64_t* dq_full = bars + 13;
-  uint64_t* dq_free = bars + 14;
-  uint64_t* dkv_done = bars + 15;
-  uint64_t* stat_full = bars + 16;
-  uint64_t* stage_free = bars + 17;
-  uint64_t* stage_full = bars + 18;
-  uint64_t* epi_full = bars + 19;  // [2]
-  uint64_t* kv_fixed = bars + 21;  // packed batches: the fixer warp has cleared the rows past the sequence
-  uint64_t* q_fixed = bars + 22;   // [2]
-  uint64_t* do_fixed = bars + 24;  // [2]
-  uint64_t* dv_done = bars + 26;   // the last dV MMA has completed (dK still has one GEMM to go)
-  uint64_t* v_full = bars + 27;    // V has landed
+  uint64_t* k_full = bars + 0;     // [2] K has landed (V has a barrier of its own: the first S^T needs only K and Q)
+  uint64_t* v_full = bars + 2;     // [2]
+  uint64_t* k_empty = bars + 4;    // [2] the tile's last dQ has read K
+  uint64_t* v_empty = bars + 6;    // [2] its last dP^T has read V
+  uint64_t* q_full = bars + 8;     // [2]
+  uint64_t* q_empty = bars + 10;   // [2]
+  uint64_t* do_full = bars + 12;   // [2]
+  uint64_t* do_empty = bars + 14;  // [2] dV has read the stage (and, in packed batches, the fixer has seen it)
+  uint64_t* s_full = bars + 16;
+  uint64_t* p_full = bars + 17;
+  uint64_t* dp_full = bars + 18;
+  uint64_t* ds_full = bars + 19;
+  uint64_t* dq_full = bars + 20;
+  uint64_t* dq_free = bars + 21;
+  uint64_t* dkv_done = bars + 22;
+  uint64_t* dv_done = bars + 23;   // the last dV MMA has completed (dK still has one GEMM to go)
+  uint64_t* stat_full = bars + 24;   // [2]
+  uint64_t* stat_empty = bars + 26;  // [2]
+  uint64_t* next_full = bars + 28;   // [2] the loader has written down the next tile
+  uint64_t* next_empty = bars + 30;  // [2] every role has read it
+  uint64_t* kv_fixed = bars + 32;  // packed batches: the fixer warp has cleared the rows past the sequence
+  uint64_t* q_fixed = bars + 33;   // [2]
+  uint64_t* do_fixed = bars + 35;  // [2]
+  uint64_t* epi_full = bars + 37;  // [2] packed batches: dK, dV are staged for their bulk store
+  uint64_t* answered = bars + 39;  // the scheduler has answered
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::kMiscOff + 8);
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::kStatOff);
@@ -216,8 +238,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   const int lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
   if (PACKED) early_wait();  // the sequences' offsets are in global memory
-  const KvTile ti = get_kv_tile(p, blockIdx.x);
-  if (!ti.valid) return;
+  const KvTile first_tile = get_kv_tile<PACKED>(p, blockIdx.x);
+  if (!first_tile.valid) return;
   const bool want_dq = (p.which & 1) != 0;
   // A dQ-only call skips the dV and dK GEMMs (their commits still hand the stages back). Only packed ones come here: dense
   // ones have bwd_dq_sm100.cu.
@@ -232,13 +254,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     tma_prefetch_desc(&p.tm_dqa);
   }
   if (warp == 0) {
-    // One barrier per lane: arrival counts by index (see the list above).
-    if (lane < Cfg::kNumBars) {
+    for (int i = lane; i < Cfg::kNumBars; i += 32) {
+      uint64_t* bar = bars + i;
       uint32_t count = 1;
-      if (lane == 10 || lane == 12 || lane == 16) count = 256;            // p_full, ds_full, stat_full
-      if (lane == 14 || lane == 18 || lane == 19 || lane == 20) count = kBlk;  // dq_free, stage_full, epi_full[2]
-      if (PACKED && (lane == 7 || lane == 8)) count = 2;  // do_empty: the dV commit and the fixer
-      mbar_init(bars + lane, count);
+      if (bar == p_full || bar == ds_full) count = 256;
+      if (bar == dq_free || bar == epi_full || bar == epi_full + 1) count = kBlk;
+      if (bar == stat_empty || bar == stat_empty + 1) count = 8;    // compute warps
+      if (bar == next_empty || bar == next_empty + 1) count = want_dq ? 14 : 10;  // issuer, statistics, compute, drain warps
+      if (PACKED && (bar == do_empty || bar == do_empty + 1)) count = 2;  // the dV commit and the fixer
+      mbar_init(bar, count);
     }
     if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
@@ -250,22 +274,23 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     // The first loads go out before the rest of the CTA is set up (TMEM allocation, the block-wide
     // barrier): their latency is the longest item of a CTA's start.
     if (!beside) early_wait();
+    const KvTile& ti = first_tile;
     if (ti.n_iter > 0) {
       const int hq0 = ti.hk * p.group + ti.g0;
       const int m00 = (ti.m_start + ti.mi0) * kBlk;
-      mbar_expect_tx(kv_full, Cfg::kTileBytes);
+      mbar_expect_tx(k_full, Cfg::kTileBytes);
       mbar_expect_tx(v_full, Cfg::kTileBytes);
-      mbar_expect_tx(&q_full[0], Cfg::kTileBytes);
-      mbar_expect_tx(&do_full[0], Cfg::kTileBytes);
+      mbar_expect_tx(q_full, Cfg::kTileBytes);
+      mbar_expect_tx(do_full, Cfg::kTileBytes);
 #pragma unroll
       for (int a = 0; a < Cfg::kAtoms; ++a) {
-        tma_load_4d(s_k + a * (kBlk * 128), &p.tm_k, kv_full, a * 64, ti.hk, ti.k_row0 + ti.n0, ti.bq);
-        tma_load_4d(s_q + a * (kBlk * 128), &p.tm_q, &q_full[0], a * 64, hq0, ti.q_row0 + m00, ti.bq);
+        tma_load_4d(s_k + a * (kBlk * 128), &p.tm_k, k_full, a * 64, ti.hk, ti.k_row0 + ti.n0, ti.bq);
+        tma_load_4d(s_q + a * (kBlk * 128), &p.tm_q, q_full, a * 64, hq0, ti.q_row0 + m00, ti.bq);
       }
 #pragma unroll
       for (int a = 0; a < Cfg::kAtoms; ++a) {
         tma_load_4d(s_v + a * (kBlk * 128), &p.tm_v, v_full, a * 64, ti.hk, ti.k_row0 + ti.n0, ti.bq);
-        tma_load_4d(s_do + a * (kBlk * 128), &p.tm_do, &do_full[0], a * 64, hq0, ti.q_row0 + m00, ti.bq);
+        tma_load_4d(s_do + a * (kBlk * 128), &p.tm_do, do_full, a * 64, hq0, ti.q_row0 + m00, ti.bq);
       }
     }
   }
@@ -279,37 +304,112 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   tc_fence_after();
   early_trigger();
   const uint32_t tmem = *tmem_slot;
-  const int n_iter = ti.n_iter;
+
+  // Dense calls: a CTA that has finished a tile goes on with one that has not started yet (the scheduler hands it the
+  // grid index of a CTA that it then leaves out). The loader asks and writes the tile down, every role reads it. Barriers,
+  // stages and TMEM carry on: the counters of a role, iterations, tiles with iterations and tiles, run through all its tiles.
+  struct Pos {
+    uint32_t it0 = 0, kv = 0, n = 0;
+  };
+  volatile int4* s_next = reinterpret_cast<volatile int4*>(smem + Cfg::kNextOff);
+  // false: no more tiles, or a wait ran out
+  auto next_tile = [&](KvTile& ti, Pos& pos) -> bool {
+    pos.it0 += ti.n_iter;
+    pos.kv += ti.n_iter > 0 ? 1 : 0;
+    const uint32_t slot = pos.n & 1;
+    if (!mbar_wait(&next_full[slot], (pos.n >> 1) & 1, ctl, kWaitBwd + 24)) return false;
+    ++pos.n;
+    const volatile int4* a = s_next + slot * 3;
+    ti.b = ti.bq = a[0].x;
+    ti.hk = a[0].y;
+    ti.n0 = a[0].z;
+    ti.n_iter = a[0].w;
+    ti.m_start = a[1].x;
+    ti.n_m = a[1].y;
+    ti.g0 = a[1].z;
+    ti.mi0 = a[1].w;
+    ti.part = a[2].x;
+    ti.parts = a[2].y;
+    return ti.n_iter >= 0;
+  };
+  auto next_tile_warp = [&](KvTile& ti, Pos& pos) -> bool {
+    const uint32_t slot = pos.n & 1;
+    const bool more = next_tile(ti, pos);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&next_empty[slot]);
+    return __all_sync(0xffffffffu, more);
+  };
 
   if (warp < 4) {
     reg_dealloc<kMiscRegs>();
     if (warp == 0 && elect_one()) {
       // ---------------------------------------------------------------- loader
-      // K, V and the first Q / dO tiles were requested during set-up.
+      // K, V and the first Q / dO tiles of the first tile were requested during set-up.
       bool ok = true;
-      Walk w{ti.g0, ti.mi0};
-      for (int it = 1; it < n_iter && ok; ++it) {
-        w = walk_next(w, ti.n_m);
-        const int hq = ti.hk * p.group + w.g;
-        const int m0 = (ti.m_start + w.mi) * kBlk;
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        ok = mbar_wait(&q_empty[st], ph ^ 1, ctl, kWaitBwd + 1);
-        if (!ok) break;
-        mbar_expect_tx(&q_full[st], Cfg::kTileBytes);
+      KvTile ti = first_tile;
+      Pos pos;
+      auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* full, int head, int row) {
+        mbar_expect_tx(full, Cfg::kTileBytes);
 #pragma unroll
-        for (int a = 0; a < Cfg::kAtoms; ++a)
-          tma_load_4d(s_q + st * Cfg::kTileBytes + a * (kBlk * 128), &p.tm_q, &q_full[st], a * 64, hq,
-                      ti.q_row0 + m0, ti.bq);
-        const int dst = it % Cfg::kDOStages;
-        ok = mbar_wait(&do_empty[dst], ((it / Cfg::kDOStages) & 1) ^ 1, ctl, kWaitBwd + 2);
+        for (int a = 0; a < Cfg::kAtoms; ++a) tma_load_4d(dst + a * (kBlk * 128), tm, full, a * 64, head, row, ti.bq);
+      };
+      do {
+        const uint32_t ks = pos.kv % Cfg::kKVStages, kph = (pos.kv / Cfg::kKVStages) & 1;
+        Walk w{ti.g0, ti.mi0};
+        for (int it = 0; it < ti.n_iter || it == 0; ++it) {
+          if (kPersistent && p.take_over && it + 1 >= ti.n_iter) {
+            mbar_expect_tx(answered, 16);
+            ask_next_cta(smem_u32(smem + Cfg::kAnswerOff), answered);
+          }
+          if (ti.n_iter == 0) break;
+          if (it > 0) w = walk_next(w, ti.n_m);
+          else if (pos.n == 0) continue;
+          const int hq = ti.hk * p.group + w.g;
+          const int row = ti.q_row0 + (ti.m_start + w.mi) * kBlk;
+          const uint32_t gi = pos.it0 + it;
+          const uint32_t st = gi & 1, dst = gi % Cfg::kDOStages;
+          ok = mbar_wait(&q_empty[st], ((gi >> 1) & 1) ^ 1, ctl, kWaitBwd + 1);
+          if (!ok) break;
+          load(s_q + st * Cfg::kTileBytes, &p.tm_q, &q_full[st], hq, row);
+          if (it == 0) {
+            ok = mbar_wait(&v_empty[ks], kph ^ 1, ctl, kWaitBwd + 26);
+            if (!ok) break;
+            load(s_v + ks * Cfg::kTileBytes, &p.tm_v, &v_full[ks], ti.hk, ti.k_row0 + ti.n0);
+          }
+          ok = mbar_wait(&do_empty[dst], ((gi / Cfg::kDOStages) & 1) ^ 1, ctl, kWaitBwd + 2);
+          if (!ok) break;
+          load(s_do + dst * Cfg::kTileBytes, &p.tm_do, &do_full[dst], hq, row);
+          if (it == 0) {
+            ok = mbar_wait(&k_empty[ks], kph ^ 1, ctl, kWaitBwd + 27);
+            if (!ok) break;
+            load(s_k + ks * Cfg::kTileBytes, &p.tm_k, &k_full[ks], ti.hk, ti.k_row0 + ti.n0);
+          }
+        }
+        if (!kPersistent || !ok) break;
+        // The tile after this one.
+        const uint32_t slot = pos.n & 1;
+        ok = (!p.take_over || mbar_wait(answered, pos.n & 1, ctl, kWaitBwd + 24)) &&
+             mbar_wait(&next_empty[slot], ((pos.n >> 1) & 1) ^ 1, ctl, kWaitBwd + 25);
         if (!ok) break;
-        mbar_expect_tx(&do_full[dst], Cfg::kTileBytes);
-#pragma unroll
-        for (int a = 0; a < Cfg::kAtoms; ++a)
-          tma_load_4d(s_do + dst * Cfg::kTileBytes + a * (kBlk * 128), &p.tm_do, &do_full[dst], a * 64, hq,
-                      ti.q_row0 + m0, ti.bq);
-      }
+        ++pos.n;
+        pos.it0 += ti.n_iter;
+        pos.kv += ti.n_iter > 0 ? 1 : 0;
+        const int t = p.take_over ? next_cta(smem_u32(smem + Cfg::kAnswerOff)) : -1;
+        if (t >= 0) ti = get_kv_tile<PACKED>(p, t);
+        else ti.n_iter = -1;
+        volatile int* a = reinterpret_cast<volatile int*>(s_next + slot * 3);
+        a[0] = ti.b;
+        a[1] = ti.hk;
+        a[2] = ti.n0;
+        a[3] = ti.n_iter;
+        a[4] = ti.m_start;
+        a[5] = ti.n_m;
+        a[6] = ti.g0;
+        a[7] = ti.mi0;
+        a[8] = ti.part;
+        a[9] = ti.parts;
+        mbar_arrive(&next_full[slot]);
+      } while (ti.n_iter >= 0);
       if (!ok) {
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000) {
@@ -330,8 +430,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       // plus a constant: its byte offset / 16, and for the MN-major views the larger leading offset.
       const uint64_t base = make_smem_desc(smem_u32(smem), 16, 1024);
       constexpr uint64_t kMn = static_cast<uint64_t>(((kBlk * 128) >> 4) - 1) << 16;
-      const uint64_t k_kmaj = base + (Cfg::kKOff >> 4), k_mn = k_kmaj + kMn;
-      const uint64_t v_kmaj = base + (Cfg::kVOff >> 4);
+      const uint64_t k0_kmaj = base + (Cfg::kKOff >> 4), v0_kmaj = base + (Cfg::kVOff >> 4);
       const uint64_t q_kmaj = base + (Cfg::kQOff >> 4), q_mn = q_kmaj + kMn;
       const uint64_t do_kmaj = base + (Cfg::kDOOff >> 4), do_mn = do_kmaj + kMn;
       const uint64_t ds_kmaj = base + (Cfg::kDSOff >> 4), ds_mn = ds_kmaj + kMn;
@@ -345,6 +444,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       // Packed batches: a tile that reaches past the end of its sequence holds rows of the next sequence; it
       // is usable once the fixer warp has cleared them. bit st of *_par: parity of the stage's next fix.
       constexpr bool packed = PACKED;
+      KvTile ti = first_tile;
+      Pos pos;
       uint32_t qfix_par = 0, dofix_par = 0;
       auto ragged_q = [&](int mi) { return packed && (ti.m_start + mi) * kBlk + kBlk > ti.sq; };
       auto q_ready = [&](int mi, uint32_t st, uint32_t ph, int code) -> bool {
@@ -361,85 +462,106 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         dofix_par ^= 1u << st;
         return mbar_wait(&do_fixed[st], par, ctl, kWaitBwd + 22);
       };
-      bool ok = n_iter > 0;
-      if (ok) ok = mbar_wait(kv_full, 0, ctl, kWaitBwd + 3);
-      if (ok && packed && ti.n0 + kBlk > ti.sk) ok = mbar_wait(kv_fixed, 0, ctl, kWaitBwd + 20);
-      if (ok) ok = q_ready(ti.mi0, 0, 0, kWaitBwd + 4);
-      if (ok) {
-        tc_fence_after();
-        kmajor_pair(tmem + Cfg::kTmemS, k_kmaj, q_kmaj);
-        mma_commit(s_full);
-        ok = do_ready(ti.mi0, 0, 0, kWaitBwd + 5);
-        if (ok) ok = mbar_wait(v_full, 0, ctl, kWaitBwd + 3);
-      }
-      if (ok) {
-        tc_fence_after();
-        kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj);
-        mma_commit(dp_full);
-      }
-      Walk wn{ti.g0, ti.mi0};  // position of iteration it + 1
-      for (int it = 0; it < n_iter && ok; ++it) {
-        wn = walk_next(wn, ti.n_m);
-        const uint32_t st = it & 1;
-        const uint32_t nph = ((it + 1) >> 1) & 1;  // phase of the Q stage barriers of iteration it + 1
-        const uint32_t dst = it % Cfg::kDOStages, ndst = (it + 1) % Cfg::kDOStages;
-        const uint32_t ndph = ((it + 1) / Cfg::kDOStages) & 1;
-        const bool has_next = it + 1 < n_iter;
-        const uint32_t acc = it > 0 ? 1u : 0u;
-        // dV += P^T dO   (P^T: two 32-column halves at S + 0 and S + 64)
-        ok = mbar_wait(p_full, it & 1, ctl, kWaitBwd + 6);
-        if (!ok) break;
-        tc_fence_after();
-        if (want_dkv) {
-          const uint64_t b = do_mn + dst * kTile16;
-          static_for<kBlk / 16>([&](auto ks) {
-            mma_ts_o<(ks.value / 4) * 64 + (ks.value % 4) * 8, ks.value * (2048 >> 4)>(
-                tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv, ks.value > 0 ? 1u : acc);
-          });
+      bool ok = true;
+      do {
+        const int n_iter = ti.n_iter;
+        const uint32_t ks = pos.kv % Cfg::kKVStages, kph = (pos.kv / Cfg::kKVStages) & 1;
+        const uint64_t k_kmaj = k0_kmaj + ks * kTile16, k_mn = k_kmaj + kMn, v_kmaj = v0_kmaj + ks * kTile16;
+        const uint32_t st0 = pos.it0 & 1, dst0 = pos.it0 % Cfg::kDOStages;
+        if (n_iter > 0) {
+          ok = mbar_wait(&k_full[ks], kph, ctl, kWaitBwd + 3);
+          if (ok && packed && ti.n0 + kBlk > ti.sk) ok = mbar_wait(kv_fixed, 0, ctl, kWaitBwd + 20);
+          if (ok) ok = q_ready(ti.mi0, st0, (pos.it0 >> 1) & 1, kWaitBwd + 4);
+          if (ok) {
+            tc_fence_after();
+            kmajor_pair(tmem + Cfg::kTmemS, k_kmaj, q_kmaj + st0 * kTile16);
+            mma_commit(s_full);
+            ok = do_ready(ti.mi0, dst0, (pos.it0 / Cfg::kDOStages) & 1, kWaitBwd + 5);
+            if (ok) ok = mbar_wait(&v_full[ks], kph, ctl, kWaitBwd + 3);
+            // the columns of dP^T still hold the last dQ of the tile before
+            if (ok && want_dq && pos.it0 > 0) ok = mbar_wait(dq_free, (pos.it0 - 1) & 1, ctl, kWaitBwd + 10);
+          }
+          if (ok) {
+            tc_fence_after();
+            kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj + dst0 * kTile16);
+            mma_commit(dp_full);
+          }
         }
-        mma_commit(&do_empty[dst]);
-        if (!has_next) mma_commit(dv_done);  // dV is final: its epilogue runs beside the last dQ and dK GEMMs
-        // S^T of the next iteration right behind dV, the last reader of P^T: the scores are there when the
-        // compute warps come out of phase B.
-        if (has_next) {
-          ok = q_ready(wn.mi, st ^ 1, nph, kWaitBwd + 8);
+        Walk wn{ti.g0, ti.mi0};  // position of iteration it + 1
+        for (int it = 0; it < n_iter && ok; ++it) {
+          wn = walk_next(wn, ti.n_m);
+          const uint32_t gi = pos.it0 + it;
+          const uint32_t st = gi & 1;
+          const uint32_t nph = ((gi + 1) >> 1) & 1;  // phase of the Q stage barriers of the next iteration
+          const uint32_t dst = gi % Cfg::kDOStages, ndst = (gi + 1) % Cfg::kDOStages;
+          const uint32_t ndph = ((gi + 1) / Cfg::kDOStages) & 1;
+          const bool has_next = it + 1 < n_iter;
+          const uint32_t acc = it > 0 ? 1u : 0u;
+          // dV += P^T dO   (P^T: two 32-column halves at S + 0 and S + 64)
+          ok = mbar_wait(p_full, gi & 1, ctl, kWaitBwd + 6);
           if (!ok) break;
           tc_fence_after();
-          kmajor_pair(tmem + Cfg::kTmemS, k_kmaj, q_kmaj + (st ^ 1) * kTile16);
-          mma_commit(s_full);
-        }
-        // dQ = dS K   (into the dP^T columns, which the compute warps have drained)
-        ok = mbar_wait(ds_full, it & 1, ctl, kWaitBwd + 7);
-        if (!ok) break;
-        tc_fence_after();
-        if (want_dq) {
-          static_for<kBlk / 16>([&](auto ks) {
-            mma_ss_o<ks.value * (2048 >> 4), ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDP, ds_mn, k_mn, idesc_dq,
-                                                                      ks.value > 0 ? 1u : 0u);
-          });
-          mma_commit(dq_full);
-        }
-        // dK += dS^T Q
-        if (want_dkv) {
-          const uint64_t b = q_mn + st * kTile16;
-          static_for<kBlk / 16>([&](auto ks) {
-            mma_ss_o<(ks.value / 4) * kAtom16 + (ks.value % 4) * 2, ks.value * (2048 >> 4)>(
-                tmem + Cfg::kTmemDK, ds_kmaj, b, idesc_dv, ks.value > 0 ? 1u : acc);
-          });
-        }
-        mma_commit(&q_empty[st]);
-        // dP^T of the next iteration, once the dQ tile has left TMEM
-        if (has_next) {
-          ok = do_ready(wn.mi, ndst, ndph, kWaitBwd + 9);
-          if (ok && want_dq) ok = mbar_wait(dq_free, it & 1, ctl, kWaitBwd + 10);
+          if (want_dkv) {
+            const uint64_t b = do_mn + dst * kTile16;
+            static_for<kBlk / 16>([&](auto ks) {
+              mma_ts_o<(ks.value / 4) * 64 + (ks.value % 4) * 8, ks.value * (2048 >> 4)>(
+                  tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv, ks.value > 0 ? 1u : acc);
+            });
+          }
+          mma_commit(&do_empty[dst]);
+          if (!has_next) {
+            mma_commit(dv_done);  // dV is final: its epilogue runs beside the last dQ and dK GEMMs
+            mma_commit(&v_empty[ks]);
+          }
+          // S^T of the next iteration right behind dV, the last reader of P^T: the scores are there when the
+          // compute warps come out of phase B.
+          if (has_next) {
+            ok = q_ready(wn.mi, st ^ 1, nph, kWaitBwd + 8);
+            if (!ok) break;
+            tc_fence_after();
+            kmajor_pair(tmem + Cfg::kTmemS, k_kmaj, q_kmaj + (st ^ 1) * kTile16);
+            mma_commit(s_full);
+          }
+          // dQ = dS K   (into the dP^T columns, which the compute warps have drained)
+          ok = mbar_wait(ds_full, gi & 1, ctl, kWaitBwd + 7);
           if (!ok) break;
           tc_fence_after();
-          kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj + ndst * kTile16);
-          mma_commit(dp_full);
+          if (want_dq) {
+            static_for<kBlk / 16>([&](auto ks) {
+              mma_ss_o<ks.value * (2048 >> 4), ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDP, ds_mn, k_mn, idesc_dq,
+                                                                        ks.value > 0 ? 1u : 0u);
+            });
+            mma_commit(dq_full);
+          }
+          if (!has_next) mma_commit(&k_empty[ks]);
+          // dK += dS^T Q
+          if (want_dkv) {
+            const uint64_t b = q_mn + st * kTile16;
+            static_for<kBlk / 16>([&](auto ks) {
+              mma_ss_o<(ks.value / 4) * kAtom16 + (ks.value % 4) * 2, ks.value * (2048 >> 4)>(
+                  tmem + Cfg::kTmemDK, ds_kmaj, b, idesc_dv, ks.value > 0 ? 1u : acc);
+            });
+          }
+          mma_commit(&q_empty[st]);
+          // dP^T of the next iteration, once the dQ tile has left TMEM
+          if (has_next) {
+            ok = do_ready(wn.mi, ndst, ndph, kWaitBwd + 9);
+            if (ok && want_dq) ok = mbar_wait(dq_free, gi & 1, ctl, kWaitBwd + 10);
+            if (!ok) break;
+            tc_fence_after();
+            kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj + ndst * kTile16);
+            mma_commit(dp_full);
+          }
         }
-      }
-      if (ok) mma_commit(dkv_done);
-    } else if (PACKED && warp == 2 && n_iter > 0) {
+        if (ok && n_iter > 0) mma_commit(dkv_done);
+        if (!ok || !kPersistent) break;
+        const uint32_t slot = pos.n & 1;
+        ok = next_tile(ti, pos);
+        mbar_arrive(&next_empty[slot]);
+      } while (ok);
+    } else if (PACKED && warp == 2 && first_tile.n_iter > 0) {
+      const KvTile& ti = first_tile;
+      const int n_iter = ti.n_iter;
       // ---------------------------------------------------------------- fixer (packed batches)
       // The reference zero-fills the rows of a tile that lie past the end of the sequence while staging it
       // (flash-attn2-rs/src/device/varlen/backward.rs:134-648 through the zfill copies of
@@ -462,7 +584,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       bool ok = true;
       const int kv_first = ti.sk - ti.n0;
       if (kv_first < kBlk) {
-        ok = __all_sync(0xffffffffu, mbar_wait(kv_full, 0, ctl, kWaitBwd + 3) && mbar_wait(v_full, 0, ctl, kWaitBwd + 3));
+        ok = __all_sync(0xffffffffu, mbar_wait(k_full, 0, ctl, kWaitBwd + 3) && mbar_wait(v_full, 0, ctl, kWaitBwd + 3));
         if (ok) {
           clear_rows(s_k, kv_first);
           clear_rows(s_v, kv_first);
@@ -488,6 +610,35 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         if (ok && lane == 0) mbar_arrive(&do_empty[dst]);
         __syncwarp();
       }
+    } else if (warp == 3) {
+      // ---------------------------------------------------------------- -LSE (log2 domain) and -delta of a query block
+      // Rows past the sequence give P = 0. Two buffers: the values of the next iteration, and of the next tile, are in
+      // shared memory before the compute warps ask for them.
+      KvTile ti = first_tile;
+      Pos pos;
+      bool ok = true;
+      do {
+        Walk w{ti.g0, ti.mi0};
+        for (int it = 0; it < ti.n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
+          const int hq = ti.hk * p.group + w.g, q0 = (ti.m_start + w.mi) * kBlk + lane;
+          const float* lse = p.lse + ti.bq * p.lse_batch_stride + hq * p.lse_head_stride + ti.q_row0;
+          const float* delta = p.delta + ti.bq * p.delta_batch_stride + hq * p.delta_head_stride + ti.q_row0 + ti.b * p.delta_seq_pad;
+          float v[8];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int q = q0 + 32 * i;
+            v[i] = q < ti.sq ? lse[q] * -kLog2e : -INFINITY;
+            v[4 + i] = q < ti.sq ? -delta[q] : 0.f;
+          }
+          const uint32_t gi = pos.it0 + it, buf = gi & 1;
+          ok = warp_wait(&stat_empty[buf], ((gi >> 1) & 1) ^ 1, ctl, kWaitBwd + 15);
+          float* stat = s_stat + buf * (2 * kBlk) + lane;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) stat[32 * i] = v[i];
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&stat_full[buf]);
+        }
+      } while (kPersistent && ok && next_tile_warp(ti, pos));
     }
   } else if (warp < 12) {
     // ------------------------------------------------------------------ compute
@@ -495,238 +646,258 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     const int cw = warp - 4;
     const int wg = cw >> 2;                 // which 64 query columns
     const int key_in = (cw & 3) * 32 + lane;
-    const int ct = tid - 128;               // 0..255
     const uint32_t lane_addr = static_cast<uint32_t>((cw & 3) * 32) << 16;
     const uint32_t t_s = tmem + lane_addr + Cfg::kTmemS + wg * 64;
     const uint32_t t_dp = tmem + lane_addr + Cfg::kTmemDP + wg * 64;
-    const int kpos = ti.n0 + key_in;
     bool ok = true;
-    // LSE (log2 domain) and delta of one query block: thread ct < 128 loads LSE of row ct, the others
-    // delta of row ct - 128; rows past the sequence give P = 0. The value for iteration it + 1 is
-    // requested while iteration it computes, so its latency never sits in front of phase A.
-    auto load_stat = [&](Walk w) -> float {
-      const int hq = ti.hk * p.group + w.g;
-      const int q = (ti.m_start + w.mi) * kBlk + (ct & 127);
-      if (ct < kBlk) {
-        float v = INFINITY;
-        if (q < ti.sq) v = p.lse[ti.bq * p.lse_batch_stride + hq * p.lse_head_stride + ti.q_row0 + q] * kLog2e;
-        return v;
-      }
-      float v = 0.f;
-      if (q < ti.sq)
-        v = p.delta[ti.bq * p.delta_batch_stride + hq * p.delta_head_stride + ti.q_row0 + ti.b * p.delta_seq_pad + q];
-      return v;
-    };
     constexpr bool fancy = MODE == kScoreAny;
     const float inv_cap1 = MODE == kScoreSoftcap ? p.scale / p.softcap : 0.f;
     const float cap1 = p.softcap * kLog2e;
-    Walk w{ti.g0, ti.mi0};
-    float stat_next = n_iter > 0 ? load_stat(w) : 0.f;
-    for (int it = 0; it < n_iter; ++it) {
-      const int m0 = (ti.m_start + w.mi) * kBlk;
-      const int g_cur = w.g;
-      w = walk_next(w, ti.n_m);
-      float* stat = s_stat + (it & 1) * (2 * kBlk);
-      stat[ct] = stat_next;
-      if (it + 1 < n_iter) stat_next = load_stat(w);
-      mbar_arrive(stat_full);
-      const bool stat_ok = mbar_wait(stat_full, it & 1, ctl, kWaitBwd + 15);  // voted on with s_full below
-      const float4* lse4 = reinterpret_cast<const float4*>(stat + wg * 64);
-      const float4* dl4 = reinterpret_cast<const float4*>(stat + kBlk + wg * 64);
+    KvTile ti = first_tile;
+    Pos pos;
+    do {
+      const int n_iter = ti.n_iter;
+      const int kpos = ti.n0 + key_in;
+      Walk w{ti.g0, ti.mi0};
+      for (int it = 0; it < n_iter; ++it) {
+        const int m0 = (ti.m_start + w.mi) * kBlk;
+        const int g_cur = w.g;
+        w = walk_next(w, ti.n_m);
+        const uint32_t gi = pos.it0 + it, par = gi & 1;
+        const float* stat = s_stat + par * (2 * kBlk);
+        const bool stat_ok = mbar_wait(&stat_full[par], (gi >> 1) & 1, ctl, kWaitBwd + 15);  // voted on with s_full below
+        const float4* lse4 = reinterpret_cast<const float4*>(stat + wg * 64);
+        const float4* dl4 = reinterpret_cast<const float4*>(stat + kBlk + wg * 64);
 
-      // ---- phase A: P^T = exp2(S^T c - lse)
-      if (!__all_sync(0xffffffffu, mbar_wait(s_full, it & 1, ctl, kWaitBwd + 11) && stat_ok)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t sr[64];
-      tmem_ld32(t_s, sr);
-      tmem_ld32(t_s + 32, sr + 32);
-      tmem_wait_ld();
-      const int qbase = m0 + wg * 64;
-      bool need_mask = (ti.n0 + kBlk > ti.sk);
-      if (p.window_right >= 0) need_mask |= (ti.n0 + kBlk - 1 > m0 + ti.off + p.window_right);
-      if (p.window_left >= 0) need_mask |= (ti.n0 < m0 + kBlk - 1 + ti.off - p.window_left);
-      int c_lo = 0, c_hi = 64;
-      if (need_mask) {
-        if (p.window_right >= 0) c_lo = kpos - ti.off - p.window_right - qbase;
-        if (p.window_left >= 0) c_hi = kpos - ti.off + p.window_left + 1 - qbase;
-        if (kpos >= ti.sk) c_hi = -1;
-      }
-      float pr[64];
-      if constexpr (MODE == kScoreSoftcap) {
-        // P = exp2(cap tanh - lse); dS takes P times the derivative of the cap, 1 - tanh^2.
-#pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          const float4 l4 = lse4[i / 4];
-          const float l[4] = {l4.x, l4.y, l4.z, l4.w};
-          float pp[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float t = tanh_approx(__uint_as_float(sr[i + e]) * inv_cap1);
-            pp[e] = ex2(fmaf(t, cap1, -l[e]));
-            if (need_mask && (i + e < c_lo || i + e >= c_hi)) pp[e] = 0.f;
-            pr[i + e] = pp[e] * fmaf(-t, t, 1.f);
-          }
-          sr[i / 2] = pack2<BF16>(pp[0], pp[1]);
-          sr[i / 2 + 1] = pack2<BF16>(pp[2], pp[3]);
-        }
-      } else if (!fancy) {
-        // The bias of a key is the same for all queries in the causal form of ALiBi.
-        float slope1 = 0.f, bias1 = 0.f;
-        if constexpr (MODE == kScoreAlibi) {
-          slope1 = p.alibi[ti.b * p.alibi_batch_stride + ti.hk * p.group + g_cur] * kLog2e;
-          bias1 = slope1 * static_cast<float>(kpos);
-          if (!p.causal_alibi) {
-            const float dist = static_cast<float>(qbase + ti.off - kpos);
-            bias1 = 0.f;
-#pragma unroll
-            for (int i = 0; i < 64; ++i)
-              sr[i] = __float_as_uint(fmaf(-slope1, fabsf(dist + static_cast<float>(i)), __uint_as_float(sr[i]) * p.scale_log2));
-          }
-        }
-        auto bias_minus = [&](float l) { return MODE == kScoreAlibi ? bias1 - l : -l; };
-        const float mul1 = MODE == kScoreAlibi && !p.causal_alibi ? 1.f : p.scale_log2;
-#pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          const float4 l4 = lse4[i / 4];
-          pr[i] = ex2(fmaf(__uint_as_float(sr[i]), mul1, bias_minus(l4.x)));
-          pr[i + 1] = ex2(fmaf(__uint_as_float(sr[i + 1]), mul1, bias_minus(l4.y)));
-          pr[i + 2] = ex2(fmaf(__uint_as_float(sr[i + 2]), mul1, bias_minus(l4.z)));
-          pr[i + 3] = ex2(fmaf(__uint_as_float(sr[i + 3]), mul1, bias_minus(l4.w)));
-        }
-        if (need_mask) {
-          fill_outside<64>(pr, c_lo, c_hi, 0.f);
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) sr[i] = pack2<BF16>(pr[2 * i], pr[2 * i + 1]);
-      } else {
-        // softcap / ALiBi: P follows the transformed scores of the forward; what goes on to dS is
-        // P times the derivative of the transform, 1 - tanh^2 (the ALiBi bias is a constant).
-        const int hq = ti.hk * p.group + g_cur;
-        const float slope = (p.alibi != nullptr) ? p.alibi[ti.b * p.alibi_batch_stride + hq] * kLog2e : 0.f;
-        const float inv_cap = (p.softcap > 0.f) ? p.scale / p.softcap : 0.f;
-        const float cap_l2 = p.softcap * kLog2e;
-#pragma unroll
-        for (int i = 0; i < 64; i += 2) {
-          float pp[2], dd[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float raw = __uint_as_float(sr[i + e]);
-            float x, deriv = 1.f;
-            if (p.softcap > 0.f) {
-              const float t = tanh_approx(raw * inv_cap);
-              x = cap_l2 * t;
-              deriv = fmaf(-t, t, 1.f);
-            } else {
-              x = raw * p.scale_log2;
-            }
-            if (p.alibi != nullptr)
-              x += p.causal_alibi ? slope * static_cast<float>(kpos)
-                                  : -slope * fabsf(static_cast<float>(qbase + i + e + ti.off - kpos));
-            const float l = reinterpret_cast<const float*>(lse4)[i + e];
-            float pv = ex2(x - l);
-            if (need_mask && (i + e < c_lo || i + e >= c_hi)) pv = 0.f;
-            pp[e] = pv;
-            dd[e] = pv * deriv;
-          }
-          sr[i / 2] = pack2<BF16>(pp[0], pp[1]);
-          pr[i] = dd[0];
-          pr[i + 1] = dd[1];
-        }
-      }
-      tmem_st32(t_s, sr);
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(p_full);
-
-      // ---- phase B: dS^T = P^T (dP^T - delta)
-      if (!warp_wait(dp_full, it & 1, ctl, kWaitBwd + 12)) { ok = false; break; }
-      tc_fence_after();
-      tmem_ld32(t_dp, sr);
-      tmem_ld32(t_dp + 32, sr + 32);
-      tmem_wait_ld();
-      tc_fence_before();
-      uint8_t* ds_row = s_ds + wg * (kBlk * 128) + key_in * 128;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 d0 = dl4[2 * c], d1 = dl4[2 * c + 1];
-        const int i = c * 8;
-        uint4 w;
-        w.x = pack2<BF16>(pr[i] * (__uint_as_float(sr[i]) - d0.x), pr[i + 1] * (__uint_as_float(sr[i + 1]) - d0.y));
-        w.y = pack2<BF16>(pr[i + 2] * (__uint_as_float(sr[i + 2]) - d0.z), pr[i + 3] * (__uint_as_float(sr[i + 3]) - d0.w));
-        w.z = pack2<BF16>(pr[i + 4] * (__uint_as_float(sr[i + 4]) - d1.x), pr[i + 5] * (__uint_as_float(sr[i + 5]) - d1.y));
-        w.w = pack2<BF16>(pr[i + 6] * (__uint_as_float(sr[i + 6]) - d1.z), pr[i + 7] * (__uint_as_float(sr[i + 7]) - d1.w));
-        *reinterpret_cast<uint4*>(ds_row + ((c ^ (key_in & 7)) << 4)) = w;
-      }
-      fence_proxy_async_smem();
-      mbar_arrive(ds_full);
-    }
-    // ---- epilogue: warpgroup 0 writes dK (scaled), warpgroup 1 writes dV
-    if (ok) {
-      const uint32_t t_acc = tmem + lane_addr + (wg == 0 ? Cfg::kTmemDK : Cfg::kTmemDV);
-      const float mul = (wg == 0) ? p.scale : 1.f;
-      const CUtensorMap* tm = (wg == 0) ? &p.tm_dk : &p.tm_dv;
-      uint16_t* gptr = reinterpret_cast<uint16_t*>(wg == 0 ? p.dk_ptr : p.dv_ptr);
-      const bool store = (p.which & 2) != 0;
-      const bool tma_store = !PACKED || (ti.n0 + kBlk <= ti.sk);
-      // Staging tile of the bulk store: the K tile for dK, the V tile for dV (their last readers have completed
-      // with dkv_done; the Q and dO stages may still hold dQ pieces of the last iteration's drain).
-      uint8_t* stage = (wg == 0) ? s_k : s_v;
-      bool done = true;
-      if (n_iter > 0) done = warp_wait(wg == 0 ? dkv_done : dv_done, 0, ctl, kWaitBwd + 13);
-      if (done && store) {
+        // ---- phase A: P^T = exp2(S^T c - lse)
+        if (!__all_sync(0xffffffffu, mbar_wait(s_full, par, ctl, kWaitBwd + 11) && stat_ok)) { ok = false; break; }
         tc_fence_after();
-        uint16_t* grow = gptr + ti.bq * p.dkv_batch_stride + static_cast<int64_t>(ti.k_row0 + kpos) * p.dkv_row_stride +
-                         ti.hk * p.dkv_head_stride;
-        uint32_t acc[D];
-        if (n_iter > 0) {
-#pragma unroll
-          for (int c = 0; c < D / 32; ++c) tmem_ld32(t_acc + c * 32, acc + c * 32);
-          tmem_wait_ld();
-        } else {
-#pragma unroll
-          for (int i = 0; i < D; ++i) acc[i] = 0;
+        uint32_t sr[64];
+        tmem_ld32(t_s, sr);
+        tmem_ld32(t_s + 32, sr + 32);
+        tmem_wait_ld();
+        const int qbase = m0 + wg * 64;
+        bool need_mask = (ti.n0 + kBlk > ti.sk);
+        if (p.window_right >= 0) need_mask |= (ti.n0 + kBlk - 1 > m0 + ti.off + p.window_right);
+        if (p.window_left >= 0) need_mask |= (ti.n0 < m0 + kBlk - 1 + ti.off - p.window_left);
+        int c_lo = 0, c_hi = 64;
+        if (need_mask) {
+          if (p.window_right >= 0) c_lo = kpos - ti.off - p.window_right - qbase;
+          if (p.window_left >= 0) c_hi = kpos - ti.off + p.window_left + 1 - qbase;
+          if (kpos >= ti.sk) c_hi = -1;
         }
-        if (!PACKED && ti.parts > 1) {
-          // A part of a split key block: fp32, 32 bytes (a whole sector) per store.
-          if (kpos < ti.sk) {
-            float* row = (wg == 0 ? p.dk_part : p.dv_part) + ti.part * p.part_stride + ti.bq * p.dkv_batch_stride +
-                         static_cast<int64_t>(kpos) * p.dkv_row_stride + ti.hk * p.dkv_head_stride;
+        float pr[64];
+        if constexpr (MODE == kScoreSoftcap) {
+          // P = exp2(cap tanh - lse); dS takes P times the derivative of the cap, 1 - tanh^2.
 #pragma unroll
-            for (int c = 0; c < D / 8; ++c)
-              if (c * 8 < p.head_dim)
-                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(row + 8 * c), "r"(acc[8 * c]),
-                             "r"(acc[8 * c + 1]), "r"(acc[8 * c + 2]), "r"(acc[8 * c + 3]), "r"(acc[8 * c + 4]),
-                             "r"(acc[8 * c + 5]), "r"(acc[8 * c + 6]), "r"(acc[8 * c + 7])
-                             : "memory");
+          for (int i = 0; i < 64; i += 4) {
+            const float4 l4 = lse4[i / 4];
+            const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+            float pp[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float t = tanh_approx(__uint_as_float(sr[i + e]) * inv_cap1);
+              pp[e] = ex2(fmaf(t, cap1, l[e]));
+              if (need_mask && (i + e < c_lo || i + e >= c_hi)) pp[e] = 0.f;
+              pr[i + e] = pp[e] * fmaf(-t, t, 1.f);
+            }
+            sr[i / 2] = pack2<BF16>(pp[0], pp[1]);
+            sr[i / 2 + 1] = pack2<BF16>(pp[2], pp[3]);
           }
+        } else if (!fancy) {
+          // The bias of a key is the same for all queries in the causal form of ALiBi.
+          float slope1 = 0.f, bias1 = 0.f;
+          if constexpr (MODE == kScoreAlibi) {
+            slope1 = p.alibi[ti.b * p.alibi_batch_stride + ti.hk * p.group + g_cur] * kLog2e;
+            bias1 = slope1 * static_cast<float>(kpos);
+            if (!p.causal_alibi) {
+              const float dist = static_cast<float>(qbase + ti.off - kpos);
+              bias1 = 0.f;
+#pragma unroll
+              for (int i = 0; i < 64; ++i)
+                sr[i] = __float_as_uint(fmaf(-slope1, fabsf(dist + static_cast<float>(i)), __uint_as_float(sr[i]) * p.scale_log2));
+            }
+          }
+          const float mul1 = MODE == kScoreAlibi && !p.causal_alibi ? 1.f : p.scale_log2;
+          const uint64_t c2 = pack_f32x2(mul1, mul1), bias2 = pack_f32x2(bias1, bias1);
+#pragma unroll
+          for (int i = 0; i < 64; i += 4) {
+            const float4 l4 = lse4[i / 4];
+            uint64_t n0 = pack_f32x2(l4.x, l4.y), n1 = pack_f32x2(l4.z, l4.w);
+            if constexpr (MODE == kScoreAlibi) {
+              n0 = add2(n0, bias2);
+              n1 = add2(n1, bias2);
+            }
+            unpack_f32x2(fma2(pack_f32x2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, n0), pr[i], pr[i + 1]);
+            unpack_f32x2(fma2(pack_f32x2(__uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3])), c2, n1), pr[i + 2], pr[i + 3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) pr[i + e] = ex2(pr[i + e]);
+          }
+          if (need_mask) {
+            fill_outside<64>(pr, c_lo, c_hi, 0.f);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sr[i] = pack2<BF16>(pr[2 * i], pr[2 * i + 1]);
         } else {
+          // softcap / ALiBi: P follows the transformed scores of the forward; what goes on to dS is
+          // P times the derivative of the transform, 1 - tanh^2 (the ALiBi bias is a constant).
+          const int hq = ti.hk * p.group + g_cur;
+          const float slope = (p.alibi != nullptr) ? p.alibi[ti.b * p.alibi_batch_stride + hq] * kLog2e : 0.f;
+          const float inv_cap = (p.softcap > 0.f) ? p.scale / p.softcap : 0.f;
+          const float cap_l2 = p.softcap * kLog2e;
 #pragma unroll
-          for (int c = 0; c < D / 8; ++c) {  // 16-byte chunks of the row
-            uint4 w;
-            w.x = pack2<BF16>(__uint_as_float(acc[8 * c]) * mul, __uint_as_float(acc[8 * c + 1]) * mul);
-            w.y = pack2<BF16>(__uint_as_float(acc[8 * c + 2]) * mul, __uint_as_float(acc[8 * c + 3]) * mul);
-            w.z = pack2<BF16>(__uint_as_float(acc[8 * c + 4]) * mul, __uint_as_float(acc[8 * c + 5]) * mul);
-            w.w = pack2<BF16>(__uint_as_float(acc[8 * c + 6]) * mul, __uint_as_float(acc[8 * c + 7]) * mul);
+          for (int i = 0; i < 64; i += 2) {
+            float pp[2], dd[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float raw = __uint_as_float(sr[i + e]);
+              float x, deriv = 1.f;
+              if (p.softcap > 0.f) {
+                const float t = tanh_approx(raw * inv_cap);
+                x = cap_l2 * t;
+                deriv = fmaf(-t, t, 1.f);
+              } else {
+                x = raw * p.scale_log2;
+              }
+              if (p.alibi != nullptr)
+                x += p.causal_alibi ? slope * static_cast<float>(kpos)
+                                    : -slope * fabsf(static_cast<float>(qbase + i + e + ti.off - kpos));
+              const float l = reinterpret_cast<const float*>(lse4)[i + e];
+              float pv = ex2(x + l);
+              if (need_mask && (i + e < c_lo || i + e >= c_hi)) pv = 0.f;
+              pp[e] = pv;
+              dd[e] = pv * deriv;
+            }
+            sr[i / 2] = pack2<BF16>(pp[0], pp[1]);
+            pr[i] = dd[0];
+            pr[i + 1] = dd[1];
+          }
+        }
+        tmem_st32(t_s, sr);
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(p_full);
+
+        // ---- phase B: dS^T = P^T (dP^T - delta)
+        if (!warp_wait(dp_full, par, ctl, kWaitBwd + 12)) { ok = false; break; }
+        tc_fence_after();
+        tmem_ld32(t_dp, sr);
+        tmem_ld32(t_dp + 32, sr + 32);
+        tmem_wait_ld();
+        tc_fence_before();
+        uint8_t* ds_row = s_ds + wg * (kBlk * 128) + key_in * 128;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float4 d0 = dl4[2 * c], d1 = dl4[2 * c + 1];
+          const int i = c * 8;
+          const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+          uint32_t ds[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int e = i + 2 * q;
+            const uint64_t dp = add2(pack_f32x2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), pack_f32x2(d[2 * q], d[2 * q + 1]));
+            float a, b;
+            unpack_f32x2(mul2(pack_f32x2(pr[e], pr[e + 1]), dp), a, b);
+            ds[q] = pack2<BF16>(a, b);
+          }
+          const uint4 w = make_uint4(ds[0], ds[1], ds[2], ds[3]);
+          *reinterpret_cast<uint4*>(ds_row + ((c ^ (key_in & 7)) << 4)) = w;
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(ds_full);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&stat_empty[par]);
+      }
+      // ---- epilogue: warpgroup 0 writes dK (scaled), warpgroup 1 writes dV
+      if (ok) {
+        const uint32_t t_acc = tmem + lane_addr + (wg == 0 ? Cfg::kTmemDK : Cfg::kTmemDV);
+        const float mul = (wg == 0) ? p.scale : 1.f;
+        uint16_t* gptr = reinterpret_cast<uint16_t*>(wg == 0 ? p.dk_ptr : p.dv_ptr);
+        const bool store = (p.which & 2) != 0;
+        if (n_iter > 0) ok = warp_wait(wg == 0 ? dkv_done : dv_done, pos.kv & 1, ctl, kWaitBwd + 13);
+        if (ok && store) {
+          tc_fence_after();
+          uint16_t* grow = gptr + ti.bq * p.dkv_batch_stride + static_cast<int64_t>(ti.k_row0 + kpos) * p.dkv_row_stride +
+                           ti.hk * p.dkv_head_stride;
+          uint32_t acc[D];
+          if (n_iter > 0) {
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) tmem_ld32(t_acc + c * 32, acc + c * 32);
+            tmem_wait_ld();
+          } else {
+#pragma unroll
+            for (int i = 0; i < D; ++i) acc[i] = 0;
+          }
+          if (!PACKED && ti.parts > 1) {
+            // A part of a split key block: fp32, 32 bytes (a whole sector) per store.
+            if (kpos < ti.sk) {
+              float* row = (wg == 0 ? p.dk_part : p.dv_part) + ti.part * p.part_stride + ti.bq * p.dkv_batch_stride +
+                           static_cast<int64_t>(kpos) * p.dkv_row_stride + ti.hk * p.dkv_head_stride;
+#pragma unroll
+              for (int c = 0; c < D / 8; ++c)
+                if (c * 8 < p.head_dim)
+                  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(row + 8 * c), "r"(acc[8 * c]),
+                               "r"(acc[8 * c + 1]), "r"(acc[8 * c + 2]), "r"(acc[8 * c + 3]), "r"(acc[8 * c + 4]),
+                               "r"(acc[8 * c + 5]), "r"(acc[8 * c + 6]), "r"(acc[8 * c + 7])
+                               : "memory");
+            }
+          } else if (kPersistent) {
+            // Straight to memory, 32 bytes (a whole sector) per store where the rows allow.
+            const bool sectors = (reinterpret_cast<uintptr_t>(gptr) & 31) == 0 && (p.head_dim & 15) == 0;
+            if (kpos < ti.sk) {
+#pragma unroll
+              for (int c = 0; c < D / 16; ++c) {
+                if (c * 16 >= p.head_dim) break;
+                uint32_t w[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  w[i] = pack2<BF16>(__uint_as_float(acc[16 * c + 2 * i]) * mul, __uint_as_float(acc[16 * c + 2 * i + 1]) * mul);
+                if (sectors) {
+                  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(grow + 16 * c), "r"(w[0]), "r"(w[1]),
+                               "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                               : "memory");
+                } else {
+                  *reinterpret_cast<uint4*>(grow + 16 * c) = make_uint4(w[0], w[1], w[2], w[3]);
+                  if (c * 16 + 8 < p.head_dim) *reinterpret_cast<uint4*>(grow + 16 * c + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                }
+              }
+            }
+          } else {
+            // Staging tile of the bulk store: the K tile for dK, the V tile for dV (their last readers have completed
+            // with dkv_done).
+            const bool tma_store = !PACKED || ti.n0 + kBlk <= ti.sk;
+            const CUtensorMap* tm = (wg == 0) ? &p.tm_dk : &p.tm_dv;
+            uint8_t* stage = (wg == 0) ? s_k : s_v;
+#pragma unroll
+            for (int c = 0; c < D / 8; ++c) {  // 16-byte chunks of the row
+              uint4 w;
+              w.x = pack2<BF16>(__uint_as_float(acc[8 * c]) * mul, __uint_as_float(acc[8 * c + 1]) * mul);
+              w.y = pack2<BF16>(__uint_as_float(acc[8 * c + 2]) * mul, __uint_as_float(acc[8 * c + 3]) * mul);
+              w.z = pack2<BF16>(__uint_as_float(acc[8 * c + 4]) * mul, __uint_as_float(acc[8 * c + 5]) * mul);
+              w.w = pack2<BF16>(__uint_as_float(acc[8 * c + 6]) * mul, __uint_as_float(acc[8 * c + 7]) * mul);
+              if (tma_store) {
+                *reinterpret_cast<uint4*>(stage + (c / 8) * (kBlk * 128) + key_in * 128 + (((c & 7) ^ (key_in & 7)) << 4)) = w;
+              } else if (kpos < ti.sk && c * 8 < p.head_dim) {
+                *reinterpret_cast<uint4*>(grow + c * 8) = w;
+              }
+            }
             if (tma_store) {
-              *reinterpret_cast<uint4*>(stage + (c / 8) * (kBlk * 128) + key_in * 128 + (((c & 7) ^ (key_in & 7)) << 4)) = w;
-            } else if (kpos < ti.sk && c * 8 < p.head_dim) {
-              *reinterpret_cast<uint4*>(grow + c * 8) = w;
-            }
-          }
-          if (tma_store) {
-            fence_proxy_async_smem();
-            mbar_arrive(&epi_full[wg]);
-            if ((ct & 127) == 0 && mbar_wait(&epi_full[wg], 0, ctl, kWaitBwd + 16)) {
+              fence_proxy_async_smem();
+              mbar_arrive(&epi_full[wg]);
+              if (key_in == 0 && mbar_wait(&epi_full[wg], 0, ctl, kWaitBwd + 16)) {
 #pragma unroll
-              for (int a = 0; a < Cfg::kAtoms; ++a)
-                if (a * 64 < p.head_dim) tma_store_4d(tm, stage + a * (kBlk * 128), a * 64, ti.hk, ti.k_row0 + ti.n0, ti.bq);
-              tma_commit_group();
-              tma_wait_group_read<0>();  // the staging tile must outlive the copy's reads, not its writes
+                for (int a = 0; a < Cfg::kAtoms; ++a)
+                  if (a * 64 < p.head_dim) tma_store_4d(tm, stage + a * (kBlk * 128), a * 64, ti.hk, ti.k_row0 + ti.n0, ti.bq);
+                tma_commit_group();
+                tma_wait_group_read<0>();  // the staging tile must outlive the copy's reads, not its writes
+              }
             }
           }
+          tc_fence_before();  // the next tile's dV and dK overwrite the accumulators behind its P^T
         }
       }
-    }
+      __syncwarp();
+    } while (kPersistent && ok && next_tile_warp(ti, pos));
   } else {
     // ------------------------------------------------------------------ dQ drain
     // The whole 128 x D fp32 tile goes to registers at once so that the dP^T / dQ columns are free
@@ -737,94 +908,99 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     const uint32_t t_dq = tmem + lane_addr + Cfg::kTmemDP;
     if (want_dq) {
       bool ok = true;
-      Walk w{ti.g0, ti.mi0};
-      for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
-        const int hq = ti.hk * p.group + w.g;
-        const int m0 = (ti.m_start + w.mi) * kBlk;
-        if (!warp_wait(dq_full, it & 1, ctl, kWaitBwd + 14)) break;
-        tc_fence_after();
-        uint32_t acc[D];
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) tmem_ld32(t_dq + c * 32, acc + c * 32);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(dq_free);
-        // Packed batches: the 32-row boxes of the reduce-adds below reach past the end of the sequence into
-        // the next sequence's rows. Rows past the end hold nothing of this sequence (and possibly NaN, when this
-        // sequence's own data is not finite): they add exact zeros.
-        if (PACKED && m0 + (warp & 3) * 32 + lane >= ti.sq) {
-#pragma unroll
-          for (int i = 0; i < D; ++i) acc[i] = 0u;
-        }
-        // Each warp drains its own 32 rows in pieces of 32 fp32 columns (4 KB) that roll through two buffers of its
-        // own, also from one tile to the next. Nothing but the warp itself has to be synchronised.
-        constexpr int kWarpPiece = Cfg::kPieceBytes / 4;
-        uint8_t* stage = smem + Cfg::kDQOff + (warp & 3) * (Cfg::kPieces * kWarpPiece);
-        int* turn = nullptr;
-        if (PACKED && p.dq_turn != nullptr) {
-          // Ordered mode: the key blocks that add into these rows take their turns in descending order,
-          // which is the order in which they get there under a causal or sliding-window mask (a higher key
-          // block starts at a later query block). This block's turn is the number of higher key blocks
-          // that cover the rows; a bounded wait for the slab's counter to reach it follows. In this mode the
-          // grid lists a head's key blocks highest first (get_kv_tile), so the blocks waited for started earlier.
-          const int mq = m0 / kBlk;
-          int rank = 0;
-          for (int nb = ti.n0 / kBlk + 1; nb < p.num_nblk; nb += 32) {
-            const int n = nb + lane;
-            bool covers = false;
-            if (n < p.num_nblk && n * kBlk < ti.sk) {
-              int ms, nm;
-              q_block_range(p, ti.sq, ti.sk, n * kBlk, ms, nm);
-              covers = (mq >= ms) && (mq < ms + nm);
-            }
-            rank += __popc(__ballot_sync(0xffffffffu, covers));
-          }
-          turn = p.dq_turn + ((static_cast<int64_t>(ti.b) * p.heads + hq) * p.num_mblk_q + mq) * 4 + (warp & 3);
-          if (lane == 0) {
-            const long long t0 = clock64();
-            while (*reinterpret_cast<volatile int*>(turn) != rank) {
-              __nanosleep(200);
-              if (*abort_flag || clock64() - t0 > FA2_WAIT_LIMIT_CYCLES) {
-                if (!*abort_flag) {
-                  *abort_flag = 1;
-                  if (p.status != nullptr) atomicCAS(p.status, 0, kWaitBwd + 19);
-                }
-                ok = false;
-                break;
-              }
-            }
-            __threadfence();
-          }
-          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      KvTile ti = first_tile;
+      Pos pos;
+      do {
+        Walk w{ti.g0, ti.mi0};
+        for (int it = 0; it < ti.n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
+          const int hq = ti.hk * p.group + w.g;
+          const int m0 = (ti.m_start + w.mi) * kBlk;
+          ok = warp_wait(dq_full, (pos.it0 + it) & 1, ctl, kWaitBwd + 14);
           if (!ok) break;
-        }
+          tc_fence_after();
+          uint32_t acc[D];
 #pragma unroll
-        for (int k = 0; k < D / 32; ++k) {
-          // The buffer is free once the reduce of the piece two before this one has read it.
-          if (lane == 0) tma_wait_group_read<Cfg::kPieces - 1>();
-          __syncwarp();
-          uint8_t* buf = stage + (k % Cfg::kPieces) * kWarpPiece;
-          uint8_t* rowp = buf + lane * 128;
+          for (int c = 0; c < D / 32; ++c) tmem_ld32(t_dq + c * 32, acc + c * 32);
+          tmem_wait_ld();
+          tc_fence_before();
+          mbar_arrive(dq_free);
+          // Packed batches: the 32-row boxes of the reduce-adds below reach past the end of the sequence into
+          // the next sequence's rows. Rows past the end hold nothing of this sequence (and possibly NaN, when this
+          // sequence's own data is not finite): they add exact zeros.
+          if (PACKED && m0 + (warp & 3) * 32 + lane >= ti.sq) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c)
-            *reinterpret_cast<uint4*>(rowp + ((c ^ (lane & 7)) << 4)) =
-                make_uint4(acc[k * 32 + 4 * c], acc[k * 32 + 4 * c + 1], acc[k * 32 + 4 * c + 2], acc[k * 32 + 4 * c + 3]);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (k * 32 < p.head_dim) tma_reduce_add_4d(&p.tm_dqa, buf, k * 32, hq, ti.q_row0 + m0 + (warp & 3) * 32, ti.bq);
-            tma_commit_group();
+            for (int i = 0; i < D; ++i) acc[i] = 0u;
+          }
+          // Each warp drains its own 32 rows in pieces of 32 fp32 columns (4 KB) that roll through two buffers of its
+          // own, also from one tile to the next. Nothing but the warp itself has to be synchronised.
+          constexpr int kWarpPiece = Cfg::kPieceBytes / 4;
+          uint8_t* stage = smem + Cfg::kDQOff + (warp & 3) * (Cfg::kPieces * kWarpPiece);
+          int* turn = nullptr;
+          if (PACKED && p.dq_turn != nullptr) {
+            // Ordered mode: the key blocks that add into these rows take their turns in descending order,
+            // which is the order in which they get there under a causal or sliding-window mask (a higher key
+            // block starts at a later query block). This block's turn is the number of higher key blocks
+            // that cover the rows; a bounded wait for the slab's counter to reach it follows. In this mode the
+            // grid lists a head's key blocks highest first (get_kv_tile), so the blocks waited for started earlier.
+            const int mq = m0 / kBlk;
+            int rank = 0;
+            for (int nb = ti.n0 / kBlk + 1; nb < p.num_nblk; nb += 32) {
+              const int n = nb + lane;
+              bool covers = false;
+              if (n < p.num_nblk && n * kBlk < ti.sk) {
+                int ms, nm;
+                q_block_range(p, ti.sq, ti.sk, n * kBlk, ms, nm);
+                covers = (mq >= ms) && (mq < ms + nm);
+              }
+              rank += __popc(__ballot_sync(0xffffffffu, covers));
+            }
+            turn = p.dq_turn + ((static_cast<int64_t>(ti.b) * p.heads + hq) * p.num_mblk_q + mq) * 4 + (warp & 3);
+            if (lane == 0) {
+              const long long t0 = clock64();
+              while (*reinterpret_cast<volatile int*>(turn) != rank) {
+                __nanosleep(200);
+                if (*abort_flag || clock64() - t0 > FA2_WAIT_LIMIT_CYCLES) {
+                  if (!*abort_flag) {
+                    *abort_flag = 1;
+                    if (p.status != nullptr) atomicCAS(p.status, 0, kWaitBwd + 19);
+                  }
+                  ok = false;
+                  break;
+                }
+              }
+              __threadfence();
+            }
+            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            if (!ok) break;
+          }
+#pragma unroll
+          for (int k = 0; k < D / 32; ++k) {
+            // The buffer is free once the reduce of the piece two before this one has read it.
+            if (lane == 0) tma_wait_group_read<Cfg::kPieces - 1>();
+            __syncwarp();
+            uint8_t* buf = stage + (k % Cfg::kPieces) * kWarpPiece;
+            uint8_t* rowp = buf + lane * 128;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<uint4*>(rowp + ((c ^ (lane & 7)) << 4)) =
+                  make_uint4(acc[k * 32 + 4 * c], acc[k * 32 + 4 * c + 1], acc[k * 32 + 4 * c + 2], acc[k * 32 + 4 * c + 3]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (k * 32 < p.head_dim) tma_reduce_add_4d(&p.tm_dqa, buf, k * 32, hq, ti.q_row0 + m0 + (warp & 3) * 32, ti.bq);
+              tma_commit_group();
+            }
+          }
+          if (!ok) break;
+          if (turn != nullptr && lane == 0) {
+            // The adds have to be in memory before the next key block may start on these rows.
+            tma_wait_group<0>();
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+            __threadfence();
+            atomicAdd(turn, 1);
           }
         }
-        if (!ok) break;
-        if (turn != nullptr && lane == 0) {
-          // The adds have to be in memory before the next key block may start on these rows.
-          tma_wait_group<0>();
-          asm volatile("fence.proxy.async.global;" ::: "memory");
-          __threadfence();
-          atomicAdd(turn, 1);
-        }
-      }
+      } while (kPersistent && ok && next_tile_warp(ti, pos));
       if (lane == 0) tma_wait_group_read<0>();
     }
   }
@@ -880,12 +1056,15 @@ cudaError_t pick_dtype(const BwdParams& p, bool bf16, int mode, bool packed, int
 
 }  // namespace
 
-cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int /*num_sms*/, cudaStream_t stream) {
+cudaError_t launch_bwd(BwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream) {
   const int num_ctas = (p.dk_part != nullptr ? p.items_per_head : p.num_nblk) * p.batch * p.heads_k;
   if (num_ctas <= 0) return cudaSuccess;
   if (head_dim <= 0 || head_dim > 128) return cudaErrorInvalidValue;
   const int mode = (p.softcap > 0.f ? kScoreSoftcap : 0) | (p.alibi != nullptr ? kScoreAlibi : 0);
   const bool packed = p.cu_q != nullptr;
+  // A CTA asks for its next tile before it has finished this one; in a call of a wave or two that takes tiles away from SMs
+  // that are about to be free (B1 H8/2 S1500 D64, bit-reproducible: 57.7 -> 59.5 us).
+  p.take_over = num_ctas > 2 * num_sms;
   return head_dim > 64 ? pick_dtype<128>(p, bf16, mode, packed, num_ctas, stream)
                        : pick_dtype<64>(p, bf16, mode, packed, num_ctas, stream);
 }

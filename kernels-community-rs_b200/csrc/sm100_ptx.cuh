@@ -127,6 +127,30 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
+// ---------------------------------------------------------------- next CTA of the grid
+// A running CTA takes over one that has not started. The request's answer (16 bytes) arrives in shared memory on an mbarrier
+// that expects them; no request may follow one that was turned down.
+__device__ __forceinline__ void ask_next_cta(uint32_t answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// Its x index, or -1 if there is none left. The fence orders the read before the answer is overwritten.
+__device__ __forceinline__ int next_cta(uint32_t answer) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 a;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 a, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n\t"
+      "fence.proxy.async.shared::cta;\n\t}"
+      : "=r"(x)
+      : "r"(answer)
+      : "memory");
+  return x;
+}
+
 // ---------------------------------------------------------------- dependent launch
 // The kernels are launched so that a grid may start while the one before it in the stream ends (launch_early). A grid
 // touches global memory only behind early_wait, which returns once everything before it in the stream has completed

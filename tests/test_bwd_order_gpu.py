@@ -48,3 +48,29 @@ def test_dkdv_beside_dq(shape):
         copies = [t.clone() for t in fa2.bwd(do, q, k, v, out, lse, is_causal=True, deterministic=True)[:3]]
     assert all(torch.equal(a, r) for a, r in zip(copies, (dq, dk, dv)))
     assert ops.device_status() == 0
+
+
+# (heads, heads_k, seqlen_q, seqlen_k, head_dim), options: more than two CTAs per SM, so that CTAs take over tiles of others
+TAKE_OVER = [((60, 60, 100, 1000, 64), dict(causal=True, window_left=300)),   # key blocks that no row sees, among the others
+             ((60, 60, 100, 1000, 40), dict(causal=True, window_left=300)),   # rows of 80 bytes
+             ((240, 240, 130, 200, 56), {}), ((700, 350, 5, 3, 64), {}), ((300, 75, 129, 129, 64), dict(causal=True, softcap=15.0))]
+
+
+@pytest.mark.parametrize("shape,opt", TAKE_OVER, ids=[str(c[0]) for c in TAKE_OVER])
+def test_tiles_taken_over_from_other_ctas(shape, opt):
+    from flash_attn2_b200 import cabi_ops as ops
+
+    h, hk, sq, sk, d = shape
+    q, k, v, do = [t.cuda() for t in make_qkv(7, 1, h, hk, sq, sk, d, torch.bfloat16, with_do=True)]
+    out, lse = ops.fwd(q, k, v, **opt)
+    delta = ops.bwd_preprocess(do, out)
+    dq, dk, dv = ops.bwd(q, k, v, do, lse, delta, **opt)
+    assert ops.device_status() == 0
+    torch.testing.assert_close(dq, ops.bwd(q, k, v, do, lse, delta, which=1, **opt)[0], atol=2e-2, rtol=2e-2)
+    g, few = h // hk, 5
+    for first in range(0, hk - few, max(1, hk // 7)):   # a few heads at a time: one wave
+        mine, own = slice(first * g, (first + few) * g), slice(first, first + few)
+        alone = ops.bwd(q[:, :, mine], k[:, :, own], v[:, :, own], do[:, :, mine], lse[:, mine].contiguous(),
+                        delta[:, mine].contiguous(), **opt)
+        assert torch.equal(alone[1], dk[:, :, own]) and torch.equal(alone[2], dv[:, :, own])
+    assert ops.device_status() == 0
