@@ -26,6 +26,12 @@ int shared_tiles(const fa2_fwd_args* a, int sms) {  // CTAs that share the call'
   fa2::plan_stream(a, sms, &p);
   return p.grid;
 }
+int few_rows_ctas(const fa2_fwd_args* a, int sms) { return fa2::decode_plan(a, sms).grid; }
+// heads whose key blocks (dq_alone: query blocks) a backward call lists together
+int head_group(const fa2_bwd_args* a, int dq_alone, int sms) {
+  const fa2::Windows w = fa2::normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
+  return dq_alone ? fa2::bwd_dq_head_group(a, w) : fa2::bwd_head_group(a, w, sms);
+}
 int64_t few_rows_workspace(const fa2_fwd_args* a, int sms) { return fa2::decode_plan(a, sms).workspace_bytes; }
 }
 '''
@@ -106,3 +112,30 @@ def test_tiles_are_shared_where_that_is_faster(plans, shape):
     h, sq, sk, d, causal = shape
     got = plans.shared_tiles(ctypes.byref(_fwd_args(1, h, h, sq, sk, d, causal=causal)), SMS)
     assert (got > 0) == (shape in SHARED)
+
+
+@pytest.mark.parametrize("sk", [2049, 4093, 6145, 8192, 9000, 30000])
+def test_a_unit_has_no_more_parts_than_shorten_the_longest(plans, sk):
+    args = _fwd_args(1, 32, 8, 1, sk, 128, causal=1)
+    tiles, most = -(-sk // 128), min(SMS // 8, 24, -(-sk // 128) // 3)
+    ctas = plans.few_rows_ctas(ctypes.byref(args), SMS)
+    assert ctas % 8 == 0
+    parts = ctas // 8
+    assert parts <= most and -(-tiles // parts) == -(-tiles // most) and (parts == 1 or -(-tiles // (parts - 1)) > -(-tiles // parts))
+
+
+# (batch, heads, heads_k, seqlen, head_dim), causal, heads in a group: all of them in a call of few CTAs; else equal groups of at
+# most 96 MB (25 MB a head: 9 groups of 32 heads; 3 MB: 9 of 256; 96 KB: 1024 heads), without a mask 16 MB (391 KB a head).
+GROUPS = [((4, 16, 4, 2048, 128), 1, 16), ((1, 32, 32, 16384, 128), 1, 4), ((16, 16, 16, 2048, 128), 1, 29),
+          ((32, 12, 12, 509, 64), 0, 43), ((1, 1, 1, 1, 8), 0, 1), ((65535, 64, 64, 128, 64), 1, 1024)]
+
+
+@pytest.mark.parametrize("shape,causal,want", GROUPS, ids=str)
+def test_heads_in_a_group(plans, shape, causal, want):
+    b, h, hk, s, d = shape
+    args = _bwd_args(b, h, hk, s, s, d)
+    args.causal = causal
+    assert plans.head_group(ctypes.byref(args), 0, SMS) == want
+    assert 1 <= plans.head_group(ctypes.byref(args), 1, SMS) <= b * h
+    args.cu_seqlens_q = 8  # packed sequences differ in length: one after the other
+    assert plans.head_group(ctypes.byref(args), 0, SMS) == 1
