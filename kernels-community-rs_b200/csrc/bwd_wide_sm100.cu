@@ -8,7 +8,7 @@
 //   S^T   = K Q^T                 smem x smem -> TMEM [128 keys x 64 q], over the whole head dim
 //   dP^T  = V dO^T                TMEM x smem: V sits in TMEM as a 16-bit A operand, written there once by the
 //                                 compute warps straight from global memory, which leaves its 64 KB of shared
-//                                 memory to a second Q / dO stage
+//                                 memory to more Q stages
 //   P^T   = exp2(S^T c - lse)     compute warps, written back over S^T as 16-bit
 //   dV_c += P^T dO_c              TMEM x smem (dO as an MN-major operand)
 //   dS^T  = P^T (dP^T - delta)    compute warps -> swizzled smem [128 keys x 64 q]
@@ -19,7 +19,7 @@
 //   dK_c += dS^T Q_c              smem x smem (Q as an MN-major operand)
 //
 // TMEM columns: dK_c [0,128) dV_c [128,256) S^T/P^T [256,320) dP^T/dQ_c^T [320,384) V [384,512).
-// Shared memory: K whole (64 KB), two stages of a Q and a dO tile of 64 rows (32 KB each), dS^T (16 KB),
+// Shared memory: K whole (64 KB), three stages of Q and one of dO, tiles of 64 rows (32 KB each), dS^T (16 KB),
 // dQ staging (16 KB).
 // Warps: 0-7 compute (two warpgroups, 32 query columns each, one key row per thread), 8-11 dQ drain (one d row of
 // dQ^T per thread), 12 loader, 13 MMA issuer, 14 fixer (packed batches: clears the rows of K, Q and dO tiles that lie
@@ -32,6 +32,9 @@
 // behind dV, the last reader of P^T: 5900. The drain has a staging buffer of its own, so the Q stage goes back to the
 // loader when dK has read it and not when the reductions have: 4800. Kernel at B4 H16/8 S2048 D256 causal bf16:
 // 833 -> 754 -> 610 us.
+// With two stages of each, S^T waited 560 cycles an iteration for Q, whose stage dK of the iteration before frees late, while
+// dO was there early: dV is its last reader, most of an iteration before the next dP^T. Three Q stages and one of dO:
+// forward and backward of that call 748 -> 705 us, B2 H16/4 S3000 D192 646 -> 630, B4 H8 S1000 D256 without a mask 223 -> 210.
 //
 // Stands in, for these head dims, for the reference kernels `backward` and `backward_kv`
 // (flash-attn2-rs/src/device/backward/dq.rs:12-302, dkv.rs:15-266, common.rs:121-152) and their packed
@@ -60,9 +63,10 @@ struct BwdWideCfg {
   static constexpr int kMaxAtoms = 4;
   static constexpr int kStageBytes = kMaxAtoms * kAtomQ;
   static constexpr int kKOff = 0;
-  static constexpr int kQOff = kMaxAtoms * kAtomK;        // 2 stages
-  static constexpr int kDOOff = kQOff + 2 * kStageBytes;  // 2 stages
-  static constexpr int kDSOff = kDOOff + 2 * kStageBytes; // [128 keys x 64 q] 16-bit, one atom
+  static constexpr int kQStages = 3;
+  static constexpr int kQOff = kMaxAtoms * kAtomK;
+  static constexpr int kDOOff = kQOff + kQStages * kStageBytes;
+  static constexpr int kDSOff = kDOOff + kStageBytes;     // [128 keys x 64 q] 16-bit, one atom
   static constexpr int kDQOff = kDSOff + kAtomK;          // dQ staging: [32 q x 32 d] fp32 per drain warp
   static constexpr int kDQPiece = 32 * 128;
   static constexpr int kBarOff = kDQOff + 4 * kDQPiece;
@@ -159,10 +163,10 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   uint8_t* s_ds = smem + Cfg::kDSOff;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kBarOff);
   uint64_t* k_full = bars + 0;
-  uint64_t* q_full = bars + 1;     // [2]
-  uint64_t* do_full = bars + 3;    // [2]
-  uint64_t* q_free = bars + 5;     // [2] S^T and dK, the readers of the Q stage, have completed
-  uint64_t* do_free = bars + 7;    // [2] dP^T and dV, the readers of the dO stage, have completed
+  uint64_t* q_full = bars + 1;     // [3]
+  uint64_t* q_free = bars + 4;     // [3] S^T and dK, the readers of the Q stage, have completed
+  uint64_t* do_full = bars + 7;
+  uint64_t* do_free = bars + 8;    // dP^T and dV, the readers of dO, have completed (packed batches: and the fixer has seen it)
   uint64_t* s_full = bars + 9;
   uint64_t* p_full = bars + 10;
   uint64_t* dp_full = bars + 11;
@@ -173,8 +177,8 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   uint64_t* stat_full = bars + 16;
   uint64_t* v_ready = bars + 17;   // V sits in TMEM
   uint64_t* k_fixed = bars + 18;   // packed batches: the fixer warp has cleared the rows past the sequence
-  uint64_t* q_fixed = bars + 19;   // [2]
-  uint64_t* do_fixed = bars + 21;  // [2]
+  uint64_t* q_fixed = bars + 19;   // [3]
+  uint64_t* do_fixed = bars + 22;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::kMiscOff + 8);
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::kStatOff);
@@ -195,14 +199,14 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   if (tid == 0) {
     *abort_flag = 0;
     mbar_init(k_full, 1);
-    for (int st = 0; st < 2; ++st) {
+    for (int st = 0; st < Cfg::kQStages; ++st) {
       mbar_init(&q_full[st], 1);
-      mbar_init(&do_full[st], 1);
       mbar_init(&q_free[st], 1);
-      mbar_init(&do_free[st], 1);
       mbar_init(&q_fixed[st], 1);
-      mbar_init(&do_fixed[st], 1);
     }
+    mbar_init(do_full, 1);
+    mbar_init(do_free, PACKED ? 2 : 1);
+    mbar_init(do_fixed, 1);
     mbar_init(s_full, 1);
     mbar_init(p_full, kBWCompute);
     mbar_init(dp_full, 1);
@@ -478,30 +482,27 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       for (int it = 0; it < n_iter && ok; ++it, w = wwalk_next(w, ti.n_m)) {
         const int hq = ti.hk * p.group + w.g;
         const int m0 = (ti.m_start + w.mi) * kBQ;
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        // A stage is free once the MMAs of its previous use that read it have completed; that of dO is first. At
-        // the start S^T waits for Q.
-#pragma unroll
-        for (int x = 0; x < 2 && ok; ++x) {
-          const bool load_q = (x == 0) == (it == 0);
-          ok = load_q ? mbar_wait(&q_free[st], ph ^ 1, ctl, kWaitBwd + 1) : mbar_wait(&do_free[st], ph ^ 1, ctl, kWaitBwd + 2);
-          if (!ok) break;
-          uint64_t* full = load_q ? &q_full[st] : &do_full[st];
-          uint8_t* dst = (load_q ? s_q : s_do) + st * Cfg::kStageBytes;
-          mbar_expect_tx(full, atoms * Cfg::kAtomQ);
-          for (int a = 0; a < atoms; ++a)
-            tma_load_4d(dst + a * Cfg::kAtomQ, load_q ? &p.tm_q : &p.tm_do, full, a * 64, hq, ti.q_row0 + m0, ti.bq);
-        }
+        const int st = it % Cfg::kQStages;
+        const uint32_t ph = (it / Cfg::kQStages) & 1;
+        // A stage is free once the MMAs of its previous use that read it have completed. Behind dV of an iteration go dO of
+        // the next one and Q of the one after that.
+        ok = mbar_wait(&q_free[st], ph ^ 1, ctl, kWaitBwd + 1);
+        if (!ok) break;
+        mbar_expect_tx(&q_full[st], atoms * Cfg::kAtomQ);
+        for (int a = 0; a < atoms; ++a)
+          tma_load_4d(s_q + st * Cfg::kStageBytes + a * Cfg::kAtomQ, &p.tm_q, &q_full[st], a * 64, hq, ti.q_row0 + m0, ti.bq);
+        ok = mbar_wait(do_free, (it & 1) ^ 1, ctl, kWaitBwd + 2);
+        if (!ok) break;
+        mbar_expect_tx(do_full, atoms * Cfg::kAtomQ);
+        for (int a = 0; a < atoms; ++a)
+          tma_load_4d(s_do + a * Cfg::kAtomQ, &p.tm_do, do_full, a * 64, hq, ti.q_row0 + m0, ti.bq);
       }
       // The loader leaves last: the commits on the free barriers of each stage's last use have landed.
-      for (int st = 0; st < 2 && ok; ++st) {
-        const int uses = (n_iter - st + 1) / 2;  // iterations st, st + 2, ...
-        if (uses > 0) {
-          ok = mbar_wait(&q_free[st], (uses - 1) & 1, ctl, kWaitBwd + 1);
-          if (ok) ok = mbar_wait(&do_free[st], (uses - 1) & 1, ctl, kWaitBwd + 2);
-        }
+      for (int st = 0; st < Cfg::kQStages && ok; ++st) {
+        const int uses = (n_iter - st + Cfg::kQStages - 1) / Cfg::kQStages;  // iterations st, st + 3, ...
+        if (uses > 0) ok = mbar_wait(&q_free[st], (uses - 1) & 1, ctl, kWaitBwd + 1);
       }
+      if (ok) ok = mbar_wait(do_free, (n_iter - 1) & 1, ctl, kWaitBwd + 2);
     }
   } else if (warp == kBWFixWarp) {
     // ---------------------------------------------------------------- fixer (packed batches)
@@ -533,18 +534,21 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       WWalk w{0, 0};
       for (int it = 0; it < n_iter && ok; ++it, w = wwalk_next(w, ti.n_m)) {
         const int first = ti.sq - (ti.m_start + w.mi) * kBQ;
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
+        const int st = it % Cfg::kQStages;
+        const uint32_t ph = (it / Cfg::kQStages) & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(&q_full[st], ph, ctl, kWaitBwd + 4));
         if (ok && first < kBQ) {
           clear_rows(s_q + st * Cfg::kStageBytes, Cfg::kAtomQ, first, kBQ);
           publish(&q_fixed[st]);
         }
-        ok = ok && __all_sync(0xffffffffu, mbar_wait(&do_full[st], ph, ctl, kWaitBwd + 5));
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(do_full, it & 1, ctl, kWaitBwd + 5));
         if (ok && first < kBQ) {
-          clear_rows(s_do + st * Cfg::kStageBytes, Cfg::kAtomQ, first, kBQ);
-          publish(&do_fixed[st]);
+          clear_rows(s_do, Cfg::kAtomQ, first, kBQ);
+          publish(do_fixed);
         }
+        // The stage is not refilled before this warp has seen it: its waits go by phase parity.
+        if (ok && lane == 0) mbar_arrive(do_free);
+        __syncwarp();
       }
     }
   } else if (warp == kBWMmaWarp && n_iter > 0 && elect_one()) {
@@ -595,12 +599,12 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       qfix_par ^= 1u << st;
       return mbar_wait(&q_fixed[st], par, ctl, kWaitBwd + 21);
     };
-    auto do_ready = [&](int mi, uint32_t st, uint32_t ph, int code) -> bool {
-      if (!mbar_wait(&do_full[st], ph, ctl, code)) return false;
+    auto do_ready = [&](int mi, uint32_t ph, int code) -> bool {
+      if (!mbar_wait(do_full, ph, ctl, code)) return false;
       if (!ragged_q(mi)) return true;
-      const uint32_t par = (dofix_par >> st) & 1;
-      dofix_par ^= 1u << st;
-      return mbar_wait(&do_fixed[st], par, ctl, kWaitBwd + 22);
+      const uint32_t par = dofix_par;
+      dofix_par ^= 1u;
+      return mbar_wait(do_fixed, par, ctl, kWaitBwd + 22);
     };
     bool ok = mbar_wait(k_full, 0, ctl, kWaitBwd + 3);
     if (ok && packed && ti.n0 + kBK > ti.sk) ok = mbar_wait(k_fixed, 0, ctl, kWaitBwd + 20);
@@ -609,7 +613,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       tc_fence_after();
       issue_st(q_kmaj);
       mma_commit(s_full);
-      ok = do_ready(0, 0, 0, kWaitBwd + 5);
+      ok = do_ready(0, 0, kWaitBwd + 5);
     }
     if (ok) ok = mbar_wait(v_ready, 0, ctl, kWaitBwd + 23);
     if (ok) {
@@ -620,8 +624,8 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
     WWalk wn{0, 0};  // position of iteration it + 1
     for (int it = 0; it < n_iter && ok; ++it) {
       wn = wwalk_next(wn, ti.n_m);
-      const uint32_t st = it & 1;
-      const uint32_t nph = ((it + 1) >> 1) & 1;  // phase of the stage barriers of iteration it + 1
+      const uint32_t st = it % Cfg::kQStages, nst = (it + 1) % Cfg::kQStages;
+      const uint32_t nph = ((it + 1) / Cfg::kQStages) & 1;  // phase of the Q stage of iteration it + 1
       const bool has_next = it + 1 < n_iter;
       const uint32_t acc = it > 0 ? 1u : 0u;
       // dV_c += P^T dO_c (P^T: two runs of 16 packed columns at S^T + 0 and S^T + 32; 16 query rows of dO are 2048 bytes)
@@ -629,20 +633,20 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       if (!ok) break;
       tc_fence_after();
       {
-        const uint64_t b = do_mn + st * kStage16;
+        const uint64_t b = do_mn;
         static_for<kBQ / 16>([&](auto ks) {
           mma_ts_o<(ks.value / 2) * 32 + (ks.value % 2) * 8, ks.value * (2048 >> 4)>(
               tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv, ks.value > 0 ? 1u : acc);
         });
       }
-      mma_commit(&do_free[st]);
+      mma_commit(do_free);
       // S^T of the next iteration right behind dV, the last reader of P^T: its scores are there when the compute
       // warps come out of phase B.
       if (has_next) {
-        ok = q_ready(wn.mi, st ^ 1, nph, kWaitBwd + 8);
+        ok = q_ready(wn.mi, nst, nph, kWaitBwd + 8);
         if (!ok) break;
         tc_fence_after();
-        issue_st(q_kmaj + (st ^ 1) * kStage16);
+        issue_st(q_kmaj + nst * kStage16);
         mma_commit(s_full);
       }
       // dQ_c^T = K_c^T dS^T over the 128 keys into the dP^T columns (the compute warps have read dP^T), then
@@ -666,11 +670,11 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
       mma_commit(&q_free[st]);
       // dP^T of the next iteration, once dQ^T has left the columns.
       if (has_next) {
-        ok = do_ready(wn.mi, st ^ 1, nph, kWaitBwd + 9);
+        ok = do_ready(wn.mi, (it + 1) & 1, kWaitBwd + 9);
         if (ok && want_dq) ok = mbar_wait(dq_free, it & 1, ctl, kWaitBwd + 10);
         if (!ok) break;
         tc_fence_after();
-        issue_dp(do_kmaj + (st ^ 1) * kStage16);
+        issue_dp(do_kmaj);
         mma_commit(dp_full);
       }
     }
