@@ -105,8 +105,7 @@ inline DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
   // incomplete round of whole units would take more than five tiles longer.
   if (units <= sms) {
     const int64_t parts = std::min<int64_t>({sms / units, 24, d.tiles / 3});
-    // No more parts than shorten the longest one (64 tiles: 16 parts of four tiles, not 18 of three or four).
-    if (parts > 1) d.grid = static_cast<int>(units * ((d.tiles + (d.tiles + parts - 1) / parts - 1) / ((d.tiles + parts - 1) / parts)));
+    if (parts > 1) d.grid = static_cast<int>(units * parts);
   } else if (per_cta * d.tiles - n / sms > 5) {
     d.grid = sm_count;
   }
