@@ -162,8 +162,8 @@ typedef struct fa2_bwd_options {
    * same with and without. */
   int32_t share_key_blocks;
   int32_t reserved; /* 0 */
-  /* 1: the last work put on the stream is a call of this library with which = 1 and otherwise the same arguments, and this
-   * one has which = 2. It may then run beside that call's kernel; what comes after it on the stream still waits for both. */
+  /* Taken and ignored: a hint that a which = 2 call may run beside the which = 1 call before it. Calls run in the order of
+   * their stream. */
   int64_t beside_dq;
 } fa2_bwd_options;
 FA2_API int64_t fa2_bwd_workspace_bytes_with_options(const fa2_bwd_args* args, const fa2_bwd_options* options);

@@ -268,12 +268,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     mbar_fence_init();
     __syncwarp();
   }
-  // Behind this library's dQ kernel, whose results it does not read, the grid starts beside it and waits at its end instead.
-  const bool beside = !PACKED && p.beside_dq != 0;
   if (tid == 0) {
     // The first loads go out before the rest of the CTA is set up (TMEM allocation, the block-wide
     // barrier): their latency is the longest item of a CTA's start.
-    if (!beside) early_wait();
+    early_wait();
     const KvTile& ti = first_tile;
     if (ti.n_iter > 0) {
       const int hq0 = ti.hk * p.group + ti.g0;
@@ -299,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
     tmem_relinquish();
   }
   tc_fence_before();
-  if (!beside) early_wait();
+  early_wait();
   __syncthreads();
   tc_fence_after();
   early_trigger();
@@ -1015,7 +1013,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 512);
-  if (beside) early_wait();
 }
 
 template <int D, bool BF16, int MODE, bool PACKED>

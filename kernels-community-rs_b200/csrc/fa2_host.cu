@@ -694,7 +694,6 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   }
   if (a->ev_kernel_start != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_start), stream);
   p.head_dim = d;
-  p.beside_dq = opt.beside_dq != 0 && opt.out == nullptr && !packed && !wide && a->which == 2 && a->ev_kernel_start == nullptr;
   p.dq_acc = static_cast<float*>(a->dq_accum);
   p.dq_rows = rows_q;
   p.v_ptr = a->v;

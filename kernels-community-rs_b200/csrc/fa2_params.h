@@ -106,7 +106,6 @@ struct BwdParams {
   int window_left, window_right;
   int which;                            // bit 0: dQ, bit 1: dK and dV
   int take_over;                        // D = 64: a CTA goes on with tiles of CTAs that have not started (set at the launch)
-  int beside_dq;                        // the grid before this one is the dQ kernel of the same gradients
   float scale, scale_log2;
   int* status;
   // Score transforms of the forward that the gradients have to follow (null / 0 when unused).

@@ -210,8 +210,6 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
   strides_of(out, opt.o_stride);
   opt.share_key_blocks = 1;
   // Bit-reproducible gradients come from the two separate calls: dQ in a fixed order, then dK and dV.
-  // The second one starts while the first one's last CTAs run: forward and backward of B2 H16/4 S777 D128 71.8 -> 69.1 us
-  // on the GPU, B1 H8/2 S1500 D64 63.3 -> 61.5.
   const int calls[2] = {deterministic ? 1 : 3, deterministic ? 2 : 0};
   for (const int which : calls) {
     if (which == 0) continue;
@@ -231,7 +229,6 @@ Gradients backward(const Tensor& dout, const Tensor& q, const Tensor& k, const T
     }
     check(fa2_bwd_with_options(&a, &opt, stream));
     opt.out = nullptr;
-    opt.beside_dq = which == 1;  // nothing else goes on this stream between the two calls
   }
   return g;
 }

@@ -145,3 +145,14 @@ def test_workspace_holds_turn_counters_only_where_they_are_used(built_libs):
         assert need(3, d, False) == need(3, d, True) == accum and need(2, d, False) == need(2, d, True) == 0
         assert need(1, d, False) == (0 if d <= 128 else accum)
         assert need(1, d, True) == accum + (2 * 4 * 2 * 4 * 4 if d <= 128 else 0)
+
+
+def test_kernels_that_start_early_wait_before_they_let_the_next_one_in():
+    """Of a kernel launched as a programmatic dependent every CTA waits for what is before it in the stream, whatever the call's
+    arguments, and only then lets the next grid start: no grid runs beside another one than the one right before it."""
+    sources = {f.name: f.read_text() for f in (ROOT / "kernels-community-rs_b200" / "csrc").glob("*.cu")}
+    early = {(f, k) for f, s in sources.items() for k in re.findall(r"launch_early\((\w+)", s)}
+    assert len(early) >= 6
+    for f, kernel in early:
+        body = sources[f][re.search(rf"__global__[^;{{]*\b{kernel}\(", sources[f]).end():]
+        assert re.search(r"^  early_wait\(\);$", body[: body.index("early_trigger();")], re.M), (f, kernel)

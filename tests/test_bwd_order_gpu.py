@@ -32,21 +32,73 @@ def test_a_head_gets_the_same_in_any_group(shape, causal):
 
 
 @pytest.mark.parametrize("shape", [(2, 16, 4, 777, 128), (1, 8, 2, 1500, 64), (3, 4, 4, 130, 96)], ids=str)
-def test_dkdv_beside_dq(shape):
-    """The second call of a bit-reproducible backward runs beside the first one's last CTAs; what follows on the stream
-    (here the next pair, into the same memory, and a copy) waits for both."""
+def test_bit_reproducible_pair_on_changing_inputs(shape):
+    """Calls without a pause, into the same memory: every one sees the delta and the inputs of its own pass."""
     import flash_attn2_b200 as fa2
     from flash_attn2_b200 import cabi_ops as ops
 
     b, h, hk, s, d = shape
-    q, k, v, do = [t.cuda() for t in make_qkv(6, b, h, hk, s, s, d, torch.bfloat16, with_do=True)]
+    sets, want = [], []
+    for seed in (6, 7, 8):
+        q, k, v, do = [t.cuda() for t in make_qkv(seed, b, h, hk, s, s, d, torch.bfloat16, with_do=True)]
+        do *= 2.0 ** (seed - 7)
+        out, lse = fa2.fwd(q, k, v, is_causal=True)[:2]
+        delta = ops.bwd_preprocess(do, out)
+        torch.cuda.synchronize()
+        dq = ops.bwd(q, k, v, do, lse, delta, causal=True, which=1)[0]
+        torch.cuda.synchronize()
+        sets.append((do, q, k, v, out, lse))
+        want.append((dq, *ops.bwd(q, k, v, do, lse, delta, causal=True, which=2, share_key_blocks=True)[1:]))
+        torch.cuda.synchronize()
+    args = [torch.empty_like(t) for t in sets[0]]
+    got = []
+    for i in range(30):
+        for a, t in zip(args, sets[i % 3]):
+            a.copy_(t)
+        got.append([t.clone() for t in fa2.bwd(*args, is_causal=True, deterministic=True)[:3]])
+    for i, grads in enumerate(got):
+        assert all(torch.equal(g, w) for g, w in zip(grads, want[i % 3])), i
+    assert ops.device_status() == 0
+
+
+def test_threads_that_share_a_stream():
+    """Bit-reproducible backward calls of one thread among forward calls of another, all on the default stream: what a call
+    frees on its return, the other thread's next call gets, scratch memory included."""
+    import threading
+
+    import flash_attn2_b200 as fa2
+    from flash_attn2_b200 import cabi_ops as ops
+
+    q, k, v, do = [t.cuda() for t in make_qkv(9, 2, 16, 4, 777, 777, 128, torch.bfloat16, with_do=True)]
     out, lse = fa2.fwd(q, k, v, is_causal=True)[:2]
-    delta = ops.bwd_preprocess(do, out)
-    dq = ops.bwd(q, k, v, do, lse, delta, causal=True, which=1)[0]
-    _, dk, dv = ops.bwd(q, k, v, do, lse, delta, causal=True, which=2, share_key_blocks=True)
-    for _ in range(20):
-        copies = [t.clone() for t in fa2.bwd(do, q, k, v, out, lse, is_causal=True, deterministic=True)[:3]]
-    assert all(torch.equal(a, r) for a, r in zip(copies, (dq, dk, dv)))
+    token = [t.cuda() for t in make_qkv(10, 1, 32, 8, 1, 8192, 128, torch.bfloat16)]
+    few = [t.cuda() for t in make_qkv(11, 1, 8, 8, 500, 4096, 128, torch.bfloat16)]   # both forwards take scratch memory
+    calls = {"backward": lambda: fa2.bwd(do, q, k, v, out, lse, is_causal=True, deterministic=True)[:3],
+             "decode": lambda: fa2.fwd(*token)[:2], "shared tiles": lambda: fa2.fwd(*few, is_causal=True)[:2]}
+    want = {}
+    for name, call in calls.items():
+        want[name] = [t.clone() for t in call()]
+        torch.cuda.synchronize()
+    wrong, errors = {name: torch.zeros((), dtype=torch.int64, device="cuda") for name in calls}, []
+    torch.cuda.synchronize()
+    start = threading.Barrier(3)
+
+    def work(name):
+        try:
+            start.wait(30)
+            for _ in range(100):
+                for g, w in zip(calls[name](), want[name]):
+                    wrong[name] += (g != w).sum()
+        except Exception as e:  # reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(name,)) for name in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert {name: int(n) for name, n in wrong.items()} == dict.fromkeys(calls, 0)
     assert ops.device_status() == 0
 
 
