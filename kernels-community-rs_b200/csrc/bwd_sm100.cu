@@ -237,7 +237,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
-  if (PACKED) early_wait();  // the sequences' offsets are in global memory
   const KvTile first_tile = get_kv_tile<PACKED>(p, blockIdx.x);
   if (!first_tile.valid) return;
   const bool want_dq = (p.which & 1) != 0;
@@ -300,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   early_wait();
   __syncthreads();
   tc_fence_after();
-  early_trigger();
+  if (!PACKED) early_trigger();
   const uint32_t tmem = *tmem_slot;
 
   // Dense calls: a CTA that has finished a tile goes on with one that has not started yet (the scheduler hands it the
@@ -1028,7 +1027,7 @@ cudaError_t launch_one(const BwdParams& p, int num_ctas, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_early(bwd_kernel<D, BF16, MODE, PACKED>, dim3(num_ctas), kThreads, Cfg::kSmemBytes, stream, p);
+  return launch_grid<!PACKED>(bwd_kernel<D, BF16, MODE, PACKED>, dim3(num_ctas), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int D, bool BF16>

@@ -187,7 +187,6 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
-  if (PACKED) early_wait();  // the sequences' offsets are in global memory
   const WKvTile ti = get_wkv_tile(p, blockIdx.x);
   if (!ti.valid) return;
   constexpr int atoms = ATOMS;
@@ -232,7 +231,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   early_wait();
   __syncthreads();
   tc_fence_after();
-  early_trigger();
+  if (!PACKED) early_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp < kBWDrainWarp) {
@@ -707,8 +706,8 @@ cudaError_t launch_bwd_wide_one(const BwdParams& p, cudaStream_t stream) {
   const int64_t blocks = 2LL * p.num_nblk * p.batch * p.heads_k;
   if (blocks <= 0) return cudaSuccess;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  return launch_early(bwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kBWThreads,
-                      BwdWideCfg::kSmemBytes, stream, p);
+  return launch_grid<!PACKED>(bwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kBWThreads,
+                              BwdWideCfg::kSmemBytes, stream, p);
 }
 
 template <bool BF16, int ATOMS>

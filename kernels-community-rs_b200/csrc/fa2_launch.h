@@ -10,9 +10,11 @@ namespace fa2 {
 // (both transforms; in the forward also a negative scale without a transform) and is what packed batches use.
 enum ScoreMode : int { kScorePlain = 0, kScoreSoftcap = 1, kScoreAlibi = 2, kScoreAny = 3 };
 
-// Launches a kernel that calls early_wait: it may start while the kernel before it in the stream ends.
-template <typename... P, typename... A>
-cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem_bytes, cudaStream_t stream, A&&... args) {
+// EARLY: the kernel, which calls early_wait, may start while the kernel before it in the stream ends. Packed batches are launched
+// the usual way, and let the next grid in when they end: the forward of a large packed batch, looped with other kernels, once
+// ended in a launch failure that was never explained, and grids that overlap are one more thing that could have a part in it.
+template <bool EARLY, typename... P, typename... A>
+cudaError_t launch_grid(void (*kernel)(P...), dim3 grid, int threads, size_t smem_bytes, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute early[1] = {};
   early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early[0].val.programmaticStreamSerializationAllowed = 1;
@@ -22,7 +24,7 @@ cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t sm
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = stream;
   cfg.attrs = early;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = EARLY ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
   if (e != cudaSuccess) cudaGetLastError();
   return e;

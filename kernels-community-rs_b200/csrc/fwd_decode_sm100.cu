@@ -576,7 +576,7 @@ cudaError_t launch_one(const DecodeParams& p, int grid, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_early(fwd_decode_kernel<A, MT, BF16>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
+  return launch_grid<true>(fwd_decode_kernel<A, MT, BF16>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int A, bool BF16>

@@ -158,7 +158,6 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const WaitCtl ctl{abort_flag, p.status};
-  if (PACKED) early_wait();  // the sequences' offsets are in global memory
   const WTile ti = get_wtile(p, blockIdx.x);
   if (!ti.valid) return;
   constexpr int atoms = ATOMS;
@@ -207,7 +206,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   early_wait();
   __syncthreads();
   tc_fence_after();
-  early_trigger();
+  if (!PACKED) early_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp < 4) {
@@ -527,8 +526,8 @@ cudaError_t launch_wide(const FwdParams& p, cudaStream_t stream) {
   const int64_t blocks = static_cast<int64_t>((p.seqlen_q + kWM - 1) / kWM) * p.batch * p.heads;
   if (blocks <= 0) return cudaSuccess;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  return launch_early(fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kWThreads,
-                      WideCfg::kSmemBytes, stream, p);
+  return launch_grid<!PACKED>(fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kWThreads,
+                              WideCfg::kSmemBytes, stream, p);
 }
 
 template <bool BF16, int ATOMS>

@@ -152,7 +152,7 @@ __device__ __forceinline__ int next_cta(uint32_t answer) {
 }
 
 // ---------------------------------------------------------------- dependent launch
-// The kernels are launched so that a grid may start while the one before it in the stream ends (launch_early). A grid
+// The kernels are launched so that a grid may start while the one before it in the stream ends (launch_grid). A grid
 // touches global memory only behind early_wait, which returns once everything before it in the stream has completed
 // and is visible; what precedes it (barriers, TMEM, descriptors) runs beside the end of that. Every CTA waits, so that a
 // grid never ends before its predecessor. early_trigger, behind the wait, lets the next grid start as soon as all CTAs
