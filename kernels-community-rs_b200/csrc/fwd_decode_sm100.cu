@@ -47,6 +47,11 @@ struct DecCfg {
   static constexpr int kBarOff = kStatOff + kConsumers * 16 * 2 * 4;
   static constexpr int kMiscOff = kBarOff + 2 * kMaxSlots * 8;
   static constexpr int kSmemBytes = kMiscOff + 16;
+  // Does the merge load twelve parts at a time, the first ones before the rows' maxima, or eight behind them? Eight, then twelve,
+  // us a call: B1 H32/8 Sk 8192 D64 11.7, 11.1 and D128 13.1, 12.7; B1 H64/8 Sq 3 Sk 8192 D64 15.9, 15.5, D128 22.0, 20.9 and
+  // D192 30.0, 29.1. Elsewhere the registers that it takes cost the loop over the key tiles more: spills at D192 with up to 16
+  // rows and with more than 32; B4 H16/2 Sk 5000 D256 19.5, 20.5; B4 H64/8 Sq 8 Sk 2000 D256 45.0, 48.7.
+  static constexpr bool kMergeAhead = A < 4 && MT < 4 && !(A == 3 && MT == 1);
 };
 
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* r) {
@@ -72,7 +77,11 @@ __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;
 // exp2(m - m_tot) with m = -inf (a part that saw no key) giving 0 also when m_tot = -inf.
 __device__ __forceinline__ float part_scale(float m, float m_tot) { return m == -INFINITY ? 0.f : ex2(m - m_tot); }
 
-template <int A, int MT, bool BF16>
+// PARTS: units may be shared by CTAs. Calls without parts have instances of their own: the merge, although they never reach it,
+// changes how the compiler lays out the loop over the key tiles: B10 H32/8 Sk 4000 D128 34.8 us a call with it, 30.8 without,
+// D64 25.3 and 22.6. With more than 32 rows the loop is the better one with it (B16 H64/8 Sq 8 Sk 4096 D128 72.0, without 73.8),
+// so there one instance takes both.
+template <int A, int MT, bool BF16, bool PARTS>
 __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_constant__ DecodeParams p) {
   using Cfg = DecCfg<A, MT>;
   constexpr int D = Cfg::D;
@@ -91,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
   // this CTA's share of the tile list; without parts (no workspace for them) it is whole units
   const int64_t n_tiles = static_cast<int64_t>(p.units) * p.tiles_per_unit;
   int lo, hi;
-  if (p.partials != nullptr) {
+  if (PARTS && p.partials != nullptr) {
     lo = static_cast<int>(blockIdx.x * n_tiles / gridDim.x);
     hi = static_cast<int>((blockIdx.x + 1) * n_tiles / gridDim.x);
   } else {
@@ -428,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
           p.lse_ptr[b * p.lse_batch_stride + h * p.lse_head_stride + q] = l > 0.f ? (m + lg2(l)) * 0.6931471805599453f : INFINITY;
         }
       };
-      const bool whole = seg_first == 0 && seg_end == p.tiles_per_unit;
+      const bool whole = !PARTS || (seg_first == 0 && seg_end == p.tiles_per_unit);
       if (whole) {
         const float i0 = ls0 > 0.f ? 1.f / ls0 : 0.f, i1 = ls1 > 0.f ? 1.f / ls1 : 0.f;
 #pragma unroll
@@ -440,7 +449,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
           store_lse(r0, t0, ls0);
           store_lse(r1, t1, ls1);
         }
-      } else {
+      } else if constexpr (PARTS) {
         // Slot 2c holds a segment that began before this share, 2c + 1 one that began in it. Layout of a slot: O
         // [row][column], then m and l of the rows; rows past the last one are neither written nor read.
         constexpr int kPart = Cfg::kRows * (D + 2);  // floats
@@ -491,13 +500,12 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
         consumers_sync();
         if (*s_last) {
           // All consumers add the parts up: the rows' maxima and sums go to shared memory, and a thread takes four columns of
-          // a row at a time, with the loads of twelve parts issued together, the first ones before the maxima: each batch is
-          // an L2 round trip. With eight at a time, behind the maxima: B4 H16/2 Sk 5000 12.1 us a call, now 11.6; B1 H32/8 Sk 8192 13.0, now 12.5.
+          // a row at a time, with the loads of a batch of parts issued together: each batch is an L2 round trip.
           auto part_of = [&](int c) { return p.partials + part_index(c) * static_cast<int64_t>(kPart); };
           const int n_parts = c_last - c_first + 1;
           float* sm = reinterpret_cast<float*>(scratch);
           float* sl = sm + n_parts * Cfg::kRows;
-          constexpr int kBatch = 12;
+          constexpr int kBatch = Cfg::kMergeAhead ? 12 : 8;
           float4 w[kBatch];
           auto fetch = [&](int i, int c0) {
 #pragma unroll
@@ -505,7 +513,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
               if (c0 + e < n_parts)
                 w[e] = __ldcg(reinterpret_cast<const float4*>(part_of(c_first + c0 + e) + i / (D / 4) * D + i % (D / 4) * 4));
           };
-          if (tid < p.rows * (D / 4)) fetch(tid, 0);
+          if (Cfg::kMergeAhead && tid < p.rows * (D / 4)) fetch(tid, 0);
           for (int i = tid; i < n_parts * Cfg::kRows; i += kConsumers * 32) {
             const int r = i % Cfg::kRows;
             if (r < p.rows) {
@@ -521,7 +529,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
             for (int c = 0; c < n_parts; ++c) m = fmaxf(m, sm[c * Cfg::kRows + r]);
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
             for (int c = 0; c < n_parts; c += kBatch) {
-              if (i != tid || c > 0) fetch(i, c);
+              if (!Cfg::kMergeAhead || i != tid || c > 0) fetch(i, c);
 #pragma unroll
               for (int e = 0; e < kBatch; ++e)
                 if (c + e < n_parts) {
@@ -565,25 +573,33 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
   __syncthreads();
 }
 
-template <int A, int MT, bool BF16>
+template <int A, int MT, bool BF16, bool PARTS>
 cudaError_t launch_one(const DecodeParams& p, int grid, cudaStream_t stream) {
   using Cfg = DecCfg<A, MT>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(fwd_decode_kernel<A, MT, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(fwd_decode_kernel<A, MT, BF16, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_grid<true>(fwd_decode_kernel<A, MT, BF16>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
+  return launch_grid<true>(fwd_decode_kernel<A, MT, BF16, PARTS>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
+}
+
+template <int A, int MT, bool BF16>
+cudaError_t pick_parts(const DecodeParams& p, int grid, cudaStream_t stream) {
+  if constexpr (MT < 4) {
+    if (p.partials == nullptr) return launch_one<A, MT, BF16, false>(p, grid, stream);
+  }
+  return launch_one<A, MT, BF16, true>(p, grid, stream);
 }
 
 template <int A, bool BF16>
 cudaError_t pick_rows(const DecodeParams& p, int grid, cudaStream_t stream) {
-  if (p.rows <= 16) return launch_one<A, 1, BF16>(p, grid, stream);
-  if (p.rows <= 32) return launch_one<A, 2, BF16>(p, grid, stream);
-  return launch_one<A, 4, BF16>(p, grid, stream);
+  if (p.rows <= 16) return pick_parts<A, 1, BF16>(p, grid, stream);
+  if (p.rows <= 32) return pick_parts<A, 2, BF16>(p, grid, stream);
+  return pick_parts<A, 4, BF16>(p, grid, stream);
 }
 
 template <bool BF16>
