@@ -346,7 +346,7 @@ cudaError_t launch_one(const DqParams& p, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_grid<true>(bwd_dq_kernel<D, BF16, MODE>, dim3(p.num_mblk * p.batch * p.heads), kThreads, Cfg::kSmemBytes, stream, p);
+  return launch_grid(true, bwd_dq_kernel<D, BF16, MODE>, dim3(p.num_mblk * p.batch * p.heads), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int D, bool BF16>

@@ -1027,7 +1027,7 @@ cudaError_t launch_one(const BwdParams& p, int num_ctas, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_grid<!PACKED>(bwd_kernel<D, BF16, MODE, PACKED>, dim3(num_ctas), kThreads, Cfg::kSmemBytes, stream, p);
+  return launch_grid(!PACKED, bwd_kernel<D, BF16, MODE, PACKED>, dim3(num_ctas), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int D, bool BF16>

@@ -706,7 +706,7 @@ cudaError_t launch_bwd_wide_one(const BwdParams& p, cudaStream_t stream) {
   const int64_t blocks = 2LL * p.num_nblk * p.batch * p.heads_k;
   if (blocks <= 0) return cudaSuccess;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  return launch_grid<!PACKED>(bwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kBWThreads,
+  return launch_grid(!PACKED, bwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kBWThreads,
                               BwdWideCfg::kSmemBytes, stream, p);
 }
 

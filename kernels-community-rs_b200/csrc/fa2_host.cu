@@ -22,6 +22,7 @@ namespace {
 using fa2::BwdSplit;
 using fa2::DecodePlan;
 using fa2::decode_plan;
+using fa2::decode_starts_early;
 using fa2::normalise_windows;
 using fa2::plan_bwd_split;
 using fa2::plan_stream;
@@ -226,7 +227,7 @@ int fwd_decode(const fa2_fwd_args* a, const DecodePlan& d, const Scratch& scratc
     p.flags = static_cast<unsigned long long*>(scratch.ptr);
     p.partials = reinterpret_cast<float*>(static_cast<char*>(scratch.ptr) + d.flag_bytes);
   }
-  const cudaError_t e = fa2::launch_fwd_decode(p, grid, a->dtype == FA2_BF16, stream);
+  const cudaError_t e = fa2::launch_fwd_decode(p, grid, a->dtype == FA2_BF16, decode_starts_early(a, d.tiles, grid, rt->sm_count), stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "forward launch failed: %s", cudaGetErrorString(e));
   return FA2_OK;
 }

@@ -10,21 +10,21 @@ namespace fa2 {
 // (both transforms; in the forward also a negative scale without a transform) and is what packed batches use.
 enum ScoreMode : int { kScorePlain = 0, kScoreSoftcap = 1, kScoreAlibi = 2, kScoreAny = 3 };
 
-// EARLY: the kernel, which calls early_wait, may start while the kernel before it in the stream ends. Packed batches are launched
+// early: the kernel, which calls early_wait, may start while the kernel before it in the stream ends. Packed batches are launched
 // the usual way, and let the next grid in when they end: the forward of a large packed batch, looped with other kernels, once
 // ended in a launch failure that was never explained, and grids that overlap are one more thing that could have a part in it.
-template <bool EARLY, typename... P, typename... A>
-cudaError_t launch_grid(void (*kernel)(P...), dim3 grid, int threads, size_t smem_bytes, cudaStream_t stream, A&&... args) {
-  cudaLaunchAttribute early[1] = {};
-  early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early[0].val.programmaticStreamSerializationAllowed = 1;
+template <typename... P, typename... A>
+cudaError_t launch_grid(bool early, void (*kernel)(P...), dim3 grid, int threads, size_t smem_bytes, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[1] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(static_cast<unsigned>(threads));
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = stream;
-  cfg.attrs = early;
-  cfg.numAttrs = EARLY ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
   if (e != cudaSuccess) cudaGetLastError();
   return e;
@@ -40,7 +40,8 @@ cudaError_t launch_fwd_wide(const FwdParams& p, int head_dim, bool bf16, cudaStr
 // Dense forward with at most kDecodeMaxRows query rows per kv head, head_dim a multiple of 8 up to 256; `grid` CTAs
 // share the tile list evenly. The workspace behind p.partials and p.flags holds 2 * grid partial results of
 // 16 * decode_row_tiles(rows) rows x (D + 2) floats (D: head_dim rounded up to 64) and as many 8-byte flags.
-cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, cudaStream_t stream);
+// early: it may start beside the end of the kernel before it (decode_starts_early).
+cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, bool early, cudaStream_t stream);
 
 // dQ / dK / dV for head_dim a multiple of 8 up to 128; the fp32 dQ accumulator behind p.tm_dqa (and the turn
 // counters p.dq_turn, when given) must be zero.

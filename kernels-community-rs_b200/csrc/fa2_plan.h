@@ -119,6 +119,16 @@ inline DecodePlan decode_plan(const fa2_fwd_args* a, int sm_count) {
   return d;
 }
 
+// Does the few-row kernel start beside the end of the kernel before it? That saves 2-3 us a call. But the CTAs of the next call
+// settle on the SMs that the present one leaves idle, the rest on whichever end first: they no longer lie evenly over the chip,
+// which costs calls that read at the memory's rate on a part of the SMs more than it saves. Without it, with it, us a call, D128:
+// 80 CTAs of 63 key tiles (4 MB of K and V each) 53.3, 66.0; 96 CTAs of 128 tiles 118, 132; 128 of 128 tiles 154, 168. On the
+// other side of the line: 80 CTAs of 8 tiles 12.3, 10.2; 128 of 16 tiles (1 MB) 27.3, 25.2; 136 of 128 tiles 178, 172.
+inline bool decode_starts_early(const fa2_fwd_args* a, int tiles_per_unit, int grid, int sm_count) {
+  const int64_t tiles = static_cast<int64_t>(a->batch) * a->heads_k * tiles_per_unit;
+  return 10 * grid >= 9 * sm_count || tiles * 128 * a->head_dim * 4 / grid <= 1 << 20;
+}
+
 // ---- dense forward with few work tiles (fwd_sm100.cu, SHARED): a work tile is 256 query rows of a head, one CTA at a
 // time works on it, and with fewer tiles than SMs some have nothing to do. Calls with more tiles are not shared, also
 // where a last, nearly empty round would gain (H32 Sq 1500 Sk 16384, 192 tiles: 454 -> 392 us): sharing makes the bits of a

@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
 }
 
 template <int A, int MT, bool BF16, bool PARTS>
-cudaError_t launch_one(const DecodeParams& p, int grid, cudaStream_t stream) {
+cudaError_t launch_one(const DecodeParams& p, int grid, bool early, cudaStream_t stream) {
   using Cfg = DecCfg<A, MT>;
   static bool configured[64] = {};
   int dev = 0;
@@ -584,37 +584,37 @@ cudaError_t launch_one(const DecodeParams& p, int grid, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_grid<true>(fwd_decode_kernel<A, MT, BF16, PARTS>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
+  return launch_grid(early, fwd_decode_kernel<A, MT, BF16, PARTS>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int A, int MT, bool BF16>
-cudaError_t pick_parts(const DecodeParams& p, int grid, cudaStream_t stream) {
+cudaError_t pick_parts(const DecodeParams& p, int grid, bool early, cudaStream_t stream) {
   if constexpr (MT < 4) {
-    if (p.partials == nullptr) return launch_one<A, MT, BF16, false>(p, grid, stream);
+    if (p.partials == nullptr) return launch_one<A, MT, BF16, false>(p, grid, early, stream);
   }
-  return launch_one<A, MT, BF16, true>(p, grid, stream);
+  return launch_one<A, MT, BF16, true>(p, grid, early, stream);
 }
 
 template <int A, bool BF16>
-cudaError_t pick_rows(const DecodeParams& p, int grid, cudaStream_t stream) {
-  if (p.rows <= 16) return pick_parts<A, 1, BF16>(p, grid, stream);
-  if (p.rows <= 32) return pick_parts<A, 2, BF16>(p, grid, stream);
-  return pick_parts<A, 4, BF16>(p, grid, stream);
+cudaError_t pick_rows(const DecodeParams& p, int grid, bool early, cudaStream_t stream) {
+  if (p.rows <= 16) return pick_parts<A, 1, BF16>(p, grid, early, stream);
+  if (p.rows <= 32) return pick_parts<A, 2, BF16>(p, grid, early, stream);
+  return pick_parts<A, 4, BF16>(p, grid, early, stream);
 }
 
 template <bool BF16>
-cudaError_t pick_dim(const DecodeParams& p, int grid, cudaStream_t stream) {
-  if (p.head_dim <= 64) return pick_rows<1, BF16>(p, grid, stream);
-  if (p.head_dim <= 128) return pick_rows<2, BF16>(p, grid, stream);
-  if (p.head_dim <= 192) return pick_rows<3, BF16>(p, grid, stream);
-  return pick_rows<4, BF16>(p, grid, stream);
+cudaError_t pick_dim(const DecodeParams& p, int grid, bool early, cudaStream_t stream) {
+  if (p.head_dim <= 64) return pick_rows<1, BF16>(p, grid, early, stream);
+  if (p.head_dim <= 128) return pick_rows<2, BF16>(p, grid, early, stream);
+  if (p.head_dim <= 192) return pick_rows<3, BF16>(p, grid, early, stream);
+  return pick_rows<4, BF16>(p, grid, early, stream);
 }
 
 }  // namespace
 
-cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, cudaStream_t stream) {
+cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, bool early, cudaStream_t stream) {
   if (p.rows <= 0 || p.rows > kDecodeMaxRows || p.head_dim <= 0 || p.head_dim > 256 || grid <= 0) return cudaErrorInvalidValue;
-  return bf16 ? pick_dim<true>(p, grid, stream) : pick_dim<false>(p, grid, stream);
+  return bf16 ? pick_dim<true>(p, grid, early, stream) : pick_dim<false>(p, grid, early, stream);
 }
 
 }  // namespace fa2

@@ -1008,9 +1008,9 @@ cudaError_t launch_one(const FwdParams& p, int num_sms, cudaStream_t stream) {
     configured[dev] = true;
   }
   const int grid = SHARED ? p.stream_grid : p.num_tiles < num_sms ? p.num_tiles : num_sms;
-  cudaError_t e = launch_grid<!PACKED>(fwd_kernel<D, BF16, MODE, PACKED, SHARED>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
+  cudaError_t e = launch_grid(!PACKED, fwd_kernel<D, BF16, MODE, PACKED, SHARED>, dim3(grid), kThreads, Cfg::kSmemBytes, stream, p);
   if (SHARED && e == cudaSuccess)
-    e = launch_grid<true>(merge_parts_kernel<D, BF16>, dim3(p.num_tiles * (256 / kMergeRows<D>)), 256, 0, stream, p);
+    e = launch_grid(true, merge_parts_kernel<D, BF16>, dim3(p.num_tiles * (256 / kMergeRows<D>)), 256, 0, stream, p);
   return e;
 }
 

@@ -526,7 +526,7 @@ cudaError_t launch_wide(const FwdParams& p, cudaStream_t stream) {
   const int64_t blocks = static_cast<int64_t>((p.seqlen_q + kWM - 1) / kWM) * p.batch * p.heads;
   if (blocks <= 0) return cudaSuccess;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  return launch_grid<!PACKED>(fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kWThreads,
+  return launch_grid(!PACKED, fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kWThreads,
                               WideCfg::kSmemBytes, stream, p);
 }
 

@@ -32,6 +32,10 @@ int head_group(const fa2_bwd_args* a, int dq_alone, int sms) {
   const fa2::Windows w = fa2::normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
   return dq_alone ? fa2::bwd_dq_head_group(a, w) : fa2::bwd_head_group(a, w, sms);
 }
+int few_rows_start_early(const fa2_fwd_args* a, int sms) {
+  const fa2::DecodePlan d = fa2::decode_plan(a, sms);
+  return fa2::decode_starts_early(a, d.tiles, d.grid, sms);
+}
 int64_t few_rows_workspace(const fa2_fwd_args* a, int sms) { return fa2::decode_plan(a, sms).workspace_bytes; }
 }
 '''
@@ -121,6 +125,19 @@ def test_parts_of_a_few_row_unit(plans, sk, parts):
     """As many equal parts as the SMs allow and leave three key tiles, at most 24."""
     assert plans.few_rows_ctas(ctypes.byref(_fwd_args(1, 32, 8, 1, sk, 128, causal=1)), SMS) == 8 * parts
     assert plans.few_rows_ctas(ctypes.byref(_fwd_args(1, 4, 1, 1, 16384, 128, causal=1)), SMS) == 24
+
+
+# (batch, heads, heads_k, seqlen_k, head_dim): timed with and without the early start.
+LATE = [(10, 32, 8, 4000, 128), (10, 32, 8, 8000, 128), (12, 32, 8, 8192, 128), (16, 64, 8, 16384, 128), (8, 64, 8, 16384, 128),
+        (76, 4, 1, 16384, 128), (16, 32, 8, 8192, 192), (10, 32, 8, 4000, 256), (16, 32, 8, 8192, 256)]
+EARLY = [(1, 32, 8, 8192, 128), (32, 32, 8, 4093, 128), (10, 32, 8, 1000, 128), (16, 64, 8, 1024, 128), (9, 32, 8, 16000, 128),
+         (17, 32, 8, 16000, 128), (10, 32, 8, 4000, 64), (37, 32, 8, 2048, 256)]
+
+
+@pytest.mark.parametrize("shape", LATE + EARLY, ids=str)
+def test_few_row_calls_start_early_where_that_is_faster(plans, shape):
+    b, h, hk, sk, d = shape
+    assert plans.few_rows_start_early(ctypes.byref(_fwd_args(b, h, hk, 1, sk, d, causal=1)), SMS) == (shape in EARLY)
 
 
 # (batch, heads, heads_k, seqlen, head_dim), causal, heads in a group: all of them in a call of few CTAs; else equal groups of at
