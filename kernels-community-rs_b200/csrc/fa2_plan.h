@@ -195,12 +195,16 @@ inline void plan_stream(const fa2_fwd_args* a, int sm_count, StreamPlan* out) {
 // ends with whatever starts last. Under a causal mask the first key block of a head sees every query row and the last one
 // only its own: listed head by head, the last head's long walks start late and most SMs wait for them. So a group of
 // heads lists all first key blocks, then all second ones ...: the call ends with short walks. What the group's CTAs read
-// and add into should stay in the L2 (126 MB), so calls of many CTAs, whose end weighs little, take groups of at most
-// 96 MB (of Q, dO, the accumulator, K and V); with up to four CTAs per SM the end weighs more than the traffic. Forward and
+// and add into should stay in the L2 (126 MB), so calls of many CTAs, whose end weighs little, take groups of about
+// 96 MB (of Q, dO, the accumulator, K and V); with up to four CTAs per SM the end weighs more than the traffic. Whole heads are
+// dealt out evenly, rounded up, so that a group of two or three large heads can be nearly twice as large: the longer list is
+// worth more than the bound (B2 H64/8 S8192 in pairs of 136 MB 7763 us, one by one 8037). Forward and
 // backward, causal bf16, head by head -> grouped: B4 H16/4 S2048 softcap 448 -> 347 us, B2 H32/8 S4096 1183 -> 1001,
 // B4 H16 S1000 128 -> 119, B4 H16/8 S2048 D256 885 -> 834, B1 H32 S16384 7444 -> 7358 (in groups of 250 MB 7602).
 // Walks of the same length have no such end, but side by side those of one head add into the same rows at the same time;
-// small groups mix them: B32 H12 S509 D64 232 -> 228 us, B16 H16 S2048 without a mask 2191 -> 2170 (all heads: 2757).
+// small groups mix them: B32 H12 S509 D64 232 -> 228 us, B16 H16 S2048 without a mask 2191 -> 2170 (all heads: 2757). Sliding
+// windows are taken for such walks; head by head, in small groups, in groups as for the causal mask: B2 H16 S4096 D64 window 1023
+// 213, 215, 207 us, B16 H16 S2048 D128 window 1023 1152, 1136, 1164, B1 H16/4 S8192 D128 window 4095 824, 815, 866.
 inline int bwd_head_group(const fa2_bwd_args* a, const Windows& w, int sm_count) {
   if (a->cu_seqlens_q != nullptr) return 1;
   const int64_t heads = std::max<int64_t>(static_cast<int64_t>(a->batch) * a->heads_k, 1);
@@ -214,7 +218,7 @@ inline int bwd_head_group(const fa2_bwd_args* a, const Windows& w, int sm_count)
 }
 
 // The same for the kernel that computes dQ alone, one CTA per 128 query rows of a head: K and V of a group, which its CTAs
-// share, take at most 64 MB.
+// share, take about 64 MB.
 inline int bwd_dq_head_group(const fa2_bwd_args* a, const Windows& w) {
   const int64_t heads = std::max<int64_t>(static_cast<int64_t>(a->batch) * a->heads, 1);
   if (w.right < 0 || w.left >= 0) return 1;

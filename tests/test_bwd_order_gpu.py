@@ -2,12 +2,15 @@
 import pytest
 import torch
 
-from tests._cases import make_qkv
+from tests._cases import alibi_slopes, make_qkv
 
 pytestmark = pytest.mark.gpu
 
-# (heads, heads_k, seqlen, head_dim), causal: enough CTAs and data for several groups, a prime number of (batch, kv head) pairs
-CASES = [((43, 43, 4096, 64), True), ((43, 43, 1024, 64), False), ((26, 13, 4000, 128), True), ((14, 7, 4096, 192), True)]
+# (heads, heads_k, seqlen, head_dim), causal: several groups of several heads and a smaller last one in the kernel for head dim 64,
+# 128 and 192 and (the last shape) in the one for dQ alone; all heads in one group. test_plans_cpu.py states which is which.
+SEVERAL = [((43, 43, 4096, 64), True), ((43, 43, 1024, 64), False), ((13, 13, 1024, 128), False), ((43, 43, 1024, 192), True),
+           ((105, 35, 4096, 128), True)]
+CASES = SEVERAL + [((26, 13, 4000, 128), True), ((14, 7, 4096, 192), True)]
 
 
 @pytest.mark.parametrize("shape,causal", CASES, ids=[str(c[0]) for c in CASES])
@@ -102,7 +105,8 @@ def test_threads_that_share_a_stream():
     assert ops.device_status() == 0
 
 
-# (heads, heads_k, seqlen_q, seqlen_k, head_dim), options: more than two CTAs per SM, so that CTAs take over tiles of others
+# (heads, heads_k, seqlen_q, seqlen_k, head_dim), options: more than two CTAs per SM, so that CTAs take over tiles of others, but
+# for the last one, which is just below that
 TAKE_OVER = [((60, 60, 100, 1000, 64), dict(causal=True, window_left=300)),   # key blocks that no row sees, among the others
              ((60, 60, 100, 1000, 40), dict(causal=True, window_left=300)),   # rows of 80 bytes
              ((240, 240, 130, 200, 56), {}), ((700, 350, 5, 3, 64), {}), ((300, 75, 129, 129, 64), dict(causal=True, softcap=15.0))]
@@ -125,4 +129,40 @@ def test_tiles_taken_over_from_other_ctas(shape, opt):
         alone = ops.bwd(q[:, :, mine], k[:, :, own], v[:, :, own], do[:, :, mine], lse[:, mine].contiguous(),
                         delta[:, mine].contiguous(), **opt)
         assert torch.equal(alone[1], dk[:, :, own]) and torch.equal(alone[2], dv[:, :, own])
+    assert ops.device_status() == 0
+
+
+# More iterations a tile (5, 8, 15), so that stages and phases carry on from one tile to the next in every position; each score
+# transform; both types. (heads, heads_k, seqlen_q, seqlen_k, head_dim), type, ALiBi, options
+FORMS = [((180, 60, 600, 600, 64), torch.bfloat16, False, dict(causal=True)), ((800, 200, 129, 129, 64), torch.bfloat16, False, dict(causal=True, softcap=15.0)),
+         ((62, 62, 600, 600, 64), torch.float16, True, dict(causal=True)), ((62, 62, 600, 600, 64), torch.bfloat16, True, {}),
+         ((130, 65, 520, 600, 48), torch.float16, True, dict(causal=True, softcap=20.0))]
+
+
+@pytest.mark.parametrize("shape,dtype,alibi,opt", FORMS, ids=[f"{c[0]}-{c[1]}" for c in FORMS])
+def test_every_form_of_tiles_taken_over(shape, dtype, alibi, opt):
+    import flash_attn2_b200 as fa2
+    from flash_attn2_b200 import cabi_ops as ops
+
+    h, hk, sq, sk, d = shape
+    assert hk * -(-sk // 128) > 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    q, k, v, do = [t.cuda() for t in make_qkv(8, 1, h, hk, sq, sk, d, dtype, with_do=True)]
+    slopes = alibi_slopes(h).cuda() if alibi else None
+    out, lse = ops.fwd(q, k, v, alibi_slopes=slopes, **opt)
+    delta = ops.bwd_preprocess(do, out)
+    dq, dk, dv = ops.bwd(q, k, v, do, lse, delta, alibi_slopes=slopes, **opt)
+    g, few = h // hk, 5
+    for first in range(0, hk - few, max(1, hk // 5)):   # a few heads at a time: one wave
+        mine, own = slice(first * g, (first + few) * g), slice(first, first + few)
+        alone = ops.bwd(q[:, :, mine], k[:, :, own], v[:, :, own], do[:, :, mine], lse[:, mine].contiguous(),
+                        delta[:, mine].contiguous(), alibi_slopes=None if slopes is None else slopes[mine].contiguous(), **opt)
+        assert torch.equal(alone[1], dk[:, :, own]) and torch.equal(alone[2], dv[:, :, own])
+    # dK and dV without dQ, and the bit-reproducible pair
+    only = ops.bwd(q, k, v, do, lse, delta, which=2, alibi_slopes=slopes, **opt)
+    assert torch.equal(only[1], dk) and torch.equal(only[2], dv)
+    dq_alone = ops.bwd(q, k, v, do, lse, delta, which=1, alibi_slopes=slopes, **opt)[0]
+    pair = fa2.bwd(do, q, k, v, out, lse, alibi_slopes=slopes, is_causal=opt.get("causal", False), softcap=opt.get("softcap", 0.0),
+                   deterministic=True)
+    assert all(torch.equal(a, b) for a, b in zip(pair, (dq_alone, dk, dv)))
+    torch.testing.assert_close(dq, dq_alone, atol=2e-2, rtol=2e-2)
     assert ops.device_status() == 0

@@ -140,10 +140,11 @@ def test_few_row_calls_start_early_where_that_is_faster(plans, shape):
     assert plans.few_rows_start_early(ctypes.byref(_fwd_args(b, h, hk, 1, sk, d, causal=1)), SMS) == (shape in EARLY)
 
 
-# (batch, heads, heads_k, seqlen, head_dim), causal, heads in a group: all of them in a call of few CTAs; else equal groups of at
-# most 96 MB (25 MB a head: 9 groups of 32 heads; 3 MB: 9 of 256; 96 KB: 1024 heads), without a mask 16 MB (391 KB a head).
+# (batch, heads, heads_k, seqlen, head_dim), causal, heads in a group: all of them in a call of few CTAs; else about 96 MB in as
+# even groups as whole heads allow (25 MB a head: 9 groups of 32 heads; 3 MB: 9 of 256; 96 KB: 1024 heads; 71 MB: pairs), without a
+# mask 16 MB (391 KB a head).
 GROUPS = [((4, 16, 4, 2048, 128), 1, 16), ((1, 32, 32, 16384, 128), 1, 4), ((16, 16, 16, 2048, 128), 1, 29),
-          ((32, 12, 12, 509, 64), 0, 43), ((1, 1, 1, 1, 8), 0, 1), ((65535, 64, 64, 128, 64), 1, 1024)]
+          ((32, 12, 12, 509, 64), 0, 43), ((1, 1, 1, 1, 8), 0, 1), ((65535, 64, 64, 128, 64), 1, 1024), ((2, 64, 8, 8192, 128), 1, 2)]
 
 
 @pytest.mark.parametrize("shape,causal,want", GROUPS, ids=str)
@@ -155,3 +156,20 @@ def test_heads_in_a_group(plans, shape, causal, want):
     assert 1 <= plans.head_group(ctypes.byref(args), 1, SMS) <= b * h
     args.cu_seqlens_q = 8  # packed sequences differ in length: one after the other
     assert plans.head_group(ctypes.byref(args), 0, SMS) == 1
+
+
+def test_the_gpu_test_of_the_order_has_several_groups(plans):
+    from tests.test_bwd_order_gpu import CASES, SEVERAL
+
+    def groups(shape, causal, dq_alone):
+        h, hk, s, d = shape
+        args = _bwd_args(1, h, hk, s, s, d)
+        args.causal = causal
+        n, heads = plans.head_group(ctypes.byref(args), dq_alone, SMS), h if dq_alone else hk
+        return n, heads
+
+    for shape, causal in CASES:
+        n, heads = groups(shape, causal, 0)
+        assert 1 < n < heads and heads % n if (shape, causal) in SEVERAL else n == heads
+    n, heads = groups(*SEVERAL[-1], 1)
+    assert 1 < n < heads and heads % n
