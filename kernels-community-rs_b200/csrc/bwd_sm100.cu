@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   uint64_t* k_empty = bars + 4;    // [2] the tile's last dQ has read K
   uint64_t* v_empty = bars + 6;    // [2] its last dP^T has read V
   uint64_t* q_full = bars + 8;     // [2]
-  uint64_t* q_empty = bars + 10;   // [2]
+  uint64_t* q_empty = bars + 10;   // [2] dK has read the stage (and, in packed batches, the fixer has seen it)
   uint64_t* do_full = bars + 12;   // [2]
   uint64_t* do_empty = bars + 14;  // [2] dV has read the stage (and, in packed batches, the fixer has seen it)
   uint64_t* s_full = bars + 16;
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
       if (bar == dq_free || bar == epi_full || bar == epi_full + 1) count = kBlk;
       if (bar == stat_empty || bar == stat_empty + 1) count = 8;    // compute warps
       if (bar == next_empty || bar == next_empty + 1) count = want_dq ? 14 : 10;  // issuer, statistics, compute, drain warps
-      if (PACKED && (bar == do_empty || bar == do_empty + 1)) count = 2;  // the dV commit and the fixer
+      if (PACKED && (bar == q_empty || bar == q_empty + 1 || bar == do_empty || bar == do_empty + 1)) count = 2;  // the commit and the fixer
       mbar_init(bar, count);
     }
     if (lane == 0) *abort_flag = 0;
@@ -598,13 +598,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           clear_rows(s_q + st * Cfg::kTileBytes, first);
           publish(&q_fixed[st]);
         }
+        // No stage is refilled before this warp has seen it: its waits go by phase parity.
+        if (ok && lane == 0) mbar_arrive(&q_empty[st]);
+        __syncwarp();
         const uint32_t dst = it % Cfg::kDOStages;
         ok = ok && __all_sync(0xffffffffu, mbar_wait(&do_full[dst], (it / Cfg::kDOStages) & 1, ctl, kWaitBwd + 5));
         if (ok && first < kBlk) {
           clear_rows(s_do + dst * Cfg::kTileBytes, first);
           publish(&do_fixed[dst]);
         }
-        // The stage is not refilled before this warp has seen it: its waits go by phase parity.
         if (ok && lane == 0) mbar_arrive(&do_empty[dst]);
         __syncwarp();
       }

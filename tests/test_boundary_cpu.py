@@ -161,3 +161,16 @@ def test_kernels_that_start_early_wait_before_they_let_the_next_one_in():
         packed = "bool PACKED" in start.group(1)
         assert when == ("!PACKED" if packed else "early" if kernel == "fwd_decode_kernel" else "true"), (f, kernel)
         assert ("if (!PACKED) early_trigger();" in body) == packed, (f, kernel)
+
+
+def test_the_backward_refills_no_stage_that_the_fixer_has_not_seen():
+    """The fixer warp of packed batches waits for every Q and dO tile by the parity of its barrier's phase. A stage that came back to
+    the loader without it could be filled again meanwhile, and the warp would wait for a phase that has gone by."""
+    body = (ROOT / "kernels-community-rs_b200" / "csrc" / "bwd_sm100.cu").read_text()
+    counted = re.search(r"if \(PACKED && \(([^;]*)\)\) count = 2;", body).group(1)
+    fixer = body[body.index("- fixer (packed batches)"):body.index("- -LSE (log2 domain)")]
+    waited = set(re.findall(r"mbar_wait\(&(\w+)_full\[", fixer))
+    assert waited == {"q", "do"}
+    for name in waited:
+        assert f"bar == {name}_empty" in counted and f"bar == {name}_empty + 1" in counted, name
+        assert re.search(rf"mbar_arrive\(&{name}_empty\[", fixer), name
