@@ -156,12 +156,12 @@ __device__ __forceinline__ int next_cta(uint32_t answer) {
 // touches global memory only behind early_wait, which returns once everything before it in the stream has completed
 // and is visible; what precedes it (barriers, TMEM, descriptors) runs beside the end of that. Every CTA waits, so that a
 // grid never ends before its predecessor. early_trigger, behind the wait, lets the next grid start as soon as all CTAs
-// of this one have started. Every grid waits, whatever its arguments: memory that a call frees on its return is given to the next
-// call in the stream, and only a grid that has waited is promised to see what was written before it. B1 H32/8 Sk 8192 decoding 16.4 -> 13.0 us a call, B4 H16/4 S2048 softcap forward and backward
-// 373 -> 366, B32 H12 S509 D64 229.4 -> 222.9. Packed batches and long few-row calls that leave SMs idle
-// (decode_starts_early) start when the grid before them has ended. The memory-bound kernels of the backward are launched the usual way: their
-// blocks otherwise settle on the SMs that the grid before them leaves first, and large calls got slower (forward and backward
-// of B16 H16 S2048 D128 causal 1330 -> 1399 us).
+// of this one have started. Every grid waits, whatever its arguments: memory that a call frees on its return is given to the
+// next call in the stream, and only a grid that has waited is promised to see what was written before it. B1 H32/8 Sk 8192
+// decoding 16.4 -> 13.0 us a call, B4 H16/4 S2048 softcap forward and backward 373 -> 366, B32 H12 S509 D64 229.4 -> 222.9.
+// Packed batches and long few-row calls that leave SMs idle (decode_starts_early) start when the grid before them has ended.
+// The memory-bound kernels of the backward are launched the usual way: their blocks otherwise settle on the SMs that the grid
+// before them leaves first, and large calls got slower (forward and backward of B16 H16 S2048 D128 causal 1330 -> 1399 us).
 __device__ __forceinline__ void early_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void early_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
