@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
     make_list_div(p, ld);
     for (int i = 0; i < Cfg::kSlots; ++i) {
       mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 2);  // one commit per issuer
+      mbar_init(&kv_empty[i], PACKED ? 3 : 2);  // one commit per issuer, and the fixer
       mbar_init(&kv_fixed[i], 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -756,8 +756,8 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
       if (ok) ok = mbar_wait(&q_empty[1], (n_q1 & 1) ^ 1, ctl, kWaitLoadQEmpty);
     } else if (warp == kFixWarp) {
       // ---------------------------------------------------------------- fixer (packed batches)
-      // Walks the ring in the loader's order and waits for every tile, which keeps it within one ring
-      // pass of the consumers; it acts on V tiles that reach past the end of their sequence.
+      // Walks the ring in the loader's order and waits for every tile by the parity of its slot's phase, so no slot is
+      // filled again before it has seen the tile; it acts on V tiles that reach past the end of their sequence.
       if (PACKED) {
         uint32_t slot = 0, ring_phase = 0;
         bool ok = true;
@@ -775,6 +775,8 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
             if (lane == 0) mbar_arrive(&kv_fixed[slot]);
             __syncwarp();
           }
+          if (lane == 0) mbar_arrive(&kv_empty[slot]);
+          __syncwarp();
           if (++slot == Cfg::kSlots) {
             slot = 0;
             ring_phase ^= 1;

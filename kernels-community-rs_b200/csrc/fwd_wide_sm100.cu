@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
     *abort_flag = 0;
     for (int i = 0; i < kWSlots; ++i) {
       mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
+      mbar_init(&kv_empty[i], PACKED ? 2 : 1);  // the commit and the fixer
       mbar_init(&kv_fixed[i], 1);
     }
     mbar_init(q_full, 1);
@@ -396,8 +396,8 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
     }
   } else if (warp == kWFixWarp) {
     // ---------------------------------------------------------------- fixer (packed batches)
-    // Walks the ring in the loader's order and waits for every tile, which keeps it within one ring pass of
-    // the issuer; it acts on V tiles that reach past the end of their sequence.
+    // Walks the ring in the loader's order and waits for every tile by the parity of its slot's phase, so no slot is
+    // filled again before it has seen the tile; it acts on V tiles that reach past the end of their sequence.
     if (PACKED) {
       uint32_t slot = 0, ring_phase = 0;
       bool ok = true;
@@ -414,6 +414,8 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
           if (lane == 0) mbar_arrive(&kv_fixed[slot]);
           __syncwarp();
         }
+        if (lane == 0) mbar_arrive(&kv_empty[slot]);
+        __syncwarp();
         if (++slot == kWSlots) {
           slot = 0;
           ring_phase ^= 1;

@@ -163,9 +163,19 @@ def test_kernels_that_start_early_wait_before_they_let_the_next_one_in():
         assert ("if (!PACKED) early_trigger();" in body) == packed, (f, kernel)
 
 
+@pytest.mark.parametrize("kernel", ["fwd_sm100.cu", "fwd_wide_sm100.cu"])
+def test_the_forward_refills_no_slot_that_the_fixer_has_not_seen(kernel):
+    """The fixer warp of packed batches waits for every tile by the parity of its barrier's phase. A stage that came back to the
+    loader without it could be filled again meanwhile, and the warp would wait for a phase that has gone by."""
+    body = (ROOT / "kernels-community-rs_b200" / "csrc" / kernel).read_text()
+    packed, dense = re.search(r"mbar_init\(&kv_empty\[i\], PACKED \? (\d) : (\d)\);", body).groups()
+    assert int(packed) == int(dense) + 1
+    fixer = body[body.index("- fixer (packed batches)"):body.index("- mma issuer")]
+    assert re.search(r"mbar_wait\(&kv_full\[slot\]", fixer) and re.search(r"mbar_arrive\(&kv_empty\[slot\]\)", fixer)
+
+
 def test_the_backward_refills_no_stage_that_the_fixer_has_not_seen():
-    """The fixer warp of packed batches waits for every Q and dO tile by the parity of its barrier's phase. A stage that came back to
-    the loader without it could be filled again meanwhile, and the warp would wait for a phase that has gone by."""
+    """The same for its Q and dO stages."""
     body = (ROOT / "kernels-community-rs_b200" / "csrc" / "bwd_sm100.cu").read_text()
     counted = re.search(r"if \(PACKED && \(([^;]*)\)\) count = 2;", body).group(1)
     fixer = body[body.index("- fixer (packed batches)"):body.index("- -LSE (log2 domain)")]
