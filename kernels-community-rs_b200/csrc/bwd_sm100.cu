@@ -27,7 +27,8 @@
 // A CTA's start and end cost 9000 cycles, a third of its time where a head has four query blocks. At D = 64 there is shared
 // memory for K and V of two tiles, so a CTA goes on with the tile of a CTA that has not started: K, V, Q and dO of the next
 // tile are loaded beside the end of this one. B32 H12 S509 D64 fp16 223.6 -> 201.0 us, B2 H16 S4096 D64 causal 378 -> 358.
-// That includes what it costs: with the tile carried through every role these instances spill 340-372 bytes of loads a thread.
+// That includes what it costs: with the tile carried through every role these instances spill 340-372 bytes of loads a thread. So
+// calls in which no CTA takes a tile over have instances without it (launch_one).
 // At D = 128 K has to wait for the last dQ and nothing is left to stage dK and dV in: B4 H16 S1000 112.8 -> 114.8 us,
 // B4 H16/4 S2048 softcap 340 -> 345, so there a CTA has one tile. Packed batches have one tile per CTA too.
 //
@@ -189,10 +190,11 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
 // MODE: what is done to the scores; PACKED: cu_seqlens batches. Both are compile-time so that the plain dense
 // kernel carries none of their code: at 156 KB the all-in-one kernel missed the SM's instruction cache on a
 // quarter of its fetches and ran 6-9 % slower than the 62 KB one.
-template <int D, bool BF16, int MODE, bool PACKED>
+// TAKE_OVER: a CTA goes on with tiles of CTAs that have not started. Calls in which no CTA does have instances without the code.
+template <int D, bool BF16, int MODE, bool PACKED, bool TAKE_OVER>
 __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = BwdCfg<D>;
-  constexpr bool kPersistent = D == 64 && !PACKED;
+  static_assert(!TAKE_OVER || (Cfg::kKVStages == 2 && !PACKED), "the next tile needs K and V stages of its own");
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
     early_wait();
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         const uint32_t ks = pos.kv % Cfg::kKVStages, kph = (pos.kv / Cfg::kKVStages) & 1;
         Walk w{ti.g0, ti.mi0};
         for (int it = 0; it < ti.n_iter || it == 0; ++it) {
-          if (kPersistent && p.take_over && it + 1 >= ti.n_iter) {
+          if (TAKE_OVER && it + 1 >= ti.n_iter) {
             mbar_expect_tx(answered, 16);
             ask_next_cta(smem_u32(smem + Cfg::kAnswerOff), answered);
           }
@@ -383,16 +385,16 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             load(s_k + ks * Cfg::kTileBytes, &p.tm_k, &k_full[ks], ti.hk, ti.k_row0 + ti.n0);
           }
         }
-        if (!kPersistent || !ok) break;
+        if (!TAKE_OVER || !ok) break;
         // The tile after this one.
         const uint32_t slot = pos.n & 1;
-        ok = (!p.take_over || mbar_wait(answered, pos.n & 1, ctl, kWaitBwd + 24)) &&
+        ok = mbar_wait(answered, pos.n & 1, ctl, kWaitBwd + 24) &&
              mbar_wait(&next_empty[slot], ((pos.n >> 1) & 1) ^ 1, ctl, kWaitBwd + 25);
         if (!ok) break;
         ++pos.n;
         pos.it0 += ti.n_iter;
         pos.kv += ti.n_iter > 0 ? 1 : 0;
-        const int t = p.take_over ? next_cta(smem_u32(smem + Cfg::kAnswerOff)) : -1;
+        const int t = next_cta(smem_u32(smem + Cfg::kAnswerOff));
         if (t >= 0) ti = get_kv_tile<PACKED>(p, t);
         else ti.n_iter = -1;
         volatile int* a = reinterpret_cast<volatile int*>(s_next + slot * 3);
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           }
         }
         if (ok && n_iter > 0) mma_commit(dkv_done);
-        if (!ok || !kPersistent) break;
+        if (!ok || !TAKE_OVER) break;
         const uint32_t slot = pos.n & 1;
         ok = next_tile(ti, pos);
         mbar_arrive(&next_empty[slot]);
@@ -638,7 +640,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(&stat_full[buf]);
         }
-      } while (kPersistent && ok && next_tile_warp(ti, pos));
+      } while (TAKE_OVER && ok && next_tile_warp(ti, pos));
     }
   } else if (warp < 12) {
     // ------------------------------------------------------------------ compute
@@ -841,7 +843,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
                                "r"(acc[8 * c + 5]), "r"(acc[8 * c + 6]), "r"(acc[8 * c + 7])
                                : "memory");
             }
-          } else if (kPersistent) {
+          } else if (TAKE_OVER) {
             // Straight to memory, 32 bytes (a whole sector) per store where the rows allow.
             const bool sectors = (reinterpret_cast<uintptr_t>(gptr) & 31) == 0 && (p.head_dim & 15) == 0;
             if (kpos < ti.sk) {
@@ -897,7 +899,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         }
       }
       __syncwarp();
-    } while (kPersistent && ok && next_tile_warp(ti, pos));
+    } while (TAKE_OVER && ok && next_tile_warp(ti, pos));
   } else {
     // ------------------------------------------------------------------ dQ drain
     // The whole 128 x D fp32 tile goes to registers at once so that the dP^T / dQ columns are free
@@ -1000,7 +1002,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             atomicAdd(turn, 1);
           }
         }
-      } while (kPersistent && ok && next_tile_warp(ti, pos));
+      } while (TAKE_OVER && ok && next_tile_warp(ti, pos));
       if (lane == 0) tma_wait_group_read<0>();
     }
   }
@@ -1017,55 +1019,64 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-template <int D, bool BF16, int MODE, bool PACKED>
-cudaError_t launch_one(const BwdParams& p, int num_ctas, cudaStream_t stream) {
+template <int D, bool BF16, int MODE, bool PACKED, bool TAKE_OVER>
+cudaError_t launch_tiles(const BwdParams& p, int num_ctas, cudaStream_t stream) {
   using Cfg = BwdCfg<D>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     cudaError_t e =
-        cudaFuncSetAttribute(bwd_kernel<D, BF16, MODE, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(bwd_kernel<D, BF16, MODE, PACKED, TAKE_OVER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_grid(!PACKED, bwd_kernel<D, BF16, MODE, PACKED>, dim3(num_ctas), kThreads, Cfg::kSmemBytes, stream, p);
+  return launch_grid(!PACKED, bwd_kernel<D, BF16, MODE, PACKED, TAKE_OVER>, dim3(num_ctas), kThreads, Cfg::kSmemBytes, stream, p);
+}
+
+template <int D, bool BF16, int MODE, bool PACKED>
+cudaError_t launch_one(const BwdParams& p, int num_ctas, int num_sms, cudaStream_t stream) {
+  // A CTA asks for its next tile before it has finished this one; in a call of a wave or two that takes tiles away from SMs
+  // that are about to be free (B1 H8/2 S1500 D64, bit-reproducible: 57.7 -> 59.5 us). Below the line the code alone costs 1-4 us;
+  // forward and backward (graph replay) with it and without: 288 CTAs, B2 H16 S1100 causal, 55.8, 52.0 us, 144 CTAs, B1 H12 S1500,
+  // 61.1, 59.6. Above it: 416 CTAs, B26 H8 S256, 45.0, 46.7, 1536 CTAs, B32 H12 S509 fp16, 207, 222.
+  if constexpr (D == 64 && !PACKED) {
+    if (num_ctas > 2 * num_sms) return launch_tiles<D, BF16, MODE, PACKED, true>(p, num_ctas, stream);
+  }
+  return launch_tiles<D, BF16, MODE, PACKED, false>(p, num_ctas, stream);
 }
 
 template <int D, bool BF16>
-cudaError_t pick_features(const BwdParams& p, int mode, bool packed, int num_ctas, cudaStream_t stream) {
+cudaError_t pick_features(const BwdParams& p, int mode, bool packed, int num_ctas, int num_sms, cudaStream_t stream) {
   if (packed) {
-    return mode != kScorePlain ? launch_one<D, BF16, kScoreAny, true>(p, num_ctas, stream)
-                               : launch_one<D, BF16, kScorePlain, true>(p, num_ctas, stream);
+    return mode != kScorePlain ? launch_one<D, BF16, kScoreAny, true>(p, num_ctas, num_sms, stream)
+                               : launch_one<D, BF16, kScorePlain, true>(p, num_ctas, num_sms, stream);
   }
   switch (mode) {
-    case kScorePlain: return launch_one<D, BF16, kScorePlain, false>(p, num_ctas, stream);
-    case kScoreSoftcap: return launch_one<D, BF16, kScoreSoftcap, false>(p, num_ctas, stream);
-    case kScoreAlibi: return launch_one<D, BF16, kScoreAlibi, false>(p, num_ctas, stream);
-    default: return launch_one<D, BF16, kScoreAny, false>(p, num_ctas, stream);
+    case kScorePlain: return launch_one<D, BF16, kScorePlain, false>(p, num_ctas, num_sms, stream);
+    case kScoreSoftcap: return launch_one<D, BF16, kScoreSoftcap, false>(p, num_ctas, num_sms, stream);
+    case kScoreAlibi: return launch_one<D, BF16, kScoreAlibi, false>(p, num_ctas, num_sms, stream);
+    default: return launch_one<D, BF16, kScoreAny, false>(p, num_ctas, num_sms, stream);
   }
 }
 
 template <int D>
-cudaError_t pick_dtype(const BwdParams& p, bool bf16, int mode, bool packed, int num_ctas, cudaStream_t stream) {
-  return bf16 ? pick_features<D, true>(p, mode, packed, num_ctas, stream)
-              : pick_features<D, false>(p, mode, packed, num_ctas, stream);
+cudaError_t pick_dtype(const BwdParams& p, bool bf16, int mode, bool packed, int num_ctas, int num_sms, cudaStream_t stream) {
+  return bf16 ? pick_features<D, true>(p, mode, packed, num_ctas, num_sms, stream)
+              : pick_features<D, false>(p, mode, packed, num_ctas, num_sms, stream);
 }
 
 }  // namespace
 
-cudaError_t launch_bwd(BwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream) {
+cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream) {
   const int num_ctas = (p.dk_part != nullptr ? p.items_per_head : p.num_nblk) * p.batch * p.heads_k;
   if (num_ctas <= 0) return cudaSuccess;
   if (head_dim <= 0 || head_dim > 128) return cudaErrorInvalidValue;
   const int mode = (p.softcap > 0.f ? kScoreSoftcap : 0) | (p.alibi != nullptr ? kScoreAlibi : 0);
   const bool packed = p.cu_q != nullptr;
-  // A CTA asks for its next tile before it has finished this one; in a call of a wave or two that takes tiles away from SMs
-  // that are about to be free (B1 H8/2 S1500 D64, bit-reproducible: 57.7 -> 59.5 us).
-  p.take_over = num_ctas > 2 * num_sms;
-  return head_dim > 64 ? pick_dtype<128>(p, bf16, mode, packed, num_ctas, stream)
-                       : pick_dtype<64>(p, bf16, mode, packed, num_ctas, stream);
+  return head_dim > 64 ? pick_dtype<128>(p, bf16, mode, packed, num_ctas, num_sms, stream)
+                       : pick_dtype<64>(p, bf16, mode, packed, num_ctas, num_sms, stream);
 }
 
 }  // namespace fa2

@@ -45,7 +45,7 @@ cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, bool e
 
 // dQ / dK / dV for head_dim a multiple of 8 up to 128; the fp32 dQ accumulator behind p.tm_dqa (and the turn
 // counters p.dq_turn, when given) must be zero.
-cudaError_t launch_bwd(BwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream);
+cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream);
 
 // The same for head_dim a multiple of 8 in 136..256: one CTA per (128 keys, half of the head dim), query blocks of
 // 64 rows; p.tm_q and p.tm_do carry boxes of 64 rows, dQ goes through p.dq_acc, dK and dV through p.dk_ptr / p.dv_ptr.

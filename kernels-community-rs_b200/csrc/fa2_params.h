@@ -105,7 +105,6 @@ struct BwdParams {
   int head_group;                       // (batch, kv head) pairs whose key blocks are listed together, heaviest first
   int window_left, window_right;
   int which;                            // bit 0: dQ, bit 1: dK and dV
-  int take_over;                        // D = 64: a CTA goes on with tiles of CTAs that have not started (set at the launch)
   float scale, scale_log2;
   int* status;
   // Score transforms of the forward that the gradients have to follow (null / 0 when unused).
