@@ -39,12 +39,12 @@
 #include "sm100_ptx.cuh"
 #include "fa2_params.h"
 #include "fa2_launch.h"
+#include "bwd_tile.cuh"
 
 namespace fa2 {
 
 namespace {
 
-constexpr int kBlk = 128;  // keys per CTA and query rows per iteration
 constexpr int kThreads = 512;
 constexpr int kComputeRegs = 152;
 constexpr int kDrainRegs = 152;
@@ -52,7 +52,6 @@ constexpr int kMiscRegs = 56;
 // setmaxnreg moves registers inside the CTA's own allocation (128 per thread at launch: 65536 / 512). What the
 // compute and drain warps take must not exceed what warps 0-3 give back: an increase beyond it never returns.
 static_assert(8 * (kComputeRegs - 128) + 4 * (kDrainRegs - 128) <= 4 * (128 - kMiscRegs), "setmaxnreg: more registers asked for than released");
-constexpr float kLog2e = 1.4426950408889634f;
 
 template <int D>
 struct BwdCfg {
@@ -99,30 +98,6 @@ __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-
-// Query blocks [m_start, m_start + n_m) whose rows can see a key of [n0, n0 + 127].
-__device__ __forceinline__ void q_block_range(const BwdParams& p, int sq, int sk, int n0, int& m_start, int& n_m) {
-  int q_lo = 0, q_hi = sq;  // [q_lo, q_hi)
-  const int off = sk - sq;
-  const int n_last = min(n0 + kBlk - 1, sk - 1);
-  if (p.window_right >= 0) q_lo = max(0, n0 - off - p.window_right);
-  if (p.window_left >= 0) q_hi = min(sq, n_last - off + p.window_left + 1);
-  m_start = q_lo / kBlk;
-  n_m = (q_hi > q_lo) ? ((q_hi + kBlk - 1) / kBlk - m_start) : 0;
-}
-
-// Position of an iteration in the CTA's walk over (query head of the GQA group, query block), advanced
-// without integer divisions: iteration it is head g = it / n_m of the group, query block m_start + it % n_m.
-struct Walk {
-  int g, mi;
-};
-__device__ __forceinline__ Walk walk_next(Walk w, int n_m) {
-  if (++w.mi == n_m) {
-    w.mi = 0;
-    ++w.g;
-  }
-  return w;
 }
 
 template <bool PACKED>
@@ -175,7 +150,7 @@ __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   }
   ti.off = ti.sk - ti.sq;
   ti.valid = ti.n0 < ti.sk;
-  q_block_range(p, ti.sq, ti.sk, ti.n0, ti.m_start, ti.n_m);
+  q_block_range(p, ti.sq, ti.sk, ti.n0, kBlk, ti.m_start, ti.n_m);
   ti.n_iter = ti.n_m * p.group;
   ti.g0 = ti.mi0 = 0;
   if (ti.parts > 1) {
@@ -951,7 +926,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
               bool covers = false;
               if (n < p.num_nblk && n * kBlk < ti.sk) {
                 int ms, nm;
-                q_block_range(p, ti.sq, ti.sk, n * kBlk, ms, nm);
+                q_block_range(p, ti.sq, ti.sk, n * kBlk, kBlk, ms, nm);
                 covers = (mq >= ms) && (mq < ms + nm);
               }
               rank += __popc(__ballot_sync(0xffffffffu, covers));

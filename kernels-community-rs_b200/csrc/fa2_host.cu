@@ -20,6 +20,7 @@
 namespace {
 
 using fa2::BwdSplit;
+using fa2::bwd_takes_pairs;
 using fa2::DecodePlan;
 using fa2::decode_plan;
 using fa2::decode_starts_early;
@@ -575,7 +576,12 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   const int64_t hd = static_cast<int64_t>(a->heads) * d, hkd = static_cast<int64_t>(a->heads_k) * d;
   // Head dims above 128 run on the kernel that takes query rows 64 at a time (bwd_wide_sm100.cu).
   const bool wide = d > 128;
-  const int q_box_rows = wide ? 64 : 128;
+  BwdSplit split;
+  plan_bwd_split(a, opt.share_key_blocks != 0, rt->sm_count, &split);
+  const bool is_split = split.fits(a->dq_accum, a->dq_accum_bytes, bwd_dq_bytes(a));
+  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, packed);
+  const bool pairs = !is_split && bwd_takes_pairs(a, w, rt->sm_count);
+  const int q_box_rows = wide || pairs ? 64 : 128;
   if ((rc = make_map(&p.tm_q, a->q, a->dtype, 2, d, a->heads, rows_q, nbatch, a->q_stride[2], a->q_stride[1],
                      a->q_stride[0], 64, q_box_rows, "q")) != FA2_OK) return rc;
   if ((rc = make_map(&p.tm_do, a->dout, a->dtype, 2, d, a->heads, rows_q, nbatch, a->do_stride[2], a->do_stride[1],
@@ -630,7 +636,6 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   p.seqlen_q = a->seqlen_q;
   p.seqlen_k = a->seqlen_k;
   p.num_nblk = (a->seqlen_k + 127) / 128;
-  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, packed);
   p.window_left = w.left;
   p.window_right = w.right;
   p.head_group = bwd_head_group(a, w, rt->sm_count);
@@ -674,11 +679,8 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
     return fail(FA2_E_RUNTIME, "memset failed: %s", cudaGetErrorString(e));
   fa2::FinishParams fin;
   fin.dk_part = nullptr;
-  BwdSplit split;
-  plan_bwd_split(a, opt.share_key_blocks != 0, rt->sm_count, &split);
-  const int64_t before = bwd_dq_bytes(a);
-  if (split.fits(a->dq_accum, a->dq_accum_bytes, before)) {
-    p.dk_part = reinterpret_cast<float*>(static_cast<char*>(a->dq_accum) + before);
+  if (is_split) {
+    p.dk_part = reinterpret_cast<float*>(static_cast<char*>(a->dq_accum) + bwd_dq_bytes(a));
     p.part_stride = (split.part_elems * 4 + 255) / 256 * 64;
     p.dv_part = p.dk_part + split.max_parts * p.part_stride;
     p.items_per_head = split.items_per_head;
@@ -701,8 +703,9 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   p.v_batch_stride = packed ? 0 : a->v_stride[0];
   p.v_row_stride = a->v_stride[1];
   p.v_head_stride = a->v_stride[2];
-  e = wide ? fa2::launch_bwd_wide(p, d, a->dtype == FA2_BF16, stream)
-           : fa2::launch_bwd(p, d, a->dtype == FA2_BF16, rt->sm_count, stream);
+  e = wide    ? fa2::launch_bwd_wide(p, d, a->dtype == FA2_BF16, stream)
+      : pairs ? fa2::launch_bwd_pair(p, a->dtype == FA2_BF16, stream)
+              : fa2::launch_bwd(p, d, a->dtype == FA2_BF16, rt->sm_count, stream);
   if (a->ev_kernel_stop != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_stop), stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "backward launch failed: %s", cudaGetErrorString(e));
   fin.dq_acc = want_dq ? static_cast<const float*>(a->dq_accum) : nullptr;
@@ -834,12 +837,15 @@ int bwd_static_impl(const fa2_bwd_args* a, void* stream_v) {
 
   fa2::BwdParams p;
   memset(&p, 0, sizeof(p));
+  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
+  const bool pairs = bwd_takes_pairs(a, w, rt->sm_count);
+  const int q_box_rows = pairs ? 64 : 128;
   const int64_t rows_q = a->seqlen_q, rows_k = a->seqlen_k, nbatch = a->batch;
   const int64_t hd = static_cast<int64_t>(a->heads) * d, hkd = static_cast<int64_t>(a->heads_k) * d;
   if ((rc = make_map(&p.tm_q, a->q, a->dtype, 2, d, a->heads, rows_q, nbatch, a->q_stride[2], a->q_stride[1],
-                     a->q_stride[0], 64, 128, "q")) != FA2_OK) return rc;
+                     a->q_stride[0], 64, q_box_rows, "q")) != FA2_OK) return rc;
   if ((rc = make_map(&p.tm_do, a->dout, a->dtype, 2, d, a->heads, rows_q, nbatch, a->do_stride[2], a->do_stride[1],
-                     a->do_stride[0], 64, 128, "dout")) != FA2_OK) return rc;
+                     a->do_stride[0], 64, q_box_rows, "dout")) != FA2_OK) return rc;
   if ((rc = make_map(&p.tm_k, a->k, a->dtype, 2, d, a->heads_k, rows_k, nbatch, a->k_stride[2], a->k_stride[1],
                      a->k_stride[0], 64, 128, "k")) != FA2_OK) return rc;
   if ((rc = make_map(&p.tm_v, a->v, a->dtype, 2, d, a->heads_k, rows_k, nbatch, a->v_stride[2], a->v_stride[1],
@@ -869,7 +875,6 @@ int bwd_static_impl(const fa2_bwd_args* a, void* stream_v) {
   p.seqlen_q = a->seqlen_q;
   p.seqlen_k = a->seqlen_k;
   p.num_nblk = (a->seqlen_k + 127) / 128;
-  const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
   p.window_left = w.left;
   p.window_right = w.right;
   p.head_group = bwd_head_group(a, w, rt->sm_count);
@@ -888,7 +893,8 @@ int bwd_static_impl(const fa2_bwd_args* a, void* stream_v) {
   cudaError_t e = cudaMemsetAsync(rt->accum, 0, static_cast<size_t>(n_dq) * 4, stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "memset failed: %s", cudaGetErrorString(e));
   p.head_dim = d;
-  if ((e = fa2::launch_bwd(p, d, a->dtype == FA2_BF16, rt->sm_count, stream)) != cudaSuccess)
+  e = pairs ? fa2::launch_bwd_pair(p, a->dtype == FA2_BF16, stream) : fa2::launch_bwd(p, d, a->dtype == FA2_BF16, rt->sm_count, stream);
+  if (e != cudaSuccess)
     return fail(FA2_E_RUNTIME, "backward launch failed: %s", cudaGetErrorString(e));
   fa2::FinishParams fin;
   fin.dk_part = nullptr;

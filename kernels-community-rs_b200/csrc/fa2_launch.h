@@ -47,6 +47,9 @@ cudaError_t launch_fwd_decode(const DecodeParams& p, int grid, bool bf16, bool e
 // counters p.dq_turn, when given) must be zero.
 cudaError_t launch_bwd(const BwdParams& p, int head_dim, bool bf16, int num_sms, cudaStream_t stream);
 
+// The same on pairs of CTAs with 256 keys, for the calls of bwd_takes_pairs; p.tm_q and p.tm_do carry boxes of 64 rows.
+cudaError_t launch_bwd_pair(const BwdParams& p, bool bf16, cudaStream_t stream);
+
 // The same for head_dim a multiple of 8 in 136..256: one CTA per (128 keys, half of the head dim), query blocks of
 // 64 rows; p.tm_q and p.tm_do carry boxes of 64 rows, dQ goes through p.dq_acc, dK and dV through p.dk_ptr / p.dv_ptr.
 cudaError_t launch_bwd_wide(const BwdParams& p, int head_dim, bool bf16, cudaStream_t stream);

@@ -227,6 +227,29 @@ inline int bwd_dq_head_group(const fa2_bwd_args* a, const Windows& w) {
   return static_cast<int>((heads + groups - 1) / groups);
 }
 
+// ---- pairs of CTAs (bwd_pair_sm100.cu). Does a backward call that is not split run on them? They add half as much into the dQ
+// accumulator, which is what large calls pay for, in time and in power; but both CTAs of a pair walk the query blocks that either of
+// them sees, and an iteration alone is no faster. Forward and backward in a steady loop (1000 W), one CTA per key block -> pairs:
+// B1 H32 S16384 causal 7709 -> 7461 us, B4 H16/4 S4096 2025 -> 1955, B16 H16 S2048 2265 -> 2220, B2 H32/8 S2048 557 -> 542,
+// B4 H16 S4096 causal 1144 -> 1133; with walks of less than 16 blocks B16 H16 S2048 causal 1364 -> 1385, B2 H16 S8192 window 1023
+// 684 -> 711; with few CTAs B1 H8/2 S8192 causal 545 -> 551; a soft cap, whose tanh makes the arithmetic the longer part, B4 H16/4 S4096
+// causal 1267 -> 1352; B2 H16 S8192 D96 3549 -> 3541.
+inline bool bwd_takes_pairs(const fa2_bwd_args* a, const Windows& w, int sm_count) {
+  if (a->cu_seqlens_q != nullptr || (a->which & 3) != 3 || a->head_dim <= 96 || a->head_dim > 128 || a->softcap > 0.f ||
+      a->alibi_slopes != nullptr)
+    return false;
+  const int64_t pairs = (static_cast<int64_t>(a->seqlen_k) + 255) / 256, off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q;
+  if (2 * pairs * a->batch * a->heads_k < sm_count * 3 / 2) return false;
+  // Query blocks of a head that the first and the last pair walk: their mean is the mean of all under a causal mask and without one.
+  auto blocks = [&](int64_t n0) {
+    const int64_t n_last = std::min<int64_t>(n0 + 255, a->seqlen_k - 1);
+    const int64_t lo = w.right >= 0 ? std::max<int64_t>(0, n0 - off - w.right) : 0;
+    const int64_t hi = w.left >= 0 ? std::min<int64_t>(a->seqlen_q, n_last - off + w.left + 1) : a->seqlen_q;
+    return hi > lo ? (hi + 127) / 128 - lo / 128 : 0;
+  };
+  return blocks(0) + blocks((pairs - 1) * 256) >= 2 * 16;
+}
+
 // ---- key blocks shared by several CTAs (bwd_sm100.cu: part_start). A CTA owns 128 keys of one kv head and walks the
 // query blocks of all the group's heads; with few (batch, kv head, key block) triples most SMs would have nothing
 // to do, or wait for the CTA with the longest walk.

@@ -293,6 +293,77 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
+// ---------------------------------------------------------------- CTA pairs
+// Two CTAs of a cluster whose tensor cores work on one MMA of M = 128 or 256 rows, half of the rows in each CTA's TMEM. One thread of
+// the CTA of rank 0 issues it; a descriptor names the same shared-memory offset in both: A has the CTA's own rows, B its half of the N
+// rows (or columns). Measured: 128x128x16 takes 32 cycles, 256x128x16 64, with either operand A in shared memory or TMEM.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// The address of a shared-memory word of this CTA in the CTA of rank `rank`.
+__device__ __forceinline__ uint32_t peer_smem(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Arrival at a barrier of either CTA. What is handed over with it is tensor memory, ordered by the tcgen05 fences, or shared memory of
+// this CTA, on which the writers' proxy fence has completed before. (With .release.cluster, which also waits for everything that the
+// thread has sent to the other CTA, an arrival takes up to 1300 cycles in place of 50: B1 H32 S16384 8377 us in place of 7356.)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Copy from this CTA's shared memory to the other one's; the bytes are counted at a barrier of the receiver.
+__device__ __forceinline__ void bulk_copy_cluster(uint32_t cluster_dst, uint32_t src, uint32_t bytes, uint32_t cluster_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(cluster_dst), "r"(src),
+               "r"(bytes), "r"(cluster_bar)
+               : "memory");
+}
+// tma_load_4d into this CTA, whose bytes are counted at a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const CUtensorMap* m, uint32_t cluster_bar, int c0, int c1, int c2,
+                                                 int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], "
+      "[%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(ncols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+template <uint32_t AOFF16, uint32_t BOFF16>
+__device__ __forceinline__ void mma_pair_ss_o(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 ra, rb;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "add.s64 ra, %1, %5;\n\tadd.s64 rb, %2, %6;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], ra, rb, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(AOFF16), "n"(BOFF16)
+      : "memory");
+}
+template <uint32_t ACOL, uint32_t BOFF16>
+__device__ __forceinline__ void mma_pair_ts_o(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 rb;\n\t.reg .b32 ta;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "add.s64 rb, %2, %6;\n\tadd.u32 ta, %1, %5;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [ta], rb, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(ACOL), "n"(BOFF16)
+      : "memory");
+}
+// Arrives at the barrier of both CTAs when every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void mma_pair_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
+}
+
 // ---------------------------------------------------------------- TMEM <-> registers
 // 32x32b: thread i of the warp owns TMEM lane (lane_base + i); register j is column (col + j).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {

@@ -1,0 +1,48 @@
+"""GPU: the backward on pairs of CTAs against the kernels with one CTA per key block, which other tests check against the oracle."""
+import pytest
+import torch
+
+from tests._cases import make_qkv
+
+pytestmark = pytest.mark.gpu
+
+# (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim, causal, window): calls that run on pairs (test_plans_cpu.py states that they
+# do). Whole tiles; a last pair of one block, of one key block and a bit, with nothing for its second CTA; bottom-right masks with more
+# keys than queries and with rows that see no key; windows; grouped heads; head dims below the kernel's.
+CASES = [(1, 28, 28, 2048, 2048, 128, False, (-1, -1)), (4, 32, 8, 2000, 1000, 128, False, (-1, -1)), (8, 16, 8, 2048, 300, 120, False, (-1, -1)),
+         (8, 16, 8, 1921, 257, 104, False, (-1, -1)), (2, 16, 8, 4200, 4200, 128, True, (-1, -1)), (2, 8, 8, 4100, 5000, 128, True, (-1, -1)),
+         (2, 8, 8, 5000, 4100, 112, True, (-1, -1)), (2, 8, 4, 5000, 5000, 128, False, (3000, 500))]
+
+
+def _check(args, causal, window, dtype):
+    from flash_attn2_b200 import cabi_ops as ops
+
+    q, k, v, do = args
+    opt = dict(causal=causal, window_left=window[0], window_right=window[1])
+    out, lse = ops.fwd(q, k, v, **opt)
+    delta = ops.bwd_preprocess(do, out)
+    dq, dk, dv = ops.bwd(q, k, v, do, lse, delta, **opt)
+    want_dq = ops.bwd(q, k, v, do, lse, delta, which=1, **opt)[0]
+    _, want_dk, want_dv = ops.bwd(q, k, v, do, lse, delta, which=2, **opt)
+    # Every value of dK and dV is the same sum in the same order; keys and rows that see nothing add exact zeros.
+    assert torch.equal(dk, want_dk) and torch.equal(dv, want_dv)
+    # dQ is summed in fp32 in another order: what lies within a few 1e-6 of a rounding boundary moves by a unit of the type (2^-8,
+    # 2^-11). That is at most one value in a hundred, so a 2-norm of at most a tenth of the unit.
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert (dq.double() - want_dq.double()).norm() <= 0.1 * unit * want_dq.double().norm()
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(str(i) for i in c[:6]))
+def test_pairs_give_what_single_ctas_give(case, dtype):
+    b, h, hk, sq, sk, d, causal, window = case
+    _check([t.cuda() for t in make_qkv(11, b, h, hk, sq, sk, d, dtype, with_do=True)], causal, window, dtype)
+
+
+def test_pairs_on_views_of_one_projection():
+    b, h, s, d = 2, 16, 2048, 128
+    gen = torch.Generator().manual_seed(12)
+    qkv = torch.randn(b, s, 3, h, d, generator=gen).to(torch.bfloat16).cuda()
+    do = torch.randn(b, s, h, d, generator=gen).to(torch.bfloat16).cuda()
+    _check([*qkv.unbind(2), do], False, (-1, -1), torch.bfloat16)

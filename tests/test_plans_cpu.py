@@ -32,6 +32,9 @@ int head_group(const fa2_bwd_args* a, int dq_alone, int sms) {
   const fa2::Windows w = fa2::normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false);
   return dq_alone ? fa2::bwd_dq_head_group(a, w) : fa2::bwd_head_group(a, w, sms);
 }
+int takes_pairs(const fa2_bwd_args* a, int sms) {
+  return fa2::bwd_takes_pairs(a, fa2::normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false), sms);
+}
 int few_rows_start_early(const fa2_fwd_args* a, int sms) {
   const fa2::DecodePlan d = fa2::decode_plan(a, sms);
   return fa2::decode_starts_early(a, d.tiles, d.grid, sms);
@@ -173,3 +176,23 @@ def test_the_gpu_test_of_the_order_has_several_groups(plans):
         assert 1 < n < heads and heads % n if (shape, causal) in SEVERAL else n == heads
     n, heads = groups(*SEVERAL[-1], 1)
     assert 1 < n < heads and heads % n
+
+
+def _takes_pairs(plans, case, **kw):
+    from flash_attn2_b200 import _cabi
+
+    b, h, hk, sq, sk, d, causal, (left, right) = case
+    a = _cabi.BwdArgs(**{**dict(batch=b, heads=h, heads_k=hk, seqlen_q=sq, seqlen_k=sk, head_dim=d, causal=causal, window_left=left,
+                                window_right=right, which=3), **kw})
+    return bool(plans.takes_pairs(ctypes.byref(a), SMS))
+
+
+def test_backward_calls_that_run_on_pairs(plans):
+    from tests.test_bwd_pair_gpu import CASES
+
+    assert all(_takes_pairs(plans, c) for c in CASES)
+    full = (4, 16, 16, 2048, 2048, 128, False, (-1, -1))
+    assert _takes_pairs(plans, full)
+    for other in (dict(which=1), dict(which=2), dict(head_dim=96), dict(head_dim=136), dict(softcap=30.0), dict(alibi_slopes=256),
+                  dict(cu_seqlens_q=256), dict(causal=True), dict(window_left=1023), dict(batch=1, heads=8, heads_k=8)):
+        assert not _takes_pairs(plans, full, **other), other
