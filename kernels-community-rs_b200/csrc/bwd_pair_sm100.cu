@@ -21,10 +21,14 @@
 // shared memory is under way, and dQ, which nothing in the iteration waits for, comes last: the drain has until the next dV.
 //
 // What bounds it: large calls run at the power limit (990 W, SM clock 1.45 GHz), where what counts is the energy of an iteration: the
-// reductions into the accumulator are 13 % of a training step of B1 H32 S16384, and a pair issues half of them (7553 -> 7307 us). In
+// reductions into the accumulator are 13 % of a training step of B1 H32 S16384, and a pair issues half of them (7478 -> 7223 us). In
 // cycles the compute warps, 3600 of an iteration: 1300 in the exponentials, both warpgroups at once; 550 for dS^T; 500 to hand dS^T on;
 // the rest in waits and TMEM accesses. The exchange takes 1100 cycles and more (32 B/clk); the same stores straight to the other CTA, with
 // their proxy fence, took 2000 that the compute warps had to wait for.
+//
+// The issuer's and the loader's steps are loops with one place in the code for each: the roles share the SM's instruction cache. With
+// a prologue of its own for each and the loader's steps written out (65 KB of machine code) B1 H32 S16384 took 7241 us, now 7223,
+// B4 H16/4 S4096 without a mask 1909, now 1893.
 //
 // Warps: 0 loader, 1 MMA issuer (CTA 0), 2 reports what CTA 1 has received, 3 statistics, 4-11 compute (two warpgroups, 64 queries each, one key per thread),
 // 12-15 dQ drain (64 queries, warps 12 and 13 columns 0-63, 14 and 15 columns 64-127).
@@ -105,9 +109,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
   uint64_t* kcol_full = bars + 1;
   uint64_t* v_full = bars + 2;
   uint64_t* q_full = bars + 3;
-  uint64_t* qcol_full = bars + 4;
+  uint64_t* qcol_full = q_full + 1;
   uint64_t* do_full = bars + 5;
-  uint64_t* docol_full = bars + 6;
+  uint64_t* docol_full = do_full + 1;
   uint64_t* p_full = bars + 7;      // P^T is in TMEM
   uint64_t* ds_full = bars + 8;     // dS^T is in TMEM
   uint64_t* dsx_full = bars + 9;    // dS^T is in shared memory: what stays in its CTA, and what CTA 1 has received
@@ -115,9 +119,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
   uint64_t* dq_free = bars + 11;    // dQ has left TMEM
   // Barriers of each CTA; commits arrive at those of both.
   uint64_t* q_empty = bars + 12;
-  uint64_t* qcol_empty = bars + 13;
+  uint64_t* qcol_empty = q_empty + 1;
   uint64_t* do_empty = bars + 14;
-  uint64_t* docol_empty = bars + 15;
+  uint64_t* docol_empty = do_empty + 1;
   uint64_t* s_full = bars + 16;
   uint64_t* dp_full = bars + 17;
   uint64_t* dq_full = bars + 18;
@@ -178,39 +182,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
   auto expect = [&](uint64_t* full, uint32_t bytes_each) {
     if (rank == 0) mbar_expect_tx(full, 2 * bytes_each);
   };
-  // [128 rows x 128]: two atoms of 64 columns
-  auto load_rows128 = [&](int dst, const CUtensorMap* tm, uint64_t* full, int head, int row) {
-    expect(full, Cfg::kTileBytes);
-#pragma unroll
-    for (int a = 0; a < 2; ++a) tma_load_4d_pair(smem + dst + a * Cfg::kAtomBytes, tm, leader(full), a * 64, head, row, ti.b);
-  };
-  // own half of a block of 128 query rows, [64 rows x 128]
-  auto load_rows64 = [&](int dst, const CUtensorMap* tm, uint64_t* full, int head, int row) {
-    expect(full, Cfg::kAtomBytes);
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-      tma_load_4d_pair(smem + dst + a * (Cfg::kAtomBytes / 2), tm, leader(full), a * 64, head, row + static_cast<int>(rank) * 64, ti.b);
-  };
-  // own columns of a block of 128 query rows, [128 rows x 64], from boxes of 64 rows
-  auto load_cols = [&](int dst, const CUtensorMap* tm, uint64_t* full, int head, int row) {
-    expect(full, Cfg::kAtomBytes);
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-      tma_load_4d_pair(smem + dst + a * (Cfg::kAtomBytes / 2), tm, leader(full), static_cast<int>(rank) * 64, head, row + a * 64, ti.b);
+  // Two pieces of a tile: 128 or 64 rows of two 64-column atoms.
+  auto load2 = [&](int dst, int step, const CUtensorMap* tm, uint64_t* full, int head, int c0, int c1, int r0, int r1) {
+    expect(full, 2 * step);
+    tma_load_4d_pair(smem + dst, tm, leader(full), c0, head, r0, ti.b);
+    tma_load_4d_pair(smem + dst + step, tm, leader(full), c1, head, r1, ti.b);
   };
   if (tid == 0 && n_iter > 0) {
-    const int hq = ti.hk * p.group, row = ti.m_start * kBlk;
-    load_rows128(Cfg::kKOff, &p.tm_k, k_full, ti.hk, n0);
-    load_rows64(Cfg::kQOff, &p.tm_q, q_full, hq, row);
-    load_rows128(Cfg::kVOff, &p.tm_v, v_full, ti.hk, n0);
-    load_rows64(Cfg::kDOOff, &p.tm_do, do_full, hq, row);
-    load_cols(Cfg::kDOColOff, &p.tm_do, docol_full, hq, row);
-    load_cols(Cfg::kQColOff, &p.tm_q, qcol_full, hq, row);
-    expect(kcol_full, Cfg::kTileBytes);
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-      tma_load_4d_pair(smem + Cfg::kKColOff + a * Cfg::kAtomBytes, &p.tm_k, leader(kcol_full), static_cast<int>(rank) * 64, ti.hk,
-                       ti.n0 + a * kBlk, ti.b);
+    const int col = static_cast<int>(rank) * 64;
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+      const bool cols = i == 2;  // K, V, K's columns
+      load2(i == 0 ? Cfg::kKOff : i == 1 ? Cfg::kVOff : Cfg::kKColOff, Cfg::kAtomBytes, i == 1 ? &p.tm_v : &p.tm_k,
+            i == 0 ? k_full : i == 1 ? v_full : kcol_full, ti.hk, cols ? col : 0, cols ? col : 64, cols ? ti.n0 : n0, cols ? ti.n0 + kBlk : n0);
+    }
   }
   __syncthreads();
   tc_fence_after();
@@ -221,31 +206,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
     reg_dealloc<kMiscRegs>();
     if (warp == 0 && elect_one()) {
       // ---------------------------------------------------------------- loader
-      // The first tiles were requested during set-up. In the order in which the stages come back.
-      Walk w{0, 0};
+      // In the order in which the stages come back: dO columns, the next Q rows, Q columns, the next dO rows. One place in the code:
+      // the roles of the CTA share the SM's instruction cache.
+      Walk w{0, -1}, next{0, 0};
       bool ok = true;
-      for (int it = 0; it + 1 < n_iter && ok; ++it) {
-        const int hq0 = ti.hk * p.group + w.g, row0 = (ti.m_start + w.mi) * kBlk;
-        w = walk_next(w, ti.n_m);
-        const int hq = ti.hk * p.group + w.g, row = (ti.m_start + w.mi) * kBlk;
-        const uint32_t ph = it & 1;
-        ok = mbar_wait(q_empty, ph, ctl, kWaitBwd + 1);
-        if (!ok) break;
-        load_rows64(Cfg::kQOff, &p.tm_q, q_full, hq, row);
-        if (it > 0) {
-          ok = mbar_wait(qcol_empty, ph ^ 1, ctl, kWaitBwd + 1);
-          if (!ok) break;
-          load_cols(Cfg::kQColOff, &p.tm_q, qcol_full, hq0, row0);
+#pragma unroll 1
+      for (int it = -1; it < n_iter && ok; ++it) {
+#pragma unroll 1
+        for (int i = 0; i < 4 && ok; ++i) {
+          const bool rows = (i & 1) != 0, is_q = i == 1 || i == 2;
+          if (rows ? it + 1 >= n_iter : it < 0) continue;
+          // own 64 rows of both halves of the head dim, or the own half of the head dim of both halves of the rows
+          const int use = rows ? it + 1 : it, r = static_cast<int>(rank) * 64;
+          const Walk& at = rows ? next : w;
+          const int row = (ti.m_start + at.mi) * kBlk;
+          ok = mbar_wait((is_q ? q_empty : do_empty) + (rows ? 0 : 1), (use & 1) ^ 1, ctl, kWaitBwd + 1);
+          if (ok)
+            load2((is_q ? Cfg::kQOff : Cfg::kDOOff) + (rows ? 0 : Cfg::kAtomBytes), Cfg::kAtomBytes / 2, is_q ? &p.tm_q : &p.tm_do,
+                  (is_q ? q_full : do_full) + (rows ? 0 : 1), ti.hk * p.group + at.g, rows ? 0 : r, rows ? 64 : r, rows ? row + r : row,
+                  rows ? row + r : row + 64);
         }
-        ok = mbar_wait(do_empty, ph, ctl, kWaitBwd + 2);
-        if (!ok) break;
-        load_rows64(Cfg::kDOOff, &p.tm_do, do_full, hq, row);
-        ok = mbar_wait(docol_empty, ph, ctl, kWaitBwd + 2);
-        if (!ok) break;
-        load_cols(Cfg::kDOColOff, &p.tm_do, docol_full, hq, row);
+        w = next;
+        next = walk_next(next, ti.n_m);
       }
-      if (ok && n_iter > 1 && mbar_wait(qcol_empty, n_iter & 1, ctl, kWaitBwd + 1))
-        load_cols(Cfg::kQColOff, &p.tm_q, qcol_full, ti.hk * p.group + w.g, (ti.m_start + w.mi) * kBlk);
     } else if (warp == 1 && rank == 0 && elect_one()) {
       // ---------------------------------------------------------------- mma issuer, for both CTAs
       constexpr uint32_t kBase = (1u << 4) | ((BF16 ? 1u : 0u) << 7) | ((BF16 ? 1u : 0u) << 10) | (static_cast<uint32_t>(kBlk >> 3) << 17);
@@ -265,39 +248,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
                         (ks.value / 4) * (Cfg::kAtomBytes >> 5) + (ks.value % 4) * 2>(d_tmem, a, b, idesc_qk, ks.value > 0 ? 1u : 0u);
         });
       };
-      bool ok = n_iter > 0;
-      if (ok) ok = mbar_wait(k_full, 0, ctl, kWaitBwd + 3) && mbar_wait(q_full, 0, ctl, kWaitBwd + 4);
-      if (ok) {
-        tc_fence_after();
-        kmajor(tmem + Cfg::kTmemS, k_d, q_d);
-        mma_pair_commit(s_full);
-        mma_pair_commit(q_empty);
-        ok = mbar_wait(v_full, 0, ctl, kWaitBwd + 3) && mbar_wait(do_full, 0, ctl, kWaitBwd + 5);
-      }
-      if (ok) {
-        tc_fence_after();
-        kmajor(tmem + Cfg::kTmemDP, v_d, do_d);
-        mma_pair_commit(dp_full);
-        mma_pair_commit(do_empty);
-      }
-      for (int it = 0; it < n_iter && ok; ++it) {
+      bool ok = true;
+#pragma unroll 1
+      for (int it = -1; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
         const bool has_next = it + 1 < n_iter;
         const uint32_t acc = it > 0 ? 1u : 0u;
         // dV += P^T dO
-        ok = mbar_wait(docol_full, ph, ctl, kWaitBwd + 5) && mbar_wait(p_full, ph, ctl, kWaitBwd + 6);
-        if (!ok) break;
-        tc_fence_after();
-        static_for<kBlk / 16>([&](auto ks) {
-          mma_pair_ts_o<ks.value * 8, ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, docol_d, idesc_dv,
-                                                              ks.value > 0 ? 1u : acc);
-        });
-        mma_pair_commit(docol_empty);
-        if (!has_next) mma_pair_commit(dv_done);
+        if (it >= 0) {
+          ok = mbar_wait(docol_full, ph, ctl, kWaitBwd + 5) && mbar_wait(p_full, ph, ctl, kWaitBwd + 6);
+          if (!ok) break;
+          tc_fence_after();
+          static_for<kBlk / 16>([&](auto ks) {
+            mma_pair_ts_o<ks.value * 8, ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, docol_d, idesc_dv,
+                                                                ks.value > 0 ? 1u : acc);
+          });
+          mma_pair_commit(docol_empty);
+          if (!has_next) mma_pair_commit(dv_done);
+        }
         // S^T of the next iteration: over P^T, which dV has read, and dQ of the iteration before, which has been drained
         if (has_next) {
-          ok = mbar_wait(q_full, ph ^ 1, ctl, kWaitBwd + 8);
-          if (ok && it > 0) ok = mbar_wait(dq_free, ph ^ 1, ctl, kWaitBwd + 10);
+          ok = mbar_wait(q_full, ph ^ 1, ctl, kWaitBwd + 8) &&
+               (it > 0 ? mbar_wait(dq_free, ph ^ 1, ctl, kWaitBwd + 10) : it == 0 || mbar_wait(k_full, 0, ctl, kWaitBwd + 3));
           if (!ok) break;
           tc_fence_after();
           kmajor(tmem + Cfg::kTmemS, k_d, q_d);
@@ -305,31 +277,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
           mma_pair_commit(q_empty);
         }
         // dK += dS^T Q
-        ok = mbar_wait(qcol_full, ph, ctl, kWaitBwd + 4) && mbar_wait(ds_full, ph, ctl, kWaitBwd + 7);
-        if (!ok) break;
-        tc_fence_after();
-        static_for<kBlk / 16>([&](auto ks) {
-          mma_pair_ts_o<(ks.value / 4) * 64 + (ks.value % 4) * 8, ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDK, tmem + Cfg::kTmemDP, qcol_d,
-                                                                                        idesc_dv, ks.value > 0 ? 1u : acc);
-        });
-        mma_pair_commit(qcol_empty);
+        if (it >= 0) {
+          ok = mbar_wait(qcol_full, ph, ctl, kWaitBwd + 4) && mbar_wait(ds_full, ph, ctl, kWaitBwd + 7);
+          if (!ok) break;
+          tc_fence_after();
+          static_for<kBlk / 16>([&](auto ks) {
+            mma_pair_ts_o<(ks.value / 4) * 64 + (ks.value % 4) * 8, ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDK, tmem + Cfg::kTmemDP, qcol_d,
+                                                                                          idesc_dv, ks.value > 0 ? 1u : acc);
+          });
+          mma_pair_commit(qcol_empty);
+        }
         // dP^T of the next iteration, over dP^T and dS^T of this one
         if (has_next) {
-          ok = mbar_wait(do_full, ph ^ 1, ctl, kWaitBwd + 9);
+          ok = mbar_wait(do_full, ph ^ 1, ctl, kWaitBwd + 9) && (it >= 0 || mbar_wait(v_full, 0, ctl, kWaitBwd + 3));
           if (!ok) break;
           tc_fence_after();
           kmajor(tmem + Cfg::kTmemDP, v_d, do_d);
           mma_pair_commit(dp_full);
           mma_pair_commit(do_empty);
         }
+        if (it < 0) continue;
         // dQ = dS K, over the second half of the next S^T, which has been read
-        if (it == 0) ok = mbar_wait(kcol_full, 0, ctl, kWaitBwd + 3);
         mbar_expect_tx(received, Cfg::kAtomBytes);
-        if (ok) ok = mbar_wait(received, ph, ctl, kWaitBwd + 19) && mbar_wait(dsx_full, ph, ctl, kWaitBwd + 7);
-        if (ok) {
-          if (has_next) ok = mbar_wait(s_read, ph ^ 1, ctl, kWaitBwd + 11);
-          else if (it > 0) ok = mbar_wait(dq_free, ph ^ 1, ctl, kWaitBwd + 10);
-        }
+        ok = (it > 0 || mbar_wait(kcol_full, 0, ctl, kWaitBwd + 3)) && mbar_wait(received, ph, ctl, kWaitBwd + 19) &&
+             mbar_wait(dsx_full, ph, ctl, kWaitBwd + 7) &&
+             (has_next ? mbar_wait(s_read, ph ^ 1, ctl, kWaitBwd + 11) : it == 0 || mbar_wait(dq_free, ph ^ 1, ctl, kWaitBwd + 10));
         if (!ok) break;
         tc_fence_after();
         static_for<2 * kBlk / 16>([&](auto ks) {
@@ -491,7 +463,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
       const uint32_t t_acc = tmem + lane_addr + (wg == 0 ? Cfg::kTmemDK : Cfg::kTmemDV);
       const float mul = (wg == 0) ? p.scale : 1.f;
       uint8_t* stage = smem + (wg == 0 ? Cfg::kKOff : Cfg::kVOff);
-#pragma unroll
+#pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         uint32_t acc[64];
         if (n_iter > 0) {
