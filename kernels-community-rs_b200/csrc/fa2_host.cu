@@ -21,6 +21,7 @@ namespace {
 
 using fa2::BwdSplit;
 using fa2::bwd_takes_pairs;
+using fa2::bwd_wide_takes_pairs;
 using fa2::DecodePlan;
 using fa2::decode_plan;
 using fa2::decode_starts_early;
@@ -113,6 +114,24 @@ int make_map(CUtensorMap* m, const void* ptr, int dtype, int esize, int64_t d, i
   CUresult r = g_encode(m, dt, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(FA2_E_VALUE, "cannot build a TMA descriptor for %s (CUresult %d)", name, (int)r);
+  return FA2_OK;
+}
+
+// The same tensor with its head dim, a multiple of 64, as 64-column atoms: 5-D over [batch][heads][atoms][rows][64]. One load brings
+// 64 rows of two atoms, each atom's rows side by side.
+int make_atom_map(CUtensorMap* m, const void* ptr, int dtype, int64_t d, int64_t heads, int64_t rows, int64_t batch, int64_t head_stride,
+                  int64_t row_stride, int64_t batch_stride, const char* name) {
+  const cuuint64_t dims[5] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(d / 64), static_cast<cuuint64_t>(heads),
+                              static_cast<cuuint64_t>(batch)};
+  // Size-1 dimensions may carry arbitrary strides; give them a legal one.
+  const cuuint64_t strides[4] = {static_cast<cuuint64_t>((rows > 1 ? row_stride : d) * 2), 128,
+                                 static_cast<cuuint64_t>((heads > 1 ? head_stride : d) * 2),
+                                 static_cast<cuuint64_t>((batch > 1 ? batch_stride : d) * 2)};
+  const cuuint32_t box[5] = {64, 64, 2, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = g_encode(m, dtype == FA2_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5,
+                        const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(FA2_E_VALUE, "cannot build a TMA descriptor for %s (CUresult %d)", name, (int)r);
   return FA2_OK;
 }
@@ -580,28 +599,36 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   plan_bwd_split(a, opt.share_key_blocks != 0, rt->sm_count, &split);
   const bool is_split = split.fits(a->dq_accum, a->dq_accum_bytes, bwd_dq_bytes(a));
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, packed);
-  const bool pairs = !is_split && bwd_takes_pairs(a, w, rt->sm_count);
-  const int q_box_rows = wide || pairs ? 64 : 128;
+  const bool pairs = wide ? bwd_wide_takes_pairs(a) : !is_split && bwd_takes_pairs(a, w, rt->sm_count);
+  const int q_box_rows = wide || pairs ? 64 : 128, k_box_rows = wide && pairs ? 64 : 128;
   if ((rc = make_map(&p.tm_q, a->q, a->dtype, 2, d, a->heads, rows_q, nbatch, a->q_stride[2], a->q_stride[1],
                      a->q_stride[0], 64, q_box_rows, "q")) != FA2_OK) return rc;
   if ((rc = make_map(&p.tm_do, a->dout, a->dtype, 2, d, a->heads, rows_q, nbatch, a->do_stride[2], a->do_stride[1],
                      a->do_stride[0], 64, q_box_rows, "dout")) != FA2_OK) return rc;
   if ((rc = make_map(&p.tm_k, a->k, a->dtype, 2, d, a->heads_k, rows_k, nbatch, a->k_stride[2], a->k_stride[1],
-                     a->k_stride[0], 64, 128, "k")) != FA2_OK) return rc;
+                     a->k_stride[0], 64, k_box_rows, "k")) != FA2_OK) return rc;
   if ((rc = make_map(&p.tm_v, a->v, a->dtype, 2, d, a->heads_k, rows_k, nbatch, a->v_stride[2], a->v_stride[1],
-                     a->v_stride[0], 64, 128, "v")) != FA2_OK) return rc;
+                     a->v_stride[0], 64, k_box_rows, "v")) != FA2_OK) return rc;
+  if (wide && pairs) {
+    const struct { CUtensorMap* map; const void* ptr; int64_t heads, rows; const int64_t* stride; const char* name; } in[4] = {
+        {&p.tm_q, a->q, a->heads, rows_q, a->q_stride, "q"}, {&p.tm_do, a->dout, a->heads, rows_q, a->do_stride, "dout"},
+        {&p.tm_k, a->k, a->heads_k, rows_k, a->k_stride, "k"}, {&p.tm_v, a->v, a->heads_k, rows_k, a->v_stride, "v"}};
+    for (const auto& t : in)
+      if ((rc = make_atom_map(t.map, t.ptr, a->dtype, d, t.heads, t.rows, nbatch, t.stride[2], t.stride[1], t.stride[0], t.name)) != FA2_OK)
+        return rc;
+  }
   if (want_dkv) {
-    if ((rc = make_map(&p.tm_dk, a->dk, a->dtype, 2, d, a->heads_k, rows_k, nbatch, d, hkd, rows_k * hkd, 64, 128,
+    if ((rc = make_map(&p.tm_dk, a->dk, a->dtype, 2, d, a->heads_k, rows_k, nbatch, d, hkd, rows_k * hkd, 64, k_box_rows,
                        "dk")) != FA2_OK) return rc;
-    if ((rc = make_map(&p.tm_dv, a->dv, a->dtype, 2, d, a->heads_k, rows_k, nbatch, d, hkd, rows_k * hkd, 64, 128,
+    if ((rc = make_map(&p.tm_dv, a->dv, a->dtype, 2, d, a->heads_k, rows_k, nbatch, d, hkd, rows_k * hkd, 64, k_box_rows,
                        "dv")) != FA2_OK) return rc;
   } else {  // a dQ-only call writes neither: the kernels never touch these maps
     p.tm_dk = p.tm_k;
     p.tm_dv = p.tm_v;
   }
   if (want_dq) {
-    // one reduce-add box: 32 columns of 32 query rows
-    if ((rc = make_map(&p.tm_dqa, a->dq_accum, 2, 4, d, a->heads, rows_q, nbatch, d, hd, rows_q * hd, 32, 32,
+    // one reduce-add box: 32 columns of 32 or 16 query rows
+    if ((rc = make_map(&p.tm_dqa, a->dq_accum, 2, 4, d, a->heads, rows_q, nbatch, d, hd, rows_q * hd, 32, wide && pairs ? 16 : 32,
                        "dq_accum")) != FA2_OK) return rc;
   } else {
     p.tm_dqa = p.tm_q;
@@ -703,8 +730,8 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   p.v_batch_stride = packed ? 0 : a->v_stride[0];
   p.v_row_stride = a->v_stride[1];
   p.v_head_stride = a->v_stride[2];
-  e = wide    ? fa2::launch_bwd_wide(p, d, a->dtype == FA2_BF16, stream)
-      : pairs ? fa2::launch_bwd_pair(p, a->dtype == FA2_BF16, stream)
+  e = pairs  ? (wide ? fa2::launch_bwd_wide_pair : fa2::launch_bwd_pair)(p, a->dtype == FA2_BF16, stream)
+      : wide ? fa2::launch_bwd_wide(p, d, a->dtype == FA2_BF16, stream)
               : fa2::launch_bwd(p, d, a->dtype == FA2_BF16, rt->sm_count, stream);
   if (a->ev_kernel_stop != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(a->ev_kernel_stop), stream);
   if (e != cudaSuccess) return fail(FA2_E_RUNTIME, "backward launch failed: %s", cudaGetErrorString(e));

@@ -250,6 +250,11 @@ inline bool bwd_takes_pairs(const fa2_bwd_args* a, const Windows& w, int sm_coun
   return blocks(0) + blocks((pairs - 1) * 256) >= 2 * 16;
 }
 
+// Head dim 256 (bwd_wide_pair_sm100.cu, which has the figures): all sizes, as many CTAs as the kernel with one per half of the head dim.
+inline bool bwd_wide_takes_pairs(const fa2_bwd_args* a) {
+  return a->cu_seqlens_q == nullptr && (a->which & 3) == 3 && a->head_dim == 256;
+}
+
 // ---- key blocks shared by several CTAs (bwd_sm100.cu: part_start). A CTA owns 128 keys of one kv head and walks the
 // query blocks of all the group's heads; with few (batch, kv head, key block) triples most SMs would have nothing
 // to do, or wait for the CTA with the longest walk.

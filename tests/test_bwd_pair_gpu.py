@@ -14,11 +14,18 @@ CASES = [(1, 28, 28, 2048, 2048, 128, False, (-1, -1)), (4, 32, 8, 2000, 1000, 1
          (2, 8, 8, 5000, 4100, 112, True, (-1, -1)), (2, 8, 4, 5000, 5000, 128, False, (3000, 500))]
 
 
-def _check(args, causal, window, dtype):
+# Head dim 256, all sizes: one query, one key block and a bit, a last pair with keys for one CTA only or too few for its first; masks as
+# above; score transforms.
+WIDE = [(1, 2, 2, 128, 128, 256, False, (-1, -1)), (2, 4, 2, 1, 300, 256, False, (-1, -1)), (3, 4, 4, 129, 65, 256, False, (-1, -1)),
+        (2, 4, 2, 577, 385, 256, False, (-1, -1)), (2, 8, 2, 777, 777, 256, True, (-1, -1)), (2, 4, 4, 300, 1021, 256, True, (-1, -1)),
+        (2, 4, 4, 700, 200, 256, True, (-1, -1)), (2, 4, 4, 1000, 1100, 256, False, (100, 50)), (1, 4, 4, 1024, 1024, 256, True, (127, 0))]
+
+
+def _check(args, causal, window, dtype, **opt):
     from flash_attn2_b200 import cabi_ops as ops
 
     q, k, v, do = args
-    opt = dict(causal=causal, window_left=window[0], window_right=window[1])
+    opt.update(causal=causal, window_left=window[0], window_right=window[1])
     out, lse = ops.fwd(q, k, v, **opt)
     delta = ops.bwd_preprocess(do, out)
     dq, dk, dv = ops.bwd(q, k, v, do, lse, delta, **opt)
@@ -46,3 +53,28 @@ def test_pairs_on_views_of_one_projection():
     qkv = torch.randn(b, s, 3, h, d, generator=gen).to(torch.bfloat16).cuda()
     do = torch.randn(b, s, h, d, generator=gen).to(torch.bfloat16).cuda()
     _check([*qkv.unbind(2), do], False, (-1, -1), torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("case", WIDE, ids=lambda c: "x".join(str(i) for i in c[:6]))
+def test_wide_pairs_give_what_single_ctas_give(case, dtype):
+    b, h, hk, sq, sk, d, causal, window = case
+    _check([t.cuda() for t in make_qkv(13, b, h, hk, sq, sk, d, dtype, with_do=True)], causal, window, dtype)
+
+
+@pytest.mark.parametrize("opt", [dict(softcap=20.0), dict(alibi=True), dict(softcap=20.0, alibi=True)], ids=lambda o: "-".join(o))
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+def test_wide_pairs_with_score_transforms(causal, opt):
+    from tests._cases import alibi_slopes
+
+    opt = dict(opt)
+    if opt.pop("alibi", False):
+        opt["alibi_slopes"] = alibi_slopes(8).cuda()
+    _check([t.cuda() for t in make_qkv(14, 2, 8, 4, 500, 450, 256, torch.bfloat16, with_do=True)], causal, (-1, -1), torch.bfloat16, **opt)
+
+
+def test_wide_pairs_on_views_of_one_projection():
+    gen = torch.Generator().manual_seed(15)
+    qkv = torch.randn(2, 300, 3, 4, 256, generator=gen).to(torch.bfloat16).cuda()
+    do = torch.randn(2, 300, 4, 256, generator=gen).to(torch.bfloat16).cuda()
+    _check([*qkv.unbind(2), do], True, (-1, -1), torch.bfloat16)

@@ -33,7 +33,7 @@ int head_group(const fa2_bwd_args* a, int dq_alone, int sms) {
   return dq_alone ? fa2::bwd_dq_head_group(a, w) : fa2::bwd_head_group(a, w, sms);
 }
 int takes_pairs(const fa2_bwd_args* a, int sms) {
-  return fa2::bwd_takes_pairs(a, fa2::normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false), sms);
+  return fa2::bwd_wide_takes_pairs(a) || fa2::bwd_takes_pairs(a, fa2::normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, false), sms);
 }
 int few_rows_start_early(const fa2_fwd_args* a, int sms) {
   const fa2::DecodePlan d = fa2::decode_plan(a, sms);
@@ -188,9 +188,10 @@ def _takes_pairs(plans, case, **kw):
 
 
 def test_backward_calls_that_run_on_pairs(plans):
-    from tests.test_bwd_pair_gpu import CASES
+    from tests.test_bwd_pair_gpu import CASES, WIDE
 
-    assert all(_takes_pairs(plans, c) for c in CASES)
+    assert all(_takes_pairs(plans, c) for c in CASES + WIDE)
+    assert not any(_takes_pairs(plans, WIDE[0], **other) for other in (dict(which=1), dict(which=2), dict(head_dim=248), dict(cu_seqlens_q=256)))
     full = (4, 16, 16, 2048, 2048, 128, False, (-1, -1))
     assert _takes_pairs(plans, full)
     for other in (dict(which=1), dict(which=2), dict(head_dim=96), dict(head_dim=136), dict(softcap=30.0), dict(alibi_slopes=256),
