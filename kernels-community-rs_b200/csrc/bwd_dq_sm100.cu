@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_kernel(const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::kMiscOff + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const WaitCtl ctl{abort_flag, p.status};
+  const WaitCtl ctl{abort_flag};
 
   const int first_bh = static_cast<int>(blockIdx.x) / (p.head_group * p.num_mblk) * p.head_group;
   const int n_bh = min(p.head_group, p.batch * p.heads - first_bh);
@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_kernel(const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
   if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
 }
 

@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const WaitCtl ctl{abort_flag, p.status};
+  const WaitCtl ctl{abort_flag};
   const KvTile first_tile = get_kv_tile<PACKED>(p, blockIdx.x);
   if (!first_tile.valid) return;
   const bool want_dq = (p.which & 1) != 0;
@@ -937,10 +937,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
               while (*reinterpret_cast<volatile int*>(turn) != rank) {
                 __nanosleep(200);
                 if (*abort_flag || clock64() - t0 > FA2_WAIT_LIMIT_CYCLES) {
-                  if (!*abort_flag) {
-                    *abort_flag = 1;
-                    if (p.status != nullptr) atomicCAS(p.status, 0, kWaitBwd + 19);
-                  }
+                  if (!*abort_flag) *abort_flag = kWaitBwd + 19;
                   ok = false;
                   break;
                 }
@@ -991,6 +988,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 

@@ -140,7 +140,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const int rank = static_cast<int>(cluster_rank());
-  const WaitCtl ctl{abort_flag, p.status};
+  const WaitCtl ctl{abort_flag};
   const WidePairTile ti = get_wide_pair_tile(p, blockIdx.x >> 1);
   const int n_iter = ti.n_iter;
   const int n0 = ti.n0 + rank * kKeys;  // first key of this CTA
@@ -595,6 +595,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
   // A CTA stays until the other one has read its operands and sent it everything.
   cluster_arrive();
   cluster_wait();

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const WaitCtl ctl{abort_flag, p.status};
+  const WaitCtl ctl{abort_flag};
   const WKvTile ti = get_wkv_tile(p, blockIdx.x);
   if (!ti.valid) return;
   constexpr int atoms = ATOMS;
@@ -689,6 +689,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
   if (warp == kBWMmaWarp) tmem_dealloc(tmem, 512);
 }
 

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::kMiscOff);
   volatile int* s_last = reinterpret_cast<volatile int*>(smem + Cfg::kMiscOff + 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const WaitCtl ctl{abort_flag, p.status};
+  const WaitCtl ctl{abort_flag};
   // this CTA's share of the tile list; without parts (no workspace for them) it is whole units
   const int64_t n_tiles = static_cast<int64_t>(p.units) * p.tiles_per_unit;
   int lo, hi;
@@ -571,6 +571,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
     }
   }
   __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
 }
 
 template <int A, int MT, bool BF16, bool PARTS>

@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const WaitCtl ctl{abort_flag, p.status};
+  const WaitCtl ctl{abort_flag};
   volatile ListDiv* ld = reinterpret_cast<volatile ListDiv*>(smem + Cfg::kMiscOff + 16);
   // Every role walks this CTA's positions of the work list.
   const int t_first = SHARED ? stream_bound(p, blockIdx.x) : static_cast<int>(blockIdx.x);
@@ -908,6 +908,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
   if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
 }
 

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const WaitCtl ctl{abort_flag, p.status};
+  const WaitCtl ctl{abort_flag};
   const WTile ti = get_wtile(p, blockIdx.x);
   if (!ti.valid) return;
   constexpr int atoms = ATOMS;
@@ -511,6 +511,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
   if (warp == kWMmaWarp) tmem_dealloc(tmem, 512);
 }
 

@@ -57,10 +57,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Shared abort state of one CTA: `abort` is set by the first wait that runs out.
+// Abort state of one CTA, a word of shared memory: the site code of a wait that ran out, or 0. report_abort hands it on when the
+// kernel ends.
 struct WaitCtl {
-  volatile int* abort_flag;   // shared memory
-  int* error_word;            // global memory, may be null
+  volatile int* abort_flag;
 };
 
 // Upper bound of one wait in SM clock cycles (about a second at B200 clocks).
@@ -68,19 +68,22 @@ struct WaitCtl {
 #define FA2_WAIT_LIMIT_CYCLES (1ll << 31)
 #endif
 
-// Returns false when the wait ran out (or the CTA already aborted).
+__device__ __forceinline__ uint32_t clock32() {
+  uint32_t c;
+  asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
+  return c;
+}
+
+// Returns false when the wait ran out (or the CTA already aborted). A kernel has 20 to 40 of these in line and its roles share the
+// SM's instruction cache, so there is no more in it than it needs.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code) {
   if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (uint32_t it = 1;; ++it) {
+  const uint32_t t0 = clock32();
+  do {
     if (mbar_try_wait(bar, parity)) return true;
     if (*ctl.abort_flag) return false;
-    if ((it & 7u) == 0u && clock64() - t0 > FA2_WAIT_LIMIT_CYCLES) break;
-  }
-  if (!*ctl.abort_flag) {
-    *ctl.abort_flag = 1;
-    if (ctl.error_word) atomicCAS(ctl.error_word, 0, code);
-  }
+  } while (clock32() - t0 < static_cast<uint32_t>(FA2_WAIT_LIMIT_CYCLES));
+  *ctl.abort_flag = code;
   return false;
 }
 
@@ -88,8 +91,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
 // hardware park the thread (a parked thread was seen to come back thousands of cycles after the phase
 // completed), at the price of issue slots while it spins.
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code) {
-  const long long t0 = clock64();
-  for (uint32_t it = 1;; ++it) {
+  const uint32_t t0 = clock32();
+  do {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -100,13 +103,15 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, c
         : "memory");
     if (ok) return true;
     if (*ctl.abort_flag) return false;
-    if ((it & 15u) == 0u && clock64() - t0 > FA2_WAIT_LIMIT_CYCLES) break;
-  }
-  if (!*ctl.abort_flag) {
-    *ctl.abort_flag = 1;
-    if (ctl.error_word) atomicCAS(ctl.error_word, 0, code);
-  }
+  } while (clock32() - t0 < static_cast<uint32_t>(FA2_WAIT_LIMIT_CYCLES));
+  *ctl.abort_flag = code;
   return false;
+}
+
+// After the CTA's last barrier, by one thread: the first site code goes to the status word (global memory, may be null).
+__device__ __forceinline__ void report_abort(const volatile int* abort_flag, int* status) {
+  const int code = *abort_flag;
+  if (code != 0 && status != nullptr) atomicCAS(status, 0, code);
 }
 
 // Wait of a whole warp. The vote brings the 32 lanes back together (they leave the polling loop in
