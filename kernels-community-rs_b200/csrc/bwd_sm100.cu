@@ -442,29 +442,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
         const int n_iter = ti.n_iter;
         const uint32_t ks = pos.kv % Cfg::kKVStages, kph = (pos.kv / Cfg::kKVStages) & 1;
         const uint64_t k_kmaj = k0_kmaj + ks * kTile16, k_mn = k_kmaj + kMn, v_kmaj = v0_kmaj + ks * kTile16;
-        const uint32_t st0 = pos.it0 & 1, dst0 = pos.it0 % Cfg::kDOStages;
-        if (n_iter > 0) {
-          ok = mbar_wait(&k_full[ks], kph, ctl, kWaitBwd + 3);
-          if (ok && packed && ti.n0 + kBlk > ti.sk) ok = mbar_wait(kv_fixed, 0, ctl, kWaitBwd + 20);
-          if (ok) ok = q_ready(ti.mi0, st0, (pos.it0 >> 1) & 1, kWaitBwd + 4);
-          if (ok) {
-            tc_fence_after();
-            kmajor_pair(tmem + Cfg::kTmemS, k_kmaj, q_kmaj + st0 * kTile16);
-            mma_commit(s_full);
-            ok = do_ready(ti.mi0, dst0, (pos.it0 / Cfg::kDOStages) & 1, kWaitBwd + 5);
-            if (ok) ok = mbar_wait(&v_full[ks], kph, ctl, kWaitBwd + 3);
-            // the columns of dP^T still hold the last dQ of the tile before
-            if (ok && want_dq && pos.it0 > 0) ok = mbar_wait(dq_free, (pos.it0 - 1) & 1, ctl, kWaitBwd + 10);
-          }
-          if (ok) {
-            tc_fence_after();
-            kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj + dst0 * kTile16);
-            mma_commit(dp_full);
-          }
-        }
+        // From one iteration before the first, of which only the next S^T and dP^T exist: the steps have one place in the code.
         Walk wn{ti.g0, ti.mi0};  // position of iteration it + 1
-        for (int it = 0; it < n_iter && ok; ++it) {
-          wn = walk_next(wn, ti.n_m);
+#pragma unroll 1
+        for (int it = -1; it < n_iter && ok; ++it) {
+          if (it >= 0) wn = walk_next(wn, ti.n_m);
           const uint32_t gi = pos.it0 + it;
           const uint32_t st = gi & 1;
           const uint32_t nph = ((gi + 1) >> 1) & 1;  // phase of the Q stage barriers of the next iteration
@@ -473,20 +455,26 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
           const bool has_next = it + 1 < n_iter;
           const uint32_t acc = it > 0 ? 1u : 0u;
           // dV += P^T dO   (P^T: two 32-column halves at S + 0 and S + 64)
-          ok = mbar_wait(p_full, gi & 1, ctl, kWaitBwd + 6);
-          if (!ok) break;
-          tc_fence_after();
-          if (want_dkv) {
-            const uint64_t b = do_mn + dst * kTile16;
-            static_for<kBlk / 16>([&](auto ks) {
-              mma_ts_o<(ks.value / 4) * 64 + (ks.value % 4) * 8, ks.value * (2048 >> 4)>(
-                  tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv, ks.value > 0 ? 1u : acc);
-            });
-          }
-          mma_commit(&do_empty[dst]);
-          if (!has_next) {
-            mma_commit(dv_done);  // dV is final: its epilogue runs beside the last dQ and dK GEMMs
-            mma_commit(&v_empty[ks]);
+          if (it >= 0) {
+            ok = mbar_wait(p_full, gi & 1, ctl, kWaitBwd + 6);
+            if (!ok) break;
+            tc_fence_after();
+            if (want_dkv) {
+              const uint64_t b = do_mn + dst * kTile16;
+              static_for<kBlk / 16>([&](auto ks) {
+                mma_ts_o<(ks.value / 4) * 64 + (ks.value % 4) * 8, ks.value * (2048 >> 4)>(
+                    tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS, b, idesc_dv, ks.value > 0 ? 1u : acc);
+              });
+            }
+            mma_commit(&do_empty[dst]);
+            if (!has_next) {
+              mma_commit(dv_done);  // dV is final: its epilogue runs beside the last dQ and dK GEMMs
+              mma_commit(&v_empty[ks]);
+            }
+          } else if (has_next) {
+            ok = mbar_wait(&k_full[ks], kph, ctl, kWaitBwd + 3);
+            if (ok && packed && ti.n0 + kBlk > ti.sk) ok = mbar_wait(kv_fixed, 0, ctl, kWaitBwd + 20);
+            if (!ok) break;
           }
           // S^T of the next iteration right behind dV, the last reader of P^T: the scores are there when the
           // compute warps come out of phase B.
@@ -498,30 +486,33 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
             mma_commit(s_full);
           }
           // dQ = dS K   (into the dP^T columns, which the compute warps have drained)
-          ok = mbar_wait(ds_full, gi & 1, ctl, kWaitBwd + 7);
-          if (!ok) break;
-          tc_fence_after();
-          if (want_dq) {
-            static_for<kBlk / 16>([&](auto ks) {
-              mma_ss_o<ks.value * (2048 >> 4), ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDP, ds_mn, k_mn, idesc_dq,
-                                                                        ks.value > 0 ? 1u : 0u);
-            });
-            mma_commit(dq_full);
+          if (it >= 0) {
+            ok = mbar_wait(ds_full, gi & 1, ctl, kWaitBwd + 7);
+            if (!ok) break;
+            tc_fence_after();
+            if (want_dq) {
+              static_for<kBlk / 16>([&](auto ks) {
+                mma_ss_o<ks.value * (2048 >> 4), ks.value * (2048 >> 4)>(tmem + Cfg::kTmemDP, ds_mn, k_mn, idesc_dq,
+                                                                          ks.value > 0 ? 1u : 0u);
+              });
+              mma_commit(dq_full);
+            }
+            if (!has_next) mma_commit(&k_empty[ks]);
+            // dK += dS^T Q
+            if (want_dkv) {
+              const uint64_t b = q_mn + st * kTile16;
+              static_for<kBlk / 16>([&](auto ks) {
+                mma_ss_o<(ks.value / 4) * kAtom16 + (ks.value % 4) * 2, ks.value * (2048 >> 4)>(
+                    tmem + Cfg::kTmemDK, ds_kmaj, b, idesc_dv, ks.value > 0 ? 1u : acc);
+              });
+            }
+            mma_commit(&q_empty[st]);
           }
-          if (!has_next) mma_commit(&k_empty[ks]);
-          // dK += dS^T Q
-          if (want_dkv) {
-            const uint64_t b = q_mn + st * kTile16;
-            static_for<kBlk / 16>([&](auto ks) {
-              mma_ss_o<(ks.value / 4) * kAtom16 + (ks.value % 4) * 2, ks.value * (2048 >> 4)>(
-                  tmem + Cfg::kTmemDK, ds_kmaj, b, idesc_dv, ks.value > 0 ? 1u : acc);
-            });
-          }
-          mma_commit(&q_empty[st]);
-          // dP^T of the next iteration, once the dQ tile has left TMEM
+          // dP^T of the next iteration, once the dQ tile, or the last one of the tile before, has left TMEM
           if (has_next) {
             ok = do_ready(wn.mi, ndst, ndph, kWaitBwd + 9);
-            if (ok && want_dq) ok = mbar_wait(dq_free, gi & 1, ctl, kWaitBwd + 10);
+            if (ok && it < 0) ok = mbar_wait(&v_full[ks], kph, ctl, kWaitBwd + 3);
+            if (ok && want_dq && gi + 1 > 0) ok = mbar_wait(dq_free, gi & 1, ctl, kWaitBwd + 10);
             if (!ok) break;
             tc_fence_after();
             kmajor_pair(tmem + Cfg::kTmemDP, v_kmaj, do_kmaj + ndst * kTile16);

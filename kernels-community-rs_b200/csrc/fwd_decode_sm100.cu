@@ -501,7 +501,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
         if (*s_last) {
           // All consumers add the parts up: the rows' maxima and sums go to shared memory, and a thread takes four columns of
           // a row at a time, with the loads of a batch of parts issued together: each batch is an L2 round trip.
-          auto part_of = [&](int c) { return p.partials + part_index(c) * static_cast<int64_t>(kPart); };
+          // Part c of the unit: every second slot, but the first one, which began in its share, has the slot behind.
+          const float* part0 = p.partials + 2 * static_cast<int64_t>(c_first) * kPart;
+          auto part_of = [&](int c) { return part0 + c * (2 * kPart) + (c == 0 ? kPart : 0); };
           const int n_parts = c_last - c_first + 1;
           float* sm = reinterpret_cast<float*>(scratch);
           float* sl = sm + n_parts * Cfg::kRows;
@@ -510,14 +512,13 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
           auto fetch = [&](int i, int c0) {
 #pragma unroll
             for (int e = 0; e < kBatch; ++e)
-              if (c0 + e < n_parts)
-                w[e] = __ldcg(reinterpret_cast<const float4*>(part_of(c_first + c0 + e) + i / (D / 4) * D + i % (D / 4) * 4));
+              if (c0 + e < n_parts) w[e] = __ldcg(reinterpret_cast<const float4*>(part_of(c0 + e)) + i);
           };
           if (Cfg::kMergeAhead && tid < p.rows * (D / 4)) fetch(tid, 0);
           for (int i = tid; i < n_parts * Cfg::kRows; i += kConsumers * 32) {
             const int r = i % Cfg::kRows;
             if (r < p.rows) {
-              const float* st = part_of(c_first + i / Cfg::kRows) + Cfg::kRows * D + r;
+              const float* st = part_of(i / Cfg::kRows) + Cfg::kRows * D + r;
               sm[i] = __ldcg(st);
               sl[i] = __ldcg(st + Cfg::kRows);
             }

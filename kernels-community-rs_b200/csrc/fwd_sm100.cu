@@ -105,25 +105,24 @@ __device__ __forceinline__ int stream_bound(const FwdParams& p, int c) {
   return static_cast<int>(static_cast<int64_t>(p.units_per_head) * p.batch * p.heads * c / p.stream_grid);
 }
 
-// Divisors of the work-list index as fixed-point reciprocals floor(2^40 / d) + 1: an integer division is a long
-// dependent chain, every role walks the list, and the softmax warps do so between two tiles. The quotient is one
-// 64-bit multiply, a shift and a correction on the integer pipes; going through float reciprocals instead put
-// int <-> float conversions on the MUFU unit, behind the other stage's exponentials (1000-3500 cycles a tile).
-// n / d for 0 <= n < 2^24; the four constants live in shared memory (written once by thread 0).
+// Divisors of the work-list index as 32-bit reciprocals floor((2^32 - 1) / d): an integer division is a long dependent chain and
+// a lot of code, every role walks the list, and the softmax warps do so between two tiles. For 0 <= n < 2^31 the high word of the
+// product is n / d or one less. (Through float reciprocals the conversions queued on the MUFU unit behind the other stage's exponentials,
+// 1000-3500 cycles a tile; with 2^40 / d in 64 bits and a division for what that did not cover the four lookups took 3 KB of code in
+// each role.) The constants live in shared memory, written once by thread 0.
 struct ListDiv {
-  unsigned long long grid, bh, heads, group;
+  uint32_t grid, bh, heads, group;  // bh: with shared tiles the units of a head
 };
+template <bool SHARED>
 __device__ __forceinline__ void make_list_div(const FwdParams& p, volatile ListDiv* d) {
-  d->grid = (1ull << 40) / gridDim.x + 1;
-  d->bh = (1ull << 40) / static_cast<unsigned>(p.batch * p.heads) + 1;
-  d->heads = (1ull << 40) / static_cast<unsigned>(p.heads) + 1;
-  d->group = (1ull << 40) / static_cast<unsigned>(p.group) + 1;
+  d->grid = 0xffffffffu / gridDim.x;
+  d->bh = 0xffffffffu / static_cast<uint32_t>(SHARED ? p.units_per_head : p.batch * p.heads);
+  d->heads = 0xffffffffu / static_cast<uint32_t>(p.heads);
+  d->group = 0xffffffffu / static_cast<uint32_t>(p.group);
 }
-__device__ __forceinline__ int div_small(int n, int d, unsigned long long m) {
-  if (n >= (1 << 24)) return n / d;
-  int q = static_cast<int>((static_cast<unsigned long long>(static_cast<unsigned>(n)) * m) >> 40);
-  if (q * d > n) --q;  // the reciprocal is rounded up: the estimate can be one too large for d >= 2^16
-  return q;
+__device__ __forceinline__ int div_list(int n, int d, uint32_t m) {
+  const int q = static_cast<int>(__umulhi(static_cast<uint32_t>(n), m));
+  return n - q * d >= d ? q + 1 : q;
 }
 
 // Key-tile ranges of the two stages of a block and their union.
@@ -158,9 +157,10 @@ __device__ __forceinline__ void key_ranges(const FwdParams& p, Tile& ti) {
 // The part of a work tile that starts at position x of the list of a launch with shared tiles; the share ends at
 // `end`. Query blocks of a head are neighbours in the list, and so are the heads of a GQA group: CTAs that run side by
 // side read the same K and V.
-__device__ __forceinline__ Tile get_segment(const FwdParams& p, int x, int end) {
+__device__ __forceinline__ Tile get_segment(const FwdParams& p, const volatile ListDiv* ldp, int x, int end) {
+  const ListDiv ld{ldp->grid, ldp->bh, ldp->heads, ldp->group};
   Tile ti;
-  const int bh = x / p.units_per_head;
+  const int bh = div_list(x, p.units_per_head, ld.bh);
   const int r = x - bh * p.units_per_head;
   int lo = 0, hi = p.num_mblk;  // block_start[lo] <= r < block_start[hi]
   while (hi - lo > 1) {
@@ -168,9 +168,9 @@ __device__ __forceinline__ Tile get_segment(const FwdParams& p, int x, int end) 
     if (p.block_start[mid] <= r) lo = mid;
     else hi = mid;
   }
-  ti.b = bh / p.heads;
+  ti.b = div_list(bh, p.heads, ld.heads);
   ti.h = bh - ti.b * p.heads;
-  ti.hk = ti.h / p.group;
+  ti.hk = div_list(ti.h, p.group, ld.group);
   ti.m0 = lo * (2 * kBlockM);
   ti.q_row0 = 0;
   ti.k_row0 = 0;
@@ -201,7 +201,7 @@ __device__ __forceinline__ Tile get_tile(const FwdParams& p, const volatile List
   // Work tiles are listed longest first; CTA c takes list entries c, 2G-1-c, 2G+c, 4G-1-c, ... (G CTAs):
   // reversing every other round evens out the work per CTA when the sizes fall off in plateaus.
   const int grid = static_cast<int>(gridDim.x);
-  const int round = div_small(t, grid, ld.grid);
+  const int round = div_list(t, grid, ld.grid);
   const int pos = (round & 1) ? round * grid + (grid - 1 - (t - round * grid)) : t;
   // Under a causal mask the upper half of a block sees one key tile more than the lower one. The stages run
   // independently through the CTA's list, so they take the halves in turns: otherwise stage 1 would end up with
@@ -212,11 +212,11 @@ __device__ __forceinline__ Tile get_tile(const FwdParams& p, const volatile List
     return ti;
   }
   const int bh = p.batch * p.heads;
-  const int mrev = div_small(pos, bh, ld.bh);
+  const int mrev = div_list(pos, bh, ld.bh);
   const int rem = pos - mrev * bh;
-  ti.b = div_small(rem, p.heads, ld.heads);
+  ti.b = div_list(rem, p.heads, ld.heads);
   ti.h = rem - ti.b * p.heads;
-  ti.hk = div_small(ti.h, p.group, ld.group);
+  ti.hk = div_list(ti.h, p.group, ld.group);
   ti.m0 = (p.num_mblk - 1 - mrev) * (2 * kBlockM);
   if (p.cu_q != nullptr) {
     ti.q_row0 = p.cu_q[ti.b];
@@ -298,12 +298,12 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   // Every role walks this CTA's positions of the work list.
   const int t_first = SHARED ? stream_bound(p, blockIdx.x) : static_cast<int>(blockIdx.x);
   const int t_end = SHARED ? stream_bound(p, blockIdx.x + 1) : p.num_tiles + static_cast<int>(blockIdx.x);
-  auto tile_at = [&](int t) { return SHARED ? get_segment(p, t, t_end) : get_tile(p, ld, t); };
+  auto tile_at = [&](int t) { return SHARED ? get_segment(p, ld, t, t_end) : get_tile(p, ld, t); };
   auto step_of = [&](const Tile& ti) { return SHARED ? max(1, ti.jhi - ti.jlo) : static_cast<int>(gridDim.x); };
 
   if (tid == 0) {
     *abort_flag = 0;
-    make_list_div(p, ld);
+    make_list_div<SHARED>(p, ld);
     for (int i = 0; i < Cfg::kSlots; ++i) {
       mbar_init(&kv_full[i], 1);
       mbar_init(&kv_empty[i], PACKED ? 3 : 2);  // one commit per issuer, and the fixer
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         if (votes & 2u) { ok = false; break; }
         if (j > nb_s && (votes & 1u)) {
           tc_fence_after();
-#pragma unroll
+#pragma unroll 1
           for (int c = 0; c < D / 16; ++c) {
             uint32_t orr[16];
             tmem_ld16(t_o + c * 16, orr);
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         mbar_arrive(&o_free[s]);
         if (row < ti.sq) {
           // No key is visible to this stage: O = 0.
-#pragma unroll
+#pragma unroll 1
           for (int q = 0; q < D / 8; ++q)
             if (q * 8 < p.head_dim) *reinterpret_cast<uint4*>(orow + q * 8) = make_uint4(0, 0, 0, 0);
         }
