@@ -1,4 +1,4 @@
-// FlashAttention-2 backward for sm_100a (B200) on pairs of CTAs, head dim 256: dQ, dK, dV of dense calls.
+// FlashAttention-2 backward for sm_100a (B200) on pairs of CTAs, head dims 192 and 256: dQ, dK, dV of dense calls.
 //
 // A pair owns 128 keys of one (batch, kv head), 64 in each CTA, and walks the 128-row query blocks (and the query heads of the GQA
 // group) that can see them. Its MMAs are issued by one thread of CTA 0 for both tensor cores:
@@ -9,7 +9,7 @@
 //   dK  += dS^T Q      128 x 256 x 128   A: own keys                    B: Q columns, 128 in each CTA
 //   dQ^T = K^T dS^T    256 x 128 x 128   A: 128 K columns in each CTA   B: dS^T of 64 queries in each CTA
 //
-// all from shared memory. In each CTA's TMEM a result of 128 rows has 64 of them: lanes 0-63 hold the first half of the columns,
+// all from shared memory (figures for head dim 256; at 192 the last 64 columns are zeros, which S^T and dP^T leave out). In each CTA's TMEM a result of 128 rows has 64 of them: lanes 0-63 hold the first half of the columns,
 // lanes 64-127 the second. So dK and dV of the pair take 128 columns each, S^T and dP^T 64, dQ^T 128. In the kernel with one CTA per
 // 128 keys and half of the head dim (bwd_wide_sm100.cu) S^T and dP^T, which contract over all of the head dim, are computed twice,
 // exponentials included, and most MMAs have N = 64, which costs 35-54 cycles in place of 32.
@@ -26,7 +26,8 @@
 // each, 88 KB of machine code, a wait for a barrier that had completed long ago took 150-400 cycles and an iteration 9000. Loops with one
 // place in the code for each step, 54 KB: 5350 cycles (the old kernel: 6600), the kernel 410 us (old: 476).
 // Forward and backward in a steady loop, old kernel -> this one, us, causal: B4 H16/8 S2048 808 -> 720, B1 H16 S8192 2544 -> 2247,
-// B2 H16/4 S2048 softcap 612 -> 477, B2 H16 S4096 window 256 479 -> 423; B4 H8 S1000 without a mask 221 -> 197, B16 H8 S300 156 -> 157.
+// B2 H16/4 S2048 softcap 612 -> 477, B2 H16 S4096 window 256 479 -> 423; B4 H8 S1000 without a mask 221 -> 197, B16 H8 S300 156 -> 157; at head dim 192
+// B4 H16/8 S2048 711 -> 638, B2 H16/4 S2048 softcap 588 -> 430, B4 H8 S1000 without a mask 194 -> 175.
 //
 // What bounds it: the latency of the ring, a turn of which takes a load's 900-1400 cycles twice an iteration, and the MMAs, 2600.
 //
@@ -100,10 +101,12 @@ __device__ __forceinline__ float tanh_approx(float x) {
 }
 
 // FANCY: a soft cap or ALiBi is in use.
-template <bool BF16, bool FANCY>
+// ATOMS: 64-column atoms of the head dim; the fourth one is zeros at head dim 192 (the loads fill it), and only the contractions over the
+// head dim leave it out.
+template <int ATOMS, bool BF16, bool FANCY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wide_pair_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = WidePairCfg;
-  constexpr int D = 256, kAtoms = D / 64, kHalf = D / 2;
+  constexpr int D = 256, kHalf = D / 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
     early_wait();
@@ -267,10 +270,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
         for (int i = 0; i < 2; ++i) {
           if (!ring_wait()) return false;
           const uint64_t b = ring_d + slot * (Cfg::kSlotBytes >> 4), aa = a + i * (2 * Cfg::kKAtom >> 4);
-          static_for<8>([&](auto ks) {
-            constexpr uint32_t o = (ks.value / 4) * (Cfg::kKAtom >> 4) + (ks.value % 4) * 2;
-            mma_pair_ss_o<o, o>(d_tmem, aa, b, idesc_qk, i + ks.value > 0 ? 1u : 0u);
-          });
+          auto steps = [&](auto atom) {
+            static_for<4>([&](auto ks) {
+              constexpr uint32_t o = atom.value * (Cfg::kKAtom >> 4) + ks.value * 2;
+              mma_pair_ss_o<o, o>(d_tmem, aa, b, idesc_qk, i + atom.value + ks.value > 0 ? 1u : 0u);
+            });
+          };
+          steps(std::integral_constant<int, 0>{});
+          if (ATOMS == 4 || i == 0) steps(std::integral_constant<int, 1>{});
           ring_next();
         }
         return true;
@@ -529,7 +536,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
       mbar_arrive(&epi_full[wg]);
       if ((tid & 127) == 0 && mbar_wait(&epi_full[wg], 0, ctl, kWaitBwd + 16)) {
 #pragma unroll
-        for (int a = 0; a < kAtoms; ++a)
+        for (int a = 0; a < ATOMS; ++a)
           if (a * 64 < p.head_dim) tma_store_4d(wg == 0 ? &p.tm_dk : &p.tm_dv, stage + a * Cfg::kKAtom, a * 64, ti.hk, n0, ti.b);
         tma_commit_group();
         tma_wait_group_read<0>();
@@ -602,13 +609,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
   if (warp == 1) tmem_dealloc_pair(tmem, 512);
 }
 
-template <bool BF16, bool FANCY>
+template <int ATOMS, bool BF16, bool FANCY>
 cudaError_t launch_one(const BwdParams& p, cudaStream_t stream) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(bwd_wide_pair_kernel<BF16, FANCY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(bwd_wide_pair_kernel<ATOMS, BF16, FANCY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          WidePairCfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
@@ -616,19 +623,21 @@ cudaError_t launch_one(const BwdParams& p, cudaStream_t stream) {
   const int64_t blocks = 2LL * p.num_nblk * p.batch * p.heads_k;
   if (blocks <= 0) return cudaSuccess;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  return launch_grid(true, bwd_wide_pair_kernel<BF16, FANCY>, dim3(static_cast<unsigned>(blocks)), kThreads, WidePairCfg::kSmemBytes,
+  return launch_grid(true, bwd_wide_pair_kernel<ATOMS, BF16, FANCY>, dim3(static_cast<unsigned>(blocks)), kThreads, WidePairCfg::kSmemBytes,
                      stream, p);
 }
 
-template <bool BF16>
+template <int ATOMS, bool BF16>
 cudaError_t pick_mode(const BwdParams& p, cudaStream_t stream) {
-  return p.softcap > 0.f || p.alibi != nullptr ? launch_one<BF16, true>(p, stream) : launch_one<BF16, false>(p, stream);
+  return p.softcap > 0.f || p.alibi != nullptr ? launch_one<ATOMS, BF16, true>(p, stream) : launch_one<ATOMS, BF16, false>(p, stream);
 }
 
 }  // namespace
 
 cudaError_t launch_bwd_wide_pair(const BwdParams& p, bool bf16, cudaStream_t stream) {
-  return bf16 ? pick_mode<true>(p, stream) : pick_mode<false>(p, stream);
+  if (p.head_dim == 192) return bf16 ? pick_mode<3, true>(p, stream) : pick_mode<3, false>(p, stream);
+  if (p.head_dim == 256) return bf16 ? pick_mode<4, true>(p, stream) : pick_mode<4, false>(p, stream);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace fa2

@@ -250,9 +250,14 @@ inline bool bwd_takes_pairs(const fa2_bwd_args* a, const Windows& w, int sm_coun
   return blocks(0) + blocks((pairs - 1) * 256) >= 2 * 16;
 }
 
-// Head dim 256 (bwd_wide_pair_sm100.cu, which has the figures): all sizes, as many CTAs as the kernel with one per half of the head dim.
+// Head dims 192 and 256 (bwd_wide_pair_sm100.cu, which has more figures). Its query blocks have 128 rows, those of the other kernel 64,
+// and at head dim 192 a quarter of what it does for dK, dV and dQ is padding: calls that pad their rows by a fifth more than in blocks
+// of 64 stay there. Without the line, before and after, us: D192 B16 H8 S300 142, 145, B16 H16/4 S300 causal 176, 183, B16 H8 S320 causal
+// 125, 129; on this side B16 H8 S450 233, 214, B32 H8 S128 89, 82. D256 B32 H8 S180 165, 164, B4 H16 Sq 64 Sk 2000 199, 194.
 inline bool bwd_wide_takes_pairs(const fa2_bwd_args* a) {
-  return a->cu_seqlens_q == nullptr && (a->which & 3) == 3 && a->head_dim == 256;
+  if (a->cu_seqlens_q != nullptr || (a->which & 3) != 3) return false;
+  const int64_t rows128 = (static_cast<int64_t>(a->seqlen_q) + 127) / 128 * 128, rows64 = (static_cast<int64_t>(a->seqlen_q) + 63) / 64 * 64;
+  return a->head_dim == 256 || (a->head_dim == 192 && 5 * rows128 < 6 * rows64);
 }
 
 // ---- key blocks shared by several CTAs (bwd_sm100.cu: part_start). A CTA owns 128 keys of one kv head and walks the

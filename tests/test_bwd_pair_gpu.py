@@ -14,11 +14,13 @@ CASES = [(1, 28, 28, 2048, 2048, 128, False, (-1, -1)), (4, 32, 8, 2000, 1000, 1
          (2, 8, 8, 5000, 4100, 112, True, (-1, -1)), (2, 8, 4, 5000, 5000, 128, False, (3000, 500))]
 
 
-# Head dim 256, all sizes: one query, one key block and a bit, a last pair with keys for one CTA only or too few for its first; masks as
+# Head dims 192 and 256: one query, one key block and a bit, a last pair with keys for one CTA only or too few for its first; masks as
 # above; score transforms.
 WIDE = [(1, 2, 2, 128, 128, 256, False, (-1, -1)), (2, 4, 2, 1, 300, 256, False, (-1, -1)), (3, 4, 4, 129, 65, 256, False, (-1, -1)),
         (2, 4, 2, 577, 385, 256, False, (-1, -1)), (2, 8, 2, 777, 777, 256, True, (-1, -1)), (2, 4, 4, 300, 1021, 256, True, (-1, -1)),
-        (2, 4, 4, 700, 200, 256, True, (-1, -1)), (2, 4, 4, 1000, 1100, 256, False, (100, 50)), (1, 4, 4, 1024, 1024, 256, True, (127, 0))]
+        (2, 4, 4, 700, 200, 256, True, (-1, -1)), (2, 4, 4, 1000, 1100, 256, False, (100, 50)), (1, 4, 4, 1024, 1024, 256, True, (127, 0)),
+        (1, 2, 2, 128, 128, 192, False, (-1, -1)), (3, 4, 4, 200, 65, 192, False, (-1, -1)), (2, 8, 2, 777, 777, 192, True, (-1, -1)),
+        (2, 4, 4, 333, 1021, 192, True, (-1, -1)), (2, 4, 4, 1000, 1100, 192, False, (100, 50))]
 
 
 def _check(args, causal, window, dtype, **opt):
@@ -63,14 +65,14 @@ def test_wide_pairs_give_what_single_ctas_give(case, dtype):
 
 
 @pytest.mark.parametrize("opt", [dict(softcap=20.0), dict(alibi=True), dict(softcap=20.0, alibi=True)], ids=lambda o: "-".join(o))
-@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
-def test_wide_pairs_with_score_transforms(causal, opt):
+@pytest.mark.parametrize("head_dim,causal", [(192, True), (256, False), (256, True)])
+def test_wide_pairs_with_score_transforms(head_dim, causal, opt):
     from tests._cases import alibi_slopes
 
     opt = dict(opt)
     if opt.pop("alibi", False):
         opt["alibi_slopes"] = alibi_slopes(8).cuda()
-    _check([t.cuda() for t in make_qkv(14, 2, 8, 4, 500, 450, 256, torch.bfloat16, with_do=True)], causal, (-1, -1), torch.bfloat16, **opt)
+    _check([t.cuda() for t in make_qkv(14, 2, 8, 4, 500, 450, head_dim, torch.bfloat16, with_do=True)], causal, (-1, -1), torch.bfloat16, **opt)
 
 
 def test_wide_pairs_on_views_of_one_projection():

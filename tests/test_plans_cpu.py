@@ -191,7 +191,8 @@ def test_backward_calls_that_run_on_pairs(plans):
     from tests.test_bwd_pair_gpu import CASES, WIDE
 
     assert all(_takes_pairs(plans, c) for c in CASES + WIDE)
-    assert not any(_takes_pairs(plans, WIDE[0], **other) for other in (dict(which=1), dict(which=2), dict(head_dim=248), dict(cu_seqlens_q=256)))
+    assert not any(_takes_pairs(plans, WIDE[0], **other) for other in (dict(which=1), dict(which=2), dict(head_dim=248), dict(head_dim=184),
+                                                               dict(cu_seqlens_q=256), dict(head_dim=192, seqlen_q=300)))
     full = (4, 16, 16, 2048, 2048, 128, False, (-1, -1))
     assert _takes_pairs(plans, full)
     for other in (dict(which=1), dict(which=2), dict(head_dim=96), dict(head_dim=136), dict(softcap=30.0), dict(alibi_slopes=256),
