@@ -416,7 +416,7 @@ def run_ours(args, rank, world):
                     frac_of_sustained_peak=None if not peak_sustained else tf(total / world, sustained["ms_per_step"]) / peak_sustained),
                 "long_context": long_context,
             },
-            "roofline": {"kernel": "bwd_kernel<128, bf16>" if D <= 128 else "bwd_wide_kernel<bf16>", "bound": "tensor", "achieved": achieved, "peak": peak,
+            "roofline": {"kernel": "bwd_kernel<128, bf16>" if D <= 128 else "bwd_wide_pair_kernel<bf16>" if D in (192, 256) else "bwd_wide_kernel<bf16>", "bound": "tensor", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind},
             "roofline_fwd": {"kernel": "fwd_kernel<128, bf16>" if D <= 128 else "fwd_wide_kernel<bf16>", "bound": "tensor", "achieved": tf(FWD_FLOPS, ms_fwd),
                              "peak": peak, "unit": "TFLOP/s", "frac": tf(FWD_FLOPS, ms_fwd) / peak},

@@ -39,7 +39,7 @@ extern "C" {
 /* Strides are in elements: {batch, row, head}; the head_dim stride is 1. In packed mode
  * the batch stride is ignored. head_dim is a multiple of 8 up to 256, the reference's range
  * (flash-attn2-rs/src/host/tiles.rs:1): up to 128 on the two-stage kernels, above on kernels with
- * smaller tiles (fwd_wide_sm100.cu, bwd_wide_sm100.cu). */
+ * smaller tiles (fwd_wide_sm100.cu, bwd_wide_sm100.cu) or on pairs of CTAs (bwd_wide_pair_sm100.cu). */
 typedef struct fa2_fwd_args {
   const void* q;
   const void* k;

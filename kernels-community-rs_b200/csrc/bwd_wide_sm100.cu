@@ -1,4 +1,6 @@
-// FlashAttention-2 backward for sm_100a (B200), head dims above 128 (136 ... 256): dQ, dK, dV in one kernel.
+// FlashAttention-2 backward for sm_100a (B200), head dims above 128 (136 ... 256): dQ, dK, dV in one kernel. Dense calls at head
+// dims 192 and 256 that want all three run on bwd_wide_pair_sm100.cu instead (bwd_wide_takes_pairs says which); packed batches, the
+// other head dims and calls for some of the gradients run here.
 //
 // dK and dV of 128 keys at head dim 256 would fill all 512 TMEM columns, so a CTA owns 128 keys of one
 // (batch, kv head) and one HALF of the head dim (columns [128 c, 128 c + 128)): it accumulates that half of dK

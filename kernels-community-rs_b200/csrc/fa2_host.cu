@@ -593,7 +593,7 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   fa2::BwdParams p;
   memset(&p, 0, sizeof(p));
   const int64_t hd = static_cast<int64_t>(a->heads) * d, hkd = static_cast<int64_t>(a->heads_k) * d;
-  // Head dims above 128 run on the kernel that takes query rows 64 at a time (bwd_wide_sm100.cu).
+  // Head dims above 128 run on bwd_wide_pair_sm100.cu or, with query rows 64 at a time, on bwd_wide_sm100.cu.
   const bool wide = d > 128;
   BwdSplit split;
   plan_bwd_split(a, opt.share_key_blocks != 0, rt->sm_count, &split);

@@ -54,8 +54,8 @@ cudaError_t launch_bwd_pair(const BwdParams& p, bool bf16, cudaStream_t stream);
 // 64 rows; p.tm_q and p.tm_do carry boxes of 64 rows, dQ goes through p.dq_acc, dK and dV through p.dk_ptr / p.dv_ptr.
 cudaError_t launch_bwd_wide(const BwdParams& p, int head_dim, bool bf16, cudaStream_t stream);
 
-// Head dims 192 and 256, dense calls that want all three, on pairs of CTAs (bwd_wide_takes_pairs); the maps of Q, K, V and dO are those of make_atom_map, the ones of dK
-// and dV have boxes of 64 rows, p.tm_dqa has boxes of 32 columns and 16 rows.
+// Head dims 192 and 256, dense calls that want all three, on pairs of CTAs (bwd_wide_takes_pairs); the maps of Q, K, V and dO
+// are those of make_atom_map, the ones of dK and dV have boxes of 64 rows, p.tm_dqa has boxes of 32 columns and 16 rows.
 cudaError_t launch_bwd_wide_pair(const BwdParams& p, bool bf16, cudaStream_t stream);
 
 // dQ alone, dense, head_dim a multiple of 8 up to 128: summed in key order, written as 16-bit.
