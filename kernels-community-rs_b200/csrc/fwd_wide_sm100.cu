@@ -3,7 +3,8 @@
 //
 // The O accumulator of one 128-row query block takes up to 256 of the 512 TMEM columns and a 128-key K or V
 // tile would take 64 KB of shared memory, so this kernel is laid out differently from the one for head dims
-// up to 128: one CTA per 128-row query block of one (batch, head), 64-key tiles, one softmax warpgroup.
+// up to 128: one CTA per 128-row query block of one (batch, head), 64-key tiles, one softmax warpgroup, or two where
+// the scores take a soft cap or a bias (the other warps' numbers below are then higher by four).
 //
 //   warps 0-3   softmax + epilogue: one S row per thread out of TMEM (two 64-column S buffers, so Q K^T of the
 //               next key tile runs under this one's softmax), mask, row max, exp2, row sum, P as 16-bit into
@@ -20,6 +21,14 @@
 // P has two buffers: with one, the exponentials of a tile were done and waited for P V of the tile before it. Together with
 // the scale folded into a packed FMA: B2 H16/8 S4096 D192 causal 250 -> 244 us, B4 H16/8 S1000 D256 58.1 -> 57.7.
 //
+// With a soft cap or ALiBi one warpgroup's arithmetic on the scores (a tanh beside each exponential, or six operations of
+// bias) is the longest part of a tile. Two share it, half of a tile's columns each, at the price of telling each other
+// their row maximum through shared memory. Forward call, one warpgroup -> two, us: B2 H16/8 S2048 D256 causal ALiBi
+// 237 -> 174, B4 H16/4 S2048 D192 soft cap 474 -> 404, B2 H16/4 S4096 D256 causal soft cap 482 -> 413, B2 H16/4 S300 D192
+// ALiBi 23.2 -> 18.2, B1 H8/4 S128 D256 soft cap 9.8 -> 9.4. The plain form loses by the exchange, which lengthens its chain
+// of waits by more than half of its exponentials are worth: B4 H16/8 S2048 D256 causal 185 -> 196, 1000 queries against 9000
+// keys 131 -> 143. It keeps one.
+//
 // Conventions as in the kernel for the smaller head dims: bottom-right aligned masks, fully masked rows give
 // O = 0 and LSE = +inf, natural-log LSE, kv_head = head / group; every wait is bounded.
 #include "sm100_ptx.cuh"
@@ -32,12 +41,12 @@ namespace {
 
 constexpr int kWM = 128;        // query rows per CTA
 constexpr int kWN = 64;         // keys per tile
-constexpr int kWThreads = 256;
-constexpr int kWLoadWarp = 4;
-constexpr int kWMmaWarp = 5;
-constexpr int kWFixWarp = 6;
 constexpr int kWSlots = 4;      // K/V ring depth
 constexpr float kWRescaleThreshold = 8.0f;  // log2 domain
+
+// Softmax warpgroups: two share the columns of a tile where the scores take a tanh or a bias each, one does the plain form.
+__host__ __device__ constexpr int wide_groups(bool fancy) { return fancy ? 2 : 1; }
+__host__ __device__ constexpr int wide_threads(bool fancy) { return (wide_groups(fancy) + 1) * 128; }
 
 struct WideCfg {
   static constexpr int kAtomQ = kWM * 128;    // bytes of one 64-column atom of Q (and of P)
@@ -48,9 +57,11 @@ struct WideCfg {
   static constexpr int kKVOff = kMaxAtoms * kAtomQ;
   static constexpr int kPOff = kKVOff + kWSlots * kKVTile;
   static constexpr int kBarOff = kPOff + 2 * kAtomQ;  // two P buffers
-  static constexpr int kNumBars = 3 * kWSlots + 9;
+  static constexpr int kNumBars = 3 * kWSlots + 9 + 8;
   static constexpr int kMiscOff = (kBarOff + kNumBars * 8 + 15) / 16 * 16;
-  static constexpr int kSmemBytes = kMiscOff + 32;
+  static constexpr int kXchgOff = kMiscOff + 32;      // [2][256] floats: what the two threads of a row tell each other
+  static constexpr int kSmemBytes = kXchgOff + 2 * 256 * 4;
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of a CTA");
   static constexpr uint32_t kTmemS = 0, kTmemO = 128;  // S buffers at columns 0 and 64
 };
 
@@ -130,8 +141,11 @@ __device__ __forceinline__ float wide_tanh(float x) {
 // FANCY (softcap or ALiBi in use) and PACKED (cu_seqlens batches) are compile-time: the plain dense kernel carries
 // none of their code, which keeps its loops within reach of the SM's instruction cache.
 template <bool BF16, int ATOMS, bool FANCY, bool PACKED>
-__global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_constant__ FwdParams p) {
+__global__ void __launch_bounds__(wide_threads(FANCY), 1) fwd_wide_kernel(const __grid_constant__ FwdParams p) {
   using Cfg = WideCfg;
+  constexpr int kGroups = wide_groups(FANCY);
+  constexpr int kWC = kWN / kGroups;  // columns of a softmax warpgroup
+  constexpr int kWSoftWarps = 4 * kGroups, kWLoadWarp = kWSoftWarps, kWMmaWarp = kWSoftWarps + 1, kWFixWarp = kWSoftWarps + 2;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
     // 128-byte swizzled tiles need a 1024-byte aligned base; report instead of computing garbage.
@@ -151,6 +165,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   uint64_t* s_free = q_full + 3;   // [2] the scores have been read out of TMEM
   uint64_t* p_full = q_full + 5;   // [2] P of this key tile is in shared memory (and O has been rescaled)
   uint64_t* pv_done = q_full + 7;  // [2] P V of this key tile has completed
+  uint64_t* x_full = q_full + 9;   // [2][4] both warps of 32 rows have written their exchange values
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::kMiscOff + 8);
 
@@ -187,9 +202,10 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
     mbar_init(q_full, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&s_full[s], 1);
-      mbar_init(&s_free[s], kWM);
-      mbar_init(&p_full[s], kWM);
+      mbar_init(&s_free[s], kWSoftWarps);
+      mbar_init(&p_full[s], kWSoftWarps);
       mbar_init(&pv_done[s], 1);
+      for (int w = 0; w < 4; ++w) mbar_init(&x_full[s * 4 + w], 2);
     }
     mbar_fence_init();
   }
@@ -209,13 +225,27 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
   if (!PACKED) early_trigger();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp < 4) {
+  if (warp < kWSoftWarps) {
     // ------------------------------------------------------------------ softmax + epilogue
-    const int row_in = tid;
+    const int half = kGroups > 1 ? warp >> 2 : 0;  // this warpgroup's half of a tile's columns, and of O's (one: all of them)
+    const int row_in = tid & (kWM - 1);
     const int row = ti.m0 + row_in;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
-    const uint32_t t_s = tmem + lane_addr + Cfg::kTmemS;
-    const uint32_t t_o = tmem + lane_addr + Cfg::kTmemO;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t t_s = tmem + lane_addr + Cfg::kTmemS + half * kWC;
+    const uint32_t t_o = tmem + lane_addr + Cfg::kTmemO + half * (n_cols / kGroups);
+    float* s_xchg = reinterpret_cast<float*>(smem + Cfg::kXchgOff);
+    // Gives x to the thread that has the other half of this row, and takes its value. The buffer of step i is written again
+    // in step i + 2, when the other warp has arrived for step i + 1 and so has read step i.
+    auto exchange = [&](int i, float x, float& other) -> bool {
+      float* slot = s_xchg + (i & 1) * 256;
+      slot[tid] = x;
+      __syncwarp();
+      uint64_t* bar = &x_full[(i & 1) * 4 + (warp & 3)];
+      if (lane == 0) mbar_arrive(bar);
+      if (!warp_wait(bar, (i >> 1) & 1, ctl, kWaitSoftmaxSFull)) return false;
+      other = slot[tid ^ kWM];
+      return true;
+    };
     // P as the K-major, 128-byte swizzled A operand of P V: key chunk c (8 keys, 16 bytes) of row r sits at
     // byte 128 r + 16 (c ^ (r % 8)) of the single atom.
     uint8_t* p_row = s_p + row_in * 128;
@@ -232,18 +262,19 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
       const int buf = i & 1;
       if (!warp_wait(&s_full[buf], (i >> 1) & 1, ctl, kWaitSoftmaxSFull)) { ok = false; break; }
       tc_fence_after();
-      uint32_t sr[kWN];
+      uint32_t sr[kWC];
       tmem_ld32(t_s + buf * kWN, sr);
-      tmem_ld32(t_s + buf * kWN + 32, sr + 32);
+      if constexpr (kGroups == 1) tmem_ld32(t_s + buf * kWN + 32, sr + 32);
       tmem_wait_ld();
       tc_fence_before();
-      mbar_arrive(&s_free[buf]);  // the scores live in registers from here on
-      const int col0 = j * kWN;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_free[buf]);  // the scores live in registers from here on
+      const int col0 = j * kWN + half * kWC;
       // The general form leaves the scores in the log2 domain (softcap, ALiBi, a scale that is not positive); otherwise
       // the scale is folded into the exponent.
       if (fancy) {
 #pragma unroll
-        for (int c = 0; c < kWN; ++c) {
+        for (int c = 0; c < kWC; ++c) {
           float x = __uint_as_float(sr[c]);
           x = (p.softcap > 0.f) ? cap_l2 * wide_tanh(x * inv_cap) : x * p.scale_log2;
           if (p.alibi != nullptr) {
@@ -261,18 +292,23 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
         if (p.window_left >= 0) lo = row + ti.off - p.window_left;
         hi -= col0;
         lo -= col0;
-        if (lo > 0 || hi < kWN) fill_outside<kWN>(sr, lo, hi, 0xff800000u);  // -inf
+        if (lo > 0 || hi < kWC) fill_outside<kWC>(sr, lo, hi, 0xff800000u);  // -inf
       }
       float mx[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) mx[c] = __uint_as_float(sr[c]);
 #pragma unroll
-      for (int c = 4; c < kWN - 4; c += 8)
+      for (int c = 4; c < kWC - 4; c += 8)
 #pragma unroll
         for (int q = 0; q < 4; ++q) mx[q] = max3(mx[q], __uint_as_float(sr[c + 2 * q]), __uint_as_float(sr[c + 2 * q + 1]));
-      mx[0] = max3(mx[0], __uint_as_float(sr[kWN - 4]), __uint_as_float(sr[kWN - 3]));
-      mx[1] = max3(mx[1], __uint_as_float(sr[kWN - 2]), __uint_as_float(sr[kWN - 1]));
-      const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * mul);
+      mx[0] = max3(mx[0], __uint_as_float(sr[kWC - 4]), __uint_as_float(sr[kWC - 3]));
+      mx[1] = max3(mx[1], __uint_as_float(sr[kWC - 2]), __uint_as_float(sr[kWC - 1]));
+      const float own = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      float other = own;
+      if constexpr (kGroups > 1) {
+        if (!exchange(i, own, other)) { ok = false; break; }
+      }
+      const float m_new = fmaxf(m, fmaxf(own, other) * mul);
       // Keep the stale max unless it grew by more than 2^8: the final O / l is exact either way.
       const bool grow = (m_new - m) > kWRescaleThreshold;
       float alpha = 1.f;
@@ -286,7 +322,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
       const uint64_t c2 = pack_f32x2(mul, mul), nm2 = pack_f32x2(neg_m, neg_m);
       uint64_t acc0 = pack_f32x2(0.f, 0.f), acc1 = acc0;
 #pragma unroll
-      for (int c = 0; c < kWN; c += 4) {
+      for (int c = 0; c < kWC; c += 4) {
         float x[4];
         unpack_f32x2(fma2(pack_f32x2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), c2, nm2), x[0], x[1]);
         unpack_f32x2(fma2(pack_f32x2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), c2, nm2), x[2], x[3]);
@@ -311,7 +347,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
         // P V of the previous key tile, the only operation that touches O, has to be complete.
         if (!warp_wait(&pv_done[buf ^ 1], ((i - 1) >> 1) & 1, ctl, kWaitSoftmaxPvDone)) { ok = false; break; }
         tc_fence_after();
-        for (int c = 0; c < n_cols / 16; ++c) {
+        for (int c = 0; c < n_cols / (16 * kGroups); ++c) {
           uint32_t orr[16];
           tmem_ld16(t_o + c * 16, orr);
           tmem_wait_ld();
@@ -325,10 +361,16 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
       }
       uint8_t* p_buf = p_row + buf * Cfg::kAtomQ;
 #pragma unroll
-      for (int c = 0; c < kWN / 8; ++c)
-        *reinterpret_cast<uint4*>(p_buf + ((c ^ p_swz) << 4)) = make_uint4(sr[4 * c], sr[4 * c + 1], sr[4 * c + 2], sr[4 * c + 3]);
+      for (int c = 0; c < kWC / 8; ++c)
+        *reinterpret_cast<uint4*>(p_buf + (((half * (kWC / 8) + c) ^ p_swz) << 4)) = make_uint4(sr[4 * c], sr[4 * c + 1], sr[4 * c + 2], sr[4 * c + 3]);
       fence_proxy_async_smem();
-      mbar_arrive(&p_full[buf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[buf]);
+    }
+    if constexpr (kGroups > 1) {
+      float l_other = 0.f;
+      if (ok) ok = exchange(n_tiles, l, l_other);
+      l += l_other;
     }
     if (ok && warp_wait(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, ctl, kWaitEpiPvDone)) {
       // ---- epilogue: O / l -> 16-bit -> global memory, 32 columns at a time; LSE = (m + log2 l) ln 2
@@ -336,7 +378,7 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
       const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
       uint16_t* orow = reinterpret_cast<uint16_t*>(p.o_ptr) + ti.bq * p.o_batch_stride +
                        static_cast<int64_t>(ti.q_row0 + row) * p.o_row_stride + ti.h * p.o_head_stride;
-      for (int c = 0; c < n_cols / 32; ++c) {
+      for (int c = 0; c < n_cols / (32 * kGroups); ++c) {
         uint32_t orr[32];
         tmem_ld32(t_o + c * 32, orr);
         tmem_wait_ld();
@@ -347,12 +389,12 @@ __global__ void __launch_bounds__(kWThreads, 1) fwd_wide_kernel(const __grid_con
           w.y = pack2<BF16>(__uint_as_float(orr[8 * q + 2]) * inv_l, __uint_as_float(orr[8 * q + 3]) * inv_l);
           w.z = pack2<BF16>(__uint_as_float(orr[8 * q + 4]) * inv_l, __uint_as_float(orr[8 * q + 5]) * inv_l);
           w.w = pack2<BF16>(__uint_as_float(orr[8 * q + 6]) * inv_l, __uint_as_float(orr[8 * q + 7]) * inv_l);
-          const int col = c * 32 + q * 8;
+          const int col = half * (n_cols / kGroups) + c * 32 + q * 8;
           if (row < ti.sq && col < p.head_dim) *reinterpret_cast<uint4*>(orow + col) = w;
         }
       }
       tc_fence_before();
-      if (row < ti.sq) {
+      if (half == 0 && row < ti.sq) {
         const float lse = (l > 0.f) ? (m + lg2(l)) * 0.6931471805599453f : INFINITY;
         p.lse_ptr[ti.bq * p.lse_batch_stride + ti.h * p.lse_head_stride + ti.q_row0 + row] = lse;
       }
@@ -529,7 +571,7 @@ cudaError_t launch_wide(const FwdParams& p, cudaStream_t stream) {
   const int64_t blocks = static_cast<int64_t>((p.seqlen_q + kWM - 1) / kWM) * p.batch * p.heads;
   if (blocks <= 0) return cudaSuccess;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  return launch_grid(!PACKED, fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), kWThreads,
+  return launch_grid(!PACKED, fwd_wide_kernel<BF16, ATOMS, FANCY, PACKED>, dim3(static_cast<unsigned>(blocks)), wide_threads(FANCY),
                               WideCfg::kSmemBytes, stream, p);
 }
 
