@@ -337,7 +337,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
         });
         mma_pair_commit(dq_full);
       }
-      mma_pair_commit(dk_done);
+      // Only for who waits: an arrival that nobody waits for could land in the other CTA after its end.
+      if (ok && n_iter > 0) mma_pair_commit(dk_done);
     } else if (warp == 2 && rank == 1 && elect_one()) {
       // ---------------------------------------------------------------- tells the issuer what this CTA has received
       bool ok = true;

@@ -8,10 +8,12 @@ pytestmark = pytest.mark.gpu
 
 # (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim, causal, window): calls that run on pairs (test_plans_cpu.py states that they
 # do). Whole tiles; a last pair of one block, of one key block and a bit, with nothing for its second CTA; bottom-right masks with more
-# keys than queries and with rows that see no key; windows; grouped heads; head dims below the kernel's.
+# keys than queries and with rows that see no key; windows; grouped heads; head dims below the kernel's; pairs whose keys no query sees
+# (EMPTY).
 CASES = [(1, 28, 28, 2048, 2048, 128, False, (-1, -1)), (4, 32, 8, 2000, 1000, 128, False, (-1, -1)), (8, 16, 8, 2048, 300, 120, False, (-1, -1)),
          (8, 16, 8, 1921, 257, 104, False, (-1, -1)), (2, 16, 8, 4200, 4200, 128, True, (-1, -1)), (2, 8, 8, 4100, 5000, 128, True, (-1, -1)),
-         (2, 8, 8, 5000, 4100, 112, True, (-1, -1)), (2, 8, 4, 5000, 5000, 128, False, (3000, 500))]
+         (2, 8, 8, 5000, 4100, 112, True, (-1, -1)), (2, 8, 4, 5000, 5000, 128, False, (3000, 500)),
+         (1, 8, 8, 4100, 4900, 128, False, (500, -1))]
 
 
 # Head dims 192 and 256: one query, one key block and a bit, a last pair with keys for one CTA only or too few for its first; masks as
@@ -20,7 +22,10 @@ WIDE = [(1, 2, 2, 128, 128, 256, False, (-1, -1)), (2, 4, 2, 1, 300, 256, False,
         (2, 4, 2, 577, 385, 256, False, (-1, -1)), (2, 8, 2, 777, 777, 256, True, (-1, -1)), (2, 4, 4, 300, 1021, 256, True, (-1, -1)),
         (2, 4, 4, 700, 200, 256, True, (-1, -1)), (2, 4, 4, 1000, 1100, 256, False, (100, 50)), (1, 4, 4, 1024, 1024, 256, True, (127, 0)),
         (1, 2, 2, 128, 128, 192, False, (-1, -1)), (3, 4, 4, 200, 65, 192, False, (-1, -1)), (2, 8, 2, 777, 777, 192, True, (-1, -1)),
-        (2, 4, 4, 333, 1021, 192, True, (-1, -1)), (2, 4, 4, 1000, 1100, 192, False, (100, 50))]
+        (2, 4, 4, 333, 1021, 192, True, (-1, -1)), (2, 4, 4, 1000, 1100, 192, False, (100, 50)),
+        (2, 4, 2, 128, 2000, 256, True, (127, 0)), (2, 4, 4, 200, 1021, 192, False, (100, 50))]
+# The cases with pairs that walk no query block: their dK and dV are zeros, and no MMA is issued.
+EMPTY = [c for c in CASES + WIDE if c[7][0] >= 0 and c[4] > c[3] + c[7][0]]
 
 
 def _check(args, causal, window, dtype, **opt):

@@ -4,6 +4,7 @@ import subprocess
 from pathlib import Path
 
 import pytest
+import torch
 
 ROOT = Path(__file__).resolve().parent.parent
 SMS = 148
@@ -187,10 +188,24 @@ def _takes_pairs(plans, case, **kw):
     return bool(plans.takes_pairs(ctypes.byref(a), SMS))
 
 
+def _empty_pairs(case):
+    """Pairs of a head (256 keys, 128 at head dims above 128) none of whose keys a query sees, from the mask itself."""
+    _, _, _, sq, sk, d, causal, (left, right) = case
+    right = 0 if causal else right
+    i, j = torch.arange(sq)[:, None] + (sk - sq), torch.arange(sk)[None, :]
+    seen = torch.ones(sq, sk, dtype=torch.bool)
+    if right >= 0:
+        seen &= j <= i + right
+    if left >= 0:
+        seen &= j >= i - left
+    return sum(not keys.any() for keys in seen.any(0).split(256 if d <= 128 else 128))
+
+
 def test_backward_calls_that_run_on_pairs(plans):
-    from tests.test_bwd_pair_gpu import CASES, WIDE
+    from tests.test_bwd_pair_gpu import CASES, EMPTY, WIDE
 
     assert all(_takes_pairs(plans, c) for c in CASES + WIDE)
+    assert {c[5] for c in EMPTY} == {128, 192, 256} and all((_empty_pairs(c) > 0) == (c in EMPTY) for c in CASES + WIDE)
     assert not any(_takes_pairs(plans, WIDE[0], **other) for other in (dict(which=1), dict(which=2), dict(head_dim=248), dict(head_dim=184),
                                                                dict(cu_seqlens_q=256), dict(head_dim=192, seqlen_q=300)))
     full = (4, 16, 16, 2048, 2048, 128, False, (-1, -1))
