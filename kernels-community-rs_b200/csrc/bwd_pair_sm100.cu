@@ -550,7 +550,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
   tc_fence_before();
   __syncthreads();
   if (tid == 0) report_abort(abort_flag, p.status);
-  // A CTA stays until the other one has read its operands and sent it everything.
+  // A CTA stays until the other one has read its operands and sent it everything. The barrier takes converged warps.
+  __syncwarp();
   cluster_arrive();
   cluster_wait();
   if (warp == 1) tmem_dealloc_pair(tmem, 512);
