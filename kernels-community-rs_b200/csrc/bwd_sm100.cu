@@ -979,8 +979,11 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_kernel(const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0) report_abort(abort_flag, p.status);
-  if (warp == 1) tmem_dealloc(tmem, 512);
+  if (warp == 1) {  // its index lives to the end anyway; the thread's (tid == 0) was spilled for it
+    if (elect_one()) report_abort(abort_flag, p.status);
+    __syncwarp();
+    tmem_dealloc(tmem, 512);
+  }
 }
 
 template <int D, bool BF16, int MODE, bool PACKED, bool TAKE_OVER>

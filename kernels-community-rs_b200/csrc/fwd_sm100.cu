@@ -908,8 +908,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
-  if (tid == 0) report_abort(abort_flag, p.status);
-  if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
+  if (warp == kMmaWarp) {  // its index lives to the end anyway; the thread's (tid == 0) was spilled for it
+    if (elect_one()) report_abort(abort_flag, p.status);
+    __syncwarp();
+    tmem_dealloc(tmem, 512);
+  }
 }
 
 // The parts of shared tiles become rows of the output: D / 4 lanes per row, 4 columns a lane, kMergeSteps rows per lane
