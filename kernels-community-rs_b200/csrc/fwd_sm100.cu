@@ -254,6 +254,17 @@ __device__ __forceinline__ float tanh_approx(float x) {
   return y;
 }
 
+// Is the rescaling of O a loop in the machine code? Its code is read by few key blocks, which is worth 1 % where the row maximum
+// soon stops growing; with ALiBi it grows along the keys, and on shared tiles the loop costs registers. Forward, rolled -> unrolled, us:
+// ALiBi B1 H8 S16384 causal D128 677 -> 644, D64 H16 1088 -> 1011, B4 H16/4 S2048 98.0 -> 95.2; soft cap D64 H16 S16384 1239 -> 1222;
+// shared tiles H20 Sq 512 Sk 4096 D64 33.3 -> 32.6, soft cap D128 52.6 -> 51.7, soft cap and ALiBi D64 121 -> 87. The other way: soft cap D128
+// B4 H16/4 S2048 102.9 -> 104.2, on shared tiles with ALiBi 114.8 -> 116.3; plain D64 B8 H16 S2048 and D128 B16 H16 S2048 within 0.2 %.
+__host__ __device__ constexpr bool rescale_rolled(int d, int mode, bool packed, bool shared) {
+  if (packed) return false;
+  if (shared) return mode == kScoreAny && d > 64;
+  return mode == kScorePlain || (mode == kScoreSoftcap && d > 64);
+}
+
 // MODE: what is done to the scores; PACKED: cu_seqlens batches. Both are compile-time so that the
 // plain dense kernel carries none of their code and stays within reach of the SM's instruction cache: without the
 // score transforms the kernel is a third smaller and ran 3-4 % faster.
@@ -518,7 +529,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         if (votes & 2u) { ok = false; break; }
         if (j > nb_s && (votes & 1u)) {
           tc_fence_after();
-#pragma unroll 1
+#pragma unroll(rescale_rolled(D, MODE, PACKED, SHARED) ? 1 : D / 16)
           for (int c = 0; c < D / 16; ++c) {
             uint32_t orr[16];
             tmem_ld16(t_o + c * 16, orr);
