@@ -304,6 +304,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
+  // In the plain form at head dim 128 the softmax warps' and the issuers' waits inside the walk are the longer ones. With none of them,
+  // with these, with all: B1 H16 S16384 causal 1032, 1003, 998 us, B2 H32/8 S8192 window 1023 305.5, 300.7, 301.0, B8 H16 S1000 85.6, 84.4, 84.1,
+  // B8 H16 S300 causal 15.3, 15.4, 15.8, B32 H16 S128 14.5, 14.7, 14.7. Head dim 64 and score transforms are up to 1.5 % faster with none.
+  using LoopCtl = std::conditional_t<D == 128 && MODE == kScorePlain && !PACKED && !SHARED, SeldomWaitCtl, WaitCtl>;
+  const LoopCtl loop_ctl{abort_flag};
   const WaitCtl ctl{abort_flag};
   volatile ListDiv* ld = reinterpret_cast<volatile ListDiv*>(smem + Cfg::kMiscOff + 16);
   // Every role walks this CTA's positions of the work list.
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
       if ((MODE == kScoreAlibi || MODE == kScoreAny) && p.alibi != nullptr) slope = p.alibi[ti.b * p.alibi_batch_stride + ti.h] * 1.4426950408889634f;
       bool ok = true;
       for (int j = nb_s; j < ne_s; ++j) {
-        if (!warp_wait(&s_full[s], n_sfull & 1, ctl, kWaitSoftmaxSFull)) { ok = false; break; }
+        if (!warp_wait(&s_full[s], n_sfull & 1, loop_ctl, kWaitSoftmaxSFull)) { ok = false; break; }
         ++n_sfull;
         tc_fence_after();
         uint32_t sr[kBlockN];
@@ -511,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         if (j > nb_s) {
           // P V(j-1) has to be complete: it reads the P buffer that this iteration overwrites, and it is the
           // only operation that touches O of this stage.
-          waited = mbar_wait(&pv_done[s], (n_pv - 1) & 1, ctl, kWaitSoftmaxPvDone);
+          waited = mbar_wait(&pv_done[s], (n_pv - 1) & 1, loop_ctl, kWaitSoftmaxPvDone);
         } else {
           // First iteration of a tile: the TMA store of the previous tile must have read the buffer.
           if (row_in == 0) {
@@ -773,7 +778,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         uint32_t slot = 0, ring_phase = 0;
         bool ok = true;
         auto fix_tile = [&](int first_stray) -> bool {
-          if (!__all_sync(0xffffffffu, mbar_wait(&kv_full[slot], ring_phase, ctl, kWaitMmaKVFull))) return false;
+          if (!__all_sync(0xffffffffu, mbar_wait(&kv_full[slot], ring_phase, loop_ctl, kWaitMmaKVFull))) return false;
           if (first_stray < kBlockN) {
             uint8_t* tile = s_kv + slot * Cfg::kTileBytes;
             // 8 lanes clear one 128-byte row of an atom (the swizzle only permutes 16-byte chunks inside it)
@@ -847,14 +852,14 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         // S_s = Q_s K_j^T over D in steps of 16 (32 bytes inside the 128-byte swizzle atom). The S region
         // is free as soon as the softmax warps hold the previous scores in registers.
         auto do_k = [&](const int j) -> bool {
-          if (!mbar_wait(&kv_full[slot], ring_phase, ctl, kWaitMmaKVFull)) return false;
+          if (!mbar_wait(&kv_full[slot], ring_phase, loop_ctl, kWaitMmaKVFull)) return false;
           if (j >= nb && j < ne) {
             if (!q_ready) {
-              if (!mbar_wait(&q_full[s], n_q & 1, ctl, kWaitMmaQFull)) return false;
+              if (!mbar_wait(&q_full[s], n_q & 1, loop_ctl, kWaitMmaQFull)) return false;
               ++n_q;
               q_ready = true;
             }
-            if (!mbar_wait(&s_free[s], (n_qk & 1) ^ 1, ctl, kWaitMmaSFree)) return false;
+            if (!mbar_wait(&s_free[s], (n_qk & 1) ^ 1, loop_ctl, kWaitMmaSFree)) return false;
             ++n_qk;
             tc_fence_after();
             const uint64_t b = k_desc + slot * kTile16;
@@ -873,10 +878,10 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
         // O_s (+)= P_s V_j, one piece of kBlockN / kPQ keys at a time (per step of 16 keys: 32 bytes of a
         // P row inside its swizzle atom, 16 rows of 128 bytes of V).
         auto do_v = [&](const int j) -> bool {
-          if (!mbar_wait(&kv_full[slot], ring_phase, ctl, kWaitMmaKVFull)) return false;
+          if (!mbar_wait(&kv_full[slot], ring_phase, loop_ctl, kWaitMmaKVFull)) return false;
           if (ragged_row<PACKED>(ti.sk, j) < kBlockN) {
             // A V tile that reaches past its sequence is usable once the fixer has cleared the stray rows.
-            if (!mbar_wait(&kv_fixed[slot], (fix_par >> slot) & 1, ctl, kWaitMmaKVFull)) return false;
+            if (!mbar_wait(&kv_fixed[slot], (fix_par >> slot) & 1, loop_ctl, kWaitMmaKVFull)) return false;
             fix_par ^= 1u << slot;
           }
           if (j >= nb && j < ne) {
@@ -885,8 +890,8 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_kernel(const __grid_constant_
             constexpr int kStepsPerPiece = kBlockN / 16 / kPQ;
 #pragma unroll
             for (int q = 0; q < kPQ; ++q) {
-              if (!mbar_wait(&p_full[s * kPQ + q], n_p & 1, ctl, kWaitMmaPFull)) return false;
-              if (q == 0 && first && !mbar_wait(&o_free[s], (n_tile & 1) ^ 1, ctl, kWaitMmaOFree)) return false;
+              if (!mbar_wait(&p_full[s * kPQ + q], n_p & 1, loop_ctl, kWaitMmaPFull)) return false;
+              if (q == 0 && first && !mbar_wait(&o_free[s], (n_tile & 1) ^ 1, loop_ctl, kWaitMmaOFree)) return false;
               tc_fence_after();
 #pragma unroll
               for (int ks = q * kStepsPerPiece; ks < (q + 1) * kStepsPerPiece; ++ks) {

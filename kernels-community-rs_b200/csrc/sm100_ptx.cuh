@@ -86,6 +86,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   *ctl.abort_flag = code;
   return false;
 }
+// The longer form, which reads the clock at every eighth try: for a kernel that names this type (the plain forward at head dim 128).
+struct SeldomWaitCtl : WaitCtl {};
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const SeldomWaitCtl& ctl, int code) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  for (uint32_t it = 1;; ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*ctl.abort_flag) return false;
+    if ((it & 7u) == 0u && clock64() - t0 > FA2_WAIT_LIMIT_CYCLES) break;
+  }
+  if (!*ctl.abort_flag) *ctl.abort_flag = code;
+  return false;
+}
 
 // The same wait for short hand-offs between the warps of one role: it probes the phase without letting the
 // hardware park the thread (a parked thread was seen to come back thousands of cycles after the phase
@@ -117,7 +130,8 @@ __device__ __forceinline__ void report_abort(const volatile int* abort_flag, int
 // Wait of a whole warp. The vote brings the 32 lanes back together (they leave the polling loop in
 // different iterations) and makes the outcome warp-uniform, so that the .sync.aligned tcgen05
 // instructions that follow are executed by the converged warp.
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code) {
+template <class Ctl>
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const Ctl& ctl, int code) {
   const bool ok = mbar_wait(bar, parity, ctl, code);
   return __all_sync(0xffffffffu, ok);
 }
