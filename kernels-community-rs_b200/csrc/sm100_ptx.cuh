@@ -57,8 +57,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Abort state of one CTA, a word of shared memory: the site code of a wait that ran out, or 0. report_abort hands it on when the
-// kernel ends.
+// Abort state of one CTA, a word of shared memory: 0, or the site code of the first wait that ran out (a wait stores its code a few
+// instructions after it has found the word clear; of two that run out within those, the later one's stays). report_abort hands it on
+// when the kernel ends.
 struct WaitCtl {
   volatile int* abort_flag;
 };
@@ -67,6 +68,7 @@ struct WaitCtl {
 #ifndef FA2_WAIT_LIMIT_CYCLES
 #define FA2_WAIT_LIMIT_CYCLES (1ll << 31)
 #endif
+static_assert(FA2_WAIT_LIMIT_CYCLES > 0 && FA2_WAIT_LIMIT_CYCLES < (1ll << 32), "waits compare 32 bits of the clock");
 
 __device__ __forceinline__ uint32_t clock32() {
   uint32_t c;
@@ -121,7 +123,8 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, c
   return false;
 }
 
-// After the CTA's last barrier, by one thread: the first site code goes to the status word (global memory, may be null).
+// After the CTA's last barrier, by one thread: the site code goes to the status word (global memory, may be null), which keeps the
+// first CTA's.
 __device__ __forceinline__ void report_abort(const volatile int* abort_flag, int* status) {
   const int code = *abort_flag;
   if (code != 0 && status != nullptr) atomicCAS(status, 0, code);

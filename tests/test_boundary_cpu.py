@@ -38,6 +38,18 @@ def test_cabi_struct_layout_matches_header(built_libs):
     assert sizes == [ctypes.sizeof(_cabi.FwdArgs), ctypes.sizeof(_cabi.BwdPreprocessArgs), ctypes.sizeof(_cabi.BwdArgs)]
 
 
+@pytest.mark.parametrize("limit,ok", [("(1ll << 31)", True), ("(1ll << 32)", False), ("(3ll << 32)", False), ("0", False)])
+def test_wait_limits_that_32_bits_cannot_hold_do_not_build(limit, ok, tmp_path):
+    """The waits compare 32 bits of the clock: 2^32 cycles would be a limit of none."""
+    import subprocess
+
+    (tmp_path / "w.cu").write_text('#include "sm100_ptx.cuh"\n')
+    run = subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", f"-DFA2_WAIT_LIMIT_CYCLES={limit}",
+                          f"-I{ROOT / 'kernels-community-rs_b200' / 'csrc'}", "-c", str(tmp_path / "w.cu"), "-o", str(tmp_path / "w.o")],
+                         capture_output=True, text=True)
+    assert (run.returncode == 0) == ok and ("32 bits of the clock" in run.stderr) != ok, run.stderr
+
+
 def test_tvm_ffi_library_exports_reference_operator_names(built_libs):
     from flash_attn2_b200 import _ops
 
