@@ -601,22 +601,14 @@ int bwd_impl(const fa2_bwd_args* a, const fa2_bwd_options& opt, void* stream_v) 
   const Windows w = normalise_windows(a->window_left, a->window_right, a->causal != 0, a->seqlen_k, packed);
   const bool pairs = wide ? bwd_wide_takes_pairs(a) : !is_split && bwd_takes_pairs(a, w, rt->sm_count);
   const int q_box_rows = wide || pairs ? 64 : 128, k_box_rows = wide && pairs ? 64 : 128;
-  if ((rc = make_map(&p.tm_q, a->q, a->dtype, 2, d, a->heads, rows_q, nbatch, a->q_stride[2], a->q_stride[1],
-                     a->q_stride[0], 64, q_box_rows, "q")) != FA2_OK) return rc;
-  if ((rc = make_map(&p.tm_do, a->dout, a->dtype, 2, d, a->heads, rows_q, nbatch, a->do_stride[2], a->do_stride[1],
-                     a->do_stride[0], 64, q_box_rows, "dout")) != FA2_OK) return rc;
-  if ((rc = make_map(&p.tm_k, a->k, a->dtype, 2, d, a->heads_k, rows_k, nbatch, a->k_stride[2], a->k_stride[1],
-                     a->k_stride[0], 64, k_box_rows, "k")) != FA2_OK) return rc;
-  if ((rc = make_map(&p.tm_v, a->v, a->dtype, 2, d, a->heads_k, rows_k, nbatch, a->v_stride[2], a->v_stride[1],
-                     a->v_stride[0], 64, k_box_rows, "v")) != FA2_OK) return rc;
-  if (wide && pairs) {
-    const struct { CUtensorMap* map; const void* ptr; int64_t heads, rows; const int64_t* stride; const char* name; } in[4] = {
-        {&p.tm_q, a->q, a->heads, rows_q, a->q_stride, "q"}, {&p.tm_do, a->dout, a->heads, rows_q, a->do_stride, "dout"},
-        {&p.tm_k, a->k, a->heads_k, rows_k, a->k_stride, "k"}, {&p.tm_v, a->v, a->heads_k, rows_k, a->v_stride, "v"}};
-    for (const auto& t : in)
-      if ((rc = make_atom_map(t.map, t.ptr, a->dtype, d, t.heads, t.rows, nbatch, t.stride[2], t.stride[1], t.stride[0], t.name)) != FA2_OK)
-        return rc;
-  }
+  auto input_map = [&](CUtensorMap* m, const void* ptr, int64_t heads, int64_t rows, const int64_t* stride, int box_rows, const char* name) {
+    return wide && pairs ? make_atom_map(m, ptr, a->dtype, d, heads, rows, nbatch, stride[2], stride[1], stride[0], name)
+                         : make_map(m, ptr, a->dtype, 2, d, heads, rows, nbatch, stride[2], stride[1], stride[0], 64, box_rows, name);
+  };
+  if ((rc = input_map(&p.tm_q, a->q, a->heads, rows_q, a->q_stride, q_box_rows, "q")) != FA2_OK) return rc;
+  if ((rc = input_map(&p.tm_do, a->dout, a->heads, rows_q, a->do_stride, q_box_rows, "dout")) != FA2_OK) return rc;
+  if ((rc = input_map(&p.tm_k, a->k, a->heads_k, rows_k, a->k_stride, 128, "k")) != FA2_OK) return rc;
+  if ((rc = input_map(&p.tm_v, a->v, a->heads_k, rows_k, a->v_stride, 128, "v")) != FA2_OK) return rc;
   if (want_dkv) {
     if ((rc = make_map(&p.tm_dk, a->dk, a->dtype, 2, d, a->heads_k, rows_k, nbatch, d, hkd, rows_k * hkd, 64, k_box_rows,
                        "dk")) != FA2_OK) return rc;
