@@ -253,11 +253,16 @@ inline bool bwd_takes_pairs(const fa2_bwd_args* a, const Windows& w, int sm_coun
 // Head dims 192 and 256 (bwd_wide_pair_sm100.cu, which has more figures). Its query blocks have 128 rows, those of the other kernel 64,
 // and at head dim 192 a quarter of what it does for dK, dV and dQ is padding: calls that pad their rows by a fifth more than in blocks
 // of 64 stay there. Without the line, before and after, us: D192 B16 H8 S300 142, 145, B16 H16/4 S300 causal 176, 183, B16 H8 S320 causal
-// 125, 129; on this side B16 H8 S450 233, 214, B32 H8 S128 89, 82. D256 B32 H8 S180 165, 164, B4 H16 Sq 64 Sk 2000 199, 194.
+// 125, 129; on this side B16 H8 S450 233, 214, B32 H8 S128 89, 82, B12 H16 S430 causal 259, 262. At head dim 256 such calls stay there if a third of
+// their keys is padding too (the second CTA of a pair then has few of them): D256 B128 H16 S32 334, 408, B64 H16 S60 208, 238, B32 H16 S130
+// 271, 286, B30 H32 S155 causal 488, 506; on this side B30 H16 S190 311, 300, causal 282, 284, B16 H16 S260 288, 275, causal 241, 242, B64 H16
+// S100 293, 282, B4 H16 Sq 64 Sk 2000 199, 194, B16 H32/4 S320 causal 385, 390.
 inline bool bwd_wide_takes_pairs(const fa2_bwd_args* a) {
   if (a->cu_seqlens_q != nullptr || (a->which & 3) != 3) return false;
-  const int64_t rows128 = (static_cast<int64_t>(a->seqlen_q) + 127) / 128 * 128, rows64 = (static_cast<int64_t>(a->seqlen_q) + 63) / 64 * 64;
-  return a->head_dim == 256 || (a->head_dim == 192 && 5 * rows128 < 6 * rows64);
+  auto padded = [](int64_t rows, int64_t block) { return (rows + block - 1) / block * block; };
+  const bool few_padded_rows = 5 * padded(a->seqlen_q, 128) < 6 * padded(a->seqlen_q, 64);
+  const bool few_padded_keys = 3 * static_cast<int64_t>(a->seqlen_k) >= 2 * padded(a->seqlen_k, 128);
+  return (a->head_dim == 192 && few_padded_rows) || (a->head_dim == 256 && (few_padded_rows || few_padded_keys));
 }
 
 // ---- key blocks shared by several CTAs (bwd_sm100.cu: part_start). A CTA owns 128 keys of one kv head and walks the

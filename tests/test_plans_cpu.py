@@ -208,6 +208,10 @@ def test_backward_calls_that_run_on_pairs(plans):
     assert {c[5] for c in EMPTY} == {128, 192, 256} and all((_empty_pairs(c) > 0) == (c in EMPTY) for c in CASES + WIDE)
     assert not any(_takes_pairs(plans, WIDE[0], **other) for other in (dict(which=1), dict(which=2), dict(head_dim=248), dict(head_dim=184),
                                                                dict(cu_seqlens_q=256), dict(head_dim=192, seqlen_q=300)))
+    # Head dim 256: rows padded by a fifth more than in blocks of 64, and a third of the keys' blocks empty.
+    for rows, keys, taken in ((60, 60, False), (64, 170, False), (130, 130, False), (170, 170, False), (171, 171, True), (192, 85, False), (192, 86, True),
+                              (65, 65, True), (193, 60, True), (320, 60, False), (60, 2000, True)):
+        assert _takes_pairs(plans, WIDE[0], seqlen_q=rows, seqlen_k=keys) == taken, (rows, keys)
     full = (4, 16, 16, 2048, 2048, 128, False, (-1, -1))
     assert _takes_pairs(plans, full)
     for other in (dict(which=1), dict(which=2), dict(head_dim=96), dict(head_dim=136), dict(softcap=30.0), dict(alibi_slopes=256),
