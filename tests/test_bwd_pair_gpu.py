@@ -85,3 +85,73 @@ def test_wide_pairs_on_views_of_one_projection():
     qkv = torch.randn(2, 300, 3, 4, 256, generator=gen).to(torch.bfloat16).cuda()
     do = torch.randn(2, 300, 4, 256, generator=gen).to(torch.bfloat16).cuda()
     _check([*qkv.unbind(2), do], True, (-1, -1), torch.bfloat16)
+
+
+# One call on each kernel, many pairs of unequal walks.
+REPEATED = [(1, 28, 28, 2048, 2048, 128, False, (-1, -1)), (2, 16, 16, 4200, 4200, 128, True, (-1, -1)), (4, 8, 4, 777, 777, 192, True, (-1, -1)),
+            (4, 8, 4, 777, 777, 256, True, (-1, -1))]
+
+
+@pytest.mark.parametrize("case", REPEATED, ids=lambda c: "x".join(str(i) for i in c[:6]))
+def test_pairs_give_the_same_bits_every_time(case):
+    """What one CTA tells the other by an arrival alone is there when it is read: three inputs in turn, so that what an earlier call left
+    in shared or tensor memory is not what belongs there, several hundred times without a pause."""
+    from flash_attn2_b200 import cabi_ops as ops
+
+    b, h, hk, sq, sk, d, causal, _ = case
+    calls, want = [], []
+    for seed in (31, 32, 33):
+        q, k, v, do = [t.cuda() for t in make_qkv(seed, b, h, hk, sq, sk, d, torch.bfloat16, with_do=True)]
+        out, lse = ops.fwd(q, k, v, causal=causal)
+        calls.append((q, k, v, do, lse, ops.bwd_preprocess(do, out)))
+        want.append(ops.bwd(*calls[-1], causal=causal, which=2)[1:])
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    for i in range(300):
+        for g, w in zip(ops.bwd(*calls[i % 3], causal=causal)[1:], want[i % 3]):
+            wrong += (g != w).any()
+    assert wrong.item() == 0
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("case", [(8, 16, 16, 2048, 250, 128), (2, 4, 4, 400, 380, 192), (2, 4, 4, 300, 200, 256)], ids=lambda c: "x".join(map(str, c)))
+def test_pairs_take_any_layout(case):
+    """Transposed, padded, strided and expanded tensors against copies of them."""
+    from flash_attn2_b200 import cabi_ops as ops
+
+    b, h, hk, sq, sk, d = case
+    gen = torch.Generator(device="cuda").manual_seed(16)
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda").to(torch.bfloat16)
+
+    def rows(s, how):
+        return {"bhsd": lambda: rand(b, h, s, d).transpose(1, 2), "sbhd": lambda: rand(s, b, h, d).transpose(0, 1),
+                "padded": lambda: rand(b, s, h, d + 24)[..., 8:8 + d], "strided": lambda: rand(b, 2 * s, 2 * h, d)[:, ::2, 1::2],
+                "one head": lambda: rand(b, s, 1, d).expand(b, s, h, d), "one batch": lambda: rand(1, s, h, d).expand(b, s, h, d)}[how]()
+
+    for how in (("bhsd", "sbhd", "padded", "strided"), ("strided", "one head", "one head", "bhsd"), ("sbhd", "one batch", "padded", "one head"),
+                ("one batch", "bhsd", "one batch", "padded")):
+        q, k, v, do = [rows(s, x) for s, x in zip((sq, sk, sk, sq), how)]
+        out, lse = ops.fwd(q, k, v)
+        delta = ops.bwd_preprocess(do, out)
+        got = ops.bwd(q, k, v, do, lse, delta)
+        want = ops.bwd(*[t.contiguous() for t in (q, k, v, do)], lse, delta)
+        assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+        # dQ: as in _check
+        assert (got[0].double() - want[0].double()).norm() <= 0.1 * 2.0 ** -8 * want[0].double().norm()
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("case,key,first_row", [((2, 16, 16, 4200, 4200, 128), 2300, 2048), ((1, 2, 2, 700, 700, 192), 300, 256),
+                                                ((1, 2, 2, 700, 700, 256), 300, 256)], ids=str)
+def test_how_far_a_key_that_is_not_finite_reaches(case, key, first_row):
+    """Into dQ of the query blocks that its pair walks, which under a causal mask start at the pair's first key; no further."""
+    from flash_attn2_b200 import cabi_ops as ops
+
+    q, k, v, do = [t.cuda() for t in make_qkv(17, *case, torch.bfloat16, with_do=True)]
+    k[:, key] = float("inf")
+    out, lse = ops.fwd(q, k, v, causal=True)
+    assert out[:, :key].isfinite().all()
+    dq = ops.bwd(q, k, v, do, lse, ops.bwd_preprocess(do, out), causal=True)[0]
+    assert dq[:, :first_row].isfinite().all() and not dq[:, key:].isfinite().any()
+    assert ops.device_status() == 0

@@ -35,8 +35,10 @@ class Canaries:
             assert (raw[-PAD:] == pattern).all(), f"buffer {i}: written past its end"
 
 
-DENSE = [(2, 4, 2, 333, 333, 128, True), (1, 3, 1, 200, 777, 64, False), (1, 2, 2, 130, 70, 96, True),
-         (2, 4, 2, 333, 333, 256, True), (1, 3, 1, 200, 777, 192, False), (1, 2, 2, 130, 70, 136, True),
+# Backward on pairs of CTAs (test_plans_cpu.py states that it is), ragged.
+PAIRS = [(1, 28, 28, 1930, 1990, 128, False), (2, 16, 16, 2041, 1000, 120, False), (2, 4, 2, 333, 333, 256, True), (2, 4, 2, 400, 333, 192, True)]
+DENSE = PAIRS + [(2, 4, 2, 333, 333, 128, True), (1, 3, 1, 200, 777, 64, False), (1, 2, 2, 130, 70, 96, True),
+         (1, 3, 1, 200, 777, 192, False), (1, 2, 2, 130, 70, 136, True),
          (1, 2, 2, 1, 200, 128, False), (1, 2, 2, 65, 129, 256, False)]
 
 

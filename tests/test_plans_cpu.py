@@ -202,9 +202,14 @@ def _empty_pairs(case):
 
 
 def test_backward_calls_that_run_on_pairs(plans):
-    from tests.test_bwd_pair_gpu import CASES, EMPTY, WIDE
+    from tests import test_canaries_gpu, test_stream_order_gpu, test_zz_no_alloc
+    from tests.test_bwd_pair_gpu import CASES, EMPTY, REPEATED, WIDE
 
-    assert all(_takes_pairs(plans, c) for c in CASES + WIDE)
+    assert all(_takes_pairs(plans, c) for c in CASES + WIDE + REPEATED)
+    none = (-1, -1)
+    assert all(_takes_pairs(plans, (*c[:6], c[6], none)) for c in test_canaries_gpu.PAIRS)
+    assert all(_takes_pairs(plans, (*shape, causal, none)) for shape, causal, _ in test_stream_order_gpu.PAIRS)
+    assert all(_takes_pairs(plans, (*shape, False, none)) for shape in test_zz_no_alloc.PAIRS)
     assert {c[5] for c in EMPTY} == {128, 192, 256} and all((_empty_pairs(c) > 0) == (c in EMPTY) for c in CASES + WIDE)
     assert not any(_takes_pairs(plans, WIDE[0], **other) for other in (dict(which=1), dict(which=2), dict(head_dim=248), dict(head_dim=184),
                                                                dict(cu_seqlens_q=256), dict(head_dim=192, seqlen_q=300)))

@@ -55,8 +55,10 @@ def _steps(seed, shape, causal, deterministic):
 FORWARDS = [((1, 32, 8, 1, 8192, 128), True), ((10, 32, 8, 1, 1500, 64), True), ((40, 8, 4, 2, 700, 192), False),
             ((1, 4, 4, 128, 128, 64), False), ((1, 8, 8, 500, 4096, 128), True), ((4, 16, 8, 700, 700, 128), True),
             ((2, 8, 4, 500, 900, 256), True)]
-# shared key blocks; few CTAs; tiles taken over; the wide kernel; bit-reproducible pairs
-STEPS = [((1, 8, 2, 777, 777, 128), True, False), ((4, 16, 16, 400, 400, 128), False, False), ((8, 16, 16, 509, 509, 64), True, False),
+# Steps on pairs of CTAs (test_plans_cpu.py states that they are).
+PAIRS = [((1, 28, 28, 2048, 2048, 128), False, False), ((2, 8, 4, 400, 400, 192), True, False), ((2, 8, 4, 300, 300, 256), True, False)]
+# shared key blocks; few CTAs; tiles taken over; the wide kernel with one CTA per key block and half of the head dim; bit-reproducible pairs
+STEPS = PAIRS + [((1, 8, 2, 777, 777, 128), True, False), ((4, 16, 16, 400, 400, 128), False, False), ((8, 16, 16, 509, 509, 64), True, False),
          ((2, 8, 4, 300, 300, 192), True, False), ((2, 16, 4, 777, 777, 128), True, True), ((10, 16, 16, 300, 300, 64), False, True)]
 CHAINS = [(_forwards, c) for c in FORWARDS] + [(_steps, c) for c in STEPS]
 
@@ -79,7 +81,7 @@ def test_a_call_sees_what_the_one_before_it_wrote(make, case):
 
 
 # (shape, causal, deterministic)
-GRAPHS = [((2, 16, 4, 777, 777, 128), True, True), ((8, 16, 16, 509, 509, 64), False, False), ((2, 16, 16, 1000, 1000, 128), True, False),
+GRAPHS = PAIRS[:2] + [((2, 16, 4, 777, 777, 128), True, True), ((8, 16, 16, 509, 509, 64), False, False), ((2, 16, 16, 1000, 1000, 128), True, False),
           ((2, 8, 4, 600, 600, 256), True, False)]
 
 
