@@ -233,21 +233,28 @@ inline int bwd_dq_head_group(const fa2_bwd_args* a, const Windows& w) {
 // B1 H32 S16384 causal 7709 -> 7461 us, B4 H16/4 S4096 2025 -> 1955, B16 H16 S2048 2265 -> 2220, B2 H32/8 S2048 557 -> 542,
 // B4 H16 S4096 causal 1144 -> 1133; with walks of less than 16 blocks B16 H16 S2048 causal 1364 -> 1385, B2 H16 S8192 window 1023
 // 684 -> 711; with few CTAs B1 H8/2 S8192 causal 545 -> 551; a soft cap, whose tanh makes the arithmetic the longer part, B4 H16/4 S4096
-// causal 1267 -> 1352; B2 H16 S8192 D96 3549 -> 3541.
+// causal 1267 -> 1352; B2 H16 S8192 D96 3549 -> 3541. With an odd number of key blocks one CTA of a head has no keys and walks for nothing, which
+// a few key blocks do not make up for: B8 H16 Sq 2048 Sk 98 179 -> 207, 354 299 -> 330, 610 425 -> 452, 1122 657 -> 680, 1634 917 -> 929; on this side 1890
+// 1029 -> 1036 (B4 Sq 4096 1003 -> 982), 2658 1423 -> 1410, B8 H16/4 S2146 1165 -> 1135, causal, where that walk is short, B4 H16 S3170 718 -> 714.
 inline bool bwd_takes_pairs(const fa2_bwd_args* a, const Windows& w, int sm_count) {
   if (a->cu_seqlens_q != nullptr || (a->which & 3) != 3 || a->head_dim <= 96 || a->head_dim > 128 || a->softcap > 0.f ||
       a->alibi_slopes != nullptr)
     return false;
   const int64_t pairs = (static_cast<int64_t>(a->seqlen_k) + 255) / 256, off = static_cast<int64_t>(a->seqlen_k) - a->seqlen_q;
   if (2 * pairs * a->batch * a->heads_k < sm_count * 3 / 2) return false;
-  // Query blocks of a head that the first and the last pair walk: their mean is the mean of all under a causal mask and without one.
+  // Query blocks of a head that the first and the last pair walk. Their mean is that of all without a mask and, with no more keys than queries,
+  // under a causal one; with more keys or a window on both sides that is larger, and the line lies further up: B2 H16 S8192 causal window
+  // 2047 1032, 1031 (a mean of 18 blocks, refused), 3071 1343, 1322 (26, refused), 4095 1593, 1560; Sq 2048 Sk 8192 causal 922, 902 (refused), Sq 4096
+  // 1520, 1474.
   auto blocks = [&](int64_t n0) {
     const int64_t n_last = std::min<int64_t>(n0 + 255, a->seqlen_k - 1);
     const int64_t lo = w.right >= 0 ? std::max<int64_t>(0, n0 - off - w.right) : 0;
     const int64_t hi = w.left >= 0 ? std::min<int64_t>(a->seqlen_q, n_last - off + w.left + 1) : a->seqlen_q;
     return hi > lo ? (hi + 127) / 128 - lo / 128 : 0;
   };
-  return blocks(0) + blocks((pairs - 1) * 256) >= 2 * 16;
+  const int64_t first = blocks(0), last = blocks((pairs - 1) * 256);
+  if ((a->seqlen_k + 127) / 128 % 2 == 1 && 16 * last > pairs * (first + last)) return false;
+  return first + last >= 2 * 16;
 }
 
 // Head dims 192 and 256 (bwd_wide_pair_sm100.cu, which has more figures). Its query blocks have 128 rows, those of the other kernel 64,

@@ -7,11 +7,11 @@ from tests._cases import make_qkv
 pytestmark = pytest.mark.gpu
 
 # (batch, heads, heads_k, seqlen_q, seqlen_k, head_dim, causal, window): calls that run on pairs (test_plans_cpu.py states that they
-# do). Whole tiles; a last pair of one block, of one key block and a bit, with nothing for its second CTA; bottom-right masks with more
+# do). Whole tiles; a last pair of one key block, of one key, with nothing for its second CTA; bottom-right masks with more
 # keys than queries and with rows that see no key; windows; grouped heads; head dims below the kernel's; pairs whose keys no query sees
 # (EMPTY).
-CASES = [(1, 28, 28, 2048, 2048, 128, False, (-1, -1)), (4, 32, 8, 2000, 1000, 128, False, (-1, -1)), (8, 16, 8, 2048, 300, 120, False, (-1, -1)),
-         (8, 16, 8, 1921, 257, 104, False, (-1, -1)), (2, 16, 8, 4200, 4200, 128, True, (-1, -1)), (2, 8, 8, 4100, 5000, 128, True, (-1, -1)),
+CASES = [(1, 28, 28, 2048, 2048, 128, False, (-1, -1)), (4, 32, 8, 2000, 1000, 128, False, (-1, -1)), (2, 16, 8, 2048, 1810, 120, False, (-1, -1)),
+         (2, 16, 8, 1921, 1793, 104, False, (-1, -1)), (2, 16, 8, 4200, 4200, 128, True, (-1, -1)), (2, 8, 8, 4100, 5000, 128, True, (-1, -1)),
          (2, 8, 8, 5000, 4100, 112, True, (-1, -1)), (2, 8, 4, 5000, 5000, 128, False, (3000, 500)),
          (1, 8, 8, 4100, 4900, 128, False, (500, -1))]
 

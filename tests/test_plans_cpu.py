@@ -219,6 +219,9 @@ def test_backward_calls_that_run_on_pairs(plans):
         assert _takes_pairs(plans, WIDE[0], seqlen_q=rows, seqlen_k=keys) == taken, (rows, keys)
     full = (4, 16, 16, 2048, 2048, 128, False, (-1, -1))
     assert _takes_pairs(plans, full)
+    # An odd number of key blocks leaves one CTA of a head without keys, which 15 blocks and more make up for, and a causal mask.
+    assert [n for n in range(1, 24) if _takes_pairs(plans, full, batch=16, seqlen_k=128 * n - 60)] == [*range(2, 14, 2), *range(14, 24)]
+    assert _takes_pairs(plans, full, causal=True, seqlen_q=4200, seqlen_k=4200)
     for other in (dict(which=1), dict(which=2), dict(head_dim=96), dict(head_dim=136), dict(softcap=30.0), dict(alibi_slopes=256),
-                  dict(cu_seqlens_q=256), dict(causal=True), dict(window_left=1023), dict(batch=1, heads=8, heads_k=8)):
+                  dict(cu_seqlens_q=256), dict(causal=True), dict(window_left=1023), dict(batch=1, heads=8, heads_k=8), dict(seqlen_k=1600)):
         assert not _takes_pairs(plans, full, **other), other
