@@ -248,7 +248,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
                         (ks.value / 4) * (Cfg::kAtomBytes >> 5) + (ks.value % 4) * 2>(d_tmem, a, b, idesc_qk, ks.value > 0 ? 1u : 0u);
         });
       };
-      bool ok = true;
+      bool ok = n_iter > 0;
 #pragma unroll 1
       for (int it = -1; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
@@ -310,7 +310,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
         mma_pair_commit(dq_full);
       }
       // Only for who waits: an arrival that nobody waits for could land in the other CTA after its end.
-      if (ok && n_iter > 0) mma_pair_commit(dk_done);
+      if (ok) mma_pair_commit(dk_done);
     } else if (warp == 2 && rank == 1 && elect_one()) {
       // ---------------------------------------------------------------- tells the issuer what this CTA has received
       bool ok = true;
@@ -323,7 +323,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
       // ---------------------------------------------------------------- -LSE (log2 domain) and -delta of a query block
       // Rows past the sequence give P = 0. Two buffers: the next iteration's values are there before the compute warps ask for them.
       Walk w{0, 0};
-      bool ok = true;
+      bool ok = n_iter > 0;
       for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
         const int hq = ti.hk * p.group + w.g, q0 = (ti.m_start + w.mi) * kBlk + lane;
         const float* lse = p.lse + ti.b * p.lse_batch_stride + hq * p.lse_head_stride;
@@ -343,6 +343,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
         __syncwarp();
         if (lane == 0) mbar_arrive(&stat_full[buf]);
       }
+      // The stages' last commits land before the CTA ends: q_empty, qcol_empty, do_empty, docol_empty.
+#pragma unroll 1
+      for (int i = 0; i < 4 && ok; ++i) ok = mbar_wait(q_empty + i, (n_iter - 1) & 1, ctl, kWaitBwd + 1);
     }
   } else if (warp < 12) {
     // ------------------------------------------------------------------ compute

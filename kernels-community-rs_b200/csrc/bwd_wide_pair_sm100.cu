@@ -295,7 +295,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
         }
         return true;
       };
-      bool ok = true;
+      bool ok = n_iter > 0;
 #pragma unroll 1
       for (int it = -1; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
@@ -338,7 +338,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
         mma_pair_commit(dq_full);
       }
       // Only for who waits: an arrival that nobody waits for could land in the other CTA after its end.
-      if (ok && n_iter > 0) mma_pair_commit(dk_done);
+      if (ok) mma_pair_commit(dk_done);
     } else if (warp == 2 && rank == 1 && elect_one()) {
       // ---------------------------------------------------------------- tells the issuer what this CTA has received
       bool ok = true;
@@ -350,7 +350,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
     } else if (warp == 3) {
       // ---------------------------------------------------------------- -LSE (log2 domain) and -delta of a query block
       Walk w{0, 0};
-      bool ok = true;
+      bool ok = n_iter > 0;
       for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
         const int hq = ti.hk * p.group + w.g, q0 = (ti.m_start + w.mi) * kBlk + lane;
         const float* lse = p.lse + ti.b * p.lse_batch_stride + hq * p.lse_head_stride;
@@ -370,6 +370,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
         __syncwarp();
         if (lane == 0) mbar_arrive(&stat_full[buf]);
       }
+      // The slots' last commits land before the CTA ends (eight loads an iteration, so all of them are in odd phases), and dK's.
+#pragma unroll 1
+      for (int i = 0; i < Cfg::kSlots && ok; ++i) ok = mbar_wait(&ring_empty[i], 1, ctl, kWaitBwd + 1);
+      if (ok) ok = mbar_wait(dk_read, (n_iter - 1) & 1, ctl, kWaitBwd + 17);
     }
   } else if (warp < 12) {
     // ------------------------------------------------------------------ compute: one key and 32 queries a thread
