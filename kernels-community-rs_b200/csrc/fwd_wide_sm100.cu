@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(wide_threads(FANCY), 1) fwd_wide_kernel(const 
       __syncwarp();
       uint64_t* bar = &x_full[(i & 1) * 4 + (warp & 3)];
       if (lane == 0) mbar_arrive(bar);
-      if (!warp_wait(bar, (i >> 1) & 1, ctl, kWaitSoftmaxSFull)) return false;
+      if (!warp_wait(bar, (i >> 1) & 1, ctl, kWaitSoftmaxExchange)) return false;
       other = slot[tid ^ kWM];
       return true;
     };
