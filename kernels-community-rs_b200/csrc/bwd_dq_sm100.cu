@@ -46,12 +46,6 @@ struct DqCfg {
   static constexpr uint32_t kTmemS = 0, kTmemDP = 256, kTmemDQ = 384;
 };
 
-__device__ __forceinline__ float tanh_approx(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <int D, bool BF16, int MODE>
 __global__ void __launch_bounds__(kThreads, 1) bwd_dq_kernel(const __grid_constant__ DqParams p) {
   using Cfg = DqCfg<D>;

@@ -12,7 +12,8 @@
 // dQ contracts over the keys of both CTAs, so each CTA sends its dS^T of the other one's 64 queries to that CTA's shared memory.
 // What leaves the pair for the fp32 dQ accumulator is one tile of 128 queries for 256 keys, half of what two CTAs with 128 keys
 // add (bwd_sm100.cu), and that traffic is what bounds those: 64 KB of reductions leave an SM in 2850-3100 cycles, of 3800 an
-// iteration. Operands are halves too: 160 KB of shared memory are read per iteration and CTA in place of 288.
+// iteration. Operands are halves too: 192 KB of shared memory are read per iteration and CTA in place of 288 (48 each for S^T and
+// dP^T, 16 each for dV and dK, 64 for dQ).
 //
 // TMEM (columns): dK 0, dV 128, S^T 256 ... 383, dP^T 384 ... 511. P^T goes over the first half of S^T as soon as both warpgroups have
 // read their scores, dQ over the second half; dS^T of a warpgroup over its own half of dP^T.
@@ -70,11 +71,6 @@ struct PairCfg {
   static constexpr int kSmemBytes = kStatOff + 2 * 2 * kBlk * 4;
   static_assert(kStatOff % 16 == 0 && kSmemBytes <= 227 * 1024, "shared memory");
   static constexpr uint32_t kTmemDK = 0, kTmemDV = 128, kTmemS = 256, kTmemDQ = 320, kTmemDP = 384;
-};
-
-struct PairTile {
-  int b, hk, n0;         // n0: first key of the pair
-  int m_start, n_m, n_iter;
 };
 
 __device__ __forceinline__ PairTile get_pair_tile(const BwdParams& p, int t) {
@@ -321,28 +317,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
       }
     } else if (warp == 3) {
       // ---------------------------------------------------------------- -LSE (log2 domain) and -delta of a query block
-      // Rows past the sequence give P = 0. Two buffers: the next iteration's values are there before the compute warps ask for them.
-      Walk w{0, 0};
-      bool ok = n_iter > 0;
-      for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
-        const int hq = ti.hk * p.group + w.g, q0 = (ti.m_start + w.mi) * kBlk + lane;
-        const float* lse = p.lse + ti.b * p.lse_batch_stride + hq * p.lse_head_stride;
-        const float* delta = p.delta + ti.b * p.delta_batch_stride + hq * p.delta_head_stride;
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int q = q0 + 32 * i;
-          v[i] = q < p.seqlen_q ? lse[q] * -kLog2e : -INFINITY;
-          v[4 + i] = q < p.seqlen_q ? -delta[q] : 0.f;
-        }
-        const uint32_t buf = it & 1;
-        ok = warp_wait(&stat_empty[buf], ((it >> 1) & 1) ^ 1, ctl, kWaitBwd + 15);
-        float* stat = s_stat + buf * (2 * kBlk) + lane;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) stat[32 * i] = v[i];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&stat_full[buf]);
-      }
+      bool ok = pair_statistics(p, ti, s_stat, stat_full, stat_empty, lane, ctl);
       // The stages' last commits land before the CTA ends: q_empty, qcol_empty, do_empty, docol_empty.
 #pragma unroll 1
       for (int i = 0; i < 4 && ok; ++i) ok = mbar_wait(q_empty + i, (n_iter - 1) & 1, ctl, kWaitBwd + 1);
@@ -543,21 +518,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_pai
     }
     if (lane == 0) tma_wait_group_read<0>();
   }
-  __syncwarp();
-  if (*abort_flag) {
-    // A wait ran out somewhere in this CTA: give MMAs, commits and copies in flight about a millisecond to land.
-    const long long t0 = clock64();
-    while (clock64() - t0 < 2000000) {
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (tid == 0) report_abort(abort_flag, p.status);
-  // A CTA stays until the other one has read its operands and sent it everything. The barrier takes converged warps.
-  __syncwarp();
-  cluster_arrive();
-  cluster_wait();
-  if (warp == 1) tmem_dealloc_pair(tmem, 512);
+  end_pair(p, abort_flag, tid, warp, tmem);
 }
 
 template <bool BF16>

@@ -94,12 +94,6 @@ struct KvTile {
   bool valid;
 };
 
-__device__ __forceinline__ float tanh_approx(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <bool PACKED>
 __device__ __forceinline__ KvTile get_kv_tile(const BwdParams& p, int t) {
   KvTile ti;

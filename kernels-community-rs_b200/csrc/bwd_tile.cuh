@@ -1,6 +1,7 @@
-// The walk over the query blocks of the backward kernels for head dims up to 128.
+// What the backward kernels with query blocks of 128 rows have in common: the walk over the blocks, and on pairs of CTAs the tail of a walk.
 #pragma once
 #include "fa2_params.h"
+#include "sm100_ptx.cuh"
 
 namespace fa2 {
 namespace {
@@ -30,6 +31,59 @@ __device__ __forceinline__ Walk walk_next(Walk w, int n_m) {
     ++w.g;
   }
   return w;
+}
+
+// What a pair of CTAs works on: 2 * kBlk or kBlk keys of one (batch, kv head) and the query blocks that see them.
+struct PairTile {
+  int b, hk, n0;  // n0: first key of the pair
+  int m_start, n_m, n_iter;
+};
+
+// A warp's part on pairs of CTAs: -LSE (log2 domain) and -delta of each query block of the walk. Rows past the sequence give P = 0. Two
+// buffers, [lse, delta][kBlk] each: the next iteration's values are there before the compute warps ask for them.
+__device__ __forceinline__ bool pair_statistics(const BwdParams& p, const PairTile& ti, float* s_stat, uint64_t* stat_full, uint64_t* stat_empty,
+                                                int lane, const WaitCtl& ctl) {
+  Walk w{0, 0};
+  bool ok = ti.n_iter > 0;
+  for (int it = 0; it < ti.n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
+    const int hq = ti.hk * p.group + w.g, q0 = (ti.m_start + w.mi) * kBlk + lane;
+    const float* lse = p.lse + ti.b * p.lse_batch_stride + hq * p.lse_head_stride;
+    const float* delta = p.delta + ti.b * p.delta_batch_stride + hq * p.delta_head_stride;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int q = q0 + 32 * i;
+      v[i] = q < p.seqlen_q ? lse[q] * -kLog2e : -INFINITY;
+      v[4 + i] = q < p.seqlen_q ? -delta[q] : 0.f;
+    }
+    const uint32_t buf = it & 1;
+    ok = warp_wait(&stat_empty[buf], ((it >> 1) & 1) ^ 1, ctl, kWaitBwd + 15);
+    float* stat = s_stat + buf * (2 * kBlk) + lane;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) stat[32 * i] = v[i];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&stat_full[buf]);
+  }
+  return ok;
+}
+
+// The end of both kernels on pairs of CTAs, by all threads.
+__device__ __forceinline__ void end_pair(const BwdParams& p, const volatile int* abort_flag, int tid, int warp, uint32_t tmem) {
+  __syncwarp();
+  if (*abort_flag) {
+    // A wait ran out somewhere in this CTA: give MMAs, commits and copies in flight about a millisecond to land.
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) {
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (tid == 0) report_abort(abort_flag, p.status);
+  // A CTA stays until the other one has read its operands and sent it everything. The barrier takes converged warps.
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (warp == 1) tmem_dealloc_pair(tmem, 512);
 }
 
 }  // namespace

@@ -74,13 +74,8 @@ struct WidePairCfg {
   static constexpr uint32_t kTmemDK = 0, kTmemDV = 128, kTmemS = 256, kTmemDP = 320, kTmemDQ = 384;
 };
 
-struct WidePairTile {
-  int b, hk, n0;  // n0: first key of the pair
-  int m_start, n_m, n_iter;
-};
-
-__device__ __forceinline__ WidePairTile get_wide_pair_tile(const BwdParams& p, int t) {
-  WidePairTile ti;
+__device__ __forceinline__ PairTile get_wide_pair_tile(const BwdParams& p, int t) {
+  PairTile ti;
   const int first_bh = t / (p.head_group * p.num_nblk) * p.head_group;
   const int n_bh = min(p.head_group, p.batch * p.heads_k - first_bh);
   const int in_group = t - first_bh * p.num_nblk;
@@ -92,12 +87,6 @@ __device__ __forceinline__ WidePairTile get_wide_pair_tile(const BwdParams& p, i
   q_block_range(p, p.seqlen_q, p.seqlen_k, ti.n0, 2 * kKeys, ti.m_start, ti.n_m);
   ti.n_iter = ti.n_m * p.group;
   return ti;
-}
-
-__device__ __forceinline__ float tanh_approx(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 
 // FANCY: a soft cap or ALiBi is in use.
@@ -144,7 +133,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
   const int lane = tid & 31;
   const int rank = static_cast<int>(cluster_rank());
   const WaitCtl ctl{abort_flag};
-  const WidePairTile ti = get_wide_pair_tile(p, blockIdx.x >> 1);
+  const PairTile ti = get_wide_pair_tile(p, blockIdx.x >> 1);
   const int n_iter = ti.n_iter;
   const int n0 = ti.n0 + rank * kKeys;  // first key of this CTA
   const int off = p.seqlen_k - p.seqlen_q;
@@ -349,27 +338,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
       }
     } else if (warp == 3) {
       // ---------------------------------------------------------------- -LSE (log2 domain) and -delta of a query block
-      Walk w{0, 0};
-      bool ok = n_iter > 0;
-      for (int it = 0; it < n_iter && ok; ++it, w = walk_next(w, ti.n_m)) {
-        const int hq = ti.hk * p.group + w.g, q0 = (ti.m_start + w.mi) * kBlk + lane;
-        const float* lse = p.lse + ti.b * p.lse_batch_stride + hq * p.lse_head_stride;
-        const float* delta = p.delta + ti.b * p.delta_batch_stride + hq * p.delta_head_stride;
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int q = q0 + 32 * i;
-          v[i] = q < p.seqlen_q ? lse[q] * -kLog2e : -INFINITY;
-          v[4 + i] = q < p.seqlen_q ? -delta[q] : 0.f;
-        }
-        const uint32_t buf = it & 1;
-        ok = warp_wait(&stat_empty[buf], ((it >> 1) & 1) ^ 1, ctl, kWaitBwd + 15);
-        float* stat = s_stat + buf * (2 * kBlk) + lane;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) stat[32 * i] = v[i];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&stat_full[buf]);
-      }
+      bool ok = pair_statistics(p, ti, s_stat, stat_full, stat_empty, lane, ctl);
       // The slots' last commits land before the CTA ends (eight loads an iteration, so all of them are in odd phases), and dK's.
 #pragma unroll 1
       for (int i = 0; i < Cfg::kSlots && ok; ++i) ok = mbar_wait(&ring_empty[i], 1, ctl, kWaitBwd + 1);
@@ -552,7 +521,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
     // ------------------------------------------------------------------ dQ drain: one column of the head dim a thread
     const int dw = warp & 3;
     const int col = rank * kHalf + dw * 32;  // of the warp's first lane
-    const bool used = dw * 32 < kHalf && col < p.head_dim;
+    const bool used = col < p.head_dim;
     const uint32_t t_dq = tmem + (static_cast<uint32_t>(dw * 32) << 16) + Cfg::kTmemDQ;
     const uint32_t free_bar = leader(dq_free);
     uint8_t* stage = smem + Cfg::kDQOff + dw * (Cfg::kPieces * Cfg::kPieceBytes);
@@ -598,21 +567,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) bwd_wid
     }
     if (lane == 0) tma_wait_group_read<0>();
   }
-  __syncwarp();
-  if (*abort_flag) {
-    // A wait ran out somewhere in this CTA: give MMAs, commits and copies in flight about a millisecond to land.
-    const long long t0 = clock64();
-    while (clock64() - t0 < 2000000) {
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (tid == 0) report_abort(abort_flag, p.status);
-  // A CTA stays until the other one has read its operands and sent it everything. The barrier takes converged warps.
-  __syncwarp();
-  cluster_arrive();
-  cluster_wait();
-  if (warp == 1) tmem_dealloc_pair(tmem, 512);
+  end_pair(p, abort_flag, tid, warp, tmem);
 }
 
 template <int ATOMS, bool BF16, bool FANCY>

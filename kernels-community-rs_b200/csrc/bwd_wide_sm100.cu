@@ -98,12 +98,6 @@ __device__ __forceinline__ WWalk wwalk_next(WWalk w, int n_m) {
   return w;
 }
 
-__device__ __forceinline__ float bw_tanh(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // The two halves of a key block are neighbours in the grid (they read the same tiles), and consecutive pairs
 // walk the key blocks of a group of heads, heaviest first under a causal mask (bwd_head_group).
 __device__ __forceinline__ WKvTile get_wkv_tile(const BwdParams& p, int t) {
@@ -351,7 +345,7 @@ __global__ void __launch_bounds__(kBWThreads, 1) bwd_wide_kernel(const __grid_co
             const float raw = __uint_as_float(sr[i + e]);
             float x, deriv = 1.f;
             if (p.softcap > 0.f) {
-              const float t = bw_tanh(raw * inv_cap);
+              const float t = tanh_approx(raw * inv_cap);
               x = cap_l2 * t;
               deriv = fmaf(-t, t, 1.f);
             } else {

@@ -251,11 +251,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_decode_kernel(const __grid_co
 #pragma unroll
           for (int i = 0; i < kNT; ++i)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float y;
-              asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(s[i][e] * inv_cap));
-              s[i][e] = cap_l2 * y;
-            }
+            for (int e = 0; e < 4; ++e) s[i][e] = cap_l2 * tanh_approx(s[i][e] * inv_cap);
         } else {
 #pragma unroll
           for (int i = 0; i < kNT; ++i)

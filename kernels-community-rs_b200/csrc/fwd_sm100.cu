@@ -248,12 +248,6 @@ __device__ __forceinline__ int ragged_row(int sk, int j) {
   return left < kBlockN ? max(left, 0) : kBlockN;
 }
 
-__device__ __forceinline__ float tanh_approx(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // Is the rescaling of O a loop in the machine code? Its code is read by few key blocks, which is worth 1 % where the row maximum
 // soon stops growing; with ALiBi it grows along the keys, and on shared tiles the loop costs registers. Forward, rolled -> unrolled, us:
 // ALiBi B1 H8 S16384 causal D128 677 -> 644, D64 H16 1088 -> 1011, B4 H16/4 S2048 98.0 -> 95.2; soft cap D64 H16 S16384 1239 -> 1222;

@@ -129,12 +129,6 @@ __device__ __forceinline__ int wide_ragged_row(int sk, int j) {
   return left < kWN ? max(left, 0) : kWN;
 }
 
-__device__ __forceinline__ float wide_tanh(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // ATOMS: 64-column atoms of the head dim that are loaded (3 for head dims up to 192, else 4). TMA fills what lies
 // past the real head dim inside them with zeros, so Q K^T runs over ATOMS * 64 columns with compile-time operand
 // offsets: a runtime bound in the issuing thread's loop doubles the cost of an MMA issue.
@@ -276,7 +270,7 @@ __global__ void __launch_bounds__(wide_threads(FANCY), 1) fwd_wide_kernel(const 
 #pragma unroll
         for (int c = 0; c < kWC; ++c) {
           float x = __uint_as_float(sr[c]);
-          x = (p.softcap > 0.f) ? cap_l2 * wide_tanh(x * inv_cap) : x * p.scale_log2;
+          x = (p.softcap > 0.f) ? cap_l2 * tanh_approx(x * inv_cap) : x * p.scale_log2;
           if (p.alibi != nullptr) {
             const int col = col0 + c;
             x += p.causal_alibi ? slope * static_cast<float>(col) : -slope * fabsf(static_cast<float>(row + ti.off - col));
