@@ -27,7 +27,7 @@
 // A CTA's start and end cost 9000 cycles, a third of its time where a head has four query blocks. At D = 64 there is shared
 // memory for K and V of two tiles, so a CTA goes on with the tile of a CTA that has not started: K, V, Q and dO of the next
 // tile are loaded beside the end of this one. B32 H12 S509 D64 fp16 223.6 -> 201.0 us, B2 H16 S4096 D64 causal 378 -> 358.
-// That includes what it costs: with the tile carried through every role these instances spill 340-372 bytes of loads a thread. So
+// That includes what it costs: with the tile carried through every role these instances spill 312-344 bytes of loads a thread. So
 // calls in which no CTA takes a tile over have instances without it (launch_one).
 // At D = 128 K has to wait for the last dQ and nothing is left to stage dK and dV in: B4 H16 S1000 112.8 -> 114.8 us,
 // B4 H16/4 S2048 softcap 340 -> 345, so there a CTA has one tile. Packed batches have one tile per CTA too.

@@ -88,6 +88,7 @@ struct DecodeParams {
 constexpr int kMaxSplitBlocks = 160;   // a grid of more key blocks fills the GPU by itself
 
 struct BwdParams {
+  // Boxes as in fa2_launch.h where a kernel has others.
   CUtensorMap tm_q, tm_k, tm_v, tm_do;  // 16-bit inputs, box (64, 1, 128, 1)
   CUtensorMap tm_dk, tm_dv;             // 16-bit outputs, box (64, 1, 128, 1)
   CUtensorMap tm_dqa;                   // fp32 dQ accumulator, box (32, 1, 32, 1): one drain warp's rows
